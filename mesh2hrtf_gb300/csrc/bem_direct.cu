@@ -6,15 +6,25 @@
 //
 // Blocked right-looking factorisation A = L U (L unit lower, U upper) in the
 // matrix's own precision (complex128 for FP64 solvers, complex64 for mixed
-// ones), in panels of kPanel columns:
-//   k_lu_panel_col  one launch per pivot column: the multipliers of the rows
-//                   below the pivot and their update inside the panel
-//   k_lu_trsm       U12 = L11^-1 A12, thread per trailing column
-//   k_lu_update     A22 -= L21 U12, 64 x 64 output tiles through shared memory
-// The substitutions run in FP64 on blocks of kPanel unknowns: a small
-// triangular solve of the diagonal block, then one grid-wide update of the
-// remaining rows (thread per row).  Like the reference, no pivoting: a zero
-// pivot is reported, not worked around.
+// ones), in panels of kPanel columns, two launches per panel:
+//   k_lu_panel   L21 = A21 U11^-1 (8 lanes per row), U12 = L11^-1 A12 (8 lanes
+//                per column), and the panel's step of the forward
+//                substitution, from the factored diagonal block
+//   k_lu_update  A22 -= L21 U12, 64 x 64 output tiles through shared memory,
+//                and the right-hand sides' remaining rows; the block that
+//                owns the next diagonal block factors it as soon as it is
+//                updated, beside the other tiles
+// The forward substitution rides along in FP64; the back substitution takes
+// one launch per panel (k_bwd): every block solves the 32 x 32 triangle
+// (a warp, lane per row) and updates its own rows, so no launch waits on a
+// single-thread solve.  Like the reference, no pivoting: a zero pivot is
+// reported, not worked around.
+//
+// What bounds it: the launch-to-launch chain of n / 32 panels below a few
+// thousand unknowns, the update's FP32 (FP64) arithmetic above.  Before, a
+// launch per pivot column (uncoalesced row walks) and one-thread diagonal
+// solves took 88.8 ms at 2420 unknowns in complex64; this form takes
+// 4.6 ms.
 #include <cuda_runtime.h>
 
 #include "../../include/bem_gb300.h"
@@ -24,17 +34,13 @@ namespace {
 
 constexpr int kPanel = 32;
 constexpr int kTile = 64;
-constexpr int kChunk = 16;
+// columns of L21 / rows of U12 staged at a time
+template <typename V> constexpr int kChunk = sizeof(V) == 8 ? 32 : 16;
+constexpr int kMaxB = bem::kMaxRhs;
+constexpr int kRowsPerBwd = kPanel;    // k_bwd: rows per block, 8 lanes each
 
 __device__ __forceinline__ double2 ld2(const double2 &v) { return v; }
 __device__ __forceinline__ double2 ld2(const float2 &v) { return make_double2(v.x, v.y); }
-__device__ __forceinline__ void st2(double2 &d, double2 v) { d = v; }
-__device__ __forceinline__ void st2(float2 &d, double2 v) { d = make_float2((float)v.x, (float)v.y); }
-
-template <typename V> struct Acc;
-template <> struct Acc<double2> { using T = double; };
-template <> struct Acc<float2> { using T = float; };
-
 template <typename V>
 __device__ __forceinline__ V cmul(V a, V b) {
     V r;
@@ -59,200 +65,356 @@ __device__ __forceinline__ V cdiv(V a, V b) {
     return r;
 }
 
-// multipliers of pivot column i for rows j > i and their update of the
-// panel's columns i+1 .. pend-1
+// a - b c with the products fused into the sum
 template <typename V>
-__global__ void __launch_bounds__(256) k_lu_panel_col(V *A, size_t lda, int n, int i, int pend, int *status) {
-    const int j = i + 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const V piv = A[(size_t)i * lda + i];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && piv.x == 0 && piv.y == 0) atomicExch(status, 1);
-    if (j >= n) return;
-    V *row = A + (size_t)j * lda;
-    const V *prow = A + (size_t)i * lda;
-    const V l = cdiv(row[i], piv);
-    row[i] = l;
-    for (int c = i + 1; c < pend; ++c) row[c] = csub(row[c], cmul(l, prow[c]));
+__device__ __forceinline__ V cfnma(V a, V b, V c) {
+    a.x = fma(-b.x, c.x, a.x);
+    a.x = fma(b.y, c.y, a.x);
+    a.y = fma(-b.x, c.y, a.y);
+    a.y = fma(-b.y, c.x, a.y);
+    return a;
 }
 
-// U12 = L11^-1 A12: thread per column c >= k0 + kb
+// Right-hand sides of the substitutions: y in (updated in place), z the
+// forward result.
+struct Rhs {
+    int count;
+    double2 *y[kMaxB], *z[kMaxB];
+};
+
+// Factor the kb x kb block D in shared memory (L below the diagonal, U on and
+// above it), 256 threads: thread t holds row t / 8, columns t % 8 + 8 q in
+// registers.  Step i needs row i and column i of the block as step i - 1 left
+// them, which their owners publish in D; one barrier per step.
 template <typename V>
-__global__ void __launch_bounds__(256) k_lu_trsm(V *A, size_t lda, int n, int k0, int kb) {
-    __shared__ V L[kPanel][kPanel];
-    for (int t = threadIdx.x; t < kb * kb; t += blockDim.x) {
-        const int r = t / kb, c = t % kb;
-        L[r][c] = A[(size_t)(k0 + r) * lda + k0 + c];
+__device__ void factor_diag(V (*D)[kPanel + 1], int kb, int *status) {
+    const int r = threadIdx.x >> 3, c0 = threadIdx.x & 7;
+    V a[kPanel / 8];
+#pragma unroll
+    for (int q = 0; q < kPanel / 8; ++q) a[q] = D[r][c0 + 8 * q];
+#pragma unroll
+    for (int p = 0; p < kPanel / 8; ++p) {
+        // rolled: straight-line code for all 32 steps would be fetched once
+        // per instruction from beyond the instruction cache
+#pragma unroll 1
+        for (int i = 8 * p; i < 8 * p + 8 && i < kb; ++i) {
+            const V piv = D[i][i];
+            if (threadIdx.x == 0 && piv.x == 0 && piv.y == 0) atomicExch(status, 1);
+            if (r > i && r < kb) {
+                const V l = cdiv(D[r][i], piv);
+                if (c0 == (i & 7)) a[p] = l;
+#pragma unroll
+                for (int q = p; q < kPanel / 8; ++q) {
+                    const int c = c0 + 8 * q;
+                    if (c > i) a[q] = cfnma(a[q], l, D[i][c]);
+                    if (c == i + 1 || r == i + 1) D[r][c] = a[q];
+                }
+            }
+            __syncthreads();
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kPanel / 8; ++q) D[r][c0 + 8 * q] = a[q];
+    __syncthreads();
+}
+
+// the first diagonal block (later ones are factored by k_lu_update)
+template <typename V>
+__global__ void __launch_bounds__(256) k_lu_diag(V *A, size_t lda, int k0, int kb, int *status) {
+    __shared__ V D[kPanel][kPanel + 1];
+    for (int t = threadIdx.x; t < kb * kb; t += 256) D[t / kb][t % kb] = A[(size_t)(k0 + t / kb) * lda + k0 + t % kb];
+    __syncthreads();
+    factor_diag(D, kb, status);
+    for (int t = threadIdx.x; t < kb * kb; t += 256) A[(size_t)(k0 + t / kb) * lda + k0 + t % kb] = D[t / kb][t % kb];
+}
+
+// Blocks [0, nt): 32 rows of L21 each; [nt, 2 nt): 32 columns of U12 each; the
+// last block: z = L11^-1 y of every right-hand side (a warp each, FP64).  Eight
+// lanes share a row (column): lane g holds entries g, g + 8, ... and the entry
+// solved in a step goes round by shuffle, so no step needs a barrier and the
+// loops stay short enough for the instruction cache (one thread per row with
+// 32 unrolled steps took 50 us per launch, most of it instruction fetches).
+template <typename V>
+__device__ __forceinline__ V shfl8(V v, int src) {
+    v.x = __shfl_sync(0xffffffffu, v.x, src, 8);
+    v.y = __shfl_sync(0xffffffffu, v.y, src, 8);
+    return v;
+}
+
+template <typename V>
+__global__ void __launch_bounds__(256) k_lu_panel(V *A, size_t lda, int n, int k0, int kb, int nt, Rhs rhs) {
+    __shared__ V D[kPanel][kPanel + 1], T[kPanel][kPanel + 1];
+    constexpr int Q = kPanel / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k1 = k0 + kb;
+    const int blk = (int)blockIdx.x;
+    const bool rows = blk < nt, ycol = blk == 2 * nt;
+    const int j0 = k1 + (rows ? blk : blk - nt) * kPanel;   // first row or column of the block
+    // the diagonal block and the block's own rows or columns, every load
+    // issued before the first is used
+    V d[Q], u[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int r = warp + 8 * q;
+        d[q].x = d[q].y = u[q].x = u[q].y = 0;
+        if (r < kb && lane < kb) d[q] = A[(size_t)(k0 + r) * lda + k0 + lane];
+        if (rows) {
+            if (j0 + r < n && lane < kb) u[q] = A[(size_t)(j0 + r) * lda + k0 + lane];
+        } else if (!ycol) {
+            if (r < kb && j0 + lane < n) u[q] = A[(size_t)(k0 + r) * lda + j0 + lane];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        D[warp + 8 * q][lane] = d[q];
+        T[warp + 8 * q][lane] = u[q];
     }
     __syncthreads();
-    const int c = k0 + kb + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    V u[kPanel];
-#pragma unroll
-    for (int r = 0; r < kPanel; ++r)
-        if (r < kb) u[r] = A[(size_t)(k0 + r) * lda + c];
-#pragma unroll
-    for (int i = 0; i < kPanel; ++i) {
-        if (i >= kb) break;
-#pragma unroll
-        for (int j = i + 1; j < kPanel; ++j)
-            if (j < kb) u[j] = csub(u[j], cmul(L[j][i], u[i]));
+    if (ycol) {
+        for (int q = warp; q < rhs.count; q += 8) {
+            double2 yv = lane < kb ? rhs.y[q][k0 + lane] : make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int i = 0; i < kPanel; ++i) {
+                const double2 yi = make_double2(__shfl_sync(0xffffffffu, yv.x, i), __shfl_sync(0xffffffffu, yv.y, i));
+                if (lane > i && lane < kb) yv = cfnma(yv, ld2(D[lane][i]), yi);
+            }
+            if (lane < kb) rhs.z[q][k0 + lane] = yv;
+        }
+        return;
     }
+    const int m = threadIdx.x >> 3, g = threadIdx.x & 7;   // row (column) of the tile, lane of its eight
+    if (rows) {
 #pragma unroll
-    for (int r = 0; r < kPanel; ++r)
-        if (r < kb) A[(size_t)(k0 + r) * lda + c] = u[r];
+        for (int q = 0; q < Q; ++q) u[q] = T[m][g + 8 * q];
+#pragma unroll
+        for (int p = 0; p < Q; ++p) {
+#pragma unroll 1
+            for (int i = 8 * p; i < 8 * p + 8 && i < kb; ++i) {
+                const V l = cdiv(shfl8(u[p], i & 7), D[i][i]);
+                if (g == (i & 7)) u[p] = l;
+#pragma unroll
+                for (int q = p; q < Q; ++q)
+                    if (g + 8 * q > i) u[q] = cfnma(u[q], l, D[i][g + 8 * q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) T[m][g + 8 * q] = u[q];
+    } else {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) u[q] = T[g + 8 * q][m];
+#pragma unroll
+        for (int p = 0; p < Q; ++p) {
+#pragma unroll 1
+            for (int i = 8 * p; i < 8 * p + 8 && i < kb; ++i) {
+                const V ui = shfl8(u[p], i & 7);
+#pragma unroll
+                for (int q = p; q < Q; ++q)
+                    if (g + 8 * q > i) u[q] = cfnma(u[q], D[g + 8 * q][i], ui);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) T[g + 8 * q][m] = u[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int r = warp + 8 * q;
+        if (rows) {
+            if (j0 + r < n && lane < kb) A[(size_t)(j0 + r) * lda + k0 + lane] = T[r][lane];
+        } else {
+            if (r < kb && j0 + lane < n) A[(size_t)(k0 + r) * lda + j0 + lane] = T[r][lane];
+        }
+    }
 }
 
 // A22 -= L21 U12 over the trailing block [k1, n) x [k1, n), k1 = k0 + kb;
-// 64 x 64 output tiles, 256 threads with 4 x 4 entries each
+// 64 x 64 output tiles, 256 threads with 4 x 4 entries each (rows ty + 16 a,
+// columns tx + 16 b: whole-segment global accesses, no bank conflicts).  The
+// tile at (k1, k1) then factors the next panel's diagonal block; the tiles of
+// the first column also update the right-hand sides' rows, y -= L21 z.
 template <typename V>
-__global__ void __launch_bounds__(256) k_lu_update(V *A, size_t lda, int n, int k0, int kb) {
-    __shared__ V Ls[kTile][kChunk + 1];
-    __shared__ V Us[kChunk][kTile + 1];
+__global__ void __launch_bounds__(256) k_lu_update(V *A, size_t lda, int n, int k0, int kb, Rhs rhs, int *status) {
+    constexpr int CH = kChunk<V>;
+    constexpr int kStage = CH * (2 * kTile + 1), kDiag = kPanel * (kPanel + 1);
+    __shared__ __align__(16) unsigned char sm[sizeof(V) * (kStage > kDiag ? kStage : kDiag)];
+    V (*Ls)[kTile + 1] = reinterpret_cast<V (*)[kTile + 1]>(sm);                                // [CH][row]
+    V (*Us)[kTile] = reinterpret_cast<V (*)[kTile]>(sm + sizeof(V) * CH * (kTile + 1));      // [CH][column]
     const int k1 = k0 + kb;
     const int j0 = k1 + blockIdx.y * kTile, c0 = k1 + blockIdx.x * kTile;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    V acc[4][4];
+    V acc[4][4], old[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b].x = acc[a][b].y = 0;
-    for (int kk = 0; kk < kb; kk += kChunk) {
-        for (int t = threadIdx.x; t < kTile * kChunk; t += 256) {
-            const int r = t / kChunk, q = t % kChunk;
-            const int j = j0 + r, col = k0 + kk + q;
-            V v;
-            v.x = v.y = 0;
-            if (j < n && kk + q < kb) v = A[(size_t)j * lda + col];
-            Ls[r][q] = v;
+        for (int b = 0; b < 4; ++b) {
+            acc[a][b].x = acc[a][b].y = 0;
+            const int j = j0 + ty + 16 * a, c = c0 + tx + 16 * b;
+            old[a][b].x = old[a][b].y = 0;
+            if (j < n && c < n) old[a][b] = A[(size_t)j * lda + c];
         }
-        for (int t = threadIdx.x; t < kTile * kChunk; t += 256) {
-            const int q = t / kTile, r = t % kTile;
-            const int row = k0 + kk + q, c = c0 + r;
+    for (int kk = 0; kk < kb; kk += CH) {
+#pragma unroll
+        for (int t = threadIdx.x; t < kTile * CH; t += 256) {
+            const int r = t / CH, q = t % CH;
             V v;
             v.x = v.y = 0;
-            if (c < n && kk + q < kb) v = A[(size_t)row * lda + c];
+            if (j0 + r < n && kk + q < kb) v = A[(size_t)(j0 + r) * lda + k0 + kk + q];
+            Ls[q][r] = v;
+        }
+#pragma unroll
+        for (int t = threadIdx.x; t < kTile * CH; t += 256) {
+            const int q = t / kTile, r = t % kTile;
+            V v;
+            v.x = v.y = 0;
+            if (c0 + r < n && kk + q < kb) v = A[(size_t)(k0 + kk + q) * lda + c0 + r];
             Us[q][r] = v;
         }
         __syncthreads();
 #pragma unroll 4
-        for (int q = 0; q < kChunk; ++q) {
+        for (int q = 0; q < CH; ++q) {
             V lv[4], uv[4];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) lv[a] = Ls[ty * 4 + a][q];
+            for (int a = 0; a < 4; ++a) lv[a] = Ls[q][ty + 16 * a];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) uv[b] = Us[q][tx * 4 + b];
+            for (int b = 0; b < 4; ++b) uv[b] = Us[q][tx + 16 * b];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    acc[a][b].x += lv[a].x * uv[b].x - lv[a].y * uv[b].y;
-                    acc[a][b].y += lv[a].x * uv[b].y + lv[a].y * uv[b].x;
+                    acc[a][b].x = fma(lv[a].x, uv[b].x, acc[a][b].x);
+                    acc[a][b].x = fma(-lv[a].y, uv[b].y, acc[a][b].x);
+                    acc[a][b].y = fma(lv[a].x, uv[b].y, acc[a][b].y);
+                    acc[a][b].y = fma(lv[a].y, uv[b].x, acc[a][b].y);
                 }
         }
         __syncthreads();
     }
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0;
+    const int nb = min(kPanel, n - k1);   // the next diagonal block
+    V (*D)[kPanel + 1] = reinterpret_cast<V (*)[kPanel + 1]>(sm);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const int j = j0 + ty * 4 + a;
+        const int r = ty + 16 * a, j = j0 + r;
         if (j >= n) continue;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int c = c0 + tx * 4 + b;
-            if (c < n) A[(size_t)j * lda + c] = csub(A[(size_t)j * lda + c], acc[a][b]);
+            const int q = tx + 16 * b, c = c0 + q;
+            if (c >= n) continue;
+            const V v = csub(old[a][b], acc[a][b]);
+            if (first && r < nb && q < nb) D[r][q] = v;
+            else A[(size_t)j * lda + c] = v;
         }
+    }
+    if (blockIdx.x == 0) {
+        // y -= L21 z: 4 lanes per row, 8 columns each
+        const int r = threadIdx.x >> 2, g = threadIdx.x & 3, j = j0 + r;
+        for (int q = 0; q < rhs.count; ++q) {
+            double2 s = make_double2(0.0, 0.0);
+            if (j < n)
+                for (int i = g; i < kb; i += 4) {
+                    const double2 l = ld2(A[(size_t)j * lda + k0 + i]), z = rhs.z[q][k0 + i];
+                    s.x += l.x * z.x - l.y * z.y;
+                    s.y += l.x * z.y + l.y * z.x;
+                }
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+            }
+            if (g == 0 && j < n) rhs.y[q][j] = csub(rhs.y[q][j], s);
+        }
+    }
+    if (first) {
+        __syncthreads();
+        factor_diag(D, nb, status);
+        for (int t = threadIdx.x; t < nb * nb; t += 256) A[(size_t)(k1 + t / nb) * lda + k1 + t % nb] = D[t / nb][t % nb];
     }
 }
 
-// forward substitution with the unit lower L on the diagonal block [k0, k0+kb)
+// Back substitution of one panel: every block solves U11 x = z[k0 .. k0 + kb)
+// (warp 0, lane per row; block 0 keeps the result) and takes x out of its own
+// kRowsPerBwd rows above, 8 lanes per row with 4 columns each, whose entries
+// of U are loaded before the triangle is solved.  blockIdx.y: right-hand side.
 template <typename V>
-__global__ void k_fwd_diag(const V *A, size_t lda, int k0, int kb, double2 *y) {
-    if (threadIdx.x != 0) return;
-    for (int i = 0; i < kb; ++i) {
-        const double2 yi = y[k0 + i];
-        for (int j = i + 1; j < kb; ++j) y[k0 + j] = csub(y[k0 + j], cmul(ld2(A[(size_t)(k0 + j) * lda + k0 + i]), yi));
-    }
-}
-// rows j >= k0 + kb: y_j -= L[j][k0 .. k0+kb) y[k0 .. k0+kb)
-template <typename V>
-__global__ void __launch_bounds__(256) k_fwd_update(const V *A, size_t lda, int n, int k0, int kb, double2 *y) {
-    __shared__ double2 ys[kPanel];
-    if (threadIdx.x < kb) ys[threadIdx.x] = y[k0 + threadIdx.x];
-    __syncthreads();
-    const int j = k0 + kb + blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const V *row = A + (size_t)j * lda + k0;
-    double2 s = y[j];
-    for (int i = 0; i < kb; ++i) s = csub(s, cmul(ld2(row[i]), ys[i]));
-    y[j] = s;
-}
-// back substitution with U on the diagonal block [k0, k0+kb)
-template <typename V>
-__global__ void k_bwd_diag(const V *A, size_t lda, int k0, int kb, double2 *y) {
-    if (threadIdx.x != 0) return;
-    for (int i = kb - 1; i >= 0; --i) {
-        const double2 xi = cdiv(y[k0 + i], ld2(A[(size_t)(k0 + i) * lda + k0 + i]));
-        y[k0 + i] = xi;
-        for (int j = 0; j < i; ++j) y[k0 + j] = csub(y[k0 + j], cmul(ld2(A[(size_t)(k0 + j) * lda + k0 + i]), xi));
-    }
-}
-// rows j < k0: y_j -= U[j][k0 .. k0+kb) x[k0 .. k0+kb)
-template <typename V>
-__global__ void __launch_bounds__(256) k_bwd_update(const V *A, size_t lda, int k0, int kb, double2 *y) {
+__global__ void __launch_bounds__(8 * kRowsPerBwd) k_bwd(const V *A, size_t lda, int k0, int kb, Rhs rhs) {
+    __shared__ V D[kPanel][kPanel + 1];
     __shared__ double2 xs[kPanel];
-    if (threadIdx.x < kb) xs[threadIdx.x] = y[k0 + threadIdx.x];
+    double2 *z = rhs.z[blockIdx.y], *x = rhs.y[blockIdx.y];
+    const int t = threadIdx.x, r = t >> 3, g = t & 7;
+    const int j = blockIdx.x * kRowsPerBwd + r;
+    const bool row = j < k0;
+    V u[kPanel / 8];
+#pragma unroll
+    for (int q = 0; q < kPanel / 8; ++q) {
+        u[q].x = u[q].y = 0;
+        if (row && g + 8 * q < kb) u[q] = A[(size_t)j * lda + k0 + g + 8 * q];
+    }
+#pragma unroll
+    for (int q = 0; q < kPanel / 8; ++q) {
+        const int c = g + 8 * q;
+        V v;
+        v.x = v.y = 0;
+        if (r < kb && c < kb) v = A[(size_t)(k0 + r) * lda + k0 + c];
+        D[r][c] = v;
+    }
     __syncthreads();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= k0) return;
-    const V *row = A + (size_t)j * lda + k0;
-    double2 s = y[j];
-    for (int i = 0; i < kb; ++i) s = csub(s, cmul(ld2(row[i]), xs[i]));
-    y[j] = s;
+    if (t < 32) {
+        // rows scaled by their pivots' inverses first, so that a step of the
+        // solve is one fused update
+        double2 v = t < kb ? z[k0 + t] : make_double2(0.0, 0.0);
+        const double2 one = make_double2(1.0, 0.0);
+        const double2 inv = t < kb ? cdiv(one, ld2(D[t][t])) : one;
+        v = cmul(v, inv);
+#pragma unroll 8
+        for (int i = kPanel - 1; i >= 0; --i) {
+            const double2 f = cmul(ld2(D[t][i]), inv);
+            const double2 xi = make_double2(__shfl_sync(0xffffffffu, v.x, i), __shfl_sync(0xffffffffu, v.y, i));
+            if (t < i && i < kb) v = cfnma(v, f, xi);
+        }
+        if (t < kb) {
+            xs[t] = v;
+            if (blockIdx.x == 0) x[k0 + t] = v;
+        }
+    }
+    __syncthreads();
+    double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < kPanel / 8; ++q) {
+        if (g + 8 * q >= kb) break;
+        const double2 l = ld2(u[q]), xv = xs[g + 8 * q];
+        s.x += l.x * xv.x - l.y * xv.y;
+        s.y += l.x * xv.y + l.y * xv.x;
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (g == 0 && row) z[j] = csub(z[j], s);
 }
 
+// A = L U in place and z = L^-1 y, then y = U^-1 z
 template <typename V>
-cudaError_t factor(V *A, size_t lda, int n, int *status, cudaStream_t st) {
-    long long launches = 0;
+cudaError_t factor_and_solve(V *A, size_t lda, int n, const Rhs &rhs, int *status, cudaStream_t st) {
+    long long launches = 1;
+    k_lu_diag<V><<<1, 256, 0, st>>>(A, lda, 0, min(kPanel, n), status);
     for (int k0 = 0; k0 < n; k0 += kPanel) {
-        const int kb = min(kPanel, n - k0), pend = k0 + kb;
-        for (int i = k0; i < pend; ++i) {
-            const int rows = n - i - 1;
-            if (rows <= 0) continue;
-            k_lu_panel_col<V><<<(rows + 255) / 256, 256, 0, st>>>(A, lda, n, i, pend, status);
-            ++launches;
-        }
-        const int rest = n - pend;
+        const int kb = min(kPanel, n - k0), rest = n - k0 - kb;
+        const int nt = (rest + kPanel - 1) / kPanel;
+        k_lu_panel<V><<<2 * nt + 1, 256, 0, st>>>(A, lda, n, k0, kb, nt, rhs);
+        ++launches;
         if (rest > 0) {
-            k_lu_trsm<V><<<(rest + 255) / 256, 256, 0, st>>>(A, lda, n, k0, kb);
             const int t = (rest + kTile - 1) / kTile;
-            k_lu_update<V><<<dim3(t, t), 256, 0, st>>>(A, lda, n, k0, kb);
-            launches += 2;
+            k_lu_update<V><<<dim3(t, t), 256, 0, st>>>(A, lda, n, k0, kb, rhs, status);
+            ++launches;
         }
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    bem::count_launches(launches);
-    return cudaSuccess;
-}
-
-template <typename V>
-cudaError_t substitute(const V *A, size_t lda, int n, double2 *y, cudaStream_t st) {
-    long long launches = 0;
-    for (int k0 = 0; k0 < n; k0 += kPanel) {
-        const int kb = min(kPanel, n - k0), rest = n - k0 - kb;
-        k_fwd_diag<V><<<1, 32, 0, st>>>(A, lda, k0, kb, y);
-        ++launches;
-        if (rest > 0) {
-            k_fwd_update<V><<<(rest + 255) / 256, 256, 0, st>>>(A, lda, n, k0, kb, y);
-            ++launches;
-        }
-    }
     for (int k0 = ((n - 1) / kPanel) * kPanel; k0 >= 0; k0 -= kPanel) {
         const int kb = min(kPanel, n - k0);
-        k_bwd_diag<V><<<1, 32, 0, st>>>(A, lda, k0, kb, y);
+        const dim3 grid(k0 > 0 ? (k0 + kRowsPerBwd - 1) / kRowsPerBwd : 1, rhs.count);
+        k_bwd<V><<<grid, 8 * kRowsPerBwd, 0, st>>>(A, lda, k0, kb, rhs);
         ++launches;
-        if (k0 > 0) {
-            k_bwd_update<V><<<(k0 + 255) / 256, 256, 0, st>>>(A, lda, k0, kb, y);
-            ++launches;
-        }
     }
     bem::count_launches(launches);
     return cudaGetLastError();
@@ -269,14 +431,16 @@ extern "C" bem_status bem_solve_direct(bem_solver_t s, bem_solve_info *info) {
     const int n = s->n;
     BEM_CU(cudaMemsetAsync(s->d.status, 0, sizeof(int), st));
     BEM_CU(cudaEventRecord(s->ev[2], st));
-    if (s->prec == BEM_PREC_FP64) BEM_CU(factor((double2 *)s->d.A, s->lda, n, s->d.status, st));
-    else BEM_CU(factor((float2 *)s->d.A, s->lda, n, s->d.status, st));
+    Rhs rhs{};
+    rhs.count = s->n_rhs;
     for (int r = 0; r < s->n_rhs; ++r) {
         const bem::SolverBufs &d = s->buf(r);
         BEM_CU(cudaMemcpyAsync(d.x, d.b, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
-        if (s->prec == BEM_PREC_FP64) BEM_CU(substitute((const double2 *)s->d.A, s->lda, n, d.x, st));
-        else BEM_CU(substitute((const float2 *)s->d.A, s->lda, n, d.x, st));
+        rhs.y[r] = d.x;
+        rhs.z[r] = d.r;   // the residual vector, idle here
     }
+    if (s->prec == BEM_PREC_FP64) BEM_CU(factor_and_solve((double2 *)s->d.A, s->lda, n, rhs, s->d.status, st));
+    else BEM_CU(factor_and_solve((float2 *)s->d.A, s->lda, n, rhs, s->d.status, st));
     BEM_CU(cudaEventRecord(s->ev[3], st));
     int zero_pivot = 0;
     BEM_CU(cudaMemcpyAsync(&zero_pivot, s->d.status, sizeof(int), cudaMemcpyDeviceToHost, st));
