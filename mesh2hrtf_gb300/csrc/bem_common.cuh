@@ -85,7 +85,49 @@ __device__ __forceinline__ void phase_sincos(float x, float *s, float *c) {
     *c = cos_approx(r);
 }
 
-__device__ __forceinline__ void sincos_t(double x, double *s, double *c) { sincos(x, s, c); }
+// FP64 counterparts for the plain path, whose kernels are bound by GB300's
+// narrow FP64 pipe: what counts is the number of FP64 instructions.
+//
+// 1 / sqrt(x): the hardware's FP64 seed (about 2^-20 relative) and one
+// third-order step, y + y e (1/2 + 3/8 e) with e = 1 - x y^2: 5 instructions,
+// within 1.5 ulp.
+__device__ __forceinline__ double rsqrt_nr(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// sin and cos of a phase (|x| below 10^9) by table look-up and a short
+// Taylor polynomial (P. T. P. Tang, "Table-driven implementation of the
+// exponential function", ACM TOMS 15, 1989, applied to the circle):
+// x = (q + f) 2 pi / 1024, q an integer, |f| <= 1/2; with the table's
+// (sin, cos) of q 2 pi / 1024 and the polynomials of f 2 pi / 1024
+// (|angle| <= 0.0031: the first terms left out are below 1e-17) the angle sum
+// takes 16 FP64 instructions, against about 35 of the general library
+// routine, whose large-argument branch is never needed here.  The
+// fraction keeps the product's low part (1024 / 2 pi in two doubles), so the
+// result is within about 2 ulp of 1.
+constexpr int kScTab = 1024;
+__device__ double2 g_sctab[kScTab];   // (sin, cos)(2 pi q / kScTab), init_device_tables
+
+__device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
+    constexpr double kShift = 6755399441055744.0;            // 1.5 * 2^52
+    constexpr double kHi = 162.97466172610083;               // 1024 / (2 pi), high and low part
+    constexpr double kLo = -1.0075482457693433e-14;
+    constexpr double a = 0.006135923151542565;                // 2 pi / 1024
+    const double t = fma(x, kHi, kShift);
+    const double q = t - kShift;
+    const double f = fma(x, kLo, fma(x, kHi, -q));
+    const double2 sc = g_sctab[__double2loint(t) & (kScTab - 1)];
+    const double f2 = f * f;
+    const double sr = f * fma(f2, fma(f2, a * a * a * a * a / 120.0, -a * a * a / 6.0), a);
+    const double cm = f2 * fma(f2, a * a * a * a / 24.0, -a * a / 2.0);   // cos - 1
+    *s = sc.x + fma(sc.y, sr, sc.x * cm);
+    *c = sc.y + fma(-sc.x, sr, sc.y * cm);
+}
+
+__device__ __forceinline__ void sincos_t(double x, double *s, double *c) { phase_sincos(x, s, c); }
 __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { phase_sincos(x, s, c); }
 __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
@@ -118,6 +160,9 @@ __constant__ float c_trif[24][3];
 // The 4-point rule's (s - 1/3, t - 1/3, 2 (s - 1/3), 2 (t - 1/3)): operands of
 // the expanded squared distance of the order-2 far pairs.
 __constant__ float c_far4[4][4];
+// (s - 1/3, t - 1/3, weight) in double for the FP64 pairs on flat triangles:
+// every triangle rule's points, in the order of QuadTables::tri
+__constant__ double c_far64[24][4];
 __constant__ float c_glxf[7][6];
 __constant__ float c_glwf[7][6];
 // local node coordinates of 6-/8-noded parents, NC_Arrays.h:126-129
@@ -320,13 +365,14 @@ __device__ __forceinline__ void map_point(const Elem64 &e, double s, double t, c
     double nx = dxs[1] * dxt[2] - dxt[1] * dxs[2];
     double ny = dxs[2] * dxt[0] - dxt[2] * dxs[0];
     double nz = dxs[0] * dxt[1] - dxt[0] * dxs[1];
-    double len = sqrt(nx * nx + ny * ny + nz * nz);
-    q.ny[0] = nx / len; q.ny[1] = ny / len; q.ny[2] = nz / len;
-    q.wj = w * len;
+    const double n2 = nx * nx + ny * ny + nz * nz, il = rsqrt_nr(n2);
+    q.ny[0] = nx * il; q.ny[1] = ny * il; q.ny[2] = nz * il;
+    q.wj = w * (n2 * il);
 #pragma unroll
     for (int k = 0; k < 3; ++k) q.d[k] = y[k] - x[k];
-    q.r = sqrt(q.d[0] * q.d[0] + q.d[1] * q.d[1] + q.d[2] * q.d[2]);
-    q.ir = 1.0 / q.r;
+    const double r2 = q.d[0] * q.d[0] + q.d[1] * q.d[1] + q.d[2] * q.d[2];
+    q.ir = rsqrt_nr(r2);
+    q.r = r2 * q.ir;
 #pragma unroll
     for (int a = 0; a < 4; ++a) q.sh[a] = sh[a];
 }

@@ -13,8 +13,10 @@
 // entries of the per-mesh near lists from a second queue and integrate them
 // cooperatively (warp_subdivide / warp_singular).
 #include <algorithm>
+#include <cmath>
 #include <memory>
 #include <type_traits>
+#include <vector>
 
 #include "bem_internal.h"
 #include "bem_pair.cuh"
@@ -279,6 +281,110 @@ __device__ __forceinline__ float2 far_entry_tri2(const FarCol4 &e, const float D
     return far_entry_tri2_bc<2>(e, D, D2, nx, c);
 }
 
+// FP64 regular pair on a flat triangle, arranged for the fewest FP64
+// instructions (the plain path is bound by GB300's narrow FP64 pipe): the
+// column's edge vectors, normal, Jacobian and, for the 4-point rule,
+// |s_g a + t_g b|^2 are formed once per thread; a point's squared distance is
+// |D|^2 + 2 s D.a + 2 t D.b + |s a + t b|^2 (the terms' cancellation costs at
+// most a factor of ten of the rounding at the smallest ratio, 1.3), and with
+// P = (D.n_y)(d.n_x), u = 1/r, E = n_x.n_y - 3 P u^2 the velocity entry's factor is
+//   u (b wr E - tau D.n_y u) + i u (b u (E + k^2 P) + tau wr D.n_y).
+// 44 FP64 instructions per point (the general form through map_point and the
+// library's square roots, divisions and sincos took about 250).  5120-triangle
+// head, 5 kHz: k_far 33.0 -> 11.9 ms; entries as close to 80-bit ones as
+// before (5.1e-15 against 5.0e-15 at 16 kHz, 1.00e-15 against 1.04e-15 at 4 kHz).
+struct FarCol64 {
+    double c[3];         // centroid
+    double a[3], b[3], n[3];
+    double aa, ab, bb;   // a.a, a.b, b.b
+    double J4;           // J / (4 pi)
+};
+struct FusedCol64 {
+    double yr, yi, tau, b, k2, wr;
+};
+
+__device__ __forceinline__ void far_col64(const DevMesh &m, int j, FarCol64 &e) {
+    double n2 = 0.0;
+    e.aa = e.ab = e.bb = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double p2 = m.v64[(6 + k) * m.n + j];
+        e.a[k] = m.v64[k * m.n + j] - p2;
+        e.b[k] = m.v64[(3 + k) * m.n + j] - p2;
+        e.c[k] = p2 + (e.a[k] + e.b[k]) * (1.0 / 3.0);
+        e.aa = fma(e.a[k], e.a[k], e.aa);
+        e.ab = fma(e.a[k], e.b[k], e.ab);
+        e.bb = fma(e.b[k], e.b[k], e.bb);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int p = (k + 1) % 3, q = (k + 2) % 3;
+        e.n[k] = e.a[p] * e.b[q] - e.b[p] * e.a[q];
+        n2 = fma(e.n[k], e.n[k], n2);
+    }
+    const double il = rsqrt_nr(n2);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) e.n[k] *= il;
+    e.J4 = n2 * il * (1.0 / kPI4);
+}
+
+// Points o0 .. o0 + np - 1 of the triangle rules; D = centroid - x.
+template <int BC>
+__device__ __forceinline__ cplx<double> far_tri64(const FarCol64 &e, const double D[3], const double nx[3], int o0,
+                                                  int np, const FusedCol64 &c) {
+    const double D2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2];
+    const double dny = D[0] * e.n[0] + D[1] * e.n[1] + D[2] * e.n[2];
+    const double dnx0 = D[0] * nx[0] + D[1] * nx[1] + D[2] * nx[2];
+    const double anx = e.a[0] * nx[0] + e.a[1] * nx[1] + e.a[2] * nx[2];
+    const double bnx = e.b[0] * nx[0] + e.b[1] * nx[1] + e.b[2] * nx[2];
+    const double nn = e.n[0] * nx[0] + e.n[1] * nx[1] + e.n[2] * nx[2];
+    const double Da2 = 2.0 * (D[0] * e.a[0] + D[1] * e.a[1] + D[2] * e.a[2]);
+    const double Db2 = 2.0 * (D[0] * e.b[0] + D[1] * e.b[1] + D[2] * e.b[2]);
+    const double ct = -c.tau * dny, cw = c.tau * c.wr * dny, bwr = c.b * c.wr;
+    double ar = 0.0, ai = 0.0;
+#pragma unroll 2
+    for (int g = 0; g < np; ++g) {
+        const double s = c_far64[o0 + g][0], t = c_far64[o0 + g][1], w = c_far64[o0 + g][2];
+        // D2 + s (2 D.a + s a.a + 2 t a.b) + t (2 D.b + t b.b)
+        const double r2 = fma(s, fma(s, e.aa, fma(2.0 * t, e.ab, Da2)), fma(t, fma(t, e.bb, Db2), D2));
+        const double dnx = fma(t, bnx, fma(s, anx, dnx0));
+        const double u = rsqrt_nr(r2), u2 = u * u;
+        double sn, cs;
+        phase_sincos(c.wr * (r2 * u), &sn, &cs);
+        double fr, fi, amp;
+        if (BC == 1) {
+            const double du = dnx * u;
+            fr = fma(-bwr, du, -c.tau);
+            fi = -c.b * du * u;
+            amp = w * e.J4 * u;
+        } else {
+            const double P = dny * dnx, E = fma(-3.0 * P, u2, nn);
+            fr = fma(bwr, E, ct * u);
+            fi = fma(c.b * u, fma(c.k2, P, E), cw);
+            amp = w * e.J4 * u2;
+            if (BC == 2) {
+                // + Y (1 + i b tau z1 re2) / u
+                const double bt = c.b * c.tau, r = r2 * u;
+                const double pr = fma(bt * c.wr, dnx, r), pi = bt * u * dnx;
+                fr += c.yr * pr - c.yi * pi;
+                fi += c.yr * pi + c.yi * pr;
+            }
+        }
+        ar = fma(amp, fma(cs, fr, -sn * fi), ar);
+        ai = fma(amp, fma(cs, fi, sn * fr), ai);
+    }
+    return {ar, ai};
+}
+
+__device__ __forceinline__ cplx<double> far_entry_tri64(const FarCol64 &e, const double x[3], const double nx[3],
+                                                        int order, int bc, const FusedCol64 &c) {
+    const double D[3] = {e.c[0] - x[0], e.c[1] - x[1], e.c[2] - x[2]};
+    const int o0 = tri_offset(order), np = tri_count(order);
+    if (bc == 0) return far_tri64<0>(e, D, nx, o0, np, c);
+    if (bc == 1) return far_tri64<1>(e, D, nx, o0, np, c);
+    return far_tri64<2>(e, D, nx, o0, np, c);
+}
+
 template <typename T>
 __device__ __forceinline__ cplx<T> col_adm(const DevFreq &f, int j, int bc) {
     if (bc != 2 || f.adm == nullptr) return {T(0), T(0)};
@@ -493,19 +599,43 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
     const int bcj = f.bc_type ? f.bc_type[j] : 0;
     const cplx<T> admj = col_adm<T>(f, j, bcj);
     if constexpr (std::is_same<T, double>::value) {
-        Elem64 e;
-        load_elem64(m, j, e);
+        const bool tri = m.nvert[j] == 3;
+        FarCol64 e4;
+        if (tri) far_col64(m, j, e4);
+        const float cjh[3] = {m.chi[j], m.chi[n + j], m.chi[2 * n + j]};
+        const float cjl[3] = {m.clo[j], m.clo[n + j], m.clo[2 * n + j]};
+        const float isq2 = m.isqa32[j] * m.isqa32[j];
+        const FusedCol64 fc = {admj.re, admj.im, f.tao, f.beta_im, f.k * f.k, f.wr};
+#pragma unroll 1
         for (int r = 0; r < kRowsPerThread; ++r) {
             const int i = i0 + r;
             if (i >= n) break;
-            // near and self entries: zero here, k_near adds their integrals
-            if (i == j) { A[(size_t)i * lda + j] = make_double2(0.0, 0.0); continue; }
-            const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
-            const double rd = ratio0_exact(m, j, x64);
-            if (rd < kTolf) { A[(size_t)i * lda + j] = make_double2(0.0, 0.0); continue; }
-            const double nx64[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
-            KVals<double> v = FarPair<double>::run(e, x64, nx64, gauss_order(rd), f.k, f.wr);
-            const cplx<double> val = combine_entry(v, bcj, admj, PT);
+            cplx<double> val = {0.0, 0.0};   // near and self entries: k_near adds their integrals
+            if (i != j) {
+                // the quadrature decision from the float distance, the exact
+                // FP64 one (a square root and a division) only near a threshold
+                const float4 rh = m.row4[3 * (size_t)i], rl = m.row4[3 * (size_t)i + 1];
+                const float d0 = (cjh[0] - rh.x) + (cjl[0] - rl.x), d1 = (cjh[1] - rh.y) + (cjl[1] - rl.y),
+                            d2 = (cjh[2] - rh.z) + (cjl[2] - rl.z);
+                const float q2 = (d0 * d0 + d1 * d1 + d2 * d2) * isq2;
+                bool near = false;
+                int order = 2;
+                if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
+                    order = far_order_exact(&mv, i, j);
+                    near = order == 0;
+                }
+                if (!near) {
+                    const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
+                    const double nx64[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
+                    if (tri) {
+                        val = far_entry_tri64(e4, x64, nx64, order, bcj, fc);
+                    } else {
+                        Elem64 e;
+                        load_elem64(m, j, e);
+                        val = combine_entry(FarPair<double>::run(e, x64, nx64, order, f.k, f.wr), bcj, admj, PT);
+                    }
+                }
+            }
             A[(size_t)i * lda + j] = make_double2(val.re, val.im);
         }
     } else {
@@ -573,8 +703,12 @@ __device__ __forceinline__ void far_tile_img(const DevMeshView &mv, const DevFre
         const DevMesh mk = image_mesh(m, kref);
         const T sg = image_negated(m, kref) ? T(-1) : T(1);
         if constexpr (std::is_same<T, double>::value) {
+            const bool tri = m.nvert[j] == 3;
+            FarCol64 e4;
             Elem64 e;
-            load_elem64(mk, j, e);
+            if (tri) far_col64(mk, j, e4);
+            else load_elem64(mk, j, e);
+            const FusedCol64 fc = {admj.re, admj.im, f.tao, f.beta_im, f.k * f.k, f.wr};
             for (int r = 0; r < kRowsPerThread; ++r) {
                 const int i = i0 + r;
                 if (i >= n) break;
@@ -583,8 +717,10 @@ __device__ __forceinline__ void far_tile_img(const DevMeshView &mv, const DevFre
                 const double rd = ratio0_exact(mk, j, x64);
                 if (rd < kTolf) continue;
                 const double nx64[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
-                KVals<double> v = FarPair<double>::run(e, x64, nx64, gauss_order(rd), f.k, f.wr);
-                const cplx<double> val = combine_entry(v, bcj, admj, PT);
+                const int order = gauss_order(rd);
+                const cplx<double> val =
+                    tri ? far_entry_tri64(e4, x64, nx64, order, bcj, fc)
+                        : combine_entry(FarPair<double>::run(e, x64, nx64, order, f.k, f.wr), bcj, admj, PT);
                 acc_re[r] += sg * val.re;
                 acc_im[r] += sg * val.im;
             }
@@ -641,7 +777,7 @@ constexpr int kFarPerSm = kFarPerSmMax;   // resident k_far blocks per SM allowe
 // operands instead of registers.  IMG: some mesh of the batch has symmetry
 // images (meshes without take the plain tile).
 template <typename T, bool ONE, bool IMG>
-__global__ void __launch_bounds__(256, kFarPerSm) k_far(const __grid_constant__ AsmBatch tb, unsigned *ctr) {
+__global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 2 : kFarPerSm) k_far(const __grid_constant__ AsmBatch tb, unsigned *ctr) {
     __shared__ int item_s;
     const int total = tb.far_off[tb.B];
     while (true) {
@@ -1664,6 +1800,23 @@ cudaError_t init_device_tables() {
         far4[g][3] = 2.0f * far4[g][1];
     }
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far4, far4, sizeof(far4));
+    double far64[24][4];
+    for (int g = 0; g < 24; ++g) {
+        far64[g][0] = kTri[g][0] - 1.0 / 3.0;
+        far64[g][1] = kTri[g][1] - 1.0 / 3.0;
+        far64[g][2] = kTri[g][2];
+        far64[g][3] = 0.0;
+    }
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far64, far64, sizeof(far64));
+    std::vector<double2> sctab(kScTab);
+    for (int q = 0; q < kScTab; ++q) {
+        const long double ang = (long double)q * 6.283185307179586476925286766559005768L / kScTab;
+        sctab[q] = make_double2((double)sinl(ang), (double)cosl(ang));
+    }
+    // exact on the axes, where the long double angle is not
+    for (int q = 0; q < 4; ++q)
+        sctab[q * (kScTab / 4)] = make_double2(q == 1 ? 1.0 : q == 3 ? -1.0 : 0.0, q == 0 ? 1.0 : q == 2 ? -1.0 : 0.0);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_sctab, sctab.data(), sctab.size() * sizeof(double2));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_glxf, glxf, sizeof(glxf));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_glwf, glwf, sizeof(glwf));
     return e;
