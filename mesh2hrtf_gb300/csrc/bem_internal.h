@@ -127,7 +127,7 @@ struct AsmBatch {
     int img;                     // some system's mesh has symmetry images
     int far_off[kMaxAsm + 1];    // tiles of 32 x 32 entries
     int near_off[kMaxAsm + 1];   // near pairs
-    int rhs_off[kMaxAsm + 1];    // blocks of 8 rows
+    int rhs_off[kMaxAsm + 1];    // blocks of 8 or 64 rows (k_rhs)
     AsmSys sys[kMaxAsm];
 };
 // Fills the offset tables from sys[0..B).

@@ -771,6 +771,7 @@ __device__ __forceinline__ void far_tile_img(const DevMeshView &mv, const DevFre
     }
 }
 
+constexpr int kRhsRows = 64;   // k_rhs without boundary columns: rows per block, a thread each
 constexpr int kFarPerSm = kFarPerSmMax;   // resident k_far blocks per SM allowed by the launch bounds
 
 // ONE: the batch holds a single system, whose table then stays in constant
@@ -967,12 +968,36 @@ __device__ cplx<double> incident_rhs(const DevSym &sy, const DevFreq &f, const d
     return zrc;
 }
 
-// Right-hand side, one warp per row (FP64): free term of the prescribed value
-// (NC_EquationSystem.cpp:233-244), incident waves, and the columns whose
+// Free term of the prescribed value (NC_EquationSystem.cpp:233-244) and
+// incident waves of row i.
+__device__ cplx<double> rhs_row(const DevMesh &m, const DevFreq &f, int i, const double x[3], const double nx[3]) {
+    const int n = m.n, nv = m.nvert[i];
+    const int bci = f.bc_type ? f.bc_type[i] : 0;
+    cplx<double> z0 = {0.0, 0.0}, zbvi = {0.0, 0.0};
+    if (f.bc_val)
+        for (int a = 0; a < nv; ++a) zbvi += ld_c(f.bc_val, a * n + i);
+    zbvi = {zbvi.re / (double)nv, zbvi.im / (double)nv};
+    const cplx<double> beta = {0.0, f.beta_im};
+    if (bci != 1) z0 += ((zbvi * beta) * f.tao) * 0.5;
+    else z0 += (zbvi * f.tao) * 0.5;
+    if (f.n_plane + f.n_point > 0) z0 += incident_rhs(m.sym, f, x, nx);
+    return z0;
+}
+
+// Right-hand side (FP64): the row's own terms (rhs_row) and the columns whose
 // prescribed values are nonzero (Zrsintel[4], NC_EquationSystem.cpp:188-198),
 // each with all its images: nodal values in the image's node order, velocity
 // values negated with the reflection factor, no factor on the term itself
 // (NC_ReflectElement, NC_3dFunctions.cpp:410-415; NC_AssembleTBEM).
+//
+// Bound by the FP64 pipe, which issues whole warps, so the lanes have to be
+// full.  Without such columns a thread takes a row (kRhsRows per block, two
+// warps, so that small systems still spread over the SMs): 19 us for 20480
+// rows and one source, 194 us with a warp per row and one lane at work.  With columns a warp takes a row and its lanes
+// the columns: far columns are integrated whole in their lane, subdivided ones
+// and the self pair by the warp, one at a time.  Integrating every column with
+// the warp left 28 of 32 lanes idle on the 4-point rule: 3072 quadrilaterals with
+// one image and 48 such columns 8.2 -> 1.5 ms.
 __global__ void __launch_bounds__(256) k_rhs(const __grid_constant__ AsmBatch tb) {
     __shared__ WarpScratch ws_all[8];
     const int sb = find_sys(tb.rhs_off, tb.B, blockIdx.x);
@@ -980,59 +1005,91 @@ __global__ void __launch_bounds__(256) k_rhs(const __grid_constant__ AsmBatch tb
     const DevMesh m = to_dev(S.m);
     const DevFreq &f = S.f;
     double2 *b = (double2 *)S.b;
-    int *status = S.status;
     const int lane = threadIdx.x, w = threadIdx.y;
-    const int n = m.n;
-    const int i = (blockIdx.x - tb.rhs_off[sb]) * 8 + w;
+    const int n = m.n, blk = blockIdx.x - tb.rhs_off[sb];
+    if (f.n_bc_cols == 0) {
+        const int t = w * 32 + lane, i = blk * kRhsRows + t;
+        if (t >= kRhsRows || i >= n) return;
+        const double x[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
+        const double nx[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
+        const cplx<double> z = rhs_row(m, f, i, x, nx);
+        b[i] = make_double2(z.re, z.im);
+        return;
+    }
+    const int i = blk * 8 + w;
     if (i >= n) return;
     WarpScratch &ws = ws_all[w];
     const double x[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
     const double nx[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
-    Phys<double> P{f.k, f.wr, f.tao, f.beta_im};
-    const cplx<double> beta = {0.0, f.beta_im};
-    cplx<double> z0 = {0.0, 0.0};
-    if (lane == 0) {
-        const int bci = f.bc_type ? f.bc_type[i] : 0;
-        cplx<double> zbvi = {0.0, 0.0};
-        const int nv = m.nvert[i];
-        if (f.bc_val)
-            for (int a = 0; a < nv; ++a) zbvi += ld_c(f.bc_val, a * n + i);
-        zbvi = {zbvi.re / (double)nv, zbvi.im / (double)nv};
-        if (bci != 1) z0 += ((zbvi * beta) * f.tao) * 0.5;
-        else z0 += (zbvi * f.tao) * 0.5;
-        if (f.n_plane + f.n_point > 0) z0 += incident_rhs(m.sym, f, x, nx);
-    }
+    const Phys<double> P{f.k, f.wr, f.tao, f.beta_im};
+    cplx<double> zw = {0.0, 0.0};   // the warp's terms (same on every lane)
     int err = kDevOk;
-    for (int c = 0; c < f.n_bc_cols; ++c) {
-        const int jc = f.bc_cols[c];
-        const int bcj = f.bc_type ? f.bc_type[jc] : 0;
-        const int nvj = m.nvert[jc];
-        for (int kref = 0; kref < m.sym.nref; ++kref) {
-            const DevMesh mk = image_mesh(m, kref);
-            Elem64 e;
-            load_elem64(mk, jc, e);
-            const double vs = (bcj != 1 && image_negated(m, kref)) ? -1.0 : 1.0;
-            cplx<double> bc[4];
+    RhsSink sink;   // the lane's far columns
+    sink.x = x; sink.nx = nx; sink.P = P;
+    sink.init();
+    for (int kref = 0; kref < m.sym.nref; ++kref) {
+        const DevMesh mk = image_mesh(m, kref);
+        const bool neg = image_negated(m, kref);
+        auto values = [&](int jc, int bcj, cplx<double> bc[4]) {
+            const double vs = (bcj != 1 && neg) ? -1.0 : 1.0;
+            const int nvj = m.nvert[jc];
             for (int a = 0; a < 4; ++a)
                 bc[a] = a < nvj ? ld_c(f.bc_val, image_node(a, kref, nvj) * n + jc) * vs : cplx<double>{0.0, 0.0};
-            cplx<double> contrib;
-            if (kref == 0 && jc == i) {
-                SingOut so = warp_singular(e, x, nx, P, bcj == 1 ? 2 : 1, bc);
-                contrib = so.rhs;
-            } else {
-                RhsSink sink;
-                sink.e = &e; sink.x = x; sink.nx = nx; sink.bc = bc; sink.bctype = bcj == 1 ? 1 : 0; sink.P = P;
-                sink.init();
-                const int rc = warp_subdivide(e, m.area64[jc], x, ws, sink);
-                if (rc != kDevOk) err = rc;
-                contrib = sink.reduce();
+        };
+        for (int base = 0; base < f.n_bc_cols; base += 32) {
+            const bool valid = base + lane < f.n_bc_cols;
+            bool whole = false;   // taken by the whole warp
+            if (valid) {
+                const int jc = f.bc_cols[base + lane];
+                const double rd = ratio0_exact(mk, jc, x);
+                whole = rd < kTolf || (kref == 0 && jc == i);
+                if (!whole) {
+                    const int order = gauss_order(rd), bcj = f.bc_type ? f.bc_type[jc] : 0;
+                    Elem64 e;
+                    load_elem64(mk, jc, e);
+                    cplx<double> bc[4];
+                    values(jc, bcj, bc);
+                    sink.e = &e; sink.bc = bc; sink.bctype = bcj == 1 ? 1 : 0;
+                    const int np = sub_npts(e.nv, order);
+                    for (int g = 0; g < np; ++g) {
+                        double s, t, wq;
+                        sub_point(e.nv, order, g, 0.0, 0.0, 1.0, s, t, wq);
+                        sink.add(s, t, wq);
+                    }
+                }
             }
-            if (lane == 0) z0 += contrib;
+            unsigned todo = __ballot_sync(0xffffffffu, whole);
+            while (todo) {
+                const int jc = f.bc_cols[base + __ffs(todo) - 1];
+                todo &= todo - 1;
+                const int bcj = f.bc_type ? f.bc_type[jc] : 0;
+                Elem64 e;
+                load_elem64(mk, jc, e);
+                cplx<double> bc[4];
+                values(jc, bcj, bc);
+                if (kref == 0 && jc == i) {
+                    zw += warp_singular(e, x, nx, P, bcj == 1 ? 2 : 1, bc).rhs;
+                } else {
+                    RhsSink ns;
+                    ns.e = &e; ns.x = x; ns.nx = nx; ns.bc = bc; ns.bctype = bcj == 1 ? 1 : 0; ns.P = P;
+                    ns.init();
+                    // float tables for the subdivision's fast decisions
+                    const float xhi[3] = {m.chi[i], m.chi[n + i], m.chi[2 * n + i]};
+                    const float xlo[3] = {m.clo[i], m.clo[n + i], m.clo[2 * n + i]};
+                    Elem32 ef;
+                    load_elem32(mk, jc, xhi, xlo, ef);
+                    const int rc = warp_subdivide(e, m.area64[jc], x, ws, ns, &ef, m.isqa32[jc]);
+                    if (rc != kDevOk) err = rc;
+                    zw += ns.reduce();
+                }
+            }
         }
     }
+    const cplx<double> zf = sink.reduce();
     if (lane == 0) {
-        b[i] = make_double2(z0.re, z0.im);
-        if (err != kDevOk) atomicMax(status, err);
+        const cplx<double> z = rhs_row(m, f, i, x, nx) + zw + zf;
+        b[i] = make_double2(z.re, z.im);
+        if (err != kDevOk) atomicMax(S.status, err);
     }
 }
 
@@ -1856,7 +1913,8 @@ void asm_batch_finish(AsmBatch &t) {
         const int nt = (n + 31) / 32;
         t.far_off[b + 1] = t.far_off[b] + nt * ((n + 8 * kRowsPerThread - 1) / (8 * kRowsPerThread));
         t.near_off[b + 1] = t.near_off[b] + (int)t.sys[b].n_near;
-        t.rhs_off[b + 1] = t.rhs_off[b] + (n + 7) / 8;
+        const int rows = t.sys[b].f.n_bc_cols > 0 ? 8 : kRhsRows;   // k_rhs: a warp or a thread per row
+        t.rhs_off[b + 1] = t.rhs_off[b] + (n + rows - 1) / rows;
     }
 }
 
