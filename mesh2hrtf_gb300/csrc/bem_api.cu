@@ -866,7 +866,7 @@ bem_status project_group(bem_solver_t *ss, int cnt, const int32_t *npts, const d
             const int np = npts ? npts[c0 + i] : 0;
             t->sys[i] = s->prsys(np, s->pts, (double *)s->pot, (double *)s->grad);
         }
-        bem::proj_batch_finish(*t);
+        bem::proj_batch_finish(*t, prec);
         CU(bem::launch_fields(*t, st));
         CU(bem::launch_project(*t, prec, st));
     }
@@ -1509,7 +1509,7 @@ bem_status bem_solve_multi(bem_solver_t s, int32_t R, const bem_frequency_desc *
         t->B = R;
         for (int r = 0; r < R; ++r)
             t->sys[r] = s->prsys(n_pts, s->pts, s->pot + 2 * (size_t)n_pts * r, s->grad + 6 * (size_t)n_pts * r, r);
-        bem::proj_batch_finish(*t);
+        bem::proj_batch_finish(*t, s->prec == BEM_PREC_FP64 ? 0 : 1);
         CU(bem::launch_fields(*t, st));
         // mixed precision: one kernel evaluation per (point, element) pair
         // for up to 8 right-hand sides at a time
@@ -1518,7 +1518,7 @@ bem_status bem_solve_multi(bem_solver_t s, int32_t R, const bem_frequency_desc *
             for (int c0 = 0; c0 < R; c0 += 8) {
                 u->B = std::min(8, R - c0);
                 for (int r = 0; r < u->B; ++r) u->sys[r] = t->sys[c0 + r];
-                bem::proj_batch_finish(*u);
+                bem::proj_batch_finish(*u, 1);
                 CU(bem::launch_project_multi(*u, st));
             }
         } else {

@@ -129,6 +129,65 @@ __device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
 
 __device__ __forceinline__ void sincos_t(double x, double *s, double *c) { phase_sincos(x, s, c); }
 __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { phase_sincos(x, s, c); }
+// ------------------------------------------------------------ two floats per register pair
+// Packed FP32 arithmetic (PTX fma/mul/add/sub.rn.f32x2): one instruction, two
+// IEEE operations.  The FMA pipe does no more of them per cycle, but the
+// kernels that are bound by instruction issue need half the slots.  Each half
+// rounds exactly as the scalar instruction.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 pk2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpk2(F2 a, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 vmul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 vsub(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ void vdup(F2 &r, float x) { r = pk2(x, x); }
+__device__ __forceinline__ void vdup(double &r, double x) { r = x; }
+// 1 / sqrt, and sin and cos of a phase, half by half (phase_sincos's steps)
+__device__ __forceinline__ F2 vrsqrt(F2 a) {
+    float lo, hi;
+    unpk2(a, lo, hi);
+    return pk2(rsqrt_approx(lo), rsqrt_approx(hi));
+}
+__device__ __forceinline__ double vrsqrt(double a) { return rsqrt_nr(a); }
+__device__ __forceinline__ void vsincos(F2 x, F2 &s, F2 &c) {
+    const F2 shift = pk2(12582912.0f, 12582912.0f);
+    const F2 q = vsub(vfma(x, pk2(0.159154943f, 0.159154943f), shift), shift);
+    F2 r = vfma(q, pk2(-6.28318548202514648f, -6.28318548202514648f), x);
+    r = vfma(q, pk2(1.74845553146951e-07f, 1.74845553146951e-07f), r);
+    float lo, hi;
+    unpk2(r, lo, hi);
+    s = pk2(sin_approx(lo), sin_approx(hi));
+    c = pk2(cos_approx(lo), cos_approx(hi));
+}
+__device__ __forceinline__ void vsincos(double x, double &s, double &c) { phase_sincos(x, &s, &c); }
+
 __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 
@@ -163,6 +222,8 @@ __constant__ float c_far4[4][4];
 // (s - 1/3, t - 1/3, weight) in double for the FP64 pairs on flat triangles:
 // every triangle rule's points, in the order of QuadTables::tri
 __constant__ double c_far64[24][4];
+// (s - 1/3, t - 1/3, weight) of the 4-point rule, each twice (a packed operand)
+__constant__ float2 c_far4d[4][3];
 __constant__ float c_glxf[7][6];
 __constant__ float c_glwf[7][6];
 // local node coordinates of 6-/8-noded parents, NC_Arrays.h:126-129

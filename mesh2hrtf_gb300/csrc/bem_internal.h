@@ -181,20 +181,23 @@ struct ProjSys {
     const double *pts;      // [npts][3]
     double *pot, *grad;     // [npts], [npts][3] complex; grad may be nullptr
     int *status;
-    float4 *part;           // float projection: partial sums [slice][point][2]
+    float4 *part;           // partial sums [slice][point], 2 float4 (FP64: 4) each
                             // (the Krylov basis, idle once the system is solved)
     long long part_cap;     // its capacity in float4
-    int nslice;             // element slices (proj_batch_finish; 0: one warp per point)
+    // work split (proj_batch_finish): element slices (0: the scratch is too
+    // short, one warp per point), elements per slice, point groups per block
+    // and points per slice of the scratch
+    int nslice, per, pgb, pstride;
 };
 struct ProjBatch {
     int B;
     int fld_off[kMaxAsm + 1];    // blocks of 256 elements
     int pt_off[kMaxAsm + 1];     // blocks of 8 points
-    int lp_off[kMaxAsm + 1];     // blocks of 8 (32-point group, element slice) warps
-    int ps_off[kMaxAsm + 1];     // blocks of 256 points (slice sums)
+    int lp_off[kMaxAsm + 1];     // blocks of (point groups, element slice)
+    int ps_off[kMaxAsm + 1];     // blocks of 4 or 32 points (slice sums)
     ProjSys sys[kMaxAsm];
 };
-void proj_batch_finish(ProjBatch &t);
+void proj_batch_finish(ProjBatch &t, int prec);
 // Element potentials and nodal normal velocities from the unknowns, then
 // potential and gradient at the points.
 cudaError_t launch_fields(const ProjBatch &t, cudaStream_t st);

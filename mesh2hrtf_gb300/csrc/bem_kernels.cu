@@ -1404,346 +1404,617 @@ __global__ void __launch_bounds__(256, 2) k_project(const __grid_constant__ Proj
     }
 }
 
-// Float projection with the roles of lanes and elements exchanged: a warp
-// takes 32 evaluation points (one per lane) and a slice of the elements,
-// and sweeps the slice one element at a time, so every element's data is a
-// warp-uniform load shared by 32 points instead of 32 loads of different
-// elements.  Partial sums go to ProjSys::part per (slice, point);
-// k_project_sum adds the slices in slice order (FP64) and finishes the
-// point.  Pair arithmetic as in k_project<float>: the fused flat-triangle
-// rule, the general rule, and the warp-wide subdivision for near pairs, here
-// one near lane at a time.
-constexpr int kProjSlice = 256;   // elements per slice (fewer slices if the scratch is short)
+// Projection with lanes = evaluation points.  A block takes some groups of
+// points (32 lanes x kP points per lane) and a slice of the elements, which it
+// stages kProjChunk at a time in shared memory; its 8 warps are pgb point
+// groups x 8 / pgb element parts (pgb < 8 when there are few groups, so that
+// a call for a few points still spreads over the SMs).  An element's data is
+// the same for all lanes: one broadcast read serves 32 kP points.
+//
+// In float a lane holds two points and the 4-point rule runs in packed
+// arithmetic: the kernel was bound by instruction issue (about 62 FP32
+// instructions per evaluation), now by the FMA pipe.  The distance, the
+// phase k r and its reduction are rounded operation by operation as in
+// map_point / phase_sincos: at k r of hundreds of radians their rounding is
+// the result's error.  The rest is regrouped: with G = w u e^{i wr r}, u = 1/r
+// and alpha = u^2 - i wr u, an element's sums over its points
+//   P0 = -sum (d.n_y) G alpha
+//   G0 = sum n_y G alpha + (d.n_y) u^2 (k^2 G - 3 G alpha) d
+// do not depend on the unknowns: the element adds W P0 to the potential and
+// W G0 to the gradient, W = phi J / 4 pi (NC_IntegrationTBEM,
+// NC_PostProcessing.cpp:1217-1322, for H = G (-u + i wr) (r^.n_y)).  So the
+// right-hand sides of one matrix (NR > 1) share them.  Elements with nodal
+// velocities add V G and V G alpha d per point, V = -(velocity at the point)
+// J / 4 pi.  d.n_y is constant on a flat triangle, so its normal terms wait
+// for the element's sum.  A right-hand side's sums are formed by the same
+// operations in the same order whatever NR is.
+//
+// Points of higher order and subdivided pairs take proj_whole and
+// warp_subdivide.  Partial sums go to ProjSys::part per (slice, point);
+// k_project_sum adds the slices (FP64) and finishes the point.  In float, 11950
+// points on 20480 elements 3.87 -> 2.15 ms (41 instructions per evaluation,
+// FMA pipe 64 % active on a smaller case), 64 points on 5120 elements 225 ->
+// 17 us (40 warps swept the elements before), 3072 quadrilaterals with an
+// image and velocities, 1730 points 1.63 -> 0.18 ms; FP64, 1730 points on 5120
+// elements 17.1 -> 5.8 ms.
+constexpr int kProjSlice = 256;   // most elements per slice
+constexpr int kProjStep = 16;     // fewest elements per slice
+// elements staged at a time (the stage and the subdivision scratch share 48 KB)
+__host__ __device__ constexpr int proj_chunk(int nr) { return nr <= 2 ? 16 : 8; }
+constexpr int kProjSlots = 304;   // resident blocks: 2 on each of 152 SMs
 
-__global__ void __launch_bounds__(256, 2) k_project_pts(const __grid_constant__ ProjBatch tb) {
+template <typename T> struct ProjLane;
+template <> struct ProjLane<float> { using R = F2; static constexpr int kP = 2, kPart = 2; };
+template <> struct ProjLane<double> { using R = double; static constexpr int kP = 1, kPart = 4; };
+
+// A staged element.  v[0..2] centre (float: high parts, v[3..5] low parts);
+// triangles: 6 a, 9 b, 12 n; quadrilaterals, per point g: 6 + 3 g offset (FP64:
+// position), 18 + 3 g normal, 30 + g weight.  Per right-hand side W (re, im,
+// -im) and, where some right-hand side has nodal velocities, V of the points.
+template <typename T, int NR> struct ProjElem {
+    typename ProjLane<T>::R v[34], W[NR][3], V[NR][4][3];
+    float hi[3], lo[3], isq2;
+    int nv, iv;
+};
+
+template <typename T>
+__device__ __forceinline__ void proj_put(typename ProjLane<T>::R *v, cplx<T> z) {
+    vdup(v[0], z.re);
+    vdup(v[1], z.im);
+    vdup(v[2], -z.im);
+}
+
+// Thread g (0..3) of element j's four: its part of the staged element.  sys:
+// the right-hand sides' systems (nr of them).
+template <typename T, int NR>
+__device__ void proj_stage(const ProjSys *sys, int nr, const DevMesh &m, const DevMesh &mk, int kref, bool neg, int j,
+                           int g, ProjElem<T, NR> &o) {
+    const int n = m.n, nv = m.nvert[j];
+    const T i4pi = T(1.0 / kPI4);
+    T fac = i4pi, sh[4];   // J / 4 pi (1 / 4 pi on quadrilaterals); shape functions at point g
+    if (nv == 3) {
+        sh[0] = (T)c_quad.tri[g][0];
+        sh[1] = (T)c_quad.tri[g][1];
+        sh[2] = T(1) - sh[0] - sh[1];
+        sh[3] = T(0);
+        T J;
+        if constexpr (std::is_same<T, float>::value) {
+            J = mk.t32[9 * n + j];
+            if (g < 3) {   // one of a, b, n each
+                for (int k = 0; k < 3; ++k) vdup(o.v[6 + 3 * g + k], mk.t32[(3 * g + k) * n + j]);
+            }
+        } else {
+            FarCol64 f;
+            far_col64(mk, j, f);
+            J = f.J4 * kPI4;
+            for (int k = 0; k < 3; ++k) {
+                if (g == 0) o.v[6 + k] = f.a[k];
+                if (g == 1) o.v[9 + k] = f.b[k];
+                if (g == 2) o.v[12 + k] = f.n[k];
+                if (g == 3) o.v[k] = f.c[k];
+            }
+        }
+        fac = J * i4pi;
+    } else {
+        QPoint<T> q;
+        if constexpr (std::is_same<T, float>::value) {
+            Elem32 e;
+            const float zero[3] = {0.f, 0.f, 0.f};
+            load_elem32(mk, j, zero, zero, e);
+            e.D[0] = e.D[1] = e.D[2] = 0.f;
+            map_point(e, c_glxf[2][g >> 1], c_glxf[2][g & 1], c_glwf[2][g >> 1] * c_glwf[2][g & 1], q);
+        } else {
+            Elem64 e;
+            load_elem64(mk, j, e);
+            const double zero[3] = {0.0, 0.0, 0.0};
+            map_point(e, c_quad.glx[2][g >> 1], c_quad.glx[2][g & 1], zero,
+                      c_quad.glw[2][g >> 1] * c_quad.glw[2][g & 1], q);
+        }
+        for (int k = 0; k < 3; ++k) {
+            vdup(o.v[6 + 3 * g + k], q.d[k]);
+            vdup(o.v[18 + 3 * g + k], q.ny[k]);
+        }
+        vdup(o.v[30 + g], q.wj);
+        for (int a = 0; a < 4; ++a) sh[a] = q.sh[a];
+    }
+    if (g == 0) {
+        o.nv = nv;
+        const float q = m.isqa32[j];
+        o.isq2 = q * q;
+        for (int k = 0; k < 3; ++k) {
+            o.hi[k] = mk.chi[k * n + j];
+            o.lo[k] = mk.clo[k * n + j];
+            if constexpr (std::is_same<T, float>::value) {
+                vdup(o.v[k], o.hi[k]);
+                vdup(o.v[3 + k], o.lo[k]);
+            }
+        }
+    }
+    bool any = false;
+#pragma unroll 1
+    for (int r = 0; r < nr; ++r) any |= sys[r].ivi[j] != 0;
+    if (g == 0) o.iv = any;
+#pragma unroll 1
+    for (int r = 0; r < nr; ++r) {
+        const ProjSys &S = sys[r];
+        const bool iv = S.ivi[j] != 0;
+        cplx<T> ph, vl[4];
+        proj_elem_data<T>((const double2 *)S.phi, (const double2 *)S.vel, (const float2 *)S.phi32,
+                          (const float2 *)S.vel32, n, j, nv, iv, kref, neg, ph, vl);
+        if (g == 0) proj_put<T>(o.W[r], ph * fac);
+        if (any) {
+            cplx<T> z = {T(0), T(0)};
+            for (int a = 0; a < 4; ++a) z += vl[a] * sh[a];
+            proj_put<T>(o.V[r][g], z * -fac);
+        }
+    }
+}
+
+template <typename R> struct RAcc { R pr, pi, gr[3], gi[3]; };
+
+// The 4-point rule of a staged element at the lane's points, for the points
+// with their bit in mask, added to the right-hand sides' sums.
+template <typename T, int NR, bool TRI, bool VEL>
+__device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const typename ProjLane<T>::R (&D)[3],
+                                         unsigned mask, typename ProjLane<T>::R wr, typename ProjLane<T>::R nwr,
+                                         typename ProjLane<T>::R k2, typename ProjLane<T>::R m3,
+                                         RAcc<typename ProjLane<T>::R> (&acc)[NR]) {
+    using R = typename ProjLane<T>::R;
+    R dny, Tr, Ti, P0r, P0i, G0r[3], G0i[3];
+    vdup(Tr, 0);
+    Ti = P0r = P0i = Tr;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) G0r[k] = G0i[k] = Tr;
+    if (TRI) dny = vfma(D[2], e.v[14], vfma(D[0], e.v[12], vmul(D[1], e.v[13])));
+    constexpr int kUnroll = std::is_same<T, float>::value ? 4 : 1;   // FP64: pipe bound, registers short
+#pragma unroll kUnroll
+    for (int g = 0; g < 4; ++g) {
+        R d[3], w;
+        if constexpr (TRI) {
+            R ss, tt;
+            if constexpr (std::is_same<T, float>::value) {
+                const float2 s2 = c_far4d[g][0], t2 = c_far4d[g][1], w2 = c_far4d[g][2];
+                ss = pk2(s2.x, s2.y);
+                tt = pk2(t2.x, t2.y);
+                w = pk2(w2.x, w2.y);
+            } else {
+                ss = c_far64[g][0];
+                tt = c_far64[g][1];
+                w = c_far64[g][2];
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d[k] = vfma(tt, e.v[9 + k], vfma(ss, e.v[6 + k], D[k]));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d[k] = vadd(D[k], e.v[6 + 3 * g + k]);
+            dny = vfma(d[2], e.v[18 + 3 * g + 2], vfma(d[0], e.v[18 + 3 * g], vmul(d[1], e.v[18 + 3 * g + 1])));
+            w = e.v[30 + g];
+        }
+        const R r2 = vfma(d[2], d[2], vfma(d[0], d[0], vmul(d[1], d[1])));
+        R u = vrsqrt(r2), sn, cs;
+        vsincos(vmul(wr, vmul(r2, u)), sn, cs);
+        if constexpr (std::is_same<T, float>::value) {
+            float lo, hi;
+            unpk2(u, lo, hi);
+            u = pk2((mask & 1u) ? lo : 0.f, (mask & 2u) ? hi : 0.f);
+        } else {
+            u = mask ? u : 0.0;
+        }
+        const R A = vmul(u, u), B = vmul(wr, u), nB = vmul(nwr, u), p = vmul(w, u);
+        const R Gr = vmul(p, cs), Gi = vmul(p, sn);
+        const R hr = vfma(Gi, B, vmul(Gr, A)), hi = vfma(Gr, nB, vmul(Gi, A));   // G alpha
+        const R Ad = vmul(A, dny);
+        const R vr = vmul(Ad, vfma(m3, hr, vmul(k2, Gr))), vi = vmul(Ad, vfma(m3, hi, vmul(k2, Gi)));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            G0r[k] = vfma(vr, d[k], G0r[k]);
+            G0i[k] = vfma(vi, d[k], G0i[k]);
+        }
+        if (TRI) {
+            Tr = vadd(Tr, hr);
+            Ti = vadd(Ti, hi);
+        } else {
+            P0r = vsub(P0r, vmul(dny, hr));
+            P0i = vsub(P0i, vmul(dny, hi));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                G0r[k] = vfma(hr, e.v[18 + 3 * g + k], G0r[k]);
+                G0i[k] = vfma(hi, e.v[18 + 3 * g + k], G0i[k]);
+            }
+        }
+        if (VEL) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                if (r >= nr) break;
+                const R *V = e.V[r][g];
+                acc[r].pr = vfma(V[0], Gr, vfma(V[2], Gi, acc[r].pr));
+                acc[r].pi = vfma(V[0], Gi, vfma(V[1], Gr, acc[r].pi));
+                const R zr = vfma(V[2], hi, vmul(V[0], hr)), zi = vfma(V[1], hr, vmul(V[0], hi));
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    acc[r].gr[k] = vfma(zr, d[k], acc[r].gr[k]);
+                    acc[r].gi[k] = vfma(zi, d[k], acc[r].gi[k]);
+                }
+            }
+        }
+    }
+    if (TRI) {
+        P0r = vsub(P0r, vmul(dny, Tr));
+        P0i = vsub(P0i, vmul(dny, Ti));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            G0r[k] = vfma(Tr, e.v[12 + k], G0r[k]);
+            G0i[k] = vfma(Ti, e.v[12 + k], G0i[k]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        if (r >= nr) break;
+        const R Wr = e.W[r][0], Wi = e.W[r][1], nWi = e.W[r][2];
+        acc[r].pr = vfma(Wr, P0r, vfma(nWi, P0i, acc[r].pr));
+        acc[r].pi = vfma(Wr, P0i, vfma(Wi, P0r, acc[r].pi));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            acc[r].gr[k] = vfma(Wr, G0r[k], vfma(nWi, G0i[k], acc[r].gr[k]));
+            acc[r].gi[k] = vfma(Wr, G0i[k], vfma(Wi, G0r[k], acc[r].gi[k]));
+        }
+    }
+}
+
+// A not subdivided pair of a higher Gauss order, by one lane.
+template <typename T>
+__device__ __noinline__ ProjAcc<T> proj_whole(const ProjSys *Sp, int kref, int j, int order, int p) {
+    const ProjSys &S = *Sp;
+    const DevMesh m = to_dev(S.m);
+    const DevMesh mk = image_mesh(m, kref);
+    const int n = m.n, nv = m.nvert[j];
+    const bool iv = S.ivi[j] != 0;
+    const double x[3] = {S.pts[3 * p], S.pts[3 * p + 1], S.pts[3 * p + 2]};
+    cplx<T> ph, vl[4];
+    proj_elem_data<T>((const double2 *)S.phi, (const double2 *)S.vel, (const float2 *)S.phi32,
+                      (const float2 *)S.vel32, n, j, nv, iv, kref, image_negated(m, kref), ph, vl);
+    ProjAcc<T> acc;
+    acc.p = acc.g[0] = acc.g[1] = acc.g[2] = cmk(T(0), T(0));
+    const T k = (T)S.f.k, wr = (T)S.f.wr;
+    const int np = sub_npts(nv, order);
+    if constexpr (std::is_same<T, double>::value) {
+        Elem64 e;
+        load_elem64(mk, j, e);
+        for (int g = 0; g < np; ++g) {
+            double s, t, w;
+            sub_point(nv, order, g, 0.0, 0.0, 1.0, s, t, w);
+            QPoint<double> q;
+            map_point(e, s, t, x, w, q);
+            proj_point(q, ph, vl, nv, iv, k, wr, acc);
+        }
+    } else {
+        float xhi[3], xlo[3];
+        for (int c = 0; c < 3; ++c) {
+            xhi[c] = (float)x[c];
+            xlo[c] = (float)(x[c] - (double)xhi[c]);
+        }
+        Elem32 e;
+        load_elem32(mk, j, xhi, xlo, e);
+        for (int g = 0; g < np; ++g) {
+            float s, t, w;
+            sub_point_f(nv, order, g, 0.f, 0.f, 1.f, s, t, w);
+            QPoint<float> q;
+            map_point(e, s, t, w, q);
+            proj_point(q, ph, vl, nv, iv, k, wr, acc);
+        }
+    }
+    return acc;
+}
+
+// A subdivided pair, by the whole warp; the reduced sum on every lane.
+template <typename T>
+__device__ __noinline__ ProjAcc<T> proj_near(const ProjSys *Sp, int kref, int j, int p, WarpScratch *ws, int *err) {
+    const ProjSys &S = *Sp;
+    const DevMesh m = to_dev(S.m);
+    const DevMesh mk = image_mesh(m, kref);
+    const int n = m.n;
+    const double x[3] = {S.pts[3 * p], S.pts[3 * p + 1], S.pts[3 * p + 2]};   // a uniform load
+    float xhi[3], xlo[3];
+    for (int c = 0; c < 3; ++c) {
+        xhi[c] = (float)x[c];
+        xlo[c] = (float)(x[c] - (double)xhi[c]);
+    }
+    Elem64 e;
+    load_elem64(mk, j, e);
+    Elem32 e32;   // float arithmetic, and the subdivision's fast decisions
+    load_elem32(mk, j, xhi, xlo, e32);
+    cplx<T> ph, vl[4];
+    proj_elem_data<T>((const double2 *)S.phi, (const double2 *)S.vel, (const float2 *)S.phi32,
+                      (const float2 *)S.vel32, n, j, e.nv, true, kref, image_negated(m, kref), ph, vl);
+    ProjSink<T> sink;
+    if constexpr (std::is_same<T, double>::value) { sink.e = &e; sink.x = x; }
+    else sink.e = &e32;
+    sink.phi = ph; sink.vel = vl; sink.ivi = S.ivi[j] != 0; sink.k = (T)S.f.k; sink.wr = (T)S.f.wr;
+    sink.init();
+    const int rc = warp_subdivide(e, m.area64[j], x, *ws, sink, &e32, m.isqa32[j]);
+    if (rc != kDevOk) *err = rc;
+    return sink.reduce();
+}
+
+__device__ __forceinline__ void racc_add(RAcc<double> &a, int, const ProjAcc<double> &b) {
+    a.pr += b.p.re;
+    a.pi += b.p.im;
+    for (int k = 0; k < 3; ++k) { a.gr[k] += b.g[k].re; a.gi[k] += b.g[k].im; }
+}
+__device__ __forceinline__ void half_add(F2 &a, int h, float x) { a = vadd(a, h ? pk2(0.f, x) : pk2(x, 0.f)); }
+__device__ __forceinline__ void racc_add(RAcc<F2> &a, int h, const ProjAcc<float> &b) {
+    half_add(a.pr, h, b.p.re);
+    half_add(a.pi, h, b.p.im);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        half_add(a.gr[k], h, b.g[k].re);
+        half_add(a.gi[k], h, b.g[k].im);
+    }
+}
+
+// acc[r] += b for the lane's point h, with every index known at compile time
+// (a runtime index would put the sums in local memory)
+template <typename T, int NR>
+__device__ __forceinline__ void racc_at(RAcc<typename ProjLane<T>::R> (&acc)[NR], int r, int h, const ProjAcc<T> &b) {
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+        if (q == r) racc_add(acc[q], h, b);
+}
+
+// NR = 1: the batch's systems, one after the other.  NR > 1: systems 0 .. nr - 1
+// are right-hand sides of one matrix (same mesh, points and split).
+template <typename T, int NR>
+__global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __grid_constant__ ProjBatch tb, int nr) {
+    using R = typename ProjLane<T>::R;
+    constexpr int P = ProjLane<T>::kP, kChunk = proj_chunk(NR);
     __shared__ WarpScratch ws_all[8];
-    const int sb = find_sys(tb.lp_off, tb.B, blockIdx.x);
+    __shared__ ProjElem<T, NR> el[kChunk];
+    static_assert(sizeof(ws_all) >= 256 * 8 * sizeof(R), "the warps' sums fit the subdivision scratch");
+    const int sb = NR > 1 ? 0 : find_sys(tb.lp_off, tb.B, blockIdx.x);
     const ProjSys &S = tb.sys[sb];
     const DevMesh m = to_dev(S.m);
     const DevFreq &f = S.f;
-    const int lane = threadIdx.x, w = threadIdx.y, n = m.n, npts = S.npts;
-    const int G = (npts + 31) >> 5, nsl = S.nslice;
-    const int item = (blockIdx.x - tb.lp_off[sb]) * 8 + w;
-    if (item >= G * nsl) return;
-    const int g = item % G, sl = item / G;
-    const int per = (n + nsl - 1) / nsl;
-    const int j0 = sl * per, j1 = min(n, j0 + per);
-    const int p = g * 32 + lane;
-    const bool pv = p < npts;
-    const int pp = pv ? p : g * 32;   // idle lanes shadow the group's first point
-    WarpScratch &ws = ws_all[w];
-    // The point as float hi/lo pair and the wave numbers in float, made opaque
-    // to the compiler: under register pressure it otherwise recomputes them
-    // from the FP64 values at every pair, and GB300 issues those conversions
-    // (and the FP64 subtraction) on its narrow FP64 pipe.
-    float xhi[3], xlo[3];
-    for (int c = 0; c < 3; ++c) {
-        const double xv = S.pts[3 * pp + c];
-        xhi[c] = (float)xv;
-        xlo[c] = (float)(xv - (double)xhi[c]);
-        asm volatile("" : "+f"(xhi[c]), "+f"(xlo[c]));
+    const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane, n = m.n, npts = S.npts;
+    const int nsl = S.nslice, pgb = S.pgb, ewb = 8 / pgb;
+    const int item = blockIdx.x - tb.lp_off[sb];
+    const int sl = item % nsl, gb = item / nsl;
+    const int ew = w / pgb;                                   // element part
+    const int p0 = (gb * pgb + w % pgb) * 32 * P + lane;     // the lane's points: p0, p0 + 32
+    const int j0 = sl * S.per, j1 = min(n, j0 + S.per);
+    const bool group = p0 - lane < npts;                      // the warp has points
+    // The points, as float hi/lo pairs for the distances of the quadrature
+    // decision and (float) the arithmetic; made opaque to the compiler: under
+    // register pressure it otherwise recomputes them from the FP64 values,
+    // and GB300 issues those conversions on its narrow FP64 pipe.  Idle
+    // points repeat the group's first.
+    float xh[P][3], xl[P][3];
+    R X[6];   // float: packed high and low parts; FP64: the point
+#pragma unroll
+    for (int h = 0; h < P; ++h) {
+        const int p = p0 + 32 * h < npts ? p0 + 32 * h : (group ? p0 - lane : 0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double xv = S.pts[3 * p + c];
+            xh[h][c] = (float)xv;
+            xl[h][c] = (float)(xv - (double)xh[h][c]);
+            asm volatile("" : "+f"(xh[h][c]), "+f"(xl[h][c]));
+            if constexpr (P == 1) X[c] = xv;
+        }
     }
-    const double2 *phi = (const double2 *)S.phi, *vel = (const double2 *)S.vel;
-    const float2 *phi32 = (const float2 *)S.phi32, *vel32 = (const float2 *)S.vel32;
-    ProjAcc<float> acc;
-    acc.p = acc.g[0] = acc.g[1] = acc.g[2] = cmk(0.f, 0.f);
-    float k = (float)f.k, wr = (float)f.wr;
-    asm volatile("" : "+f"(k), "+f"(wr));
-    const float k2 = k * k;
+    if constexpr (P == 2) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            X[c] = pk2(xh[0][c], xh[P - 1][c]);
+            X[3 + c] = pk2(xl[0][c], xl[P - 1][c]);
+        }
+    }
+    T k = (T)f.k, wrs = (T)f.wr;
+    if constexpr (P == 2) asm volatile("" : "+f"(k), "+f"(wrs));
+    R wr, nwr, k2, m3;
+    vdup(wr, wrs);
+    vdup(nwr, -wrs);
+    vdup(k2, k * k);
+    vdup(m3, T(-3));
+    RAcc<R> acc[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        vdup(acc[r].pr, 0);
+        acc[r].pi = acc[r].pr;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[r].gr[c] = acc[r].gi[c] = acc[r].pr;
+    }
+    if (NR == 1) nr = 1;
     int err = kDevOk;
     for (int kref = 0; kref < m.sym.nref; ++kref) {
         const DevMesh mk = image_mesh(m, kref);
         const bool neg = image_negated(m, kref);
-        for (int j = j0; j < j1; ++j) {
-            const bool iv = S.ivi[j] != 0;
-            const int nv = m.nvert[j];
-            cplx<float> ph, vl[4];
-            proj_elem_data<float>(phi, vel, phi32, vel32, n, j, nv, iv, kref, neg, ph, vl);
-            Elem32 e;
-            load_elem32(mk, j, xhi, xlo, e);
-            const float isq = m.isqa32[j];
-            const float q2 = (e.D[0] * e.D[0] + e.D[1] * e.D[1] + e.D[2] * e.D[2]) * (isq * isq);
-            bool near = false;
-            int order = 2;
-            if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
-                const double xp[3] = {S.pts[3 * pp], S.pts[3 * pp + 1], S.pts[3 * pp + 2]};
-                const double rd = ratio0_exact(mk, j, xp);
-                near = rd < kTolf;
-                if (!near) order = gauss_order(rd);
-            }
-            if (!near && e.nv == 3 && !iv) {
-                float2 P = make_float2(0.f, 0.f), U[3], Tn = make_float2(0.f, 0.f);
-                U[0] = U[1] = U[2] = make_float2(0.f, 0.f);
-                const float dny = e.D[0] * e.n[0] + e.D[1] * e.n[1] + e.D[2] * e.n[2];
-                if (order <= 2) proj_tri_points<4, 0>(e, dny, k2, wr, P, U, Tn);
-                else if (order == 3) proj_tri_points<7, 4>(e, dny, k2, wr, P, U, Tn);
-                else proj_tri_points<13, 11>(e, dny, k2, wr, P, U, Tn);
-                const cplx<float> pq = ph * cplx<float>{P.x, P.y};
-                acc.p.re += pq.re;
-                acc.p.im += pq.im;
+        for (int base = j0; base < j1; base += kChunk) {
+            const int cnt = min(kChunk, j1 - base);
+            __syncthreads();   // the previous chunk has been read
+            if (tid < 4 * kChunk && (tid >> 2) < cnt)
+                proj_stage<T, NR>(&S, nr, m, mk, kref, neg, base + (tid >> 2), tid & 3, el[tid >> 2]);
+            __syncthreads();
+            if (!group) continue;
+            for (int q = ew; q < cnt; q += ewb) {
+                const ProjElem<T, NR> &e = el[q];
+                const bool tri = e.nv == 3;
+                // distances and quadrature orders of the lane's points
+                R D[3];
+                float q2[P];
+                if constexpr (P == 2) {
 #pragma unroll
-                for (int kk = 0; kk < 3; ++kk) {
-                    const cplx<float> gg = ph * cplx<float>{fmaf(Tn.x, e.n[kk], U[kk].x), fmaf(Tn.y, e.n[kk], U[kk].y)};
-                    acc.g[kk].re += gg.re;
-                    acc.g[kk].im += gg.im;
-                }
-            } else if (!near) {
-                const int np = e.nv == 3 ? tri_count(order) : quad_count(order);
-                for (int gq = 0; gq < np; ++gq) {
-                    float s, t, wq;
-                    if (e.nv == 3) {
-                        const int o = tri_offset(order) + gq;
-                        s = c_trif[o][0]; t = c_trif[o][1]; wq = c_trif[o][2];
-                    } else {
-                        const int a = gq / order, b = gq - a * order;
-                        s = c_glxf[order][a]; t = c_glxf[order][b];
-                        wq = c_glwf[order][a] * c_glwf[order][b];
-                    }
-                    QPoint<float> q;
-                    map_point(e, s, t, wq, q);
-                    proj_point(q, ph, vl, e.nv, iv, k, wr, acc);
-                }
-            }
-            // near pairs: the whole warp subdivides for one lane's point at a time
-            unsigned todo = __ballot_sync(0xffffffffu, pv && near);
-            if (todo) {
-                Elem64 e64;
-                load_elem64(mk, j, e64);
-                cplx<float> phn, vln[4];
-                proj_elem_data<float>(phi, vel, phi32, vel32, n, j, nv, true, kref, neg, phn, vln);
-                while (todo) {
-                    const int L = __ffs(todo) - 1;
-                    todo &= todo - 1;
-                    double xl[3];
-                    float lh[3], ll[3];
+                    for (int c = 0; c < 3; ++c) D[c] = vadd(vsub(e.v[c], X[c]), vsub(e.v[3 + c], X[3 + c]));
+                    const F2 d2 = vfma(D[2], D[2], vfma(D[0], D[0], vmul(D[1], D[1])));
+                    unpk2(vmul(d2, pk2(e.isq2, e.isq2)), q2[0], q2[P - 1]);
+                } else {
+                    float d[3];
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        xl[c] = S.pts[3 * (g * 32 + L) + c];   // lane L's point, a uniform load
-                        lh[c] = __shfl_sync(0xffffffffu, xhi[c], L);
-                        ll[c] = __shfl_sync(0xffffffffu, xlo[c], L);
+                        D[c] = tri ? e.v[c] - X[c] : -X[c];
+                        d[c] = (e.hi[c] - xh[0][c]) + (e.lo[c] - xl[0][c]);
                     }
-                    Elem32 e32;
-                    load_elem32(mk, j, lh, ll, e32);
-                    ProjSink<float> sink;
-                    sink.e = &e32; sink.phi = phn; sink.vel = vln; sink.ivi = iv; sink.k = k; sink.wr = wr;
-                    sink.init();
-                    const int rc = warp_subdivide(e64, m.area64[j], xl, ws, sink, &e32, isq);
-                    if (rc != kDevOk) err = rc;
-                    const ProjAcc<float> r = sink.reduce();
-                    if (lane == L) {
-                        acc.p += r.p;
-                        for (int kk = 0; kk < 3; ++kk) acc.g[kk] += r.g[kk];
-                    }
+                    q2[0] = (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]) * e.isq2;
                 }
-            }
-        }
-    }
-    float4 *out = S.part + 2 * ((size_t)(sl * G + g) * 32 + lane);
-    out[0] = make_float4(acc.p.re, acc.p.im, acc.g[0].re, acc.g[0].im);
-    out[1] = make_float4(acc.g[1].re, acc.g[1].im, acc.g[2].re, acc.g[2].im);
-    if (err != kDevOk && lane == 0) atomicMax(S.status, err);
-}
-
-// Several right-hand sides of one matrix (bem_solve_multi): systems
-// 0 .. nr-1 of the batch share the mesh, the points and the slicing and
-// differ in their element data.  The pass over (32-point group, element
-// slice) items is the one of k_project_pts, but a far flat triangle whose
-// elements carry no velocity term in any right-hand side is evaluated once
-// (P, U, T of proj_tri_points, independent of phi) and applied to every
-// right-hand side's phi: the kernel evaluations, which dominate, are shared,
-// and each right-hand side adds 4 complex multiply-adds per element.  Other
-// pairs (velocity terms, quadrilaterals, subdivided near pairs) are evaluated
-// per right-hand side as in k_project_pts.  Each right-hand side's partial
-// sums go to its own scratch; k_project_sum finishes them.
-// acc[r] += a with every index known at compile time (a runtime index
-// would put the accumulators in local memory)
-template <int RMAX>
-__device__ __forceinline__ void acc_add(ProjAcc<float> (&acc)[RMAX], int r, const ProjAcc<float> &a) {
+                unsigned far = 0;
+                int ord[P];   // 0: subdivided
 #pragma unroll
-    for (int q = 0; q < RMAX; ++q)
-        if (q == r) {
-            acc[q].p += a.p;
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk) acc[q].g[kk] += a.g[kk];
-        }
-}
-
-template <int RMAX>
-__global__ void __launch_bounds__(256, RMAX <= 4 ? 2 : 1) k_project_pts_multi(const __grid_constant__ ProjBatch tb, int nr) {
-    __shared__ WarpScratch ws_all[8];
-    const ProjSys &S = tb.sys[0];
-    const DevMesh m = to_dev(S.m);
-    const DevFreq &f = S.f;
-    const int lane = threadIdx.x, w = threadIdx.y, n = m.n, npts = S.npts;
-    const int G = (npts + 31) >> 5, nsl = S.nslice;
-    const int item = blockIdx.x * 8 + w;
-    if (item >= G * nsl) return;
-    const int g = item % G, sl = item / G;
-    const int per = (n + nsl - 1) / nsl;
-    const int j0 = sl * per, j1 = min(n, j0 + per);
-    const int p = g * 32 + lane;
-    const bool pv = p < npts;
-    const int pp = pv ? p : g * 32;
-    WarpScratch &ws = ws_all[w];
-    float xhi[3], xlo[3];
-    for (int c = 0; c < 3; ++c) {
-        const double xv = S.pts[3 * pp + c];
-        xhi[c] = (float)xv;
-        xlo[c] = (float)(xv - (double)xhi[c]);
-        asm volatile("" : "+f"(xhi[c]), "+f"(xlo[c]));
-    }
-    ProjAcc<float> acc[RMAX];
-#pragma unroll
-    for (int r = 0; r < RMAX; ++r) acc[r].p = acc[r].g[0] = acc[r].g[1] = acc[r].g[2] = cmk(0.f, 0.f);
-    float k = (float)f.k, wr = (float)f.wr;
-    asm volatile("" : "+f"(k), "+f"(wr));
-    const float k2 = k * k;
-    int err = kDevOk;
-    for (int kref = 0; kref < m.sym.nref; ++kref) {
-        const DevMesh mk = image_mesh(m, kref);
-        const bool neg = image_negated(m, kref);
-        for (int j = j0; j < j1; ++j) {
-            bool iv_any = false;
-#pragma unroll
-            for (int r = 0; r < RMAX; ++r)
-                if (r < nr && tb.sys[r].ivi[j] != 0) iv_any = true;
-            const int nv = m.nvert[j];
-            Elem32 e;
-            load_elem32(mk, j, xhi, xlo, e);
-            const float isq = m.isqa32[j];
-            const float q2 = (e.D[0] * e.D[0] + e.D[1] * e.D[1] + e.D[2] * e.D[2]) * (isq * isq);
-            bool near = false;
-            int order = 2;
-            if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
-                const double xp[3] = {S.pts[3 * pp], S.pts[3 * pp + 1], S.pts[3 * pp + 2]};
-                const double rd = ratio0_exact(mk, j, xp);
-                near = rd < kTolf;
-                if (!near) order = gauss_order(rd);
-            }
-            if (!near && e.nv == 3 && !iv_any) {
-                float2 P = make_float2(0.f, 0.f), U[3], Tn = make_float2(0.f, 0.f);
-                U[0] = U[1] = U[2] = make_float2(0.f, 0.f);
-                const float dny = e.D[0] * e.n[0] + e.D[1] * e.n[1] + e.D[2] * e.n[2];
-                if (order <= 2) proj_tri_points<4, 0>(e, dny, k2, wr, P, U, Tn);
-                else if (order == 3) proj_tri_points<7, 4>(e, dny, k2, wr, P, U, Tn);
-                else proj_tri_points<13, 11>(e, dny, k2, wr, P, U, Tn);
-                cplx<float> gk[3];
-#pragma unroll
-                for (int kk = 0; kk < 3; ++kk) gk[kk] = cplx<float>{fmaf(Tn.x, e.n[kk], U[kk].x), fmaf(Tn.y, e.n[kk], U[kk].y)};
-#pragma unroll
-                for (int r = 0; r < RMAX; ++r) {
-                    if (r >= nr) break;
-                    const float2 p2 = ((const float2 *)tb.sys[r].phi32)[j];
-                    const cplx<float> ph = neg ? cplx<float>{-p2.x, -p2.y} : cplx<float>{p2.x, p2.y};
-                    const cplx<float> pq = ph * cplx<float>{P.x, P.y};
-                    acc[r].p.re += pq.re;
-                    acc[r].p.im += pq.im;
-#pragma unroll
-                    for (int kk = 0; kk < 3; ++kk) {
-                        const cplx<float> gg = ph * gk[kk];
-                        acc[r].g[kk].re += gg.re;
-                        acc[r].g[kk].im += gg.im;
-                    }
-                }
-            } else if (!near) {
-                const int np = e.nv == 3 ? tri_count(order) : quad_count(order);
-#pragma unroll 1
-                for (int r = 0; r < RMAX; ++r) {
-                    if (r >= nr) break;
-                    const ProjSys &Sr = tb.sys[r];
-                    const bool iv = Sr.ivi[j] != 0;
-                    cplx<float> ph, vl[4];
-                    proj_elem_data<float>((const double2 *)Sr.phi, (const double2 *)Sr.vel, (const float2 *)Sr.phi32,
-                                          (const float2 *)Sr.vel32, n, j, nv, iv, kref, neg, ph, vl);
-                    ProjAcc<float> tmp;
-                    tmp.p = tmp.g[0] = tmp.g[1] = tmp.g[2] = cmk(0.f, 0.f);
-                    for (int gq = 0; gq < np; ++gq) {
-                        float s, t, wq;
-                        if (e.nv == 3) {
-                            const int o = tri_offset(order) + gq;
-                            s = c_trif[o][0]; t = c_trif[o][1]; wq = c_trif[o][2];
-                        } else {
-                            const int a = gq / order, b = gq - a * order;
-                            s = c_glxf[order][a]; t = c_glxf[order][b];
-                            wq = c_glwf[order][a] * c_glwf[order][b];
+                for (int h = 0; h < P; ++h) {
+                    bool near = false;
+                    ord[h] = 2;
+                    if (q2[h] <= c_quad.far2_sq) {
+                        if (!classify_fast(sqrtf(q2[h]), near, ord[h])) {
+                            const int p = p0 + 32 * h < npts ? p0 + 32 * h : p0 - lane;
+                            const double xp[3] = {S.pts[3 * p], S.pts[3 * p + 1], S.pts[3 * p + 2]};
+                            const double rd = ratio0_exact(mk, base + q, xp);
+                            near = rd < kTolf;
+                            if (!near) ord[h] = gauss_order(rd);
                         }
-                        QPoint<float> q;
-                        map_point(e, s, t, wq, q);
-                        proj_point(q, ph, vl, e.nv, iv, k, wr, tmp);
+                        if (near) ord[h] = 0;
                     }
-                    acc_add<RMAX>(acc, r, tmp);
+                    if (ord[h] == 2) far |= 1u << h;
                 }
-            }
-            // near pairs: the whole warp subdivides for one lane's point at a
-            // time, once per right-hand side
-            unsigned todo = __ballot_sync(0xffffffffu, pv && near);
-            if (todo) {
-                Elem64 e64;
-                load_elem64(mk, j, e64);
-                while (todo) {
-                    const int L = __ffs(todo) - 1;
-                    todo &= todo - 1;
-                    double xl[3];
-                    float lh[3], ll[3];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        xl[c] = S.pts[3 * (g * 32 + L) + c];
-                        lh[c] = __shfl_sync(0xffffffffu, xhi[c], L);
-                        ll[c] = __shfl_sync(0xffffffffu, xlo[c], L);
+                if (__any_sync(0xffffffffu, far != 0)) {
+                    if (tri) {
+                        if (!e.iv) proj_far<T, NR, true, false>(e, nr, D, far, wr, nwr, k2, m3, acc);
+                        else proj_far<T, NR, true, true>(e, nr, D, far, wr, nwr, k2, m3, acc);
+                    } else {
+                        if (!e.iv) proj_far<T, NR, false, false>(e, nr, D, far, wr, nwr, k2, m3, acc);
+                        else proj_far<T, NR, false, true>(e, nr, D, far, wr, nwr, k2, m3, acc);
                     }
-                    Elem32 e32;
-                    load_elem32(mk, j, lh, ll, e32);
+                }
+                if (__all_sync(0xffffffffu, far == (1u << P) - 1u)) continue;
+#pragma unroll
+                for (int h = 0; h < P; ++h) {
+                    const bool pv = p0 + 32 * h < npts;
+                    if (pv && ord[h] > 2)
 #pragma unroll 1
-                    for (int r = 0; r < RMAX; ++r) {
-                        if (r >= nr) break;
-                        const ProjSys &Sr = tb.sys[r];
-                        const bool iv = Sr.ivi[j] != 0;
-                        cplx<float> phn, vln[4];
-                        proj_elem_data<float>((const double2 *)Sr.phi, (const double2 *)Sr.vel,
-                                              (const float2 *)Sr.phi32, (const float2 *)Sr.vel32, n, j, nv, true, kref,
-                                              neg, phn, vln);
-                        ProjSink<float> sink;
-                        sink.e = &e32; sink.phi = phn; sink.vel = vln; sink.ivi = iv; sink.k = k; sink.wr = wr;
-                        sink.init();
-                        const int rc = warp_subdivide(e64, m.area64[j], xl, ws, sink, &e32, isq);
-                        if (rc != kDevOk) err = rc;
-                        const ProjAcc<float> rs = sink.reduce();
-                        if (lane == L) acc_add<RMAX>(acc, r, rs);
+                        for (int r = 0; r < nr; ++r)
+                            racc_at<T, NR>(acc, r, h, proj_whole<T>(&tb.sys[sb + r], kref, base + q, ord[h], p0 + 32 * h));
+                    unsigned todo = __ballot_sync(0xffffffffu, pv && ord[h] == 0);
+                    while (todo) {
+                        const int L = __ffs(todo) - 1;
+                        todo &= todo - 1;
+#pragma unroll 1
+                        for (int r = 0; r < nr; ++r) {
+                            const ProjAcc<T> z = proj_near<T>(&tb.sys[sb + r], kref, base + q, p0 - lane + 32 * h + L,
+                                                              &ws_all[w], &err);
+                            if (lane == L) racc_at<T, NR>(acc, r, h, z);
+                        }
                     }
                 }
             }
         }
     }
-#pragma unroll
-    for (int r = 0; r < RMAX; ++r) {
-        if (r >= nr) break;
-        float4 *out = tb.sys[r].part + 2 * ((size_t)(sl * G + g) * 32 + lane);
-        out[0] = make_float4(acc[r].p.re, acc[r].p.im, acc[r].g[0].re, acc[r].g[0].im);
-        out[1] = make_float4(acc[r].g[1].re, acc[r].g[1].im, acc[r].g[2].re, acc[r].g[2].im);
-    }
     if (err != kDevOk && lane == 0) atomicMax(S.status, err);
+    // the element parts of a point group meet in shared memory, in order
+    R *red = reinterpret_cast<R *>(ws_all);   // [warp][8][lane]
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        if (r >= nr) break;
+        RAcc<R> &a = acc[r];
+        if (ewb > 1) {
+            __syncthreads();
+            if (ew > 0) {
+                R *o = red + (size_t)w * 8 * 32 + lane;
+                o[0] = a.pr;
+                o[32] = a.pi;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) { o[(2 + 2 * c) * 32] = a.gr[c]; o[(3 + 2 * c) * 32] = a.gi[c]; }
+            }
+            __syncthreads();
+            for (int q = 1; q < ewb && ew == 0; ++q) {
+                const R *o = red + (size_t)(w + q * pgb) * 8 * 32 + lane;
+                a.pr = vadd(a.pr, o[0]);
+                a.pi = vadd(a.pi, o[32]);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    a.gr[c] = vadd(a.gr[c], o[(2 + 2 * c) * 32]);
+                    a.gi[c] = vadd(a.gi[c], o[(3 + 2 * c) * 32]);
+                }
+            }
+        }
+        if (ew > 0 || !group) continue;
+        float4 *part = tb.sys[sb + r].part;
+        if constexpr (P == 2) {
+            float v[2][8];
+            unpk2(a.pr, v[0][0], v[1][0]);
+            unpk2(a.pi, v[0][1], v[1][1]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                unpk2(a.gr[c], v[0][2 + 2 * c], v[1][2 + 2 * c]);
+                unpk2(a.gi[c], v[0][3 + 2 * c], v[1][3 + 2 * c]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 *out = part + 2 * ((size_t)sl * S.pstride + p0 + 32 * h);
+                out[0] = make_float4(v[h][0], v[h][1], v[h][2], v[h][3]);
+                out[1] = make_float4(v[h][4], v[h][5], v[h][6], v[h][7]);
+            }
+        } else {
+            double2 *out = reinterpret_cast<double2 *>(part) + 4 * ((size_t)sl * S.pstride + p0);
+            out[0] = make_double2(a.pr, a.pi);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) out[1 + c] = make_double2(a.gr[c], a.gi[c]);
+        }
+    }
 }
 
-// Thread per point: the slices' partial sums in slice order (FP64), then the
-// point's tau factor and incident field.
+// Sums of the slices (FP64) and the finish of a point (tau factor, incident
+// field).  A block of 256 threads takes PT points, 256 / PT threads each adding
+// every (256 / PT)th slice; the threads' sums are added in order by the thread
+// that finishes the point.  The additions and conversions run on an SM's
+// narrow FP64 pipe, so few points (up to kSumSpread) go 4 to a block to reach
+// more SMs: 64 points x 320 slices on 2 SMs took 56 us, on 16 they take 15.
+constexpr int kSumSpread = 2432;   // 4 points per block: up to 4 blocks per SM
+__host__ __device__ inline int sum_points(int npts) { return npts <= kSumSpread ? 4 : 32; }
+
+template <typename T>
 __global__ void __launch_bounds__(256) k_project_sum(const __grid_constant__ ProjBatch tb) {
+    __shared__ double red[256][8];   // [slice thread][point][component]
     const int sb = find_sys(tb.ps_off, tb.B, blockIdx.x);
     const ProjSys &S = tb.sys[sb];
-    const int p = (blockIdx.x - tb.ps_off[sb]) * 256 + threadIdx.x;
-    if (p >= S.npts) return;
-    const DevMesh m = to_dev(S.m);
-    const int G = (S.npts + 31) >> 5;
-    cplx<double> sp = {0.0, 0.0}, sg[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    for (int sl = 0; sl < S.nslice; ++sl) {
-        const float4 *in = S.part + 2 * ((size_t)sl * G * 32 + p);
-        const float4 a = in[0], b = in[1];
-        sp += cplx<double>{(double)a.x, (double)a.y};
-        sg[0] += cplx<double>{(double)a.z, (double)a.w};
-        sg[1] += cplx<double>{(double)b.x, (double)b.y};
-        sg[2] += cplx<double>{(double)b.z, (double)b.w};
+    const int PT = sum_points(S.npts), per = 256 / PT;
+    const int pi = threadIdx.x % PT, w = threadIdx.x / PT;
+    const int p = (blockIdx.x - tb.ps_off[sb]) * PT + pi;
+    double a[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) a[q] = 0.0;
+    if (p < S.npts) {
+#pragma unroll 4
+        for (int sl = w; sl < S.nslice; sl += per) {
+            if constexpr (std::is_same<T, float>::value) {
+                const float4 *in = S.part + 2 * ((size_t)sl * S.pstride + p);
+                const float4 u = in[0], v = in[1];
+                a[0] += (double)u.x; a[1] += (double)u.y; a[2] += (double)u.z; a[3] += (double)u.w;
+                a[4] += (double)v.x; a[5] += (double)v.y; a[6] += (double)v.z; a[7] += (double)v.w;
+            } else {
+                const double2 *in = reinterpret_cast<const double2 *>(S.part) + 4 * ((size_t)sl * S.pstride + p);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double2 u = in[q];
+                    a[2 * q] += u.x;
+                    a[2 * q + 1] += u.y;
+                }
+            }
+        }
     }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) red[threadIdx.x][q] = a[q];
+    __syncthreads();
+    // 8 PT threads: component c of point e
+    if (threadIdx.x < 8 * PT) {
+        const int e = threadIdx.x >> 3, c = threadIdx.x & 7, top = min(per, S.nslice);
+        double t = red[e][c];
+        for (int u = 1; u < top; ++u) t += red[u * PT + e][c];
+        red[e][c] = t;
+    }
+    __syncthreads();
+    if (w != 0 || p >= S.npts) return;
+    const double *t = red[pi];
+    cplx<double> sg[3] = {{t[2], t[3]}, {t[4], t[5]}, {t[6], t[7]}};
+    const DevMesh m = to_dev(S.m);
     const double x64[3] = {S.pts[3 * p], S.pts[3 * p + 1], S.pts[3 * p + 2]};
-    project_finish(m, S.f, x64, p, sp, sg, (double2 *)S.pot, (double2 *)S.grad);
+    project_finish(m, S.f, x64, p, {t[0], t[1]}, sg, (double2 *)S.pot, (double2 *)S.grad);
 }
 
 // ---------------------------------------------------------------- tables
@@ -1857,6 +2128,13 @@ cudaError_t init_device_tables() {
         far4[g][3] = 2.0f * far4[g][1];
     }
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far4, far4, sizeof(far4));
+    float2 far4d[4][3];
+    for (int g = 0; g < 4; ++g) {
+        far4d[g][0] = make_float2(far4[g][0], far4[g][0]);
+        far4d[g][1] = make_float2(far4[g][1], far4[g][1]);
+        far4d[g][2] = make_float2(trif[g][2], trif[g][2]);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far4d, far4d, sizeof(far4d));
     double far64[24][4];
     for (int g = 0; g < 24; ++g) {
         far64[g][0] = kTri[g][0] - 1.0 / 3.0;
@@ -1918,19 +2196,38 @@ void asm_batch_finish(AsmBatch &t) {
     }
 }
 
-void proj_batch_finish(ProjBatch &t) {
+// Work split of the projection, from the system's own sizes only (a system's
+// result does not depend on the rest of its batch).  Point groups per block:
+// the most, up to 8, that pad the groups by less than a fourteenth (a wide
+// block stages its elements for more points; 28 groups of 1730 points go in
+// fours).  Slices: of at most kProjSlice elements (the length of an FP32 sum),
+// more where that leaves SMs idle, down to kProjStep elements; the number of
+// blocks is then rounded down to whole rounds of the resident ones (2 per SM
+// of 152; 26 slices of 24 blocks ran a third round for 16 of them: 11950 points
+// on 20480 elements 2.43 ms, with whole rounds 2.15), and the scratch may hold fewer.
+void proj_batch_finish(ProjBatch &t, int prec) {
     t.fld_off[0] = t.pt_off[0] = t.lp_off[0] = t.ps_off[0] = 0;
+    const int gpts = 32 * (prec == 0 ? ProjLane<double>::kP : ProjLane<float>::kP);
+    const int part = prec == 0 ? ProjLane<double>::kPart : ProjLane<float>::kPart;
     for (int b = 0; b < t.B; ++b) {
         ProjSys &S = t.sys[b];
         t.fld_off[b + 1] = t.fld_off[b] + (S.m.n + 255) / 256;
         t.pt_off[b + 1] = t.pt_off[b] + (S.npts + 7) / 8;
-        // element slices of the float projection, as many as the scratch holds
-        const long long G = (S.npts + 31) / 32;
-        const long long want = (S.m.n + kProjSlice - 1) / kProjSlice;
-        const long long fit = G > 0 ? S.part_cap / (2 * 32 * G) : 0;
-        S.nslice = S.part ? (int)std::min(want, fit) : 0;
-        t.lp_off[b + 1] = t.lp_off[b] + (int)((G * S.nslice + 7) / 8);
-        t.ps_off[b + 1] = t.ps_off[b] + (S.npts + 255) / 256;
+        const int G = ceil_div(S.npts, gpts);
+        S.pgb = 8;
+        while (S.pgb > 1 && 14 * (ceil_div(G, S.pgb) * S.pgb - G) >= G) S.pgb /= 2;
+        const int GB = G > 0 ? ceil_div(G, S.pgb) : 1;
+        S.pstride = G * gpts;
+        const long long fit = G > 0 && S.part ? S.part_cap / ((long long)part * S.pstride) : 0;
+        const long long least = ceil_div(S.m.n, kProjSlice), most = ceil_div(S.m.n, kProjStep);
+        long long nsl = std::max(least, std::min<long long>(most, ceil_div(4 * kProjSlots, GB)));
+        nsl = std::min(nsl, fit);
+        const long long rounds = nsl * GB / kProjSlots;
+        if (rounds > 0 && rounds <= 4) nsl = std::max(std::min(least, fit), rounds * kProjSlots / GB);
+        S.per = nsl > 0 ? ceil_div(S.m.n, nsl) : 0;
+        S.nslice = nsl > 0 ? ceil_div(S.m.n, S.per) : 0;
+        t.lp_off[b + 1] = t.lp_off[b] + (G > 0 ? GB * S.nslice : 0);
+        t.ps_off[b + 1] = t.ps_off[b] + ceil_div(S.npts, sum_points(S.npts));
     }
 }
 
@@ -2019,41 +2316,43 @@ cudaError_t launch_fields(const ProjBatch &t, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+namespace {
+// lanes = points (NR right-hand sides at a time), then the slice sums
+template <typename T, int NR>
+void project_sliced(const ProjBatch &t, cudaStream_t st) {
+    k_project_pts<T, NR><<<NR > 1 ? t.lp_off[1] : t.lp_off[t.B], dim3(32, 8), 0, st>>>(t, t.B);
+    k_project_sum<T><<<t.ps_off[t.B], 256, 0, st>>>(t);
+    count_launches(2);
+}
+}  // namespace
+
 cudaError_t launch_project_multi(const ProjBatch &t, cudaStream_t st) {
-    // the right-hand sides of one solver: same mesh, points and slicing
+    // the right-hand sides of one solver: same mesh, points and split
     bool shared = t.B >= 2 && t.B <= 8 && t.sys[0].nslice > 0;
     for (int b = 1; b < t.B && shared; ++b)
         shared = t.sys[b].npts == t.sys[0].npts && t.sys[b].pts == t.sys[0].pts &&
-                 t.sys[b].nslice == t.sys[0].nslice && t.sys[b].m.n == t.sys[0].m.n;
+                 t.sys[b].nslice == t.sys[0].nslice && t.sys[b].per == t.sys[0].per && t.sys[b].m.n == t.sys[0].m.n;
     if (!shared) return launch_project(t, 1, st);
     if (t.sys[0].npts == 0) return cudaSuccess;
-    dim3 block(32, 8);
-    const int items = ((t.sys[0].npts + 31) / 32) * t.sys[0].nslice;
-    const int grid = (items + 7) / 8;
-    count_launches(2);
-    if (t.B <= 2) k_project_pts_multi<2><<<grid, block, 0, st>>>(t, t.B);
-    else if (t.B <= 4) k_project_pts_multi<4><<<grid, block, 0, st>>>(t, t.B);
-    else k_project_pts_multi<8><<<grid, block, 0, st>>>(t, t.B);
-    k_project_sum<<<t.ps_off[t.B], 256, 0, st>>>(t);
+    if (t.B <= 2) project_sliced<float, 2>(t, st);
+    else if (t.B <= 4) project_sliced<float, 4>(t, st);
+    else project_sliced<float, 8>(t, st);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project(const ProjBatch &t, int prec, cudaStream_t st) {
     if (t.B <= 0 || t.pt_off[t.B] == 0) return cudaSuccess;
-    dim3 block(32, 8);
-    bool sliced = prec != 0;
+    bool sliced = true;
     for (int b = 0; b < t.B; ++b)
         if (t.sys[b].npts > 0 && t.sys[b].nslice == 0) sliced = false;   // scratch too short
-    if (prec == 0) {
+    if (!sliced) {
         count_launches(1);
-        k_project<double><<<t.pt_off[t.B], block, 0, st>>>(t);
-    } else if (!sliced) {
-        count_launches(1);
-        k_project<float><<<t.pt_off[t.B], block, 0, st>>>(t);
+        if (prec == 0) k_project<double><<<t.pt_off[t.B], dim3(32, 8), 0, st>>>(t);
+        else k_project<float><<<t.pt_off[t.B], dim3(32, 8), 0, st>>>(t);
+    } else if (prec == 0) {
+        project_sliced<double, 1>(t, st);
     } else {
-        count_launches(2);
-        k_project_pts<<<t.lp_off[t.B], block, 0, st>>>(t);
-        k_project_sum<<<t.ps_off[t.B], 256, 0, st>>>(t);
+        project_sliced<float, 1>(t, st);
     }
     return cudaGetLastError();
 }

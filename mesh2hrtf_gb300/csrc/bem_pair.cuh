@@ -108,12 +108,13 @@ __device__ __forceinline__ void proj_point(const QPoint<T> &q, cplx<T> phi, cons
 #pragma unroll
     for (int kk = 0; kk < 3; ++kk) a.g[kk] += (zfac1 * dh[kk] + zfac2 * q.ny[kk]) * z1;
     if (ivi) {
-        for (int v = 0; v < nv; ++v) {
-            cplx<T> zz = vel[v] * (q.wj * q.sh[v]);
-            a.p -= zgr * zz;
+        // the nodal velocities interpolated to the point first
+        cplx<T> zz = {T(0), T(0)};
+        for (int v = 0; v < nv; ++v) zz += vel[v] * (q.wj * q.sh[v]);
+        a.p -= zgr * zz;
+        const cplx<T> zi = zgikr * zz;
 #pragma unroll
-            for (int kk = 0; kk < 3; ++kk) a.g[kk] -= (zgikr * (-dh[kk])) * zz;
-        }
+        for (int kk = 0; kk < 3; ++kk) a.g[kk] += zi * dh[kk];
     }
 }
 

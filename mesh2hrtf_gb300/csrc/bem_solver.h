@@ -229,8 +229,10 @@ struct bem_solver_s {
         q.pot = pot_dev;
         q.grad = grad_dev;
         q.status = d.status;
+        // the basis and the Krylov vectors behind it, idle once the system is
+        // solved (solver_layout places V ... hsum before phi)
         q.part = reinterpret_cast<float4 *>(d.V);
-        q.part_cap = (long long)((size_t)(restart + 1) * (size_t)n * (prec == BEM_PREC_FP64 ? 16 : 8) / 16);
+        q.part_cap = (long long)((reinterpret_cast<const char *>(d.phi) - reinterpret_cast<const char *>(d.V)) / 16);
         return q;
     }
 };

@@ -21,9 +21,9 @@ namespace {
 constexpr int kStaticMaxElem = BEM_STATIC_MAX_ELEMENTS;
 // per element: phi (16 B) + 4 nodal velocities (64 B) + their float copies
 // (8 + 32 B) + flag (4 B); then the error word (256 B); then the partial
-// sums of the float projection.  With fewer partial-sum slots than a call
-// needs, the projection takes wider element slices, and below one slice per
-// 32-point group it runs one warp per point (same quadrature, FP32 sums).
+// sums of the projection.  With fewer partial-sum slots than a call
+// needs, the projection takes wider element slices, and without room for one
+// slice it runs one warp per point (same quadrature and sum precision).
 constexpr size_t kElemBytes = (size_t)kStaticMaxElem * (16 + 64 + 8 + 32 + 4);
 constexpr size_t kPartBytes = (size_t)8 << 20;
 constexpr size_t kScratchBytes = kElemBytes + 256 + kPartBytes;
@@ -100,7 +100,7 @@ extern "C" bem_status bem_project_static(bem_solver_t solver, int32_t n_pts, con
     S.pot = pot_dev;
     S.grad = grad_dev;
     t.B = 1;
-    bem::proj_batch_finish(t);
+    bem::proj_batch_finish(t, prec);
     cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), st);
     if (e == cudaSuccess) e = bem::launch_fields(t, st);
     if (e == cudaSuccess && n_pts > 0) e = bem::launch_project(t, prec, st);
