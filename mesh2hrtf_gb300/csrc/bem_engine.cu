@@ -71,6 +71,9 @@ Engine::~Engine() {
         if (x) cudaGraphExecDestroy(x);
     for (auto &e : ev_)
         if (e) cudaEventDestroy(e);
+    if (side_.fork) cudaEventDestroy(side_.fork);
+    if (side_.join) cudaEventDestroy(side_.join);
+    if (side_.st) cudaStreamDestroy(side_.st);
     cudaFree(d_tab_);
     cudaFree(d_st_);
     cudaFree(d_items_);
@@ -87,6 +90,9 @@ cudaError_t Engine::ensure_init() {
     if (e == cudaSuccess) e = cudaMallocHost(&h_st_, sizeof(KState) * kMaxSys);
     for (auto &ev : ev_)
         if (e == cudaSuccess) e = cudaEventCreate(&ev);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side_.st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&side_.fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&side_.join, cudaEventDisableTiming);
     if (e == cudaSuccess) {
         std::memset(h_tab_, 0, sizeof(KTable));
         std::memset(h_st_, 0, sizeof(KState) * kMaxSys);
@@ -227,7 +233,7 @@ cudaError_t Engine::run_body() {
         e = cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
         cudaError_t le = launch_krylov_body(prec_, d_tab_, ev_, st_, &body_launches_[v], (v & 1) != 0,
-                                                   (v & 2) != 0, (v & 4) != 0);
+                                                   (v & 2) != 0, (v & 4) != 0, side_);
         e = cudaStreamEndCapture(st_, &g);
         if (le != cudaSuccess) e = le;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_[v], g, 0);

@@ -63,6 +63,7 @@ private:
     int blr_ = 0;      // systems of the current batch with a block low-rank copy
     int dense_ = 0;    // single systems whose Krylov products read A or its fp16 copy
     cudaEvent_t ev_[2 * (kSteps + 1)] = {};
+    SideStream side_{};   // the captured body's second branch
     double mv_ms_ = 0.0;
     long long bodies_ = 0;
     bool timing_ok_ = true;

@@ -55,6 +55,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "bem_engine.h"
 #include "bem_internal.h"
@@ -1734,8 +1735,10 @@ __global__ void __launch_bounds__(kBlrThreads, 4 * kBlrRowsPerThread) k_mv_blr(K
 
 // ------------------------------------------------------------ block helpers
 // dp[l * nvb + blk] = sum over the block's rows of conj(V_l[row]) w[row], l < nv.
+// The warps' sums of all vectors wait in shared memory for one pair of
+// barriers, so the loads of the next eight vectors overlap the sums.
 __device__ void block_dots(const double2 *__restrict__ V, long long ldv, int nv, double2 wv, bool ok, int row,
-                           double2 *__restrict__ dp, int nvb, int blk, double (*red)[16]) {
+                           double2 *__restrict__ dp, int nvb, int blk, double (*red)[2 * kMaxV]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int l0 = 0; l0 < nv; l0 += 8) {
 #pragma unroll
@@ -1748,25 +1751,24 @@ __device__ void block_dots(const double2 *__restrict__ V, long long ldv, int nv,
             }
             re = warp_sum_d(re);
             im = warp_sum_d(im);
-            if (lane == 0) {
-                red[warp][2 * q] = re;
-                red[warp][2 * q + 1] = im;
+            if (lane == 0 && l0 + q < nv) {
+                red[warp][2 * (l0 + q)] = re;
+                red[warp][2 * (l0 + q) + 1] = im;
             }
         }
-        __syncthreads();
-        if (threadIdx.x < 16) {
-            double t = 0.0;
-#pragma unroll
-            for (int w8 = 0; w8 < 8; ++w8) t += red[w8][threadIdx.x];
-            const int q = threadIdx.x >> 1;
-            if (l0 + q < nv) reinterpret_cast<double *>(dp + (size_t)(l0 + q) * nvb + blk)[threadIdx.x & 1] = t;
-        }
-        __syncthreads();
     }
+    __syncthreads();
+    if (threadIdx.x < 2 * nv) {
+        double t = 0.0;
+#pragma unroll
+        for (int w8 = 0; w8 < 8; ++w8) t += red[w8][threadIdx.x];
+        reinterpret_cast<double *>(dp + (size_t)(threadIdx.x >> 1) * nvb + blk)[threadIdx.x & 1] = t;
+    }
+    __syncthreads();
 }
 
 // nrmp[blk] = sum over the block's rows of |w|^2
-__device__ void block_norm(double2 wv, bool ok, double *__restrict__ nrmp, int blk, double (*red)[16]) {
+__device__ void block_norm(double2 wv, bool ok, double *__restrict__ nrmp, int blk, double (*red)[2 * kMaxV]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double t = ok ? fma(wv.x, wv.x, wv.y * wv.y) : 0.0;
     t = warp_sum_d(t);
@@ -1781,19 +1783,19 @@ __device__ void block_norm(double2 wv, bool ok, double *__restrict__ nrmp, int b
     __syncthreads();
 }
 
-// sum of the squared-norm partials, in block order
-__device__ __forceinline__ double norm_total(const double *__restrict__ nrmp, int nvb) {
+// sum of the squared-norm partials by a warp (the same value on every lane);
+// a thread adding them one by one took 0.2 us each on the FP64 pipe's latency
+__device__ __forceinline__ double warp_norm_total(const double *__restrict__ nrmp, int nvb, int lane) {
     double t = 0.0;
-#pragma unroll 8
-    for (int c = 0; c < nvb; ++c) t += nrmp[c];
-    return t;
+    for (int c = lane; c < nvb; c += 32) t += nrmp[c];
+    return warp_sum_d(t);
 }
 
 // The same for the float Krylov basis of complex64 systems: FP32 products
 // and sums (GB300's FP64 pipe would bound these loops), one float2 inner-
 // product partial per block and vector, the norm partial converted once.
 __device__ void block_dots_f(const float2 *__restrict__ V, long long ldv, int nv, float2 wv, bool ok, int row,
-                             float2 *__restrict__ dp, int nvb, int blk, float (*red)[16]) {
+                             float2 *__restrict__ dp, int nvb, int blk, float (*red)[2 * kMaxV]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int l0 = 0; l0 < nv; l0 += 8) {
 #pragma unroll
@@ -1806,24 +1808,23 @@ __device__ void block_dots_f(const float2 *__restrict__ V, long long ldv, int nv
             }
             re = warp_sum_f(re);
             im = warp_sum_f(im);
-            if (lane == 0) {
-                red[warp][2 * q] = re;
-                red[warp][2 * q + 1] = im;
+            if (lane == 0 && l0 + q < nv) {
+                red[warp][2 * (l0 + q)] = re;
+                red[warp][2 * (l0 + q) + 1] = im;
             }
         }
-        __syncthreads();
-        if (threadIdx.x < 16) {
-            float t = 0.f;
-#pragma unroll
-            for (int w8 = 0; w8 < 8; ++w8) t += red[w8][threadIdx.x];
-            const int q = threadIdx.x >> 1;
-            if (l0 + q < nv) reinterpret_cast<float *>(dp + (size_t)(l0 + q) * nvb + blk)[threadIdx.x & 1] = t;
-        }
-        __syncthreads();
     }
+    __syncthreads();
+    if (threadIdx.x < 2 * nv) {
+        float t = 0.f;
+#pragma unroll
+        for (int w8 = 0; w8 < 8; ++w8) t += red[w8][threadIdx.x];
+        reinterpret_cast<float *>(dp + (size_t)(threadIdx.x >> 1) * nvb + blk)[threadIdx.x & 1] = t;
+    }
+    __syncthreads();
 }
 
-__device__ void block_norm_f(float2 wv, bool ok, double *__restrict__ nrmp, int blk, float (*red)[16]) {
+__device__ void block_norm_f(float2 wv, bool ok, double *__restrict__ nrmp, int blk, float (*red)[2 * kMaxV]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float t = ok ? fmaf(wv.x, wv.x, wv.y * wv.y) : 0.f;
     t = warp_sum_f(t);
@@ -1864,8 +1865,10 @@ __device__ __forceinline__ double2 apply_minv(const void *Minv, int n, int blk, 
 // V in float (C128 = false).
 template <bool C128>
 __global__ void __launch_bounds__(kThreads) k_dot1(const KTable *tb) {
-    __shared__ double red[8][16];
-    __shared__ float redf[8][16];
+    // one of the two is used: FP64 or float sums
+    __shared__ double red_s[8][2 * kMaxV];
+    double (*red)[2 * kMaxV] = red_s;
+    float (*redf)[2 * kMaxV] = reinterpret_cast<float (*)[2 * kMaxV]>(red_s);
     for (int it = blockIdx.x; it < tb->vb_total; it += gridDim.x) {
         const int2 bi = tb->vb_items[it];
         const KSys &S = tb->sys[bi.x];
@@ -1878,6 +1881,7 @@ __global__ void __launch_bounds__(kThreads) k_dot1(const KTable *tb) {
             float2 wv = make_float2(0.f, 0.f);
             if (ok) {
                 const float2 *mp = reinterpret_cast<const float2 *>(S.mvp);
+#pragma unroll 8
                 for (int c = 0; c < S.nchunk; ++c) {
                     const float2 p = mp[(size_t)c * n + row];
                     wv.x += p.x;
@@ -1890,6 +1894,7 @@ __global__ void __launch_bounds__(kThreads) k_dot1(const KTable *tb) {
         } else {
             double2 wv = make_double2(0.0, 0.0);
             if (ok) {
+#pragma unroll 8
                 for (int c = 0; c < S.nchunk; ++c) {
                     const double2 p = S.mvp[(size_t)c * n + row];
                     wv.x += p.x;
@@ -1911,8 +1916,10 @@ template <int PASS, bool C128>
 __global__ void __launch_bounds__(kThreads) k_axpy(const KTable *tb) {
     __shared__ double2 hs[kMaxV];
     __shared__ float2 hsf[kMaxV];
-    __shared__ double red[8][16];
-    __shared__ float redf[8][16];
+    // one of the two is used: FP64 or float sums
+    __shared__ double red_s[8][2 * kMaxV];
+    double (*red)[2 * kMaxV] = red_s;
+    float (*redf)[2 * kMaxV] = reinterpret_cast<float (*)[2 * kMaxV]>(red_s);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int it = blockIdx.x; it < tb->vb_total; it += gridDim.x) {
         const int2 bi = tb->vb_items[it];
@@ -2011,21 +2018,25 @@ __device__ __forceinline__ float2 apply_minv_f(const void *Minv, int n, int blk,
     const float2 *M = (const float2 *)Minv + (size_t)pb * kBlock * kBlock;
     float sh = 0.f, sl = 0.f, th = 0.f, tl = 0.f;
     if (nb == kBlock) {
-        // full block: each chunk's 16 loads issued before its arithmetic
-        for (int c0 = 0; c0 < kBlock; c0 += 16) {
-            float2 mv[16];
+        // full block: the loads of two chunks of 16 issued before their
+        // arithmetic (four round trips to L2 instead of eight)
+        for (int c0 = 0; c0 < kBlock; c0 += 32) {
+            float2 mv[32];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) mv[u] = M[(size_t)(c0 + u) * kBlock + rr];
-            float ar = 0.f, ai = 0.f;
+            for (int u = 0; u < 32; ++u) mv[u] = M[(size_t)(c0 + u) * kBlock + rr];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const float2 xv = x[c0 + u];
-                ar = fmaf(mv[u].x, xv.x, ar); ar = fmaf(-mv[u].y, xv.y, ar);
-                ai = fmaf(mv[u].x, xv.y, ai); ai = fmaf(mv[u].y, xv.x, ai);
+            for (int h = 0; h < 32; h += 16) {
+                float ar = 0.f, ai = 0.f;
+#pragma unroll
+                for (int u = h; u < h + 16; ++u) {
+                    const float2 xv = x[c0 + u];
+                    ar = fmaf(mv[u].x, xv.x, ar); ar = fmaf(-mv[u].y, xv.y, ar);
+                    ai = fmaf(mv[u].x, xv.y, ai); ai = fmaf(mv[u].y, xv.x, ai);
+                }
+                float t, e;
+                two_sum(sh, ar, t, e); sh = t; sl += e;
+                two_sum(th, ai, t, e); th = t; tl += e;
             }
-            float t, e;
-            two_sum(sh, ar, t, e); sh = t; sl += e;
-            two_sum(th, ai, t, e); th = t; tl += e;
         }
         return make_float2(sh + sl, th + tl);
     }
@@ -2045,64 +2056,140 @@ __device__ __forceinline__ float2 apply_minv_f(const void *Minv, int n, int blk,
     return make_float2(sh + sl, th + tl);
 }
 
+// The block-Jacobi application of the step kernels (k_scale, k_pcfin): a block
+// takes 32 rows of a 128-row inverse, warp w its columns 16 w .. 16 w + 15, all
+// of a thread's loads in flight at once and issued before the vector is there
+// (the product streams A through L2 in between, so the inverses come from
+// DRAM: with 256 rows per block and eight rounds of loads k_scale took 18 us at
+// 5120 unknowns, on 20 SMs; now 6 us).  The eight partial sums of a row are
+// added in order, in float-float pairs, as apply_minv_f adds its chunks.
+constexpr int kXRows = 32;
+constexpr int kXItems = kThreads / kXRows;
+constexpr int kXCols = kBlock / (kThreads / 32);   // columns per warp
+static_assert(kXCols == 16, "chunks as in apply_minv_f");
+
+// Groups of 32 rows per item of those kernels: one, or four in a batch with many
+// rows (fewer items to look at for the systems that are in another phase).
+__device__ __forceinline__ int x_groups(int vb_total) { return vb_total * kXItems > 4 * (int)gridDim.x ? 4 : 1; }
+
+template <bool C128> struct XTile {
+    using V = typename std::conditional<C128, double2, float2>::type;
+    V m[kXCols];
+    // the inverse's columns 16 warp .. + 15 at row r0 + lane
+    __device__ __forceinline__ void load(const void *Minv, int n, int r0) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int pb = r0 / kBlock, nb = min(kBlock, n - pb * kBlock), rr = r0 - pb * kBlock + lane;
+        const V *M = (const V *)Minv + (size_t)pb * kBlock * kBlock + (size_t)warp * kXCols * kBlock + rr;
+#pragma unroll
+        for (int u = 0; u < kXCols; ++u) {
+            m[u].x = m[u].y = 0;
+            if (rr < nb && warp * kXCols + u < nb) m[u] = M[(size_t)u * kBlock];
+        }
+    }
+    // the product with x (shared memory, the block's 128 entries, zeros past
+    // the system); the row's sum on warp 0.  Two block barriers.
+    __device__ __forceinline__ V apply(const V *x, V (*red)[32]) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        V t;
+        t.x = t.y = 0;
+#pragma unroll
+        for (int u = 0; u < kXCols; ++u) {
+            const V v = x[warp * kXCols + u];
+            t.x = fma(m[u].x, v.x, t.x);
+            t.x = fma(-m[u].y, v.y, t.x);
+            t.y = fma(m[u].x, v.y, t.y);
+            t.y = fma(m[u].y, v.x, t.y);
+        }
+        red[warp][lane] = t;
+        __syncthreads();
+        V o;
+        o.x = o.y = 0;
+        if (warp == 0) {
+            if constexpr (C128) {
+#pragma unroll
+                for (int w = 0; w < kThreads / 32; ++w) {
+                    o.x += red[w][lane].x;
+                    o.y += red[w][lane].y;
+                }
+            } else {
+                float sh = 0.f, sl = 0.f, th = 0.f, tl = 0.f, q, e;
+#pragma unroll
+                for (int w = 0; w < kThreads / 32; ++w) {
+                    two_sum(sh, red[w][lane].x, q, e); sh = q; sl += e;
+                    two_sum(th, red[w][lane].y, q, e); th = q; tl += e;
+                }
+                o = make_float2(sh + sl, th + tl);
+            }
+        }
+        return o;
+    }
+};
+
 template <bool C128, bool RESTART>
-__global__ void __launch_bounds__(kThreads) k_scale(const KTable *tb) {
-    __shared__ double2 vs[kThreads];
-    __shared__ float2 vf[kThreads];
-    __shared__ double nrm_s;
-    for (int it = blockIdx.x; it < tb->vb_total; it += gridDim.x) {
-        const int2 bi = tb->vb_items[it];
+__global__ void __launch_bounds__(kThreads, C128 ? 2 : 4) k_scale(const KTable *tb) {
+    using V = typename XTile<C128>::V;
+    __shared__ V xs[kBlock], red[kThreads / 32][32];
+    __shared__ double inv_s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = x_groups(tb->vb_total), items = kXItems / grp;
+    for (int it = blockIdx.x; it < tb->vb_total * items; it += gridDim.x) {
+        const int2 bi = tb->vb_items[it / items];
         const KSys &S = tb->sys[bi.x];
         const KState *st = S.st;
         if (st->phase != kPhaseArnoldi) continue;
         if (RESTART && st->k != 0) continue;
-        const int n = S.n, blk = bi.y, row = blk * kThreads + threadIdx.x;
-        if (!RESTART) {
-            // the norm once per block (same sum, same order as k_givens)
-            if (threadIdx.x == 0) nrm_s = norm_total(S.nrmp, S.nvb);
+        for (int q = 0; q < grp; ++q) {
+            const int n = S.n, r0 = bi.y * kThreads + ((it % items) * grp + q) * kXRows, row = r0 + lane;
+            if (r0 >= n) break;
+            XTile<C128> X;
+            if (S.pc) X.load(S.Minv, n, r0);
+            const int dst = RESTART ? 0 : st->k + 1, b0 = r0 / kBlock * kBlock;
+            // the vector's 128 entries, and 1 / |w| (1 / |r|) by one warp: a square
+            // root and a division on every thread would hold the FP64 pipe
+            if (warp == 4 && q == 0) {
+                const double nrm = RESTART ? 0.0 : warp_norm_total(S.nrmp, S.nvb, lane);
+                if (lane == 0) {
+                    inv_s = RESTART ? 1.0 / st->beta : 1.0 / sqrt(nrm);
+                    if (!RESTART && r0 == 0) S.st->wnorm2 = nrm;   // for k_givens
+                }
+            }
+            double2 wd = make_double2(0.0, 0.0);
+            if (threadIdx.x < kBlock && b0 + threadIdx.x < n) {
+                if (C128 || RESTART) wd = (RESTART ? S.r : S.w)[b0 + threadIdx.x];
+            }
+            // float: X v = (X w) / |w|, so the product does not wait for the norm
+            // (v_0 = r / beta from the FP64 r)
+            if constexpr (!C128) {
+                if (!RESTART && threadIdx.x < kBlock)
+                    xs[threadIdx.x] = b0 + threadIdx.x < n ? reinterpret_cast<const float2 *>(S.w)[b0 + threadIdx.x]
+                                                            : make_float2(0.f, 0.f);
+            }
+            __syncthreads();
+            const double s = inv_s;
+            if constexpr (C128) {
+                if (threadIdx.x < kBlock) xs[threadIdx.x] = make_double2(wd.x * s, wd.y * s);
+                __syncthreads();
+            } else if (RESTART) {
+                if (threadIdx.x < kBlock) xs[threadIdx.x] = make_float2((float)(wd.x * s), (float)(wd.y * s));
+                __syncthreads();
+            }
+            // with the window correction, X v goes to pcy and k_pcwin / k_pcfin
+            // form the product's input
+            V u = xs[row - b0];
+            if (S.pc) u = X.apply(xs, red);
+            if (warp == 0 && row < n) {
+                V v = xs[row - b0];
+                if constexpr (C128) {
+                    S.V[(size_t)dst * S.ldv + row] = v;
+                    if (S.pc) (S.pcw ? (double2 *)S.pcy : S.z)[row] = u;
+                } else {
+                    const float sf = RESTART ? 1.f : (float)s;
+                    reinterpret_cast<float2 *>(S.V)[(size_t)dst * S.ldv + row] = make_float2(v.x * sf, v.y * sf);
+                    (S.pcw ? (float2 *)S.pcy : S.xh)[row] = make_float2(u.x * sf, u.y * sf);
+                }
+            }
             __syncthreads();
         }
-        const double s = RESTART ? 1.0 / st->beta : 1.0 / sqrt(nrm_s);
-        const int dst = RESTART ? 0 : st->k + 1;
-        // with the window correction, X v goes to pcy and k_pcwin / k_pcfin
-        // form the product's input
-        if (C128) {
-            const double2 *src = RESTART ? S.r : S.w;
-            double2 v = make_double2(0.0, 0.0);
-            if (row < n) {
-                const double2 a = src[row];
-                v = make_double2(a.x * s, a.y * s);
-                S.V[(size_t)dst * S.ldv + row] = v;
-            }
-            double2 u = v;   // input of the next product
-            if (S.pc) {
-                vs[threadIdx.x] = v;
-                __syncthreads();
-                u = apply_minv(S.Minv, n, blk, vs);
-                if (row < n) (S.pcw ? (double2 *)S.pcy : S.z)[row] = u;
-            }
-        } else {
-            // float basis: v = w / |w| in FP32 (v_0 = r / beta from the FP64 r)
-            float2 u = make_float2(0.f, 0.f);
-            if (row < n) {
-                if (RESTART) {
-                    const double2 a = S.r[row];
-                    u = make_float2((float)(a.x * s), (float)(a.y * s));
-                } else {
-                    const float2 a = reinterpret_cast<const float2 *>(S.w)[row];
-                    const float sf = (float)s;
-                    u = make_float2(a.x * sf, a.y * sf);
-                }
-                reinterpret_cast<float2 *>(S.V)[(size_t)dst * S.ldv + row] = u;
-            }
-            if (S.pc) {
-                vf[threadIdx.x] = u;
-                __syncthreads();
-                u = apply_minv_f(S.Minv, n, blk, vf);
-            }
-            if (row < n) (S.pcw ? (float2 *)S.pcy : S.xh)[row] = u;
-        }
-        __syncthreads();
     }
 }
 
@@ -2114,22 +2201,22 @@ __device__ void givens_step(const KSys &S) {
     KState *st = S.st;
     const int k = st->k, m = st->m;
     double2 *H = S.H, *cs = S.cs, *sn = S.sn, *g = S.g, *hsum = S.hsum;
-    const double hn = sqrt(norm_total(S.nrmp, S.nvb));
+    const double hn = sqrt(st->wnorm2);   // |w|^2 from k_scale
     // column k of H from hsum (cleared for the next step) with the previous
-    // rotations applied on the way: [a; b] <- [[conj(c), conj(s)], [-s, c]]
-    // [a; b]; the running entry stays in registers, the loads do not depend
-    // on it
+    // rotations applied on the way: [a; b] <- [[conj(c), s], [-s, c]] [a; b],
+    // s real; the running entry stays in registers and takes one fused
+    // operation per rotation (c b does not depend on it)
     double2 a = hsum[0];
     hsum[0] = make_double2(0.0, 0.0);
-#pragma unroll 4
+#pragma unroll 8
     for (int l = 0; l < k; ++l) {
         const double2 bb = hsum[l + 1];
         hsum[l + 1] = make_double2(0.0, 0.0);
-        const double2 c = cs[l], s = sn[l];
-        H[(size_t)l * m + k] = make_double2(c.x * a.x + c.y * a.y + s.x * bb.x + s.y * bb.y,
-                                            c.x * a.y - c.y * a.x + s.x * bb.y - s.y * bb.x);
-        a = make_double2(-(s.x * a.x - s.y * a.y) + c.x * bb.x - c.y * bb.y,
-                         -(s.x * a.y + s.y * a.x) + c.x * bb.y + c.y * bb.x);
+        const double2 c = cs[l];
+        const double s = sn[l].x;
+        const double tx = c.x * bb.x - c.y * bb.y, ty = c.x * bb.y + c.y * bb.x;
+        H[(size_t)l * m + k] = make_double2(c.x * a.x + c.y * a.y + s * bb.x, c.x * a.y - c.y * a.x + s * bb.y);
+        a = make_double2(fma(-s, a.x, tx), fma(-s, a.y, ty));
     }
     const double den = sqrt(a.x * a.x + a.y * a.y + hn * hn);
     double2 c, s;
@@ -2173,9 +2260,12 @@ __global__ void __launch_bounds__(kMaxSys) k_givens(KTable *tb) {
 }
 
 // ------------------------------------------------------------ end of cycle
-// y = H^{-1} g (k x k upper triangular), one warp per system.
+// y = H^{-1} g (k x k upper triangular), one warp per system: lane l keeps the
+// entries l and l + 32 of the right-hand side; a step broadcasts one unknown
+// and takes its column out of the entries above, so its latency is a shuffle,
+// a product with the pivot's inverse (formed beforehand) and a fused update.
+static_assert(kMaxRestart <= 64, "two entries per lane");
 __global__ void __launch_bounds__(128) k_trisolve(const KTable *tb) {
-    __shared__ double2 ys[4][kMaxV];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * 4 + warp;
     if (b >= tb->B) return;
@@ -2183,24 +2273,31 @@ __global__ void __launch_bounds__(128) k_trisolve(const KTable *tb) {
     const KState *st = S.st;
     if (st->phase != kPhaseUpdate || st->k == 0) return;
     const int kk = st->k, m = st->m;
-    for (int i = kk - 1; i >= 0; --i) {
-        double re = 0.0, im = 0.0;
-        for (int l = i + 1 + lane; l < kk; l += 32) {
-            const double2 h = S.H[(size_t)i * m + l], yl = ys[warp][l];
-            re += h.x * yl.x - h.y * yl.y;
-            im += h.x * yl.y + h.y * yl.x;
-        }
-        re = warp_sum_d(re);
-        im = warp_sum_d(im);
-        if (lane == 0) {
-            const double2 gi = S.g[i], d = S.H[(size_t)i * m + i];
-            const double ar = gi.x - re, ai = gi.y - im;
+    double2 v[2], inv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        v[h] = inv[h] = make_double2(0.0, 0.0);
+        if (i < kk) {
+            const double2 d = S.H[(size_t)i * m + i];
             const double dd = d.x * d.x + d.y * d.y;
-            const double2 y = make_double2((ar * d.x + ai * d.y) / dd, (ai * d.x - ar * d.y) / dd);
-            ys[warp][i] = y;
-            S.y[i] = y;
+            v[h] = S.g[i];
+            inv[h] = make_double2(d.x / dd, -d.y / dd);
         }
-        __syncwarp();
+    }
+#pragma unroll 4
+    for (int i = kk - 1; i >= 0; --i) {
+        double2 h0 = make_double2(0.0, 0.0), h1 = h0;
+        if (lane < i) h0 = S.H[(size_t)lane * m + i];
+        if (lane + 32 < i) h1 = S.H[(size_t)(lane + 32) * m + i];
+        const double2 g = i < 32 ? v[0] : v[1], q = i < 32 ? inv[0] : inv[1];
+        const double2 p = make_double2(g.x * q.x - g.y * q.y, g.x * q.y + g.y * q.x);
+        const double2 y = make_double2(__shfl_sync(0xffffffffu, p.x, i & 31), __shfl_sync(0xffffffffu, p.y, i & 31));
+        if (lane == (i & 31)) S.y[i] = y;
+        v[0].x = fma(-h0.x, y.x, fma(h0.y, y.y, v[0].x));
+        v[0].y = fma(-h0.x, y.y, fma(-h0.y, y.x, v[0].y));
+        v[1].x = fma(-h1.x, y.x, fma(h1.y, y.y, v[1].x));
+        v[1].y = fma(-h1.x, y.y, fma(-h1.y, y.x, v[1].y));
     }
 }
 
@@ -2305,8 +2402,11 @@ __device__ __forceinline__ bool pcw_active(const KSys &S, int mode) {
     return st->phase == kPhaseArnoldi && (mode == 0 || st->k == 0);
 }
 
-constexpr int kPcRows = 32;                  // rows per k_pcwin item
-constexpr int kPcItems = kThreads / kPcRows; // items per vector block
+// Rows per k_pcwin item: 32 (four per warp) when that makes enough items for
+// the SMs, else 16: 5120 unknowns 12.3 -> 10 us,
+// 20480 unknowns 20 us with 32; 8 rows with early loads took 33 there.
+constexpr int kPcRowsMost = 32;
+__device__ __forceinline__ int pc_rows(int vb_total) { return vb_total >= 64 ? kPcRowsMost : kPcRowsMost / 2; }
 static_assert(kPcWin % kThreads == 0, "windows hold whole vector blocks");
 static_assert(kPcWin == kMvChunk, "a window is one column chunk: one fp16 segment scale per row");
 
@@ -2323,14 +2423,15 @@ __global__ void __launch_bounds__(kThreads) k_pcwin(const KTable *tb, int mode) 
     __shared__ __align__(16) double2 ysh[kPcWin];
     if (!tb->pcw_any) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int it = blockIdx.x; it < tb->vb_total * kPcItems; it += gridDim.x) {
-        const int2 bi = tb->vb_items[it / kPcItems];
+    const int rows = pc_rows(tb->vb_total), items = kThreads / rows;
+    for (int it = blockIdx.x; it < tb->vb_total * items; it += gridDim.x) {
+        const int2 bi = tb->vb_items[it / items];
         const KSys &S = tb->sys[bi.x];
-        if (!pcw_active(S, mode)) continue;
-        const int n = S.n, r0 = bi.y * kThreads + (it % kPcItems) * kPcRows;
+        if (!__syncthreads_or(pcw_active(S, mode))) continue;   // one answer per block: k_givens may run beside this
+        const int n = S.n, r0 = bi.y * kThreads + (it % items) * rows;
         if (r0 >= n) continue;
         const int c0 = r0 / kPcWin * kPcWin, nw = min(kPcWin, n - c0);
-        const int r1 = min(r0 + kPcRows, n);
+        const int r1 = min(r0 + rows, n);
         __syncthreads();   // the previous item's rows are done with ysh
         if (C128) {
             const double2 *y = (const double2 *)S.pcy + c0;
@@ -2403,46 +2504,49 @@ __global__ void __launch_bounds__(kThreads) k_pcwin(const KTable *tb, int mode) 
 // (mode 2).
 template <bool C128>
 __global__ void __launch_bounds__(kThreads) k_pcfin(const KTable *tb, int mode) {
-    __shared__ double2 vs[kThreads];
-    __shared__ float2 vf[kThreads];
+    using V = typename XTile<C128>::V;
+    __shared__ V xs[kBlock], red[kThreads / 32][32];
     if (!tb->pcw_any) return;
-    for (int it = blockIdx.x; it < tb->vb_total; it += gridDim.x) {
-        const int2 bi = tb->vb_items[it];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = x_groups(tb->vb_total), items = kXItems / grp;
+    for (int it = blockIdx.x; it < tb->vb_total * items; it += gridDim.x) {
+        const int2 bi = tb->vb_items[it / items];
         const KSys &S = tb->sys[bi.x];
-        if (!pcw_active(S, mode)) continue;
-        const int n = S.n, blk = bi.y, row = blk * kThreads + threadIdx.x;
-        const bool ok = row < n;
-        if (C128) {
-            const double2 *Y = (const double2 *)S.pcy, *Z = (const double2 *)S.pcz;
-            vs[threadIdx.x] = ok ? Z[row] : make_double2(0.0, 0.0);
-            __syncthreads();
-            const double2 q = apply_minv(S.Minv, n, blk, vs);
-            if (ok) {
-                const double2 y = Y[row];
-                const double2 u = make_double2(2.0 * y.x - q.x, 2.0 * y.y - q.y);
-                if (mode == 2) xupdate_finish<true>(S, S.st, row, u);
-                else S.z[row] = u;
+        if (!__syncthreads_or(pcw_active(S, mode))) continue;   // one answer per block: k_givens may run beside this
+        for (int g = 0; g < grp; ++g) {
+            const int n = S.n, r0 = bi.y * kThreads + ((it % items) * grp + g) * kXRows, row = r0 + lane;
+            if (r0 >= n) break;
+            XTile<C128> X;
+            X.load(S.Minv, n, r0);
+            const int b0 = r0 / kBlock * kBlock;
+            if (threadIdx.x < kBlock) {
+                V z;
+                z.x = z.y = 0;
+                if (b0 + threadIdx.x < n) z = ((const V *)S.pcz)[b0 + threadIdx.x];
+                xs[threadIdx.x] = z;
             }
-        } else {
-            const float2 *Y = (const float2 *)S.pcy, *Z = (const float2 *)S.pcz;
-            vf[threadIdx.x] = ok ? Z[row] : make_float2(0.f, 0.f);
+            V y;
+            y.x = y.y = 0;
+            if (warp == 0 && row < n) y = ((const V *)S.pcy)[row];
             __syncthreads();
-            const float2 q = apply_minv_f(S.Minv, n, blk, vf);
-            if (ok) {
-                const float2 y = Y[row];
-                const float2 u = make_float2(2.f * y.x - q.x, 2.f * y.y - q.y);
-                if (mode == 2) xupdate_finish<false>(S, S.st, row, make_double2((double)u.x, (double)u.y));
+            const V q = X.apply(xs, red);
+            if (warp == 0 && row < n) {
+                V u;
+                u.x = 2 * y.x - q.x;
+                u.y = 2 * y.y - q.y;
+                if (mode == 2) xupdate_finish<C128>(S, S.st, row, make_double2((double)u.x, (double)u.y));
+                else if constexpr (C128) S.z[row] = u;
                 else S.xh[row] = u;
             }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
 // r = b - A x, or r - A d (complex64 after the first cycle), or r = b before
 // the first cycle; |r|^2 partials
 __global__ void __launch_bounds__(kThreads) k_resid(const KTable *tb) {
-    __shared__ double red[8][16];
+    __shared__ double red[8][2 * kMaxV];
     for (int it = blockIdx.x; it < tb->vb_total; it += gridDim.x) {
         const int2 bi = tb->vb_items[it];
         const KSys &S = tb->sys[bi.x];
@@ -2456,6 +2560,7 @@ __global__ void __launch_bounds__(kThreads) k_resid(const KTable *tb) {
             r = (tb->prec == 1 && st->cycles >= 2) ? S.r[row] : S.b[row];
             if (st->cycles > 0) {
                 double ax = 0.0, ay = 0.0;
+#pragma unroll 8
                 for (int c = 0; c < S.nchunk; ++c) {
                     const double2 p = S.mvp[(size_t)c * n + row];
                     ax += p.x;
@@ -2472,9 +2577,9 @@ __global__ void __launch_bounds__(kThreads) k_resid(const KTable *tb) {
 
 // One thread per system: convergence decision after a cycle (or the initial
 // residual), then the restart: g = beta e_1, hsum = 0, the cycle's target.
-__device__ void decide_step(const KSys &S) {
+__device__ void decide_step(const KSys &S, double nrm2) {
     KState *st = S.st;
-    const double beta = sqrt(norm_total(S.nrmp, S.nvb));
+    const double beta = sqrt(nrm2);
     if (st->cycles == 0) {
         st->bnorm = beta;
         st->beta = beta;
@@ -2522,8 +2627,16 @@ __device__ void decide_step(const KSys &S) {
 // plans from the new phases (k_givens rebuilds them only when a phase changes
 // in its step).
 __global__ void __launch_bounds__(kMaxSys) k_decide(KTable *tb) {
-    const int b = threadIdx.x;
-    if (b < tb->B && tb->sys[b].st->phase == kPhaseUpdate) decide_step(tb->sys[b]);
+    __shared__ double nrm[kMaxSys];
+    const int b = threadIdx.x, lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < tb->B; q += kMaxSys / 32) {   // a warp per system
+        const KSys &S = tb->sys[q];
+        if (S.st->phase != kPhaseUpdate) continue;
+        const double t = warp_norm_total(S.nrmp, S.nvb, lane);
+        if (lane == 0) nrm[q] = t;
+    }
+    __syncthreads();
+    if (b < tb->B && tb->sys[b].st->phase == kPhaseUpdate) decide_step(tb->sys[b], nrm[b]);
     __syncthreads();
     plan_build(tb, 0);
     plan_build(tb, 1);
@@ -2622,7 +2735,7 @@ static void pc_window(bool c128, const KTable *d_tab, int mode, int gv, cudaStre
 }
 
 cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev, cudaStream_t st,
-                               int *launches_out, bool groups, bool blr, bool dense) {
+                               int *launches_out, bool groups, bool blr, bool dense, const SideStream &side) {
     KTable *tb = const_cast<KTable *>(d_tab);
     const bool c128 = prec == 0;
     if (!g_vec_grid) return cudaErrorNotReady;   // krylov_prepare() first
@@ -2658,8 +2771,17 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev
         }
         if (c128) k_scale<true, false><<<gv, kThreads, 0, st>>>(d_tab);
         else k_scale<false, false><<<gv, kThreads, 0, st>>>(d_tab);
+        // the rotations beside the window correction: both follow k_scale and
+        // precede the next product.  A system whose cycle ends here may see
+        // its phase change under the correction, whose result it then does
+        // not read (the cycle's update forms pcy, pcz and xh anew); a block of
+        // the correction decides as a whole whether it takes part.
+        cudaEventRecord(side.fork, st);
+        cudaStreamWaitEvent(side.st, side.fork, 0);
+        k_givens<<<1, kMaxSys, 0, side.st>>>(tb);
+        cudaEventRecord(side.join, side.st);
         pc_window(c128, d_tab, 0, gv, st);
-        k_givens<<<1, kMaxSys, 0, st>>>(tb);
+        cudaStreamWaitEvent(st, side.join, 0);
         nl += 8;
     }
     k_trisolve<<<(kMaxSys + 3) / 4, 128, 0, st>>>(d_tab);

@@ -307,6 +307,7 @@ struct KState {
     double floor_rel;    // inner cycle stops at floor_rel * beta (mixed: 3e-4
                          // with the fp16 copy, 1e-5 without)
     double bnorm, beta, prev_beta, thr, res, rel;
+    double wnorm2;       // |w|^2 of the current Arnoldi step (k_scale, for k_givens)
 };
 
 struct KSys {
@@ -411,8 +412,14 @@ constexpr int kSteps = 8;
 // product from A or its fp16 copy (k_mv_tma / k_mv64), for batches with
 // single systems without one (always for complex128).  Returns the number of
 // kernel launches enqueued through *launches_out.
+// side: a second stream for the branch that runs beside the main one (joined
+// again before the next product), and the events that fork and join it.
+struct SideStream {
+    cudaStream_t st;
+    cudaEvent_t fork, join;
+};
 cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev, cudaStream_t st,
-                               int *launches_out, bool groups, bool blr, bool dense);
+                               int *launches_out, bool groups, bool blr, bool dense, const SideStream &side);
 // complex64 matrices: the product streams row segments with bulk copies
 // (TMA) in strips of `strip` rows (a multiple of kTmaRows, chosen per system
 // by the tuner; kTmaStrip by default); complex128: tiles of kMvRows rows.
