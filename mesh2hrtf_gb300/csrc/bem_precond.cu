@@ -10,11 +10,12 @@
 // windows of kPcWin unknowns, M = X (2 I - A_w X) (bem_gmres.cu), which
 // needs no further set-up.
 //
-// Inversion: one CTA per block of any system in the batch, in-place
-// Gauss-Jordan with partial pivoting.  complex64 blocks live in shared memory
-// (128 KB); complex128 blocks are inverted in a global workspace (L2
-// resident).  Inverses are stored transposed so that the application (inside
-// the Krylov kernels, bem_gmres.cu) reads them coalesced.
+// Inversion: in-place Gauss-Jordan with partial pivoting, one block of kBlock
+// rows per cluster of CTAs that share its columns, entries in registers
+// (gauss_jordan_reg); the last, partial block of a system goes through shared
+// memory or a global workspace (gauss_jordan).  Inverses are stored transposed
+// so that the application (inside the Krylov kernels, bem_gmres.cu) reads them
+// coalesced.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -43,6 +44,21 @@ template <typename V> __device__ __forceinline__ V cinv2(V a) {
     r.x = ar / (d * s);
     r.y = -ai / (d * s);
     return r;
+}
+
+// The same with one division, for a chain that waits for it: scaled by a power
+// of two (exact) instead of the larger component.
+__device__ __forceinline__ float2 cinv_pow2(float2 a) {
+    const int e = (int)((__float_as_uint(fmaxf(fabsf(a.x), fabsf(a.y))) >> 23) & 255u);   // biased exponent
+    const float s = __uint_as_float((unsigned)min(max(254 - e, 1), 254) << 23);
+    const float ar = a.x * s, ai = a.y * s, q = s / fmaf(ar, ar, ai * ai);
+    return make_float2(ar * q, -ai * q);
+}
+__device__ __forceinline__ double2 cinv_pow2(double2 a) {
+    const int e = (__double2hiint(fmax(fabs(a.x), fabs(a.y))) >> 20) & 2047;
+    const double s = __hiloint2double(min(max(2046 - e, 1), 2046) << 20, 0);
+    const double ar = a.x * s, ai = a.y * s, q = s / fma(ar, ar, ai * ai);
+    return make_double2(ar * q, -ai * q);
 }
 
 // In-place Gauss-Jordan on the nb x nb block W (row-major, leading dim ld),
@@ -115,78 +131,152 @@ __device__ void gauss_jordan(typename C2<T>::t *W, int ld, int nb, typename C2<T
     }
 }
 
-// The same on a full kBlock x kBlock block by NT threads, with compile-time
-// indexing and three barriers per pivot: warp 0 finds the pivot (largest
-// |a|^2, lowest row on ties) and gathers the pivot column with the rows
-// interchanged, the first kBlock threads interchange the rows and scale the
-// pivot row, then thread t updates column t % kBlock of rows t / kBlock,
-// + NT / kBlock, ...
-template <typename T, int NT>
-__device__ void gauss_jordan_full(typename C2<T>::t *W, typename C2<T>::t *colk, int *piv, int *pivrow,
-                                  int *singular) {
+// The same on a full kBlock x kBlock block held in registers by CL CTAs of a
+// cluster: CTA r has the columns r kBlock / CL .. , thread t of NT its column
+// t % C (C = kBlock / CL) at rows kR (t / C) .. + kR - 1.  A step needs the
+// pivot column (published by the threads that hold it as soon as the step
+// before has updated it, in one of two buffers; the other CTAs fetch it through
+// distributed shared memory), the pivot with its inverse (one warp: square and
+// divisions on every warp took longer than the update) and the pivot row
+// (published by the threads that hold it).  Rows are not interchanged:
+// step k's pivot is the largest |a|^2 among the rows not used yet, lowest row
+// on ties, and with p_k its row the inverse is Ainv[k][p_c] = W[p_k][c].
+//
+// A full block in shared memory (three barriers a step, every entry loaded and
+// stored each step) was bound by shared-memory traffic: 306 us in complex64,
+// whatever the system's size; in registers 205 us.  complex128 is bound by
+// an SM's narrow FP64 pipe (4 FMA per entry and step), so its blocks spread
+// over four SMs: 40 blocks 3.9 ms in an L2 workspace, 1.24 ms now.
+template <typename T, int CL, int NT>
+__device__ void gauss_jordan_reg(const typename C2<T>::t *A, size_t lda, typename C2<T>::t *out, int *status) {
     using V = typename C2<T>::t;
-    constexpr int kG = NT / kBlock;
-    static_assert(NT % kBlock == 0 && kBlock % 32 == 0, "threads cover whole columns");
+    constexpr int C = kBlock / CL, G = NT / C, kR = kBlock / G;
+    static_assert(G * kR == kBlock && C % 32 == 0, "threads cover the block, a warp one row group");
+    __shared__ __align__(16) V colb[2][kBlock];       // pivot column, by step parity (own CTA's threads)
+    __shared__ V col[CL > 1 ? kBlock : 1];   // the pivot column fetched from its CTA
+    __shared__ V rowb[C], inv_s;
+    __shared__ int piv[kBlock], singular_s;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int j = tid % kBlock, g = tid / kBlock;
+    unsigned rank = 0;
+    if (CL > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int j = tid % C, i0 = tid / C * kR, jg = (int)rank * C + j;   // own column (in the CTA, in the block)
+    V a[kR];
+#pragma unroll
+    for (int q = 0; q < kR; ++q) a[q] = A[(size_t)(i0 + q) * lda + jg];
+    if (jg == 0) {
+#pragma unroll
+        for (int q = 0; q < kR; ++q) colb[0][i0 + q] = a[q];
+    }
+    unsigned used = 0;   // warp 0, bit q: row lane + 32 q has been a pivot row
+    if (tid == 0) singular_s = 0;
+#pragma unroll 1
     for (int k = 0; k < kBlock; ++k) {
+        const V *pc = colb[k & 1];
+        if (CL > 1) {
+            // the column is complete in its CTA, and the others are done with
+            // the buffer of two steps ago
+            asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+            if (tid < kBlock) {
+                const unsigned src = (unsigned)__cvta_generic_to_shared(&colb[k & 1][tid]);
+                unsigned rem;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rem) : "r"(src), "r"(k / C));
+                V v;
+                if constexpr (sizeof(V) == 16)
+                    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(rem) : "memory");
+                else
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(rem) : "memory");
+                col[tid] = v;
+            }
+            pc = col;
+        }
+        __syncthreads();
         if (tid < 32) {
             T best = -1;
-            int bi = k;
-            for (int i = k + lane; i < kBlock; i += 32) {
-                const V a = W[i * kBlock + k];
-                const T m = a.x * a.x + a.y * a.y;
-                if (m > best) { best = m; bi = i; }
+            int p = kBlock;
+#pragma unroll
+            for (int q = 0; q < kBlock / 32; ++q) {
+                const V v = pc[lane + 32 * q];
+                const T m = v.x * v.x + v.y * v.y;
+                if (!((used >> q) & 1u) && m > best) {
+                    best = m;
+                    p = lane + 32 * q;
+                }
             }
-            // butterfly: every lane ends with the same (best, bi)
+#pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const T ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+                const int oi = __shfl_xor_sync(0xffffffffu, p, o);
+                if (ob > best || (ob == best && oi < p)) { best = ob; p = oi; }
             }
-            for (int i = lane; i < kBlock; i += 32) {
-                const int src = i == k ? bi : (i == bi ? k : i);
-                colk[i] = W[src * kBlock + k];
+            if (!(best > 0)) {
+                if (lane == 0) singular_s = 1;
+                // nothing comparable (NaN): the lowest unused row
+                if (p >= kBlock) {
+                    int cand = kBlock;
+#pragma unroll
+                    for (int q = kBlock / 32 - 1; q >= 0; --q)
+                        if (!((used >> q) & 1u)) cand = lane + 32 * q;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
+                    p = cand;
+                }
             }
+            if (lane == (p & 31)) used |= 1u << (p >> 5);
             if (lane == 0) {
-                *pivrow = bi;
-                piv[k] = bi;
-                if (!(best > 0)) *singular = 1;
+                piv[k] = p;
+                inv_s = cinv_pow2(pc[p]);
             }
         }
         __syncthreads();
-        const int p = *pivrow;
-        if (tid < kBlock) {
-            const V inv = cinv2(colk[k]);
-            const V tk = W[k * kBlock + j], tp = W[p * kBlock + j];
-            if (p != k) W[p * kBlock + j] = tk;
-            const V a = j == k ? V{1, 0} : tp;
-            W[k * kBlock + j] = cmul2(a, inv);
+        const int p = piv[k] - i0;   // the pivot row among this warp's rows
+        // the pivot row, scaled (its own column: 1 / pivot)
+        if (p >= 0 && p < kR) {
+            V r = a[0];
+#pragma unroll
+            for (int q = 1; q < kR; ++q)
+                if (p == q) r = a[q];
+            if (jg == k) { r.x = 1; r.y = 0; }
+            rowb[j] = cmul2(r, inv_s);
         }
         __syncthreads();
-        const V r = W[k * kBlock + j];
-#pragma unroll 4
-        for (int i = g; i < kBlock; i += kG) {
-            if (i == k) continue;
-            const V f = colk[i];
-            V a = j == k ? V{0, 0} : W[i * kBlock + j];
-            a.x -= f.x * r.x - f.y * r.y;
-            a.y -= f.x * r.y + f.y * r.x;
-            W[i * kBlock + j] = a;
-        }
-        __syncthreads();
-    }
-    // undo the row interchanges as column interchanges, last first
-    for (int k = kBlock - 1; k >= 0; --k) {
-        const int p = piv[k];
-        if (p != k)
-            for (int i = tid; i < kBlock; i += NT) {
-                V t = W[i * kBlock + k];
-                W[i * kBlock + k] = W[i * kBlock + p];
-                W[i * kBlock + p] = t;
+        const V r = rowb[j];
+        if ((jg >> 5) == (k >> 5)) {   // the warps with column k
+            if (jg == k) {
+#pragma unroll
+                for (int q = 0; q < kR; ++q) a[q].x = a[q].y = 0;
             }
-        __syncthreads();
+        }
+#pragma unroll
+        for (int q = 0; q < kR; ++q) {
+            const V f = pc[i0 + q];
+            a[q].x = fma(-f.x, r.x, a[q].x);
+            a[q].x = fma(f.y, r.y, a[q].x);
+            a[q].y = fma(-f.x, r.y, a[q].y);
+            a[q].y = fma(-f.y, r.x, a[q].y);
+        }
+        if (p >= 0 && p < kR) {
+#pragma unroll
+            for (int q = 0; q < kR; ++q)
+                if (p == q) a[q] = r;
+        }
+        if (jg == k + 1) {
+#pragma unroll
+            for (int q = 0; q < kR; ++q) colb[(k + 1) & 1][i0 + q] = a[q];
+        }
     }
+    __syncthreads();
+    // row i was the pivot of step inv_p(i), column jg holds the inverse's column
+    // p_jg: Minv[c][r] (transposed) with r the step, c = piv[jg]
+    int *step = reinterpret_cast<int *>(rowb);   // C * sizeof(V) >= 4 kBlock
+    static_assert(C * sizeof(V) >= kBlock * sizeof(int), "the steps fit the row buffer");
+    if (tid < kBlock) step[piv[tid]] = tid;
+    __syncthreads();
+    const int c = piv[jg];
+#pragma unroll
+    for (int q = 0; q < kR; ++q) out[(size_t)c * kBlock + step[i0 + q]] = a[q];
+    if (tid == 0 && rank == 0 && singular_s) atomicMax(status, 1);
+    // no CTA leaves while another may still read its column buffer
+    if (CL > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ int find_blk(const int *off, int B, int item) {
@@ -198,74 +288,64 @@ __device__ __forceinline__ int find_blk(const int *off, int B, int item) {
     return lo;
 }
 
-// complex64: block in shared memory
 constexpr int kBinv32Threads = 1024;
-__global__ void __launch_bounds__(kBinv32Threads) k_binv32(const __grid_constant__ PcBatch tb) {
-    extern __shared__ float2 smem[];
-    __shared__ float2 colk[kBlock];
+constexpr int kBinv64Threads = 256, kBinv64Cluster = 4;
+
+// The system's last, partial block by one CTA on the nb x nb work array w
+// (leading dimension kBlock); the rest of the stored block is zero.
+template <typename T>
+__device__ void invert_partial(const PcSys &S, int r0, int nb, typename C2<T>::t *w, typename C2<T>::t *out) {
+    using V = typename C2<T>::t;
+    __shared__ V colk[kBlock];
     __shared__ int piv[kBlock];
     __shared__ int pivrow, singular;
-    const int sb = find_blk(tb.off, tb.B, blockIdx.x);
-    const PcSys &S = tb.sys[sb];
-    const float2 *A = (const float2 *)S.A;
-    const size_t lda = S.lda;
-    const int b = blockIdx.x - tb.off[sb], r0 = b * kBlock;
-    const int nb = min(kBlock, S.n - r0);
+    const V *A = (const V *)S.A;
     if (threadIdx.x == 0) singular = 0;
-    if (nb == kBlock) {
-        for (int e = threadIdx.x; e < kBlock * kBlock; e += kBinv32Threads)
-            smem[e] = A[(size_t)(r0 + e / kBlock) * lda + r0 + e % kBlock];
-        __syncthreads();
-        gauss_jordan_full<float, kBinv32Threads>(smem, colk, piv, &pivrow, &singular);
-    } else {   // the last, partial block of a system
-        for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-            const int i = e / nb, j = e - i * nb;
-            smem[i * kBlock + j] = A[(size_t)(r0 + i) * lda + r0 + j];
-        }
-        __syncthreads();
-        gauss_jordan<float>(smem, kBlock, nb, colk, piv, &pivrow, &singular);
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+        const int i = e / nb, j = e - i * nb;
+        w[i * kBlock + j] = A[(size_t)(r0 + i) * S.lda + r0 + j];
     }
-    // store transposed: Minv[b][c][r] = inv[r][c]
-    float2 *out = (float2 *)S.Minv + (size_t)b * kBlock * kBlock;
+    __syncthreads();
+    gauss_jordan<T>(w, kBlock, nb, colk, piv, &pivrow, &singular);
     for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
         const int c = e / kBlock, r = e - c * kBlock;
-        out[e] = (r < nb && c < nb) ? smem[r * kBlock + c] : make_float2(0.f, 0.f);
+        V v;
+        v.x = v.y = 0;
+        if (r < nb && c < nb) v = w[r * kBlock + c];
+        out[e] = v;
     }
     if (threadIdx.x == 0 && singular) atomicMax(S.status, 1);
 }
 
-// complex128: block in a global workspace
-__global__ void __launch_bounds__(512) k_binv64(const __grid_constant__ PcBatch tb) {
-    __shared__ double2 colk[kBlock];
-    __shared__ int piv[kBlock];
-    __shared__ int pivrow, singular;
+// complex64: one CTA per block; a partial block's work array in shared memory
+__global__ void __launch_bounds__(kBinv32Threads) k_binv32(const __grid_constant__ PcBatch tb) {
+    extern __shared__ float2 smem[];
     const int sb = find_blk(tb.off, tb.B, blockIdx.x);
     const PcSys &S = tb.sys[sb];
-    const double2 *A = (const double2 *)S.A;
-    const size_t lda = S.lda;
     const int b = blockIdx.x - tb.off[sb], r0 = b * kBlock;
     const int nb = min(kBlock, S.n - r0);
-    double2 *w = (double2 *)S.work + (size_t)b * kBlock * kBlock;
-    if (threadIdx.x == 0) singular = 0;
-    if (nb == kBlock) {
-        for (int e = threadIdx.x; e < kBlock * kBlock; e += 512)
-            w[e] = A[(size_t)(r0 + e / kBlock) * lda + r0 + e % kBlock];
-        __syncthreads();
-        gauss_jordan_full<double, 512>(w, colk, piv, &pivrow, &singular);
-    } else {
-        for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-            const int i = e / nb, j = e - i * nb;
-            w[i * kBlock + j] = A[(size_t)(r0 + i) * lda + r0 + j];
-        }
-        __syncthreads();
-        gauss_jordan<double>(w, kBlock, nb, colk, piv, &pivrow, &singular);
-    }
+    float2 *out = (float2 *)S.Minv + (size_t)b * kBlock * kBlock;
+    if (nb == kBlock)
+        gauss_jordan_reg<float, 1, kBinv32Threads>((const float2 *)S.A + (size_t)r0 * S.lda + r0, S.lda, out, S.status);
+    else
+        invert_partial<float>(S, r0, nb, smem, out);
+}
+
+// complex128: a cluster of CTAs per block; a partial block by its first CTA,
+// in the global workspace
+__global__ void __cluster_dims__(kBinv64Cluster, 1, 1) __launch_bounds__(kBinv64Threads)
+    k_binv64(const __grid_constant__ PcBatch tb) {
+    const int item = blockIdx.x / kBinv64Cluster;
+    const int sb = find_blk(tb.off, tb.B, item);
+    const PcSys &S = tb.sys[sb];
+    const int b = item - tb.off[sb], r0 = b * kBlock;
+    const int nb = min(kBlock, S.n - r0);
     double2 *out = (double2 *)S.Minv + (size_t)b * kBlock * kBlock;
-    for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
-        const int c = e / kBlock, r = e - c * kBlock;
-        out[e] = (r < nb && c < nb) ? w[r * kBlock + c] : make_double2(0.0, 0.0);
-    }
-    if (threadIdx.x == 0 && singular) atomicMax(S.status, 1);
+    if (nb == kBlock)
+        gauss_jordan_reg<double, kBinv64Cluster, kBinv64Threads>((const double2 *)S.A + (size_t)r0 * S.lda + r0, S.lda,
+                                                                 out, S.status);
+    else if (blockIdx.x % kBinv64Cluster == 0)
+        invert_partial<double>(S, r0, nb, (double2 *)S.work + (size_t)b * kBlock * kBlock, out);
 }
 
 // fp16 copy of complex64 rows (SplitBatch): one warp per (row, column
@@ -427,7 +507,7 @@ cudaError_t launch_block_inverse(const PcBatch &t, int prec, cudaStream_t st) {
     if (t.B <= 0 || t.off[t.B] == 0) return cudaSuccess;
     count_launches(1);
     if (prec == 0) {
-        k_binv64<<<t.off[t.B], 512, 0, st>>>(t);
+        k_binv64<<<t.off[t.B] * kBinv64Cluster, kBinv64Threads, 0, st>>>(t);
     } else {
         const int smem = kBlock * kBlock * sizeof(float2);
         cudaError_t e = cudaFuncSetAttribute(k_binv32, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
