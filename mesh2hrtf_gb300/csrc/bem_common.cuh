@@ -158,15 +158,17 @@ __device__ __forceinline__ F2 vadd(F2 a, F2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
-__device__ __forceinline__ F2 vsub(F2 a, F2 b) {
-    F2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+// A packed constant kept in registers: as an immediate the compiler forms it
+// with two moves at every use.
+__device__ __forceinline__ F2 opaque2(float x) {
+    F2 r = pk2(x, x);
+    asm volatile("" : "+l"(r.v));
     return r;
 }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ double vmul(double a, double b) { return a * b; }
 __device__ __forceinline__ double vadd(double a, double b) { return a + b; }
-__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ double opaque2(double x) { return x; }
 __device__ __forceinline__ void vdup(F2 &r, float x) { r = pk2(x, x); }
 __device__ __forceinline__ void vdup(double &r, double x) { r = x; }
 // 1 / sqrt, and sin and cos of a phase, half by half (phase_sincos's steps)
@@ -176,17 +178,32 @@ __device__ __forceinline__ F2 vrsqrt(F2 a) {
     return pk2(rsqrt_approx(lo), rsqrt_approx(hi));
 }
 __device__ __forceinline__ double vrsqrt(double a) { return rsqrt_nr(a); }
-__device__ __forceinline__ void vsincos(F2 x, F2 &s, F2 &c) {
-    const F2 shift = pk2(12582912.0f, 12582912.0f);
-    const F2 q = vsub(vfma(x, pk2(0.159154943f, 0.159154943f), shift), shift);
-    F2 r = vfma(q, pk2(-6.28318548202514648f, -6.28318548202514648f), x);
-    r = vfma(q, pk2(1.74845553146951e-07f, 1.74845553146951e-07f), r);
+// Constants of phase_sincos in packed form.
+template <typename R> struct ScConst {};
+template <> struct ScConst<F2> {
+    F2 inv2pi, shift, nshift, m2pi, lo2pi;
+    __device__ __forceinline__ void init() {
+        inv2pi = opaque2(0.159154943f);
+        shift = opaque2(12582912.0f);
+        nshift = opaque2(-12582912.0f);
+        m2pi = opaque2(-6.28318548202514648f);
+        lo2pi = opaque2(1.74845553146951e-07f);
+    }
+};
+template <> struct ScConst<double> {
+    __device__ __forceinline__ void init() {}
+};
+__device__ __forceinline__ void vsincos(const ScConst<F2> &k, F2 x, F2 &s, F2 &c) {
+    const F2 q = vadd(vfma(x, k.inv2pi, k.shift), k.nshift);
+    const F2 r = vfma(q, k.lo2pi, vfma(q, k.m2pi, x));
     float lo, hi;
     unpk2(r, lo, hi);
     s = pk2(sin_approx(lo), sin_approx(hi));
     c = pk2(cos_approx(lo), cos_approx(hi));
 }
-__device__ __forceinline__ void vsincos(double x, double &s, double &c) { phase_sincos(x, &s, &c); }
+__device__ __forceinline__ void vsincos(const ScConst<double> &, double x, double &s, double &c) {
+    phase_sincos(x, &s, &c);
+}
 
 __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }

@@ -125,7 +125,7 @@ struct AsmSys {
 struct AsmBatch {
     int B;
     int img;                     // some system's mesh has symmetry images
-    int far_off[kMaxAsm + 1];    // tiles of 32 x 32 entries
+    int far_off[kMaxAsm + 1];    // items of 32 columns x some rows (k_far)
     int near_off[kMaxAsm + 1];   // near pairs
     int rhs_off[kMaxAsm + 1];    // blocks of 8 or 64 rows (k_rhs)
     AsmSys sys[kMaxAsm];
@@ -159,10 +159,10 @@ inline size_t image_table_bytes(int n, int nref) {
 // k_far, at most kFarPerSmMax, and of k_near, at most 2); the results do not
 // depend on them.
 struct AsmShape {
-    int far_per_sm = 3;
+    int far_per_sm = 2;
     int near_per_sm = 2;
 };
-constexpr int kFarPerSmMax = 3;
+constexpr int kFarPerSmMax = 2;
 cudaError_t launch_assemble(const AsmBatch &t, int prec, unsigned *ctr, cudaStream_t st,
                             AsmShape shape = AsmShape());
 

@@ -4,14 +4,14 @@
 // table travels in kernel parameter space (__grid_constant__); a single solve
 // is a batch of one.
 //
-// Regular pairs (k_far): a persistent grid pulls tiles of 32 rows x 32
-// columns from a work queue that spans all systems of the batch; in a tile,
-// each of 8 warps owns 4 rows and each lane one column, so the column
-// element's tables are loaded once per lane and reused for 4 rows, and the
-// entries go out as coalesced row segments.  Pairs that NumCalc subdivides
-// and the self pairs are skipped there and integrated by k_near: warps pull
-// entries of the per-mesh near lists from a second queue and integrate them
-// cooperatively (warp_subdivide / warp_singular).
+// Regular pairs (k_far): the warps of a persistent grid take items of 32
+// columns x 2 .. 16 rows, dealt in turn over all systems of the batch; each
+// lane owns one column, so the column element's tables are loaded once per
+// lane and reused for the rows, and the entries go out as coalesced row
+// segments.  Pairs that NumCalc subdivides and the self pairs are skipped
+// there and integrated by k_near: warps pull entries of the per-mesh near
+// lists from a queue and integrate them cooperatively (warp_subdivide /
+// warp_singular).
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -192,93 +192,166 @@ __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3]
     return make_float2(ar, ai);
 }
 
-// Order-2 far pair on a flat triangle (the 4-point rule) with the column
-// element's data hoisted out of the row loop: point g's squared distance is
-// |D|^2 + 2 s_g D.a + 2 t_g D.b + C_g with C_g = |s_g a + t_g b|^2 (at the
-// order-2 ratio, |D| > 4 sqrt(area), the terms do not cancel), and the
-// kernel terms of fused_point regrouped around u = 1/r.
-struct FarCol4 {
-    float a[3], b[3], n[3];
-    float C[4];    // |s_g a + t_g b|^2
-    float J4;      // J / (4 pi)
+// Order-2 far pairs on a flat triangle (the 4-point rule), two rows at a time
+// in packed FP32, with the column element's data hoisted out of the row loop:
+// point g's squared distance is |D|^2 + 2 s_g D.a + 2 t_g D.b + C_g with
+// C_g = |s_g a + t_g b|^2 (at the order-2 ratio, |D| > 4 sqrt(area), the terms
+// do not cancel).  The distance, the phase and its reduction are rounded
+// operation by operation (the phase's rounding is the entry's error); the
+// kernel terms of fused_point are regrouped around u = 1/r as in far_tri64.
+//
+// Bound by the FMA pipe and the special-function unit together (27 packed and
+// 2 scalar FP32 operations and 6 special functions per two evaluations, and
+// about 45 per pair of entries); one entry at a time it was bound by
+// instruction issue at 79 per evaluation.  20480-triangle head, 10 kHz: k_far
+// 4.07 -> 3.33 ms (1280 triangles 50 us as before, 1536 quadrilaterals and their
+// images 690 -> 673).  Three blocks per SM with the column's data in shared
+// memory instead of two with it in registers: 3.77 ms.
+struct FarCol2 {
+    F2 a[3], b[3], n[3];
+    F2 C[3];       // |s_g a + t_g b|^2 of points 1 .. 3 (point 0 is the centroid)
+    F2 wJ0, wJ1;   // weight J / (4 pi) of point 0 and of the others
 };
+static_assert(sizeof(FarCol2) == 14 * sizeof(F2), "28 registers");
 
-__device__ __forceinline__ void far_col4(const DevMesh &m, int j, FarCol4 &e) {
+__device__ __forceinline__ F2 dup2(float x) { return pk2(x, x); }
+
+// Constants of the packed evaluation, each twice.
+struct FarConst {
+    ScConst<F2> sc;
+    F2 m1, m3;       // -1, -3
+    F2 p, q;         // the 4-point rule's s - 1/3: -2/15 and 4/15
+};
+__device__ __forceinline__ void far_const(FarConst &k) {
+    k.sc.init();
+    k.m1 = opaque2(-1.f);
+    k.m3 = opaque2(-3.f);
+    k.p = opaque2(c_far4[1][0]);
+    k.q = opaque2(c_far4[2][0]);
+}
+
+__device__ __forceinline__ void far_col2(const DevMesh &m, int j, FarCol2 &e) {
+    float a[3], b[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        e.a[k] = m.t32[k * m.n + j];
-        e.b[k] = m.t32[(3 + k) * m.n + j];
-        e.n[k] = m.t32[(6 + k) * m.n + j];
+        a[k] = m.t32[k * m.n + j];
+        b[k] = m.t32[(3 + k) * m.n + j];
+        vdup(e.a[k], a[k]);
+        vdup(e.b[k], b[k]);
+        vdup(e.n[k], m.t32[(6 + k) * m.n + j]);
     }
-    const float J = m.t32[9 * m.n + j];
+    const float J4 = m.t32[9 * m.n + j] * (float)(1.0 / kPI4);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
+    for (int g = 1; g < 4; ++g) {
         float c = 0.f;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float d = fmaf(c_far4[g][1], e.b[k], c_far4[g][0] * e.a[k]);
+            const float d = fmaf(c_far4[g][1], b[k], c_far4[g][0] * a[k]);
             c = fmaf(d, d, c);
         }
-        e.C[g] = c;
+        vdup(e.C[g - 1], c);
     }
-    e.J4 = J * (float)(1.0 / kPI4);
+    vdup(e.wJ0, c_trif[0][2] * J4);
+    vdup(e.wJ1, c_trif[1][2] * J4);
 }
 
-// BC: the column's boundary condition (0 velocity, 1 pressure, 2 velocity
-// with admittance), fixed per instantiation so the point loop has no branch
+// Constants of a column, each twice.
+struct FusedCol2 {
+    F2 wr, b, bwr, k2, nt, tw;    // wr, beta / i, b wr, k^2, -tau, tau wr
+    F2 yr, yi, nyi, bt, btw;      // admittance, -its imaginary part, b tau, b tau wr (BC 2)
+};
+// Sums of an entry pair: cos F_re, sin F_im (apart, so that no negation is
+// needed) and the imaginary part.
+struct FarSum2 { F2 rr, ri, ai; };
+
+__device__ __forceinline__ F2 dot2(const F2 x[3], const F2 y[3]) {
+    return vfma(x[2], y[2], vfma(x[0], y[0], vmul(x[1], y[1])));
+}
+
+// One quadrature point of two entries: squared distance, d.n_y, d.n_x, n_x.n_y,
+// weight / (4 pi).  BC: the column's boundary condition (0 velocity, 1
+// pressure, 2 velocity with admittance), fixed per instantiation so that the
+// point has no branch.
 template <int BC>
-__device__ __forceinline__ float2 far_entry_tri2_bc(const FarCol4 &e, const float D[3], float D2, const float nx[3],
-                                                    const FusedCol &c) {
-    const float dny = D[0] * e.n[0] + D[1] * e.n[1] + D[2] * e.n[2];
-    const float dnx0 = D[0] * nx[0] + D[1] * nx[1] + D[2] * nx[2];
-    const float anx = e.a[0] * nx[0] + e.a[1] * nx[1] + e.a[2] * nx[2];
-    const float bnx = e.b[0] * nx[0] + e.b[1] * nx[1] + e.b[2] * nx[2];
-    const float nn = e.n[0] * nx[0] + e.n[1] * nx[1] + e.n[2] * nx[2];
-    const float Da = D[0] * e.a[0] + D[1] * e.a[1] + D[2] * e.a[2];
-    const float Db = D[0] * e.b[0] + D[1] * e.b[1] + D[2] * e.b[2];
-    const float ct = -c.tau * dny;          // velocity: -tau d.n_y / r^2
-    const float cw = c.tau * c.wr * dny;    // velocity: tau wr d.n_y / r
-    const float bwr = c.b * c.wr;
-    float ar = 0.f, ai = 0.f;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const float r2 = fmaf(c_far4[g][2], Da, fmaf(c_far4[g][3], Db, D2 + e.C[g]));
-        const float dnx = fmaf(c_far4[g][1], bnx, fmaf(c_far4[g][0], anx, dnx0));
-        const float u = rsqrt_approx(r2);
-        float sn, cs;
-        phase_sincos(c.wr * (r2 * u), &sn, &cs);
-        float fr, fi;
-        if (BC == 1) {
-            // -tau - i b z1 re2, z1 = -1/r + i wr, re2 = -d.n_x / r
-            const float du = dnx * u;
-            fr = fmaf(-bwr, du, -c.tau);
-            fi = -c.b * du * u;
-        } else {
-            // tau z1 re1 + i b ze1 (re1 = d.n_y / r)
-            const float u2 = u * u;
-            const float rq = -(dny * dnx) * u2;
-            fr = fmaf(bwr * u, fmaf(3.f, rq, nn), ct * u2);
-            fi = fmaf(c.b, fmaf(fmaf(3.f, u2, -c.k2), rq, nn * u2), cw * u);
-            if (BC == 2) {
-                // + Y (1 + i b tau z1 re2)
-                const float du = dnx * u, bt = c.b * c.tau;
-                const float pr = fmaf(bt * c.wr, du, 1.f), pi = bt * u * du;
-                fr += c.yr * pr - c.yi * pi;
-                fi += c.yr * pi + c.yi * pr;
-            }
+__device__ __forceinline__ void far_point2(const FarConst &k, const FusedCol2 &c, F2 r2, F2 dny, F2 dnx, F2 nn, F2 wj,
+                                           FarSum2 &o) {
+    const F2 u = vrsqrt(r2), r = vmul(r2, u);
+    F2 sn, cs, fr, fi, amp;
+    vsincos(k.sc, vmul(c.wr, r), sn, cs);
+    if (BC == 1) {
+        // -tau - i b z1 re2, z1 = -1/r + i wr, re2 = -d.n_x / r
+        const F2 ndu = vmul(vmul(dnx, u), k.m1);
+        fr = vfma(c.bwr, ndu, c.nt);
+        fi = vmul(vmul(c.b, ndu), u);
+        amp = vmul(wj, u);
+    } else {
+        // tau z1 re1 + i b ze1 (re1 = d.n_y / r), times r
+        const F2 P = vmul(dny, dnx), u2 = vmul(u, u);
+        const F2 E = vfma(vmul(P, u2), k.m3, nn);   // n_x.n_y - 3 P / r^2
+        fr = vfma(c.bwr, E, vmul(vmul(c.nt, dny), u));
+        fi = vfma(vmul(c.b, u), vfma(c.k2, P, E), vmul(c.tw, dny));
+        amp = vmul(wj, u2);
+        if (BC == 2) {
+            // + Y (1 + i b tau z1 re2), times r
+            const F2 pr = vfma(c.btw, dnx, r), pi = vmul(vmul(c.bt, u), dnx);
+            fr = vfma(c.yr, pr, vfma(c.nyi, pi, fr));
+            fi = vfma(c.yr, pi, vfma(c.yi, pr, fi));
         }
-        const float amp = c_trif[g][2] * e.J4 * u;
-        ar = fmaf(amp, fmaf(cs, fr, -sn * fi), ar);
-        ai = fmaf(amp, fmaf(cs, fi, sn * fr), ai);
     }
-    return make_float2(ar, ai);
+    const F2 qr = vmul(amp, fr), qi = vmul(amp, fi);
+    o.rr = vfma(cs, qr, o.rr);
+    o.ri = vfma(sn, qi, o.ri);
+    o.ai = vfma(cs, qi, vfma(sn, qr, o.ai));
 }
 
-__device__ __forceinline__ float2 far_entry_tri2(const FarCol4 &e, const float D[3], float D2, const float nx[3],
-                                                 const FusedCol &c) {
-    if (c.bc == 0) return far_entry_tri2_bc<0>(e, D, D2, nx, c);
-    if (c.bc == 1) return far_entry_tri2_bc<1>(e, D, D2, nx, c);
-    return far_entry_tri2_bc<2>(e, D, D2, nx, c);
+template <int BC>
+__device__ __forceinline__ void far_tri2(const FarConst &k, const FarCol2 &e, const F2 D[3], F2 D2, const F2 nx[3],
+                                         const FusedCol2 &c, FarSum2 &o) {
+    const F2 dny = dot2(D, e.n), dnx = dot2(D, nx), nn = dot2(e.n, nx);
+    const F2 anx = dot2(e.a, nx), bnx = dot2(e.b, nx);
+    F2 Da = dot2(D, e.a), Db = dot2(D, e.b);
+    Da = vadd(Da, Da);   // exact: 2 s D.a = s (2 D.a)
+    Db = vadd(Db, Db);
+    far_point2<BC>(k, c, D2, dny, dnx, nn, e.wJ0, o);
+    far_point2<BC>(k, c, vfma(k.p, Da, vfma(k.p, Db, vadd(D2, e.C[0]))), dny, vfma(k.p, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
+    far_point2<BC>(k, c, vfma(k.q, Da, vfma(k.p, Db, vadd(D2, e.C[1]))), dny, vfma(k.p, bnx, vfma(k.q, anx, dnx)), nn, e.wJ1, o);
+    far_point2<BC>(k, c, vfma(k.p, Da, vfma(k.q, Db, vadd(D2, e.C[2]))), dny, vfma(k.q, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
+}
+
+// The same for a quadrilateral column, whose four points (offset from the
+// centre, normal, weight) were mapped once by far_quad_stage into the lane's
+// column of shared memory.
+constexpr int kQuadRows = 28;
+__device__ __forceinline__ void far_quad_stage(const DevMesh &m, int j, float (*st)[32], int lane) {
+    Elem32 e;
+    const float zero[3] = {0.f, 0.f, 0.f};
+    load_elem32(m, j, zero, zero, e);
+    e.D[0] = e.D[1] = e.D[2] = 0.f;
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) {
+        QPoint<float> q;
+        map_point(e, c_glxf[2][g >> 1], c_glxf[2][g & 1], c_glwf[2][g >> 1] * c_glwf[2][g & 1], q);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            st[7 * g + k][lane] = q.d[k];
+            st[7 * g + 3 + k][lane] = q.ny[k];
+        }
+        st[7 * g + 6][lane] = q.wj * (float)(1.0 / kPI4);
+    }
+}
+template <int BC>
+__device__ __forceinline__ void far_quad2(const FarConst &k, float (*st)[32], int lane, const F2 D[3], const F2 nx[3],
+                                          const FusedCol2 &c, FarSum2 &o) {
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) {
+        F2 d[3], ny[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            d[q] = vadd(D[q], dup2(st[7 * g + q][lane]));
+            ny[q] = dup2(st[7 * g + 3 + q][lane]);
+        }
+        far_point2<BC>(k, c, dot2(d, d), dot2(d, ny), dot2(d, nx), dot2(ny, nx), dup2(st[7 * g + 6][lane]), o);
+    }
 }
 
 // FP64 regular pair on a flat triangle, arranged for the fewest FP64
@@ -556,27 +629,35 @@ __global__ void __launch_bounds__(256) k_near_list(DevMeshView mv, const float4 
 }
 
 // ------------------------------------------------------------ regular pairs
-// Regular (not subdivided) pairs: block of 8 warps, every warp 4 rows x 32
-// columns, one column per lane.  The column element is loaded once per lane
-// and reused for its 4 rows; entries go out as coalesced row segments.  Near
-// and self pairs are skipped here and written by k_near.
-constexpr int kRowsPerThread = 4;
+// Regular (not subdivided) pairs: a warp takes 32 columns, one per lane, and
+// some rows.  The column element is loaded once per lane and reused for its
+// rows; entries go out as coalesced row segments.  Near and self pairs are
+// zero here; k_near adds their integrals.
+//
+// Rows per item (an item is one warp's 32 columns x far_rows rows): the more,
+// the further the column's preparation is spread; small systems take fewer so
+// that the 2432 warps of the grid get about six items or more each (with one
+// or two the last round would leave most of them idle).
+__host__ __device__ inline int far_rows(int n) {
+    const long long e = (long long)n * n / (32 * 6 * 2432);   // rows for six items per warp
+    return e >= 16 ? 16 : e >= 8 ? 8 : e >= 4 ? 4 : 2;
+}
 
 // Out-of-line parts of the float tile, taken by few pairs: keeping them out
 // of the row loop keeps the mesh pointers they read out of its registers.
 // Exact (FP64) decision for a pair within the float test's margin of a
 // threshold: 0 for a near pair, else the Gauss order.
-__device__ __noinline__ int far_order_exact(const DevMeshView *mv, int i, int j) {
+__device__ __noinline__ int far_order_exact(const DevMeshView *mv, int kref, int i, int j) {
     const DevMesh m = to_dev(*mv);
     const int n = m.n;
     const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
-    const double rd = ratio0_exact(m, j, x64);
+    const double rd = ratio0_exact(image_mesh(m, kref), j, x64);
     return rd < kTolf ? 0 : gauss_order(rd);
 }
 // Entry of a quadrilateral column or of a Gauss order above 2.
-__device__ __noinline__ float2 far_entry_general(const DevMeshView *mv, int j, float D0, float D1, float D2,
+__device__ __noinline__ float2 far_entry_general(const DevMeshView *mv, int kref, int j, float D0, float D1, float D2,
                                                  float nx0, float nx1, float nx2, int order, FusedCol fc) {
-    const DevMesh m = to_dev(*mv);
+    const DevMesh m = image_mesh(to_dev(*mv), kref);
     Elem32 e;
     const float zero[3] = {0.f, 0.f, 0.f};
     load_elem32(m, j, zero, zero, e);
@@ -585,33 +666,52 @@ __device__ __noinline__ float2 far_entry_general(const DevMeshView *mv, int j, f
     return far_entry_f(e, nx, order, fc);
 }
 
+// One warp's item of image kref of the columns: rows from i0, column block tx.
+// st: the warp's shared memory for quadrilateral columns.
+// kref = 0 writes the entries; the images add theirs (reflection factor
+// applied, NC_AssembleTBEM, NC_EquationSystem.cpp:181-206) in image order.
+// Near images and the self pair contribute zero here; k_near adds them.
 template <typename T>
 __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f,
-                                         typename Vec2<T>::type *__restrict__ A, size_t lda, int tx, int ty) {
+                                         typename Vec2<T>::type *__restrict__ A, size_t lda, int tx, int i0, int kref,
+                                         const FarConst &fk, float (*st)[32]) {
     const DevMesh m = to_dev(mv);
-    const int lane = threadIdx.x, n = m.n;
-    const int i0 = (ty * 8 + threadIdx.y) * kRowsPerThread;
+    const DevMesh mk = image_mesh(m, kref);
+    const int lane = threadIdx.x, n = m.n, rpt = far_rows(n);
     const int j = tx * 32 + lane;
-    if (i0 >= n || j >= n) return;
+    if (j >= n) return;
     Phys<T> PT;
     if constexpr (std::is_same<T, double>::value) PT = {f.k, f.wr, f.tao, f.beta_im};
     else PT = {f.kf, f.wrf, f.taof, f.beta_imf};
     const int bcj = f.bc_type ? f.bc_type[j] : 0;
     const cplx<T> admj = col_adm<T>(f, j, bcj);
+    const bool neg = image_negated(m, kref);
+    const bool tri = m.nvert[j] == 3;
+    const float cjh[3] = {mk.chi[j], mk.chi[n + j], mk.chi[2 * n + j]};
+    const float cjl[3] = {mk.clo[j], mk.clo[n + j], mk.clo[2 * n + j]};
+    const float isq2 = m.isqa32[j] * m.isqa32[j];
+    auto put = [&](int i, T re, T im) {
+        typename Vec2<T>::type *p = A + (size_t)i * lda + j, o;
+        if (kref > 0) {
+            o = *p;
+            o.x += neg ? -re : re;
+            o.y += neg ? -im : im;
+        } else {
+            o.x = re;
+            o.y = im;
+        }
+        *p = o;
+    };
     if constexpr (std::is_same<T, double>::value) {
-        const bool tri = m.nvert[j] == 3;
         FarCol64 e4;
-        if (tri) far_col64(m, j, e4);
-        const float cjh[3] = {m.chi[j], m.chi[n + j], m.chi[2 * n + j]};
-        const float cjl[3] = {m.clo[j], m.clo[n + j], m.clo[2 * n + j]};
-        const float isq2 = m.isqa32[j] * m.isqa32[j];
+        if (tri) far_col64(mk, j, e4);
         const FusedCol64 fc = {admj.re, admj.im, f.tao, f.beta_im, f.k * f.k, f.wr};
 #pragma unroll 1
-        for (int r = 0; r < kRowsPerThread; ++r) {
+        for (int r = 0; r < rpt; ++r) {
             const int i = i0 + r;
             if (i >= n) break;
-            cplx<double> val = {0.0, 0.0};   // near and self entries: k_near adds their integrals
-            if (i != j) {
+            cplx<double> val = {0.0, 0.0};
+            if (i != j || kref > 0) {
                 // the quadrature decision from the float distance, the exact
                 // FP64 one (a square root and a division) only near a threshold
                 const float4 rh = m.row4[3 * (size_t)i], rl = m.row4[3 * (size_t)i + 1];
@@ -621,7 +721,7 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
                 bool near = false;
                 int order = 2;
                 if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
-                    order = far_order_exact(&mv, i, j);
+                    order = far_order_exact(&mv, kref, i, j);
                     near = order == 0;
                 }
                 if (!near) {
@@ -631,20 +731,17 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
                         val = far_entry_tri64(e4, x64, nx64, order, bcj, fc);
                     } else {
                         Elem64 e;
-                        load_elem64(m, j, e);
+                        load_elem64(mk, j, e);
                         val = combine_entry(FarPair<double>::run(e, x64, nx64, order, f.k, f.wr), bcj, admj, PT);
                     }
                 }
             }
-            A[(size_t)i * lda + j] = make_double2(val.re, val.im);
+            put(i, val.re, val.im);
         }
     } else {
-        const bool tri = m.nvert[j] == 3;
-        FarCol4 e4;
-        if (tri) far_col4(m, j, e4);
-        const float cjh[3] = {m.chi[j], m.chi[n + j], m.chi[2 * n + j]};
-        const float cjl[3] = {m.clo[j], m.clo[n + j], m.clo[2 * n + j]};
-        const float isq2 = m.isqa32[j] * m.isqa32[j];
+        FarCol2 e2;
+        if (tri) far_col2(mk, j, e2);
+        else far_quad_stage(mk, j, st, lane);
         FusedCol fc;
         fc.bc = bcj;
         fc.yr = admj.re;
@@ -653,150 +750,95 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
         fc.b = PT.beta_im;
         fc.k2 = PT.k * PT.k;
         fc.wr = PT.wr;
-        #pragma unroll 1
-        for (int r = 0; r < kRowsPerThread; ++r) {
+        const FusedCol2 f2 = {dup2(fc.wr), dup2(fc.b), dup2(fc.b * fc.wr), dup2(fc.k2), dup2(-fc.tau),
+                              dup2(fc.tau * fc.wr), dup2(fc.yr), dup2(fc.yi), dup2(-fc.yi), dup2(fc.b * fc.tau),
+                              dup2(fc.b * fc.tau * fc.wr)};
+#pragma unroll 1
+        for (int r = 0; r < rpt; r += 2) {
             const int i = i0 + r;
             if (i >= n) break;
-            if (i == j) { A[(size_t)i * lda + j] = make_float2(0.f, 0.f); continue; }
-            // the row's data (the same for the warp's 32 columns)
-            const float4 rh = m.row4[3 * (size_t)i], rl = m.row4[3 * (size_t)i + 1], rn = m.row4[3 * (size_t)i + 2];
-            const float D[3] = {(cjh[0] - rh.x) + (cjl[0] - rl.x), (cjh[1] - rh.y) + (cjl[1] - rl.y),
-                                (cjh[2] - rh.z) + (cjl[2] - rl.z)};
-            const float D2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2];
-            const float q2 = D2 * isq2;
-            bool near = false;
-            int order = 2;
-            if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
-                order = far_order_exact(&mv, i, j);
-                near = order == 0;
-            }
-            if (near) { A[(size_t)i * lda + j] = make_float2(0.f, 0.f); continue; }
-            const float nx[3] = {rn.x, rn.y, rn.z};
-            if (tri && order <= 2)
-                A[(size_t)i * lda + j] = far_entry_tri2(e4, D, D2, nx, fc);
-            else
-                A[(size_t)i * lda + j] = far_entry_general(&mv, j, D[0], D[1], D[2], nx[0], nx[1], nx[2], order, fc);
-        }
-    }
-}
-
-// The same tile for a mesh with symmetry images: every entry sums the far
-// images of its column element (reflection factor applied, NC_AssembleTBEM,
-// NC_EquationSystem.cpp:181-206), in image order; near images and the self
-// pair are left to k_near, which adds them to the entry.
-template <typename T>
-__device__ __forceinline__ void far_tile_img(const DevMeshView &mv, const DevFreq &f,
-                                             typename Vec2<T>::type *__restrict__ A, size_t lda, int tx, int ty) {
-    const DevMesh m = to_dev(mv);
-    const int lane = threadIdx.x, n = m.n;
-    const int i0 = (ty * 8 + threadIdx.y) * kRowsPerThread;
-    const int j = tx * 32 + lane;
-    if (i0 >= n || j >= n) return;
-    Phys<T> PT;
-    if constexpr (std::is_same<T, double>::value) PT = {f.k, f.wr, f.tao, f.beta_im};
-    else PT = {f.kf, f.wrf, f.taof, f.beta_imf};
-    const int bcj = f.bc_type ? f.bc_type[j] : 0;
-    const cplx<T> admj = col_adm<T>(f, j, bcj);
-    T acc_re[kRowsPerThread], acc_im[kRowsPerThread];
-    for (int r = 0; r < kRowsPerThread; ++r) acc_re[r] = acc_im[r] = T(0);
-    for (int kref = 0; kref < m.sym.nref; ++kref) {
-        const DevMesh mk = image_mesh(m, kref);
-        const T sg = image_negated(m, kref) ? T(-1) : T(1);
-        if constexpr (std::is_same<T, double>::value) {
-            const bool tri = m.nvert[j] == 3;
-            FarCol64 e4;
-            Elem64 e;
-            if (tri) far_col64(mk, j, e4);
-            else load_elem64(mk, j, e);
-            const FusedCol64 fc = {admj.re, admj.im, f.tao, f.beta_im, f.k * f.k, f.wr};
-            for (int r = 0; r < kRowsPerThread; ++r) {
-                const int i = i0 + r;
-                if (i >= n) break;
-                if (kref == 0 && i == j) continue;
-                const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
-                const double rd = ratio0_exact(mk, j, x64);
-                if (rd < kTolf) continue;
-                const double nx64[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
-                const int order = gauss_order(rd);
-                const cplx<double> val =
-                    tri ? far_entry_tri64(e4, x64, nx64, order, bcj, fc)
-                        : combine_entry(FarPair<double>::run(e, x64, nx64, order, f.k, f.wr), bcj, admj, PT);
-                acc_re[r] += sg * val.re;
-                acc_im[r] += sg * val.im;
-            }
-        } else {
-            Elem32 e;
-            const float zero[3] = {0.f, 0.f, 0.f};
-            load_elem32(mk, j, zero, zero, e);
-            const float cjh[3] = {mk.chi[j], mk.chi[n + j], mk.chi[2 * n + j]};
-            const float cjl[3] = {mk.clo[j], mk.clo[n + j], mk.clo[2 * n + j]};
-            const float isq2 = m.isqa32[j] * m.isqa32[j];
-            FusedCol fc;
-            fc.bc = bcj;
-            fc.yr = admj.re;
-            fc.yi = admj.im;
-            fc.tau = PT.tao;
-            fc.b = PT.beta_im;
-            fc.k2 = PT.k * PT.k;
-            fc.wr = PT.wr;
-            for (int r = 0; r < kRowsPerThread; ++r) {
-                const int i = i0 + r;
-                if (i >= n) break;
-                if (kref == 0 && i == j) continue;
-                for (int k = 0; k < 3; ++k) e.D[k] = (cjh[k] - m.chi[k * n + i]) + (cjl[k] - m.clo[k * n + i]);
-                const float q2 = (e.D[0] * e.D[0] + e.D[1] * e.D[1] + e.D[2] * e.D[2]) * isq2;
-                bool near = false;
-                int order = 2;
-                if (q2 <= c_quad.far2_sq && !classify_fast(sqrtf(q2), near, order)) {
-                    const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
-                    const double rd = ratio0_exact(mk, j, x64);
-                    near = rd < kTolf;
-                    if (!near) order = gauss_order(rd);
+            // the two rows' data (the same for the warp's 32 columns)
+            const float4 *row = m.row4 + 3 * (size_t)i, *row1 = i + 1 < n ? row + 3 : row;
+            const float4 h0 = row[0], l0 = row[1], n0 = row[2], h1 = row1[0], l1 = row1[1], n1 = row1[2];
+            const F2 D[3] = {vadd(vfma(pk2(h0.x, h1.x), fk.m1, dup2(cjh[0])), vfma(pk2(l0.x, l1.x), fk.m1, dup2(cjl[0]))),
+                             vadd(vfma(pk2(h0.y, h1.y), fk.m1, dup2(cjh[1])), vfma(pk2(l0.y, l1.y), fk.m1, dup2(cjl[1]))),
+                             vadd(vfma(pk2(h0.z, h1.z), fk.m1, dup2(cjh[2])), vfma(pk2(l0.z, l1.z), fk.m1, dup2(cjl[2])))};
+            const F2 D2 = vfma(D[2], D[2], vfma(D[0], D[0], vmul(D[1], D[1])));
+            const F2 nx[3] = {pk2(n0.x, n1.x), pk2(n0.y, n1.y), pk2(n0.z, n1.z)};
+            float q2[2];
+            unpk2(vmul(D2, dup2(isq2)), q2[0], q2[1]);
+            // quadrature orders; 0: near or self
+            int ord[2] = {2, 2};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (q2[h] <= c_quad.far2_sq) {
+                    bool near = false;
+                    if (i + h == j && kref == 0) near = true;
+                    else if (!classify_fast(sqrtf(q2[h]), near, ord[h])) {
+                        ord[h] = far_order_exact(&mv, kref, i + h < n ? i + h : i, j);
+                        near = ord[h] == 0;
+                    }
+                    if (near) ord[h] = 0;
                 }
-                if (near) continue;
-                const float nx[3] = {m.n32[i], m.n32[n + i], m.n32[2 * n + i]};
-                const float2 v = far_entry_f(e, nx, order, fc);
-                acc_re[r] += sg * v.x;
-                acc_im[r] += sg * v.y;
             }
+            FarSum2 o = {dup2(0.f), dup2(0.f), dup2(0.f)};
+            if (ord[0] == 2 || ord[1] == 2) {
+                if (tri) {
+                    if (bcj == 0) far_tri2<0>(fk, e2, D, D2, nx, f2, o);
+                    else if (bcj == 1) far_tri2<1>(fk, e2, D, D2, nx, f2, o);
+                    else far_tri2<2>(fk, e2, D, D2, nx, f2, o);
+                } else {
+                    if (bcj == 0) far_quad2<0>(fk, st, lane, D, nx, f2, o);
+                    else if (bcj == 1) far_quad2<1>(fk, st, lane, D, nx, f2, o);
+                    else far_quad2<2>(fk, st, lane, D, nx, f2, o);
+                }
+            }
+            float er[2], ei[2], d[3][2];
+            unpk2(vfma(o.ri, fk.m1, o.rr), er[0], er[1]);
+            unpk2(o.ai, ei[0], ei[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (ord[h] == 0) er[h] = ei[h] = 0.f;
+                else if (ord[h] > 2) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) unpk2(D[c], d[c][0], d[c][1]);
+                    const float2 v = far_entry_general(&mv, kref, j, d[0][h], d[1][h], d[2][h], h ? n1.x : n0.x,
+                                                       h ? n1.y : n0.y, h ? n1.z : n0.z, ord[h], fc);
+                    er[h] = v.x;
+                    ei[h] = v.y;
+                }
+            }
+            put(i, er[0], ei[0]);
+            if (i + 1 < n) put(i + 1, er[1], ei[1]);
         }
-    }
-    for (int r = 0; r < kRowsPerThread; ++r) {
-        const int i = i0 + r;
-        if (i >= n) break;
-        typename Vec2<T>::type o;
-        o.x = acc_re[r];
-        o.y = acc_im[r];
-        A[(size_t)i * lda + j] = o;
     }
 }
 
 constexpr int kRhsRows = 64;   // k_rhs without boundary columns: rows per block, a thread each
 constexpr int kFarPerSm = kFarPerSmMax;   // resident k_far blocks per SM allowed by the launch bounds
 
+// The grid's warps take the items in turn.  A queue of eight-warp tiles in place
+// of that: 20480 triangles 3.23 against 3.33 ms, but 66 against 50 us at 1280,
+// where its last tiles leave most SMs idle.
 // ONE: the batch holds a single system, whose table then stays in constant
 // operands instead of registers.  IMG: some mesh of the batch has symmetry
-// images (meshes without take the plain tile).
+// images.
 template <typename T, bool ONE, bool IMG>
-__global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 2 : kFarPerSm) k_far(const __grid_constant__ AsmBatch tb, unsigned *ctr) {
-    __shared__ int item_s;
+__global__ void __launch_bounds__(256, kFarPerSm) k_far(const __grid_constant__ AsmBatch tb) {
+    __shared__ float st[std::is_same<T, float>::value ? 8 : 1][kQuadRows][32];
     const int total = tb.far_off[tb.B];
-    while (true) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) item_s = (int)atomicAdd(ctr, 1u);
-        __syncthreads();
-        const int item = item_s;
-        __syncthreads();
-        if (item >= total) break;
+    FarConst fk;
+    if constexpr (std::is_same<T, float>::value) far_const(fk);
+    for (int item = blockIdx.x * 8 + threadIdx.y; item < total; item += gridDim.x * 8) {
         const int b = ONE ? 0 : find_sys(tb.far_off, tb.B, item);
         const AsmSys &S = tb.sys[ONE ? 0 : b];
         const int local = item - tb.far_off[b];
         const int ntx = (S.m.n + 31) / 32;
-        if (IMG && S.m.sym.nref > 1)
-            far_tile_img<T>(S.m, S.f, (typename Vec2<T>::type *)S.A, S.lda, local % ntx, local / ntx);
-        else
-            far_tile<T>(S.m, S.f, (typename Vec2<T>::type *)S.A, S.lda, local % ntx, local / ntx);
+        const int nref = IMG ? S.m.sym.nref : 1;
+        for (int kref = 0; kref < nref; ++kref)
+            far_tile<T>(S.m, S.f, (typename Vec2<T>::type *)S.A, S.lda, local % ntx, local / ntx * far_rows(S.m.n), kref,
+                        fk, st[std::is_same<T, float>::value ? threadIdx.y : 0]);
     }
-    queue_exit(ctr);
 }
 
 // ------------------------------------------------------------ near pairs
@@ -1450,9 +1492,9 @@ template <> struct ProjLane<double> { using R = double; static constexpr int kP 
 // A staged element.  v[0..2] centre (float: high parts, v[3..5] low parts);
 // triangles: 6 a, 9 b, 12 n; quadrilaterals, per point g: 6 + 3 g offset (FP64:
 // position), 18 + 3 g normal, 30 + g weight.  Per right-hand side W (re, im,
-// -im) and, where some right-hand side has nodal velocities, V of the points.
+// -im, -re) and, where some right-hand side has nodal velocities, V of the points.
 template <typename T, int NR> struct ProjElem {
-    typename ProjLane<T>::R v[34], W[NR][3], V[NR][4][3];
+    typename ProjLane<T>::R v[34], W[NR][4], V[NR][4][3];
     float hi[3], lo[3], isq2;
     int nv, iv;
 };
@@ -1541,7 +1583,10 @@ __device__ void proj_stage(const ProjSys *sys, int nr, const DevMesh &m, const D
         cplx<T> ph, vl[4];
         proj_elem_data<T>((const double2 *)S.phi, (const double2 *)S.vel, (const float2 *)S.phi32,
                           (const float2 *)S.vel32, n, j, nv, iv, kref, neg, ph, vl);
-        if (g == 0) proj_put<T>(o.W[r], ph * fac);
+        if (g == 0) {
+            proj_put<T>(o.W[r], ph * fac);
+            vdup(o.W[r][3], -(ph.re * fac));
+        }
         if (any) {
             cplx<T> z = {T(0), T(0)};
             for (int a = 0; a < 4; ++a) z += vl[a] * sh[a];
@@ -1558,6 +1603,7 @@ template <typename T, int NR, bool TRI, bool VEL>
 __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const typename ProjLane<T>::R (&D)[3],
                                          unsigned mask, typename ProjLane<T>::R wr, typename ProjLane<T>::R nwr,
                                          typename ProjLane<T>::R k2, typename ProjLane<T>::R m3,
+                                         const ScConst<typename ProjLane<T>::R> &sc,
                                          RAcc<typename ProjLane<T>::R> (&acc)[NR]) {
     using R = typename ProjLane<T>::R;
     R dny, Tr, Ti, P0r, P0i, G0r[3], G0i[3];
@@ -1592,7 +1638,7 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
         }
         const R r2 = vfma(d[2], d[2], vfma(d[0], d[0], vmul(d[1], d[1])));
         R u = vrsqrt(r2), sn, cs;
-        vsincos(vmul(wr, vmul(r2, u)), sn, cs);
+        vsincos(sc, vmul(wr, vmul(r2, u)), sn, cs);
         if constexpr (std::is_same<T, float>::value) {
             float lo, hi;
             unpk2(u, lo, hi);
@@ -1614,8 +1660,8 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
             Tr = vadd(Tr, hr);
             Ti = vadd(Ti, hi);
         } else {
-            P0r = vsub(P0r, vmul(dny, hr));
-            P0i = vsub(P0i, vmul(dny, hi));
+            P0r = vfma(dny, hr, P0r);   // -P0 until the end
+            P0i = vfma(dny, hi, P0i);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 G0r[k] = vfma(hr, e.v[18 + 3 * g + k], G0r[k]);
@@ -1639,8 +1685,8 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
         }
     }
     if (TRI) {
-        P0r = vsub(P0r, vmul(dny, Tr));
-        P0i = vsub(P0i, vmul(dny, Ti));
+        P0r = vmul(dny, Tr);
+        P0i = vmul(dny, Ti);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             G0r[k] = vfma(Tr, e.v[12 + k], G0r[k]);
@@ -1650,9 +1696,9 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
         if (r >= nr) break;
-        const R Wr = e.W[r][0], Wi = e.W[r][1], nWi = e.W[r][2];
-        acc[r].pr = vfma(Wr, P0r, vfma(nWi, P0i, acc[r].pr));
-        acc[r].pi = vfma(Wr, P0i, vfma(Wi, P0r, acc[r].pi));
+        const R Wr = e.W[r][0], Wi = e.W[r][1], nWi = e.W[r][2], nWr = e.W[r][3];
+        acc[r].pr = vfma(nWr, P0r, vfma(Wi, P0i, acc[r].pr));
+        acc[r].pi = vfma(nWr, P0i, vfma(nWi, P0r, acc[r].pi));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             acc[r].gr[k] = vfma(Wr, G0r[k], vfma(nWi, G0i[k], acc[r].gr[k]));
@@ -1788,7 +1834,7 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
     // and GB300 issues those conversions on its narrow FP64 pipe.  Idle
     // points repeat the group's first.
     float xh[P][3], xl[P][3];
-    R X[6];   // float: packed high and low parts; FP64: the point
+    R X[6];   // float: packed high and low parts, negated; FP64: the point
 #pragma unroll
     for (int h = 0; h < P; ++h) {
         const int p = p0 + 32 * h < npts ? p0 + 32 * h : (group ? p0 - lane : 0);
@@ -1804,8 +1850,8 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
     if constexpr (P == 2) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            X[c] = pk2(xh[0][c], xh[P - 1][c]);
-            X[3 + c] = pk2(xl[0][c], xl[P - 1][c]);
+            X[c] = pk2(-xh[0][c], -xh[P - 1][c]);
+            X[3 + c] = pk2(-xl[0][c], -xl[P - 1][c]);
         }
     }
     T k = (T)f.k, wrs = (T)f.wr;
@@ -1814,7 +1860,9 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
     vdup(wr, wrs);
     vdup(nwr, -wrs);
     vdup(k2, k * k);
-    vdup(m3, T(-3));
+    m3 = opaque2(T(-3));
+    ScConst<R> sc;
+    sc.init();
     RAcc<R> acc[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
@@ -1843,7 +1891,7 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
                 float q2[P];
                 if constexpr (P == 2) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) D[c] = vadd(vsub(e.v[c], X[c]), vsub(e.v[3 + c], X[3 + c]));
+                    for (int c = 0; c < 3; ++c) D[c] = vadd(vadd(e.v[c], X[c]), vadd(e.v[3 + c], X[3 + c]));   // X holds -x
                     const F2 d2 = vfma(D[2], D[2], vfma(D[0], D[0], vmul(D[1], D[1])));
                     unpk2(vmul(d2, pk2(e.isq2, e.isq2)), q2[0], q2[P - 1]);
                 } else {
@@ -1875,11 +1923,11 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
                 }
                 if (__any_sync(0xffffffffu, far != 0)) {
                     if (tri) {
-                        if (!e.iv) proj_far<T, NR, true, false>(e, nr, D, far, wr, nwr, k2, m3, acc);
-                        else proj_far<T, NR, true, true>(e, nr, D, far, wr, nwr, k2, m3, acc);
+                        if (!e.iv) proj_far<T, NR, true, false>(e, nr, D, far, wr, nwr, k2, m3, sc, acc);
+                        else proj_far<T, NR, true, true>(e, nr, D, far, wr, nwr, k2, m3, sc, acc);
                     } else {
-                        if (!e.iv) proj_far<T, NR, false, false>(e, nr, D, far, wr, nwr, k2, m3, acc);
-                        else proj_far<T, NR, false, true>(e, nr, D, far, wr, nwr, k2, m3, acc);
+                        if (!e.iv) proj_far<T, NR, false, false>(e, nr, D, far, wr, nwr, k2, m3, sc, acc);
+                        else proj_far<T, NR, false, true>(e, nr, D, far, wr, nwr, k2, m3, sc, acc);
                     }
                 }
                 if (__all_sync(0xffffffffu, far == (1u << P) - 1u)) continue;
@@ -2189,7 +2237,7 @@ void asm_batch_finish(AsmBatch &t) {
         if (t.sys[b].m.sym.nref > 1) t.img = 1;
         const int n = t.sys[b].m.n;
         const int nt = (n + 31) / 32;
-        t.far_off[b + 1] = t.far_off[b] + nt * ((n + 8 * kRowsPerThread - 1) / (8 * kRowsPerThread));
+        t.far_off[b + 1] = t.far_off[b] + nt * ceil_div(n, far_rows(n));
         t.near_off[b + 1] = t.near_off[b] + (int)t.sys[b].n_near;
         const int rows = t.sys[b].f.n_bc_cols > 0 ? 8 : kRhsRows;   // k_rhs: a warp or a thread per row
         t.rhs_off[b + 1] = t.rhs_off[b] + (n + rows - 1) / rows;
@@ -2252,14 +2300,14 @@ cudaError_t launch_assemble(const AsmBatch &t, int prec, unsigned *ctr, cudaStre
     // bounds allow kFarPerSm), near_per_sm of k_near (launch bounds allow 2)
     const int fps = std::max(1, std::min(shape.far_per_sm, kFarPerSm));
     const int nps = std::max(1, std::min(shape.near_per_sm, 2));
-    const int gfar = std::max(1, std::min(far_items, fps * sm_count()));
+    const int gfar = std::max(1, std::min((far_items + 7) / 8, fps * sm_count()));
     const int gnear = std::max(1, std::min((near_items + 7) / 8, nps * sm_count()));
     // Systems that fill the GPU on their own take one single-system launch
     // each: the single-system kernel keeps the table in constant operands
-    // (fewer registers, no spills), which beat the shared work queue.
+    // (fewer registers, no spills), which beat one launch over the batch.
     bool split = t.B > 1;
     for (int b = 0; b < t.B && split; ++b)
-        if (t.far_off[b + 1] - t.far_off[b] < fps * sm_count()) split = false;
+        if (t.far_off[b + 1] - t.far_off[b] < 8 * fps * sm_count()) split = false;
     std::unique_ptr<AsmBatch> one_sys;
     if (split) one_sys.reset(new AsmBatch());
     count_launches((split ? t.B : 1) + (near_items ? 1 : 0));
@@ -2267,29 +2315,28 @@ cudaError_t launch_assemble(const AsmBatch &t, int prec, unsigned *ctr, cudaStre
         const bool one = a.B == 1;
         if (prec == 0) {
             if (a.img) {
-                if (one) k_far<double, true, true><<<grid, block, 0, st>>>(a, ctr);
-                else k_far<double, false, true><<<grid, block, 0, st>>>(a, ctr);
+                if (one) k_far<double, true, true><<<grid, block, 0, st>>>(a);
+                else k_far<double, false, true><<<grid, block, 0, st>>>(a);
             } else {
-                if (one) k_far<double, true, false><<<grid, block, 0, st>>>(a, ctr);
-                else k_far<double, false, false><<<grid, block, 0, st>>>(a, ctr);
+                if (one) k_far<double, true, false><<<grid, block, 0, st>>>(a);
+                else k_far<double, false, false><<<grid, block, 0, st>>>(a);
             }
         } else {
             if (a.img) {
-                if (one) k_far<float, true, true><<<grid, block, 0, st>>>(a, ctr);
-                else k_far<float, false, true><<<grid, block, 0, st>>>(a, ctr);
+                if (one) k_far<float, true, true><<<grid, block, 0, st>>>(a);
+                else k_far<float, false, true><<<grid, block, 0, st>>>(a);
             } else {
-                if (one) k_far<float, true, false><<<grid, block, 0, st>>>(a, ctr);
-                else k_far<float, false, false><<<grid, block, 0, st>>>(a, ctr);
+                if (one) k_far<float, true, false><<<grid, block, 0, st>>>(a);
+                else k_far<float, false, false><<<grid, block, 0, st>>>(a);
             }
         }
     };
     if (split) {
-        // launches run in order on st; each ends by resetting the queue counter
         for (int b = 0; b < t.B; ++b) {
             one_sys->B = 1;
             one_sys->sys[0] = t.sys[b];
             asm_batch_finish(*one_sys);
-            far(*one_sys, std::max(1, std::min(one_sys->far_off[1], fps * sm_count())));
+            far(*one_sys, std::max(1, std::min((one_sys->far_off[1] + 7) / 8, fps * sm_count())));
         }
     } else {
         far(t, gfar);

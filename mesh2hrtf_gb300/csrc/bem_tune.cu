@@ -87,9 +87,9 @@ void load_locked() {
         if (!std::strcmp(what, "asm")) {
             int fa, ne;
             double ms;
-            if (std::sscanf(rest, "%d %d %lf", &fa, &ne, &ms) == 3 && fa >= 1 && fa <= kFarPerSmMax && ne >= 1 &&
-                ne <= 2) {
-                c.asm_shape.far_per_sm = fa;
+            // (k_far took up to three blocks per SM when older lines were written)
+            if (std::sscanf(rest, "%d %d %lf", &fa, &ne, &ms) == 3 && fa >= 1 && fa <= 3 && ne >= 1 && ne <= 2) {
+                c.asm_shape.far_per_sm = fa < kFarPerSmMax ? fa : kFarPerSmMax;
                 c.asm_shape.near_per_sm = ne;
                 c.asm_ms = ms;
                 c.asm_tuned = true;
