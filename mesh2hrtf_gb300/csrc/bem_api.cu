@@ -286,10 +286,8 @@ size_t solver_layout(int n, int prec, int m, bool pc, unsigned char *base, Solve
         q.z = (double2 *)take(N * 16);
         q.V = (double2 *)take((size_t)(m + 1) * N * vsz);
         q.mvp = (double2 *)take(mvp_elems(n) * 16);
-        if (prec != 0) {   // complex64: float copies of the product's input
-            q.xh = (float2 *)take(xsplit_elems(n) * 8);
-            q.xf = (float4 *)take(xsplit_elems(n) * 16);
-        }
+        // complex64: float copy of the product's input
+        if (prec != 0) q.xh = (float2 *)take(xsplit_elems(n) * 8);
         if (pc) {
             q.pcy = take(N * 16);
             q.pcz = take(N * 16);

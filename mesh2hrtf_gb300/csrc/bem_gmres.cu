@@ -58,6 +58,7 @@
 #include <type_traits>
 
 #include "bem_engine.h"
+#include "bem_f32x2.cuh"
 #include "bem_internal.h"
 #include "bem_umma.h"
 
@@ -108,13 +109,26 @@ __device__ __forceinline__ void warp_sum_ff(float &s, float &e) {
         e = (e + e2) + u;
     }
 }
-__device__ __forceinline__ void acc_exact(float &s, float &e, float a, float b) {
-    const float p = a * b;
-    const float q = fmaf(a, b, -p);
-    float t, u;
-    two_sum(s, p, t, u);
+// (s, e) += a b for two pairs at once (packed FP32), each half by the FMA
+// two-product and Knuth's two-sum; na = -a, m1 = (-1, -1).
+__device__ __forceinline__ void two_sum2(F2 a, F2 b, F2 m1, F2 &s, F2 &e) {
+    s = vadd(a, b);
+    const F2 bb = vfma(a, m1, s), t = vfma(bb, m1, s);
+    e = vadd(vfma(t, m1, a), vfma(bb, m1, b));
+}
+__device__ __forceinline__ void acc_exact2(F2 &s, F2 &e, F2 a, F2 na, F2 b, F2 m1) {
+    const F2 p = vmul(a, b), nq = vfma(na, b, p);   // -q, the product's error
+    F2 t, u;
+    two_sum2(s, p, m1, t, u);
     s = t;
-    e += u + q;
+    e = vadd(e, vfma(nq, m1, u));
+}
+// The same where s is known to stay at least twice as large as any product
+// left to add: t - s is exact, so the fused product's error needs no two-sum.
+__device__ __forceinline__ void acc_biased2(F2 &s, F2 &e, F2 a, F2 b, F2 m1) {
+    const F2 t = vfma(a, b, s);
+    e = vadd(e, vfma(a, b, vfma(t, m1, s)));
+    s = t;
 }
 
 // Does a system take part in a product of this kind?  0: Krylov product;
@@ -305,14 +319,15 @@ __global__ void __launch_bounds__(256, 4) k_mv64(KTable *tb, int kind) {
 // (system, 1024-column chunk, strip of 64 rows) from the queue and streams
 // them through a ring of kTmaStages stages of kTmaRows row segments (8 KB
 // each, one cp.async.bulk per segment) into shared memory; the chunk of x
-// (float hi parts, or hi/lo pairs for the refinement residual) goes into one
-// of two x buffers.  mbarriers carry the byte counts (full) and the
+// goes into one of two x buffers.  mbarriers carry the byte counts (full) and the
 // consumers' releases (empty).  Consumer warp w < 8 takes row w of a stage.
 // Krylov products of systems with an fp16 copy of A (KSys::A16) stream that
 // copy instead, with items of two column chunks so that row segments stay
 // 8 KB (the number of bulk copies an SM completes per second, not their
 // size, limits 4 KB segments); consumer warp w takes row w & 7 over chunk
 // w >> 3 of the item and scales its sum by the row's power-of-two scale.
+// The residual's error-free products (20 packed operations per entry) bound it by the FMA pipe: both sets of eight warps work, on
+// alternate stages, 20480 unknowns 888 -> 647 us (490 at HBM speed).
 // Every wait is bounded (kWaitCycles); on expiry the kernel sets tb->err,
 // lets its own copies land and returns.
 constexpr int kTmaStages = 3;
@@ -332,12 +347,9 @@ __device__ __forceinline__ float2 h2f(unsigned u) {
     return __half22float2(h);
 }
 
-// x buffers: hi/lo pairs of one chunk (refinement residual) or hi parts of
-// two chunks (fp16 Krylov items)
-__host__ __device__ constexpr int tma_x_bytes(bool) { return kMvChunk * 16; }
-__host__ __device__ constexpr int tma_smem_bytes(bool exact) {
-    return kTmaStages * kStageBytes + 2 * tma_x_bytes(exact) + 256;
-}
+// x buffers: one chunk, or two (fp16 Krylov items)
+constexpr int kTmaXBytes = 2 * kMvChunk * 8;
+constexpr int kTmaSmem = kTmaStages * kStageBytes + 2 * kTmaXBytes + 256;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
@@ -409,7 +421,7 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *ring = smem;                                       // kTmaStages x 64 KB
     unsigned char *xbuf = smem + kTmaStages * kStageBytes;           // 2 x chunk of x
-    uint64_t *bars = reinterpret_cast<uint64_t *>(xbuf + 2 * tma_x_bytes(EXACT));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(xbuf + 2 * kTmaXBytes);
     // bars: full[3], empty[3], xfull[2], xempty[2]; then the stage metadata
     TmaMeta *meta = reinterpret_cast<TmaMeta *>(bars + 2 * kTmaStages + 4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -476,14 +488,9 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
             if (!__shfl_sync(kAll, w, 0)) { ok = false; break; }
             xeph[xs] ^= 1;
             if (lane == 0) {
-                const uint32_t xdst = smem_u32(xbuf + xs * tma_x_bytes(EXACT));
-                if (EXACT) {
-                    mbar_expect_tx(xfull0 + 8 * xs, kMvChunk * 16);
-                    bulk_g2s(xdst, S.xf + c0, kMvChunk * 16, xfull0 + 8 * xs);
-                } else {
-                    mbar_expect_tx(xfull0 + 8 * xs, lenp * 8);
-                    bulk_g2s(xdst, S.xh + c0, lenp * 8, xfull0 + 8 * xs);
-                }
+                const uint32_t xdst = smem_u32(xbuf + xs * kTmaXBytes);
+                mbar_expect_tx(xfull0 + 8 * xs, lenp * 8);
+                bulk_g2s(xdst, S.xh + c0, lenp * 8, xfull0 + 8 * xs);
             }
             xiss[xs] = 1;
             xfp[xs] ^= 1;
@@ -535,9 +542,12 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
         }
         return;
     }
-    // ---------------- consumers: warp w takes row w of each stage
-    int stage = 0;
+    // ---------------- consumers: warp w takes row w of each stage; for the
+    // residual, whose arithmetic would leave eight warps waiting on their own
+    // chains, warps 0 - 7 and 8 - 15 take row w & 7 of every other stage
+    int stage = 0, turn = 0;
     uint32_t fph = 0, xph[2] = {0, 0};
+    const int row = EXACT ? warp & (kTmaRows - 1) : warp;
     while (true) {
         if (!mbar_wait(full0 + 8 * stage, fph, err, lim)) return;
         const TmaMeta mt = meta[stage];
@@ -546,7 +556,7 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
         if (mt.first) {
             if (!mbar_wait(xfull0 + 8 * mt.xslot, xph[mt.xslot], err, lim)) return;
         }
-        const unsigned char *xb = xbuf + mt.xslot * tma_x_bytes(EXACT);
+        const unsigned char *xb = xbuf + mt.xslot * kTmaXBytes;
         // this warp's row sum as float-float (hi, lo) pairs of the real and
         // imaginary parts, written after the stage is released
         float4 o0 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -626,12 +636,12 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
                 o0 = make_float4(warp_sum_f(ar + br) * sca, 0.f, warp_sum_f(ai + bi) * sca, 0.f);
                 nout = 1;
             }
-        } else if (warp < mt.nrows) {
-            const float4 *A4 = reinterpret_cast<const float4 *>(ring + stage * kStageBytes) + warp * (kMvChunk / 2);
+        } else if (row < mt.nrows && (!EXACT || turn == (warp >> 3))) {
+            const float4 *A4 = reinterpret_cast<const float4 *>(ring + stage * kStageBytes) + row * (kMvChunk / 2);
             const int len = mt.len, len2 = len >> 1;
             float sr = 0.f, si = 0.f, er = 0.f, ei = 0.f;
             if (!EXACT) {
-                const float4 *x4 = reinterpret_cast<const float4 *>(xb);   // hi parts of entries 2c, 2c + 1
+                const float4 *x4 = reinterpret_cast<const float4 *>(xb);   // entries 2c, 2c + 1
 #pragma unroll 4
                 for (int c = lane; c < len2; c += 32) {
                     const float4 a = A4[c], xv = x4[c];
@@ -647,43 +657,47 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
                     si = fmaf(a.x, xv.y, si); si = fmaf(a.y, xv.x, si);
                 }
             } else {
-                // x chunk permuted: entry 2c at xa[c], entry 2c + 1 at xb2[c].
-                // Even and odd entries, and the two terms of each component,
-                // accumulate into separate float-float pairs (one exact
-                // product per pair and iteration), merged below.
-                const float4 *xa = reinterpret_cast<const float4 *>(xb), *xb2 = xa + kMvChunk / 2;
-                float sr2 = 0.f, si2 = 0.f, er2 = 0.f, ei2 = 0.f;   // odd entries
-                float sr3 = 0.f, si3 = 0.f, er3 = 0.f, ei3 = 0.f;   // second terms, even
-                float sr4 = 0.f, si4 = 0.f, er4 = 0.f, ei4 = 0.f;   // second terms, odd
+                // pairs (re re, im im) and (im re, re im) of the products; even
+                // and odd entries accumulate into separate float-float pairs,
+                // merged below
+                const float4 *x4 = reinterpret_cast<const float4 *>(xb);
+                const F2 m1 = opaque2(-1.f);
+                F2 sv[4], ev[4];   // entry parity, + 2 for the crossed products
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sv[q] = ev[q] = pk2(0.f, 0.f);
+                auto entry = [&](int h, float ax, float ay, F2 x) {
+                    acc_exact2(sv[h], ev[h], pk2(ax, ay), pk2(-ax, -ay), x, m1);
+                    acc_exact2(sv[2 + h], ev[2 + h], pk2(ay, ax), pk2(-ay, -ax), x, m1);
+                };
 #pragma unroll 2
                 for (int c = lane; c < len2; c += 32) {
-                    const float4 a = A4[c], x0 = xa[c], x1 = xb2[c];
-                    acc_exact(sr, er, a.x, x0.x); acc_exact(sr3, er3, -a.y, x0.y);
-                    acc_exact(si, ei, a.x, x0.y); acc_exact(si3, ei3, a.y, x0.x);
-                    er = fmaf(a.x, x0.z, er); er3 = fmaf(-a.y, x0.w, er3);
-                    ei = fmaf(a.x, x0.w, ei); ei3 = fmaf(a.y, x0.z, ei3);
-                    acc_exact(sr2, er2, a.z, x1.x); acc_exact(sr4, er4, -a.w, x1.y);
-                    acc_exact(si2, ei2, a.z, x1.y); acc_exact(si4, ei4, a.w, x1.x);
-                    er2 = fmaf(a.z, x1.z, er2); er4 = fmaf(-a.w, x1.w, er4);
-                    ei2 = fmaf(a.z, x1.w, ei2); ei4 = fmaf(a.w, x1.z, ei4);
-                }
-                {
-                    float t, u;
-                    two_sum(sr, sr3, t, u); sr = t; er += er3 + u;
-                    two_sum(si, si3, t, u); si = t; ei += ei3 + u;
-                    two_sum(sr2, sr4, t, u); sr2 = t; er2 += er4 + u;
-                    two_sum(si2, si4, t, u); si2 = t; ei2 += ei4 + u;
-                    two_sum(sr, sr2, t, u); sr = t; er += er2 + u;
-                    two_sum(si, si2, t, u); si = t; ei += ei2 + u;
+                    const float4 a = A4[c], xv = x4[c];
+                    entry(0, a.x, a.y, pk2(xv.x, xv.y));
+                    entry(1, a.z, a.w, pk2(xv.z, xv.w));
                 }
                 if ((len & 1) && lane == 0) {
                     const float2 a = reinterpret_cast<const float2 *>(A4)[len - 1];
-                    const float4 x0 = xa[(len - 1) >> 1];
-                    acc_exact(sr, er, a.x, x0.x); acc_exact(sr, er, -a.y, x0.y);
-                    acc_exact(si, ei, a.x, x0.y); acc_exact(si, ei, a.y, x0.x);
-                    er = fmaf(a.x, x0.z, er); er = fmaf(-a.y, x0.w, er);
-                    ei = fmaf(a.x, x0.w, ei); ei = fmaf(a.y, x0.z, ei);
+                    const float2 xv = reinterpret_cast<const float2 *>(xb)[len - 1];
+                    entry(0, a.x, a.y, pk2(xv.x, xv.y));
                 }
+                F2 t, u;
+#pragma unroll
+                for (int h = 0; h < 4; h += 2) {
+                    two_sum2(sv[h], sv[h + 1], m1, t, u);
+                    sv[h] = t;
+                    ev[h] = vadd(ev[h], vadd(ev[h + 1], u));
+                }
+                float s0, s1, e0, e1, tt, uu;
+                unpk2(sv[0], s0, s1);
+                unpk2(ev[0], e0, e1);
+                two_sum(s0, -s1, tt, uu);
+                sr = tt;
+                er = (e0 - e1) + uu;
+                unpk2(sv[2], s0, s1);
+                unpk2(ev[2], e0, e1);
+                two_sum(s0, s1, tt, uu);
+                si = tt;
+                ei = (e0 + e1) + uu;
             }
             if (EXACT) {
                 warp_sum_ff(sr, er);
@@ -702,7 +716,7 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
             // the Krylov products (summed in FP32 by k_dot1), FP64 for the
             // residuals (summed in FP64 by k_resid)
             const size_t o = (size_t)mt.chunk * S.n + mt.row0 +
-                             ((!EXACT && mt.h) ? (size_t)(warp >> 3) * S.n + (warp & (kTmaRows - 1)) : (size_t)warp);
+                             ((!EXACT && mt.h) ? (size_t)(warp >> 3) * S.n + (warp & (kTmaRows - 1)) : (size_t)row);
             if (nout > 0) {
                 if (!EXACT && kind == 0)
                     reinterpret_cast<float2 *>(S.mvp)[o] = make_float2(o0.x + o0.y, o0.z + o0.w);
@@ -711,48 +725,53 @@ __global__ void __launch_bounds__(32 * (kTmaConsumers + 1), 1) k_mv_tma(KTable *
             }
         }
         if (mt.first) xph[mt.xslot] ^= 1;
+        turn ^= 1;
         if (++stage == kTmaStages) { stage = 0; fph ^= 1; }
     }
 }
 
-// ------------------------------------------------------------ shared-matrix product
-// Right-hand sides of one solver share A (complex64).  One launch streams
-// every tile of A once: an item is a strip of rows of one group over all
-// columns; a stage holds the strip's rows x kGrpCols columns of A (one bulk
-// copy per 2 KB row segment) and the x chunks of the group's members that
-// take part (2 KB each for the Krylov product, 4 KB of hi/lo pairs for the
-// residual).
-// Consumer warps own 4 rows x 4 members each and keep, in registers, one
-// accumulator per (row, member) across all column chunks; at the strip's
-// last chunk they write the members' full-row products (nchunk = 1).
-// Krylov product: 16 consumer warps, 32-row strips, 2 stages of 80 KB.
-// Refinement residual (twice the registers): 8 warps, 16 rows, 3 x 64 KB.
-template <bool EXACT> struct GrpCfg {
-    static constexpr int kWarps = EXACT ? 8 : 16;
-    static constexpr int kRows = 2 * kWarps;          // 4 rows per warp pair
-    static constexpr int kStages = EXACT ? 3 : 2;
-    static constexpr int kXBytes = EXACT ? kGrpCols * 16 : kGrpCols * 8;
-    static constexpr int kABytes = kRows * kGrpCols * 8;
-    static constexpr int kStageBytes = kABytes + kMaxGroup * kXBytes;
-    static constexpr int kSmem = kStages * kStageBytes + 512;
-};
-static_assert(GrpCfg<false>::kSmem <= 227 * 1024 && GrpCfg<true>::kSmem <= 227 * 1024, "shared memory");
-static_assert(GrpCfg<false>::kRows == kGrpRowsInner && GrpCfg<true>::kRows == kGrpRowsExact, "plan strip heights");
-__host__ __device__ constexpr int grp_smem_bytes(bool exact) {
-    return exact ? GrpCfg<true>::kSmem : GrpCfg<false>::kSmem;
-}
+// ------------------------------------------------------------ shared-matrix residual
+// Right-hand sides of one solver share A (complex64).  The first cycle's
+// residual (error-free products, as k_mv_tma<true>) for up to eight of them:
+// one launch streams every tile of A once: an item is a strip of rows of one
+// group over all columns; a stage holds the strip's rows x kGrpCols columns of
+// A (one bulk copy per 2 KB row segment) and the 2 KB x chunks of the group's
+// members that take part.
+// Consumer warps own 2 rows x 4 members each and keep one float-float
+// accumulator per lane and (row, member) across all column chunks; at the
+// strip's last chunk they write the members' full-row products (nchunk = 1).
+//
+// Bound by the FMA pipe and issue: each component's 16 products of a lane and
+// stage are added onto a bias of twice their bound, sum |a| max |x|
+// (acc_biased2), and the stage's sum and error then go to the row's pair: 4.7
+// operations a product instead of 11.  69620 unknowns, 8 right-hand sides:
+// 61.5 -> 36.9 ms (the matrix alone 5.7); 8 warps of 4 rows each, too few to
+// hide their chains, 50.8.
+// The bias costs three bits in the stage that holds the row's largest entry
+// and saves the error term of a long sum: measured against 64-bit sums its
+// error is 1 .. 0.1 of the two-sum form's from 4096 unknowns on (5120: 0.5,
+// 69620: 0.1), up to three times below, so small systems keep that.
+constexpr int kGrpBiasedMin = 4096;
+constexpr int kGrpWarps = 16;
+constexpr int kGrpRows = kGrpWarps;              // 2 rows per warp pair
+constexpr int kGrpStages = 3;
+constexpr int kGrpSumBytes = kGrpWarps * 32 * 2 * (kMaxGroup / 2) * 16;   // the lanes' row sums
+constexpr int kGrpXBytes = kGrpCols * 8;
+constexpr int kGrpABytes = kGrpRows * kGrpCols * 8;
+constexpr int kGrpStageBytes = kGrpABytes + kMaxGroup * kGrpXBytes;
+constexpr int kGrpSmem = kGrpStages * kGrpStageBytes + kGrpSumBytes + 512;
+static_assert(kGrpSmem <= 227 * 1024, "shared memory");
+static_assert(kGrpRows == kGrpRowsExact, "plan strip heights");
 
 struct GrpMeta {
     int first, chunk, row0, nrows, len, last, mask, pad;
 };
 
-template <bool EXACT>
-__global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(KTable *tb, int kind) {
+__global__ void __launch_bounds__(32 * (kGrpWarps + 1), 1) k_mv_grp(KTable *tb, int kind) {
     extern __shared__ __align__(128) unsigned char smem[];
-    using Cfg = GrpCfg<EXACT>;
-    constexpr int SB = Cfg::kStageBytes, XB = Cfg::kXBytes, NW = Cfg::kWarps, ROWS = Cfg::kRows;
-    constexpr int NS = Cfg::kStages, ASTAGE = Cfg::kABytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NS * SB);
+    constexpr int SB = kGrpStageBytes, XB = kGrpXBytes, NW = kGrpWarps, ROWS = kGrpRows;
+    constexpr int NS = kGrpStages, ASTAGE = kGrpABytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NS * SB + kGrpSumBytes);
     GrpMeta *meta = reinterpret_cast<GrpMeta *>(bars + 2 * NS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + NS);
@@ -770,8 +789,7 @@ __global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(
     const long long lim = (tb->wait_cycles > 0 && ((tb->wait_kinds >> kind) & 1)) ? tb->wait_cycles : kWaitCycles;
     if (warp == NW) {
         // ---------------- producer warp: lane 0 takes the strips and keeps the
-        // barriers; lane r < ROWS issues row r's copy, the other copies (the
-        // members' x chunks) go round the lanes
+        // barriers; lane r < ROWS issues row r's copy, lane q member q's x chunk
         const unsigned kAll = 0xffffffffu;
         const int total = pl.off[pl.n];
         int stage = 0;
@@ -795,37 +813,24 @@ __global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(
             const float2 *A = (const float2 *)S0.A;
             const size_t lda = (size_t)S0.lda;
             const int nmem = __popc(mask & ((1u << g.count) - 1u));
-            constexpr int XPER = EXACT ? 2 : 1;   // copies per member and stage
             for (int ck = 0; ck < nck && ok; ++ck) {
                 int w = 1;
                 if (lane == 0) w = mbar_wait(empty0 + 8 * stage, eph, err, lim);
                 if (!__shfl_sync(kAll, w, 0)) { ok = false; break; }
                 const int c0 = ck * kGrpCols, len = min(kGrpCols, n - c0), lenp = (len + 1) & ~1;
-                const uint32_t xbytes = EXACT ? (uint32_t)XB : (uint32_t)(lenp * 8);
                 const uint32_t fb = full0 + 8 * stage;
                 if (lane == 0) {
                     GrpMeta mt;
                     mt.first = g.first; mt.chunk = ck; mt.row0 = row0; mt.nrows = nrows; mt.len = len;
                     mt.last = ck == nck - 1; mt.mask = (int)mask; mt.pad = 0;
                     meta[stage] = mt;
-                    mbar_expect_tx(fb, (uint32_t)(nrows * lenp * 8) + nmem * xbytes);
+                    mbar_expect_tx(fb, (uint32_t)((nrows + nmem) * lenp * 8));
                 }
                 __syncwarp();
                 const uint32_t dst = smem_u32(smem + stage * SB);
                 if (lane < nrows) bulk_g2s(dst + lane * kGrpCols * 8, A + (size_t)(row0 + lane) * lda + c0, lenp * 8, fb);
-                for (int t = lane; t < kMaxGroup * XPER; t += 32) {
-                    const int q = t / XPER, h = t - q * XPER;
-                    if (q >= g.count || !((mask >> q) & 1)) continue;
-                    const uint32_t xd = dst + ASTAGE + q * XB;
-                    if (EXACT) {
-                        // chunk-permuted (hi, lo) pairs: the stage's even entries, then its odd ones
-                        const float4 *base = (const float4 *)tb->sys[g.first + q].xf + (size_t)(c0 & ~(kMvChunk - 1));
-                        const int o = (c0 & (kMvChunk - 1)) >> 1;
-                        bulk_g2s(xd + h * kGrpCols * 8, base + h * (kMvChunk / 2) + o, kGrpCols * 8, fb);
-                    } else {
-                        bulk_g2s(xd, (const float2 *)tb->sys[g.first + q].xh + c0, lenp * 8, fb);
-                    }
-                }
+                if (lane < g.count && ((mask >> lane) & 1))
+                    bulk_g2s(dst + ASTAGE + lane * XB, (const float2 *)tb->sys[g.first + lane].xh + c0, lenp * 8, fb);
                 issued[stage] = 1;
                 fph[stage] ^= 1;
                 if (++stage == NS) { stage = 0; eph ^= 1; }
@@ -852,11 +857,24 @@ __global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(
         }
         return;
     }
-    // ---------------- consumers: warp w takes rows 4(w/2) .. 4(w/2)+3 of each
+    // ---------------- consumers: warp w takes rows 2(w/2), 2(w/2)+1 of each
     // strip and members 4(w%2) .. 4(w%2)+3: every A value loaded from shared
-    // memory serves 4 members, every x value 4 rows
-    constexpr int RW = 4, MW = kMaxGroup / 2;
-    float ar[RW][MW], ai[RW][MW], er[RW][MW], ei[RW][MW];
+    // memory serves 4 members, every x value 2 rows
+    constexpr int RW = 2, MW = kMaxGroup / 2;
+    const F2 m1 = opaque2(-1.f), zero = pk2(0.f, 0.f);
+    // (re, im) sums of (row r, member q) and their errors, between stages
+    float4 *sum = reinterpret_cast<float4 *>(smem + NS * SB) + warp * (RW * MW * 32) + lane;
+    auto sum_get = [&](int r, int q, F2 &v, F2 &e) {
+        const float4 f = sum[(r * MW + q) * 32];
+        v = pk2(f.x, f.y);
+        e = pk2(f.z, f.w);
+    };
+    auto sum_put = [&](int r, int q, F2 v, F2 e) {
+        float4 f;
+        unpk2(v, f.x, f.y);
+        unpk2(e, f.z, f.w);
+        sum[(r * MW + q) * 32] = f;
+    };
     const int rbase = RW * (warp >> 1), mbase = MW * (warp & 1);
     int stage = 0;
     uint32_t fph = 0;
@@ -868,79 +886,111 @@ __global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(
 #pragma unroll
             for (int r = 0; r < RW; ++r)
 #pragma unroll
-                for (int q = 0; q < MW; ++q) ar[r][q] = ai[r][q] = er[r][q] = ei[r][q] = 0.f;
+                for (int q = 0; q < MW; ++q) sum_put(r, q, zero, zero);
         }
         const unsigned char *sb = smem + stage * SB;
-        const unsigned mymask = ((unsigned)mt.mask >> mbase) & ((1u << MW) - 1u);
+        const unsigned mymask =
+            rbase < mt.nrows ? ((unsigned)mt.mask >> mbase) & ((1u << MW) - 1u) : 0u;
         const int len = mt.len, len2 = len >> 1;
-        const float4 *Ab = reinterpret_cast<const float4 *>(sb) + rbase * (kGrpCols / 2);
-        if (mymask) {
-#pragma unroll 2
-            for (int c = lane; c < len2; c += 32) {
-                float4 a[RW];
+        // the strip's last row stands in for rows past its end
+        const float4 *Ar[RW];
 #pragma unroll
-                for (int r = 0; r < RW; ++r)
-                    a[r] = rbase + r < mt.nrows ? Ab[r * (kGrpCols / 2) + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < RW; ++r)
+            Ar[r] = reinterpret_cast<const float4 *>(sb) + min(rbase + r, mt.nrows - 1) * (kGrpCols / 2);
+        auto xrow = [&](int q) { return reinterpret_cast<const float4 *>(sb + ASTAGE + (mbase + q) * XB); };
+        // entries 2c, 2c + 1; of an odd stage's last pair only the first counts
+        auto load = [&](const float4 *p, int c) {
+            float4 v = p[c];
+            if (c >= len2) v.z = v.w = 0.f;
+            return v;
+        };
+        const int c1 = (len & 1) && lane == (len2 & 31) ? len2 + 1 : len2;
+        if (mymask && tb->sys[mt.first].n >= kGrpBiasedMin) {
+            float asum[RW], xmax[MW];
 #pragma unroll
-                for (int q = 0; q < MW; ++q) {
-                    if (!((mymask >> q) & 1)) continue;
-                    const unsigned char *xq = sb + ASTAGE + (mbase + q) * XB;
-                    if (!EXACT) {
-                        const float4 xv = reinterpret_cast<const float4 *>(xq)[c];   // hi of entries 2c, 2c + 1
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            ar[r][q] = fmaf(a[r].x, xv.x, ar[r][q]); ar[r][q] = fmaf(-a[r].y, xv.y, ar[r][q]);
-                            ai[r][q] = fmaf(a[r].x, xv.y, ai[r][q]); ai[r][q] = fmaf(a[r].y, xv.x, ai[r][q]);
-                            ar[r][q] = fmaf(a[r].z, xv.z, ar[r][q]); ar[r][q] = fmaf(-a[r].w, xv.w, ar[r][q]);
-                            ai[r][q] = fmaf(a[r].z, xv.w, ai[r][q]); ai[r][q] = fmaf(a[r].w, xv.z, ai[r][q]);
-                        }
-                    } else {
-                        const float4 x0 = reinterpret_cast<const float4 *>(xq)[c];
-                        const float4 x1 = reinterpret_cast<const float4 *>(xq + kGrpCols * 8)[c];
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            acc_exact(ar[r][q], er[r][q], a[r].x, x0.x); acc_exact(ar[r][q], er[r][q], -a[r].y, x0.y);
-                            acc_exact(ai[r][q], ei[r][q], a[r].x, x0.y); acc_exact(ai[r][q], ei[r][q], a[r].y, x0.x);
-                            er[r][q] = fmaf(a[r].x, x0.z, er[r][q]); er[r][q] = fmaf(-a[r].y, x0.w, er[r][q]);
-                            ei[r][q] = fmaf(a[r].x, x0.w, ei[r][q]); ei[r][q] = fmaf(a[r].y, x0.z, ei[r][q]);
-                            acc_exact(ar[r][q], er[r][q], a[r].z, x1.x); acc_exact(ar[r][q], er[r][q], -a[r].w, x1.y);
-                            acc_exact(ai[r][q], ei[r][q], a[r].z, x1.y); acc_exact(ai[r][q], ei[r][q], a[r].w, x1.x);
-                            er[r][q] = fmaf(a[r].z, x1.z, er[r][q]); er[r][q] = fmaf(-a[r].w, x1.w, er[r][q]);
-                            ei[r][q] = fmaf(a[r].z, x1.w, ei[r][q]); ei[r][q] = fmaf(a[r].w, x1.z, ei[r][q]);
-                        }
-                    }
+            for (int r = 0; r < RW; ++r) {
+                asum[r] = 0.f;
+                for (int c = lane; c < c1; c += 32) {
+                    const float4 a = load(Ar[r], c);
+                    asum[r] += (fabsf(a.x) + fabsf(a.y)) + (fabsf(a.z) + fabsf(a.w));
                 }
             }
-            if ((len & 1) && lane == 0) {   // odd tail: entry len - 1
-                float2 b[RW];
 #pragma unroll
-                for (int r = 0; r < RW; ++r)
-                    b[r] = rbase + r < mt.nrows ? reinterpret_cast<const float2 *>(Ab + r * (kGrpCols / 2))[len - 1]
-                                                : make_float2(0.f, 0.f);
+            for (int q = 0; q < MW; ++q) {
+                xmax[q] = 0.f;
+                if (!((mymask >> q) & 1)) continue;
+                for (int c = lane; c < c1; c += 32) {
+                    const float4 x = load(xrow(q), c);
+                    xmax[q] = fmaxf(xmax[q], fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+                }
+            }
+            // twice the bound, with room for its rounding; the cap keeps the bias
+            // finite (sums near the type's end lose the error term there)
+            auto bias = [&](int r, int q) {
+                const float b = fminf(2.001f * asum[r] * xmax[q], 4e37f);
+                return pk2(b, b);
+            };
+            F2 s[RW][MW], e[RW][MW];
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int q = 0; q < MW; ++q) {
+                    s[r][q] = bias(r, q);
+                    e[r][q] = zero;
+                }
+            auto step = [&](int c, bool tail) {
+                F2 ax[RW][2], ay[RW][2];
+#pragma unroll
+                for (int r = 0; r < RW; ++r) {
+                    const float4 a = tail ? load(Ar[r], c) : Ar[r][c];
+                    ax[r][0] = pk2(a.x, a.x);
+                    ay[r][0] = pk2(a.y, a.y);
+                    ax[r][1] = pk2(a.z, a.z);
+                    ay[r][1] = pk2(a.w, a.w);
+                }
 #pragma unroll
                 for (int q = 0; q < MW; ++q) {
                     if (!((mymask >> q) & 1)) continue;
-                    const unsigned char *xq = sb + ASTAGE + (mbase + q) * XB;
-                    float xr, xi, lr = 0.f, li = 0.f;
-                    if (!EXACT) {
-                        const float2 xv = reinterpret_cast<const float2 *>(xq)[len - 1];
-                        xr = xv.x; xi = xv.y;
-                    } else {
-                        const float4 x0 = reinterpret_cast<const float4 *>(xq)[(len - 1) >> 1];
-                        xr = x0.x; xi = x0.y; lr = x0.z; li = x0.w;
-                    }
+                    const float4 x = tail ? load(xrow(q), c) : xrow(q)[c];
 #pragma unroll
-                    for (int r = 0; r < RW; ++r) {
-                        if (!EXACT) {
-                            ar[r][q] = fmaf(b[r].x, xr, ar[r][q]); ar[r][q] = fmaf(-b[r].y, xi, ar[r][q]);
-                            ai[r][q] = fmaf(b[r].x, xi, ai[r][q]); ai[r][q] = fmaf(b[r].y, xr, ai[r][q]);
-                        } else {
-                            acc_exact(ar[r][q], er[r][q], b[r].x, xr); acc_exact(ar[r][q], er[r][q], -b[r].y, xi);
-                            acc_exact(ai[r][q], ei[r][q], b[r].x, xi); acc_exact(ai[r][q], ei[r][q], b[r].y, xr);
-                            er[r][q] = fmaf(b[r].x, lr, er[r][q]); er[r][q] = fmaf(-b[r].y, li, er[r][q]);
-                            ei[r][q] = fmaf(b[r].x, li, ei[r][q]); ei[r][q] = fmaf(b[r].y, lr, ei[r][q]);
-                        }
+                    for (int r = 0; r < RW; ++r) acc_biased2(s[r][q], e[r][q], ax[r][0], pk2(x.x, x.y), m1);
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) acc_biased2(s[r][q], e[r][q], ay[r][0], pk2(-x.y, x.x), m1);
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) acc_biased2(s[r][q], e[r][q], ax[r][1], pk2(x.z, x.w), m1);
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) acc_biased2(s[r][q], e[r][q], ay[r][1], pk2(-x.w, x.z), m1);
+                }
+            };
+#pragma unroll 1
+            for (int c = lane; c < len2; c += 32) step(c, false);
+            if (c1 > len2) step(len2, true);
+#pragma unroll
+            for (int q = 0; q < MW; ++q)
+#pragma unroll
+                for (int r = 0; r < RW; ++r) {
+                    F2 v, l, t, u;
+                    sum_get(r, q, v, l);
+                    two_sum2(v, vfma(bias(r, q), m1, s[r][q]), m1, t, u);
+                    sum_put(r, q, t, vadd(l, vadd(u, e[r][q])));
+                }
+        } else if (mymask) {
+#pragma unroll 1
+            for (int q = 0; q < MW; ++q) {
+                if (!((mymask >> q) & 1)) continue;
+#pragma unroll
+                for (int r = 0; r < RW; ++r) {
+                    F2 v, l;
+                    sum_get(r, q, v, l);
+#pragma unroll 1
+                    for (int c = lane; c < c1; c += 32) {
+                        const float4 a = load(Ar[r], c), x = load(xrow(q), c);
+                        acc_exact2(v, l, pk2(a.x, a.x), pk2(-a.x, -a.x), pk2(x.x, x.y), m1);
+                        acc_exact2(v, l, pk2(a.y, a.y), pk2(-a.y, -a.y), pk2(-x.y, x.x), m1);
+                        acc_exact2(v, l, pk2(a.z, a.z), pk2(-a.z, -a.z), pk2(x.z, x.w), m1);
+                        acc_exact2(v, l, pk2(a.w, a.w), pk2(-a.w, -a.w), pk2(-x.w, x.z), m1);
                     }
+                    sum_put(r, q, v, l);
                 }
             }
         }
@@ -953,8 +1003,8 @@ __global__ void __launch_bounds__(32 * (GrpCfg<EXACT>::kWarps + 1), 1) k_mv_grp(
                 const KSys &S = tb->sys[mt.first + mbase + q];
 #pragma unroll
                 for (int r = 0; r < RW; ++r) {
-                    const double tr = warp_sum_d((double)ar[r][q] + (double)er[r][q]);
-                    const double ti = warp_sum_d((double)ai[r][q] + (double)ei[r][q]);
+                    const float4 v = sum[(r * MW + q) * 32];
+                    const double tr = warp_sum_d((double)v.x + (double)v.z), ti = warp_sum_d((double)v.y + (double)v.w);
                     if (lane == 0 && rbase + r < mt.nrows) S.mvp[mt.row0 + rbase + r] = make_double2(tr, ti);
                 }
             }
@@ -2301,26 +2351,16 @@ __global__ void __launch_bounds__(128) k_trisolve(const KTable *tb) {
     }
 }
 
-// x += d for the thread's row; complex64 systems also keep the float forms
-// of x (first cycle) or d (later cycles) that the residual products read
+// x += d for the thread's row; complex64 systems also keep the float copy of d
+// that the residual products read (x = 0 before the first cycle and d is formed
+// in floats, so there it is x itself, exactly)
 template <bool C128>
-__device__ __forceinline__ void xupdate_finish(const KSys &S, const KState *st, int row, double2 t) {
+__device__ __forceinline__ void xupdate_finish(const KSys &S, int row, double2 t) {
     double2 xv = S.x[row];
     xv.x += t.x;
     xv.y += t.y;
     S.x[row] = xv;
-    if (!C128 && st->cycles == 1) {
-        // first residual: (hi, lo) float split of x, stored so that
-        // chunk entries 2c and 2c + 1 land in the chunk's first and
-        // second half (conflict-free reads in the product)
-        const float hr = (float)xv.x, hi = (float)xv.y;
-        const int c = row & (kMvChunk - 1);
-        S.xf[(size_t)(row - c) + (c & 1) * (kMvChunk / 2) + (c >> 1)] =
-            make_float4(hr, hi, (float)(xv.x - (double)hr), (float)(xv.y - (double)hi));
-    } else if (!C128) {
-        // later residuals: r -= A d, with the float copy of d
-        S.xh[row] = make_float2((float)t.x, (float)t.y);
-    }
+    if (!C128) S.xh[row] = make_float2((float)t.x, (float)t.y);
 }
 
 // x += M^{-1} (V y)
@@ -2356,7 +2396,7 @@ __global__ void __launch_bounds__(kThreads) k_xupdate(const KTable *tb) {
                 tf = apply_minv_f(S.Minv, n, blk, vf);
             }
             if (row < n) {
-                if (!S.pcw) xupdate_finish<false>(S, st, row, make_double2((double)tf.x, (double)tf.y));
+                if (!S.pcw) xupdate_finish<false>(S, row, make_double2((double)tf.x, (double)tf.y));
                 else reinterpret_cast<float2 *>(S.pcy)[row] = tf;   // k_pcfin adds the corrected d
             }
             __syncthreads();
@@ -2378,7 +2418,7 @@ __global__ void __launch_bounds__(kThreads) k_xupdate(const KTable *tb) {
                 t = apply_minv(S.Minv, n, blk, vs);
             }
             if (row < n) {
-                if (!S.pcw) xupdate_finish<true>(S, st, row, t);
+                if (!S.pcw) xupdate_finish<true>(S, row, t);
                 else ((double2 *)S.pcy)[row] = t;   // k_pcfin adds the corrected d
             }
             __syncthreads();
@@ -2534,7 +2574,7 @@ __global__ void __launch_bounds__(kThreads) k_pcfin(const KTable *tb, int mode) 
                 V u;
                 u.x = 2 * y.x - q.x;
                 u.y = 2 * y.y - q.y;
-                if (mode == 2) xupdate_finish<C128>(S, S.st, row, make_double2((double)u.x, (double)u.y));
+                if (mode == 2) xupdate_finish<C128>(S, row, make_double2((double)u.x, (double)u.y));
                 else if constexpr (C128) S.z[row] = u;
                 else S.xh[row] = u;
             }
@@ -2671,16 +2711,12 @@ cudaError_t krylov_prepare() {
         if (sms <= 0) sms = 1;
         if (err == cudaSuccess)
             err = cudaFuncSetAttribute(k_mv_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       tma_smem_bytes(false));
+                                       kTmaSmem);
         if (err == cudaSuccess)
             err = cudaFuncSetAttribute(k_mv_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       tma_smem_bytes(true));
+                                       kTmaSmem);
         if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(k_mv_grp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       grp_smem_bytes(false));
-        if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(k_mv_grp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       grp_smem_bytes(true));
+            err = cudaFuncSetAttribute(k_mv_grp, cudaFuncAttributeMaxDynamicSharedMemorySize, kGrpSmem);
         if (err == cudaSuccess)
             err = cudaFuncSetAttribute(k_mv_grp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (err == cudaSuccess)
@@ -2713,7 +2749,7 @@ cudaError_t launch_product(KTable *d_tab, int prec, cudaStream_t st) {
     if (!g_vec_grid) return cudaErrorNotReady;   // krylov_prepare() first
     constexpr int kTmaThreads = 32 * (kTmaConsumers + 1);
     if (prec == 0) k_mv64<false><<<g_mv_grid[0], 256, 0, st>>>(d_tab, 0);
-    else k_mv_tma<false><<<g_mv_grid[1], kTmaThreads, tma_smem_bytes(false), st>>>(d_tab, 0);
+    else k_mv_tma<false><<<g_mv_grid[1], kTmaThreads, kTmaSmem, st>>>(d_tab, 0);
     return cudaGetLastError();
 }
 
@@ -2747,7 +2783,7 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev
         if (mv_ev) cudaEventRecordWithFlags(mv_ev[2 * q], st, cudaEventRecordExternal);
         if (c128) k_mv64<false><<<gmv, 256, 0, st>>>(tb, 0);
         else {
-            if (dense) k_mv_tma<false><<<gmv, kTmaThreads, tma_smem_bytes(false), st>>>(tb, 0);
+            if (dense) k_mv_tma<false><<<gmv, kTmaThreads, kTmaSmem, st>>>(tb, 0);
             else --nl;   // counted with the step's 8 below
             if (groups) {
                 k_mv_grp_tc<<<gmv, 32 * (kTcWarps + 1), kTcSmem, st>>>(tb, 0);
@@ -2792,9 +2828,9 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev
     if (c128) k_mv64<true><<<gmv, 256, 0, st>>>(tb, 1);
     else {
         // first-cycle residuals with error-free products, then the recursive updates
-        k_mv_tma<true><<<gmv, kTmaThreads, tma_smem_bytes(true), st>>>(tb, 1);
-        if (groups) k_mv_grp<true><<<gmv, 32 * (GrpCfg<true>::kWarps + 1), grp_smem_bytes(true), st>>>(tb, 1);
-        k_mv_tma<false><<<gmv, kTmaThreads, tma_smem_bytes(false), st>>>(tb, 2);
+        k_mv_tma<true><<<gmv, kTmaThreads, kTmaSmem, st>>>(tb, 1);
+        if (groups) k_mv_grp<<<gmv, 32 * (kGrpWarps + 1), kGrpSmem, st>>>(tb, 1);
+        k_mv_tma<false><<<gmv, kTmaThreads, kTmaSmem, st>>>(tb, 2);
         if (groups) k_mv_grp_tc<<<gmv, 32 * (kTcWarps + 1), kTcSmem, st>>>(tb, 2);
         nl += groups ? 3 : 1;
     }

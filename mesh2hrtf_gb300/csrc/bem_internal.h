@@ -320,7 +320,6 @@ struct KSys {
                                       // complex64 systems: w, V (and the inner-
                                       // product partials) hold float pairs
     float2 *xh;             // complex64 systems: float copy of the next product's input
-    float4 *xf;             // complex64 systems: x as (hi, lo) floats, chunk-permuted
     long long ldv;
     double2 *mvp;           // matvec partials [nchunk][n]
     double2 *dpa, *dpb;     // inner-product partials [kMaxRestart + 1][nvb]

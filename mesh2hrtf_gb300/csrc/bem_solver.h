@@ -77,7 +77,6 @@ struct SolverBufs {
     double2 *b = nullptr, *x = nullptr, *r = nullptr, *w = nullptr, *z = nullptr, *V = nullptr;
     double2 *mvp = nullptr, *dpa = nullptr, *dpb = nullptr;
     float2 *xh = nullptr;
-    float4 *xf = nullptr;
     double *nrmp = nullptr;
     double2 *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr, *y = nullptr, *hsum = nullptr;
     void *Minv = nullptr, *Mwork = nullptr;
@@ -162,7 +161,7 @@ struct bem_solver_s {
         k.nvb = bem::vec_blocks(n);
         k.Minv = d.Minv;
         k.x = d.x; k.b = d.b; k.r = d.r; k.w = d.w; k.z = d.z; k.V = d.V;
-        k.xh = d.xh; k.xf = d.xf;
+        k.xh = d.xh;
         k.ldv = n;
         k.mvp = d.mvp; k.dpa = d.dpa; k.dpb = d.dpb; k.nrmp = d.nrmp;
         k.H = d.H; k.cs = d.cs; k.sn = d.sn; k.g = d.g; k.y = d.y; k.hsum = d.hsum;
