@@ -2467,6 +2467,7 @@ __global__ void __launch_bounds__(kThreads) k_pcwin(const KTable *tb, int mode) 
     for (int it = blockIdx.x; it < tb->vb_total * items; it += gridDim.x) {
         const int2 bi = tb->vb_items[it / items];
         const KSys &S = tb->sys[bi.x];
+        if (S.shared) continue;   // k_pcwin_grp
         if (!__syncthreads_or(pcw_active(S, mode))) continue;   // one answer per block: k_givens may run beside this
         const int n = S.n, r0 = bi.y * kThreads + (it % items) * rows;
         if (r0 >= n) continue;
@@ -2535,6 +2536,113 @@ __global__ void __launch_bounds__(kThreads) k_pcwin(const KTable *tb, int mode) 
                 sr = warp_sum_f(sr);
                 si = warp_sum_f(si);
                 if (lane == 0) ((float2 *)S.pcz)[r] = make_float2(sr * scale, si * scale);
+            }
+        }
+    }
+}
+
+// z = A_w y of the right-hand sides that share A (complex64): one read of the
+// windows for all of them.  A warp takes 4 rows; its lanes' entries of A serve
+// every member's y, in shared memory.  A row is summed in k_pcwin's order.  HBM
+// takes 84 us for the windows of 69620 unknowns, a right-hand side alone 135
+// (one load ahead per lane and row), eight 188; each on its own read them in
+// turn, 700 us for eight.  y staged half a window at a time through registers:
+// 307.
+constexpr int kPcgThreads = 128, kPcgRows = 4;
+constexpr int kPcgSmem = kMaxGroup * kPcWin * 8;
+__global__ void __launch_bounds__(kPcgThreads, 3) k_pcwin_grp(const KTable *tb, int mode) {
+    extern __shared__ __align__(16) unsigned char pcg_raw[];
+    float2 (*ysh)[kPcWin] = reinterpret_cast<float2 (*)[kPcWin]>(pcg_raw);
+    __shared__ unsigned active;
+    if (!tb->pcw_any) return;
+    constexpr int kItemRows = kPcgThreads / 32 * kPcgRows;
+    static_assert(kPcWin % kItemRows == 0, "an item's rows lie in one window");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int first_item = 0;
+    for (int q = 0; q < tb->n_groups; ++q) {
+        const KGroup g = tb->grp[q];
+        const KSys &S = tb->sys[g.first];
+        const int n = S.n, items = ceil_div(n, kItemRows);
+        // one answer per group and block: k_givens may run beside this
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned b = __ballot_sync(0xffffffffu, lane < g.count && pcw_active(tb->sys[g.first + min(lane, g.count - 1)], mode));
+            if (lane == 0) active = b;
+        }
+        __syncthreads();
+        const unsigned mask = active;
+        if (!mask) continue;
+        // items go round the blocks across the groups
+        int it = (int)((blockIdx.x + gridDim.x - (unsigned)first_item % gridDim.x) % gridDim.x);
+        first_item += items;
+        for (; it < items; it += gridDim.x) {
+            const int r0 = it * kItemRows + warp * kPcgRows, c0 = it * kItemRows / kPcWin * kPcWin;
+            float sr[kPcgRows][kMaxGroup], si[kPcgRows][kMaxGroup];
+#pragma unroll
+            for (int r = 0; r < kPcgRows; ++r)
+#pragma unroll
+                for (int m = 0; m < kMaxGroup; ++m) sr[r][m] = si[r][m] = 0.f;
+            const float4 *a[kPcgRows];   // rows past the end repeat the last
+#pragma unroll
+            for (int r = 0; r < kPcgRows; ++r)
+                a[r] = reinterpret_cast<const float4 *>((const float2 *)S.A + (size_t)min(r0 + r, n - 1) * S.lda + c0);
+            const int nw = min(kPcWin, n - c0);   // columns of the window
+            // entries 2c, 2c + 1; an odd window's last column alone
+            auto get = [&](int r, int c) {
+                if (2 * c + 1 < nw) return a[r][c];
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (2 * c < nw) {
+                    const float2 f = *reinterpret_cast<const float2 *>(a[r] + c);
+                    v.x = f.x;
+                    v.y = f.y;
+                }
+                return v;
+            };
+            float4 nx[kPcgRows];
+#pragma unroll
+            for (int r = 0; r < kPcgRows; ++r) nx[r] = get(r, lane);
+            __syncthreads();   // the previous item's rows are done with ysh
+            for (int m = 0; m < g.count; ++m) {
+                if (!((mask >> m) & 1)) continue;
+                const float2 *y = (const float2 *)tb->sys[g.first + m].pcy + c0;
+                for (int c = 2 * threadIdx.x; c < kPcWin; c += 2 * kPcgThreads) {
+                    // zero past the window's end
+                    const int bytes = 8 * max(0, min(2, nw - c));
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&ysh[m][c])),
+                                 "l"(bytes ? y + c : y), "r"(bytes)
+                                 : "memory");
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+#pragma unroll 1
+            for (int c = lane; c < kPcWin / 2; c += 32) {
+                float4 v[kPcgRows];
+#pragma unroll
+                for (int r = 0; r < kPcgRows; ++r) {
+                    v[r] = nx[r];
+                    if (c + 32 < kPcWin / 2) nx[r] = get(r, c + 32);
+                }
+#pragma unroll
+                for (int m = 0; m < kMaxGroup; ++m) {
+                    if (!((mask >> m) & 1)) continue;
+                    const float4 y = reinterpret_cast<const float4 *>(ysh[m])[c];
+#pragma unroll
+                    for (int r = 0; r < kPcgRows; ++r) {
+                        cmac(sr[r][m], si[r][m], make_float2(v[r].x, v[r].y), make_float2(y.x, y.y));
+                        cmac(sr[r][m], si[r][m], make_float2(v[r].z, v[r].w), make_float2(y.z, y.w));
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < kMaxGroup; ++m) {
+                if (!((mask >> m) & 1)) continue;
+                float2 *z = (float2 *)tb->sys[g.first + m].pcz;
+#pragma unroll
+                for (int r = 0; r < kPcgRows; ++r) {
+                    const float2 t = make_float2(warp_sum_f(sr[r][m]), warp_sum_f(si[r][m]));
+                    if (lane == 0 && r0 + r < n) z[r0 + r] = t;
+                }
             }
         }
     }
@@ -2693,6 +2801,7 @@ __global__ void __launch_bounds__(kMaxSys) k_plans(KTable *tb) {
 int g_mv_grid[2] = {0, 0};
 int g_vec_grid = 0;
 int g_pcw_grid = 0;   // k_pcwin: every block it can keep resident (loads in flight)
+int g_pcg_grid = 0;   // k_pcwin_grp, likewise
 int g_blr_grid = 0;   // k_mv_blr: every block it can keep resident
 std::atomic<long long> g_launches{0};
 
@@ -2734,6 +2843,11 @@ cudaError_t krylov_prepare() {
         if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcwin<false>, kThreads, 0);
         g_pcw_grid = sms * (per > 0 ? per : 1);
         per = 0;
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_pcwin_grp, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgSmem);
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcwin_grp, kPcgThreads, kPcgSmem);
+        g_pcg_grid = sms * (per > 0 ? per : 1);
+        per = 0;
         if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mv_blr, kBlrThreads, 0);
         g_blr_grid = sms * (per > 0 ? per : 1);
     });
@@ -2759,15 +2873,18 @@ cudaError_t launch_plans(KTable *d_tab, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// the two launches of the preconditioner's window correction
-static void pc_window(bool c128, const KTable *d_tab, int mode, int gv, cudaStream_t st) {
+// the launches of the preconditioner's window correction (two, or three with
+// both shared-matrix groups and other systems); returns those beyond two
+static int pc_window(bool c128, const KTable *d_tab, int mode, int gv, cudaStream_t st, bool groups, bool single) {
     if (c128) {
         k_pcwin<true><<<g_pcw_grid, kThreads, 0, st>>>(d_tab, mode);
         k_pcfin<true><<<gv, kThreads, 0, st>>>(d_tab, mode);
     } else {
-        k_pcwin<false><<<g_pcw_grid, kThreads, 0, st>>>(d_tab, mode);
+        if (groups) k_pcwin_grp<<<g_pcg_grid, kPcgThreads, kPcgSmem, st>>>(d_tab, mode);
+        if (single || !groups) k_pcwin<false><<<g_pcw_grid, kThreads, 0, st>>>(d_tab, mode);
         k_pcfin<false><<<gv, kThreads, 0, st>>>(d_tab, mode);
     }
+    return !c128 && groups && single ? 1 : 0;
 }
 
 cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev, cudaStream_t st,
@@ -2816,14 +2933,14 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev
         cudaStreamWaitEvent(side.st, side.fork, 0);
         k_givens<<<1, kMaxSys, 0, side.st>>>(tb);
         cudaEventRecord(side.join, side.st);
-        pc_window(c128, d_tab, 0, gv, st);
+        nl += pc_window(c128, d_tab, 0, gv, st, groups, dense || blr);
         cudaStreamWaitEvent(st, side.join, 0);
         nl += 8;
     }
     k_trisolve<<<(kMaxSys + 3) / 4, 128, 0, st>>>(d_tab);
     if (c128) k_xupdate<true><<<gv, kThreads, 0, st>>>(d_tab);
     else k_xupdate<false><<<gv, kThreads, 0, st>>>(d_tab);
-    pc_window(c128, d_tab, 2, gv, st);
+    nl += pc_window(c128, d_tab, 2, gv, st, groups, dense || blr);
     if (mv_ev) cudaEventRecordWithFlags(mv_ev[2 * kSteps], st, cudaEventRecordExternal);
     if (c128) k_mv64<true><<<gmv, 256, 0, st>>>(tb, 1);
     else {
@@ -2839,7 +2956,7 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev
     k_decide<<<1, kMaxSys, 0, st>>>(tb);
     if (c128) k_scale<true, true><<<gv, kThreads, 0, st>>>(d_tab);
     else k_scale<false, true><<<gv, kThreads, 0, st>>>(d_tab);
-    pc_window(c128, d_tab, 1, gv, st);
+    nl += pc_window(c128, d_tab, 1, gv, st, groups, dense || blr);
     nl += 10;
     e = cudaGetLastError();
     if (launches_out) *launches_out = nl;
