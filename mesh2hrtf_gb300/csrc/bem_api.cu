@@ -814,7 +814,7 @@ bem_status solve_group(bem_solver_t *ss, int cnt, bem::Engine *eng, cudaStream_t
             s->info.iterations = q.iters;
             s->info.restarts = q.cycles;
             s->info.rel_residual = q.rel;
-            s->info.matvec_ms = eng->timing_ok() ? eng->matvec_ms() : 0.0;
+            s->info.matvec_ms = eng->matvec_ms();
             s->info.n_matvec = q.n_mv;
             s->solved = true;
             if (q.phase != bem::kPhaseFinished) rcs[c0 + i] = fail(BEM_ERR_DEVICE_TIMEOUT, "GMRES did not finish");
@@ -1487,7 +1487,7 @@ bem_status bem_solve_multi(bem_solver_t s, int32_t R, const bem_frequency_desc *
     float sms = 0.f;
     CU(cudaEventElapsedTime(&sms, s->ev[2], s->ev[3]));
     s->info.solve_ms = sms;
-    s->info.matvec_ms = eng->timing_ok() ? eng->matvec_ms() : 0.0;
+    s->info.matvec_ms = eng->matvec_ms();
     s->solved = true;
     bem_status first = BEM_OK;
     std::vector<bem::KState> fin(eng->states(), eng->states() + R);

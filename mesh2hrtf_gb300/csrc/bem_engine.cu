@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdlib>
+#include <cstddef>
 #include <cstring>
 
 #include <cudaTypedefs.h>
@@ -181,7 +182,6 @@ cudaError_t Engine::set_batch(const std::vector<KSys> &sys, const std::vector<KS
     if (e == cudaSuccess) e = launch_plans(d_tab_, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     B_ = B;
-    mv_ms_ = 0.0;
     bodies_ = 0;
     return e;
 }
@@ -232,8 +232,8 @@ cudaError_t Engine::run_body() {
         cudaGraph_t g = nullptr;
         e = cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
-        cudaError_t le = launch_krylov_body(prec_, d_tab_, ev_, st_, &body_launches_[v], (v & 1) != 0,
-                                                   (v & 2) != 0, (v & 4) != 0, side_);
+        cudaError_t le = launch_krylov_body(prec_, d_tab_, st_, &body_launches_[v], (v & 1) != 0,
+                                            (v & 2) != 0, (v & 4) != 0, side_);
         e = cudaStreamEndCapture(st_, &g);
         if (le != cudaSuccess) e = le;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_[v], g, 0);
@@ -246,23 +246,14 @@ cudaError_t Engine::run_body() {
     e = cudaGraphLaunch(exec_[v], st_);
     if (e == cudaSuccess && B_ > 0)
         e = cudaMemcpyAsync(h_st_, d_st_, sizeof(KState) * B_, cudaMemcpyDeviceToHost, st_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_tab_->err, &d_tab_->err, sizeof(int), cudaMemcpyDeviceToHost, st_);
+    if (e == cudaSuccess)   // err and mv_ns
+        e = cudaMemcpyAsync(&h_tab_->err, &d_tab_->err, offsetof(KTable, mv_t0) - offsetof(KTable, err),
+                            cudaMemcpyDeviceToHost, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     if (e != cudaSuccess) return e;
     if (h_tab_->err) return cudaErrorLaunchTimeout;   // a bounded wait in the product gave up
     count_launches(body_launches_[v]);
     ++bodies_;
-    if (timing_ok_) {
-        for (int q = 0; q <= kSteps; ++q) {
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, ev_[2 * q], ev_[2 * q + 1]) != cudaSuccess) {
-                cudaGetLastError();
-                timing_ok_ = false;
-                break;
-            }
-            mv_ms_ += ms;
-        }
-    }
     return cudaSuccess;
 }
 

@@ -39,9 +39,8 @@ public:
     // the tuner, before set_batch (it overwrites the launch table).
     cudaError_t time_product(const KSys &sys, float *ms);
     // device time of the matrix-vector products (ms) and body replays since set_batch
-    double matvec_ms() const { return mv_ms_; }
+    double matvec_ms() const { return h_tab_ ? 1e-6 * (double)h_tab_->mv_ns : 0.0; }
     long long bodies() const { return bodies_; }
-    bool timing_ok() const { return timing_ok_; }
 
 private:
     cudaError_t ensure_init();
@@ -62,11 +61,9 @@ private:
     int groups_ = 0;   // shared-matrix groups of the current batch
     int blr_ = 0;      // systems of the current batch with a block low-rank copy
     int dense_ = 0;    // single systems whose Krylov products read A or its fp16 copy
-    cudaEvent_t ev_[2 * (kSteps + 1)] = {};
+    cudaEvent_t ev_[2] = {};   // time_product
     SideStream side_{};   // the captured body's second branch
-    double mv_ms_ = 0.0;
     long long bodies_ = 0;
-    bool timing_ok_ = true;
 };
 
 }  // namespace bem

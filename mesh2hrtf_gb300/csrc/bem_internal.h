@@ -364,6 +364,7 @@ struct KTable {
     int prec;               // 0: complex128 tiles, 1: complex64 strips
     int vb_total;           // vector blocks of all systems
     int err;                // set when a bounded device wait gave up
+    unsigned long long mv_ns, mv_t0;   // device time of the products so far, start of the one under way
     int pcw_any;            // some system applies the window correction
     long long wait_cycles;  // bound of the products' mbarrier waits in clock
                             // cycles (0: the default of about 2 s); a test
@@ -403,8 +404,7 @@ constexpr int kGrpCols = 256;
 // Arnoldi steps per iteration body.
 constexpr int kSteps = 8;
 // Enqueues one iteration body for the systems of *d_tab (device memory) on
-// st.  mv_ev: 2 * (kSteps + 1) events recorded around the matrix-vector
-// products (may be nullptr).  prec: 0 complex128, 1 complex64 matrices.
+// st.  prec: 0 complex128, 1 complex64 matrices.
 // groups: include the shared-matrix (group) products, for batches that have
 // groups; blr: include the block low-rank product (k_mv_blr), for batches
 // with systems that have a block low-rank copy; dense: include the Krylov
@@ -417,7 +417,7 @@ struct SideStream {
     cudaStream_t st;
     cudaEvent_t fork, join;
 };
-cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaEvent_t *mv_ev, cudaStream_t st,
+cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaStream_t st,
                                int *launches_out, bool groups, bool blr, bool dense, const SideStream &side);
 // complex64 matrices: the product streams row segments with bulk copies
 // (TMA) in strips of `strip` rows (a multiple of kTmaRows, chosen per system
