@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 
 #include <cstdlib>
+#include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstring>
 
@@ -68,8 +70,9 @@ long long test_wait_cycles() {
 
 Engine::~Engine() {
     if (st_) cudaStreamSynchronize(st_);
-    for (auto &x : exec_)
-        if (x) cudaGraphExecDestroy(x);
+    for (auto &part : exec_)
+        for (auto &x : part)
+            if (x) cudaGraphExecDestroy(x);
     for (auto &e : ev_)
         if (e) cudaEventDestroy(e);
     if (side_.fork) cudaEventDestroy(side_.fork);
@@ -182,6 +185,7 @@ cudaError_t Engine::set_batch(const std::vector<KSys> &sys, const std::vector<KS
     if (e == cudaSuccess) e = launch_plans(d_tab_, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     B_ = B;
+    rate_.assign(B, 0.0);
     bodies_ = 0;
     return e;
 }
@@ -224,26 +228,53 @@ cudaError_t Engine::time_product(const KSys &sys, float *ms) {
     return e;
 }
 
+cudaError_t Engine::capture(int part, int v) {
+    if (exec_[part][v]) return cudaSuccess;
+    const bool groups = v & 1, blr = v & 2, dense = v & 4;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    const cudaError_t le =
+        part == 0 ? launch_krylov_step(prec_, d_tab_, st_, &launches_[0][v], groups, blr, dense, side_)
+                  : launch_krylov_cycle_end(prec_, d_tab_, st_, &launches_[1][v], groups, blr, dense);
+    e = cudaStreamEndCapture(st_, &g);
+    if (le != cudaSuccess) e = le;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_[part][v], g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) exec_[part][v] = nullptr;
+    return e;
+}
+
+// Arnoldi steps of the next body: what the system furthest from the end of its
+// cycle is expected to need (at the rate of its cycle so far, or of its last
+// one; kSteps without either), at most kSteps, none before the first residual.
+// A step too many is some ten empty launches (1280 triangles: 16 us), one too
+// few an empty end of cycle and a wait for the host (40 us), hence the half
+// step on top.  The number changes when a cycle's end is seen, not its result.
+int Engine::steps_ahead() const {
+    int most = 0;
+    for (int b = 0; b < B_; ++b) {
+        const KState &q = h_st_[b];
+        if (q.phase != kPhaseArnoldi) continue;
+        const double from = q.k > 0 ? q.res : q.beta, rate = q.k > 0 ? std::log(q.beta / q.res) / q.k : rate_[b];
+        const double need = std::log(from / q.thr) / rate + 0.5;
+        int s = kSteps;
+        if (rate > 0.0 && need < kSteps) s = need > 1.0 ? (int)std::ceil(need) : 1;
+        most = std::max(most, std::min(s, q.m - q.k));
+    }
+    return std::min(most, kSteps);
+}
+
 cudaError_t Engine::run_body() {
     cudaError_t e = ensure_init();
     if (e != cudaSuccess) return e;
     const int v = (groups_ > 0 ? 1 : 0) | (blr_ > 0 ? 2 : 0) | (dense_ > 0 ? 4 : 0);
-    if (!exec_[v]) {
-        cudaGraph_t g = nullptr;
-        e = cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        cudaError_t le = launch_krylov_body(prec_, d_tab_, st_, &body_launches_[v], (v & 1) != 0,
-                                            (v & 2) != 0, (v & 4) != 0, side_);
-        e = cudaStreamEndCapture(st_, &g);
-        if (le != cudaSuccess) e = le;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_[v], g, 0);
-        if (g) cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            exec_[v] = nullptr;
-            return e;
-        }
-    }
-    e = cudaGraphLaunch(exec_[v], st_);
+    const int steps = steps_ahead();
+    if (steps > 0) e = capture(0, v);
+    if (e == cudaSuccess) e = capture(1, v);
+    for (int q = 0; q < steps && e == cudaSuccess; ++q) e = cudaGraphLaunch(exec_[0][v], st_);
+    if (e == cudaSuccess) e = cudaGraphLaunch(exec_[1][v], st_);
+    std::vector<KState> was(h_st_, h_st_ + B_);
     if (e == cudaSuccess && B_ > 0)
         e = cudaMemcpyAsync(h_st_, d_st_, sizeof(KState) * B_, cudaMemcpyDeviceToHost, st_);
     if (e == cudaSuccess)   // err and mv_ns
@@ -252,7 +283,12 @@ cudaError_t Engine::run_body() {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     if (e != cudaSuccess) return e;
     if (h_tab_->err) return cudaErrorLaunchTimeout;   // a bounded wait in the product gave up
-    count_launches(body_launches_[v]);
+    count_launches(steps * launches_[0][v] + launches_[1][v]);
+    for (int b = 0; b < B_; ++b) {   // the rate of a cycle that ended
+        const KState &q = h_st_[b];
+        const int len = q.iters - (was[b].iters - was[b].k);
+        if (q.cycles > was[b].cycles && len > 0) rate_[b] = std::log(q.prev_beta / q.res) / len;
+    }
     ++bodies_;
     return cudaSuccess;
 }

@@ -52,12 +52,15 @@ private:
     int2 *d_items_ = nullptr;
     size_t items_cap_ = 0;
     std::vector<int2> items_;
-    // the iteration body's variants: with the shared-matrix (group) products
-    // (bit 0), with the block low-rank product (bit 1), with the product of
-    // single systems from A or its fp16 copy (bit 2); each captured at its
-    // first replay
-    cudaGraphExec_t exec_[8] = {};
-    int body_launches_[8] = {};
+    int steps_ahead() const;
+    cudaError_t capture(int part, int v);
+    // the graphs of the Arnoldi step and the end of cycle, in variants: with
+    // the shared-matrix (group) products (bit 0), with the block low-rank
+    // product (bit 1), with the product of single systems from A or its fp16
+    // copy (bit 2); each captured at its first replay
+    cudaGraphExec_t exec_[2][8] = {};
+    int launches_[2][8] = {};
+    std::vector<double> rate_;   // per system: log reduction per step of its last cycle (0: none yet)
     int groups_ = 0;   // shared-matrix groups of the current batch
     int blr_ = 0;      // systems of the current batch with a block low-rank copy
     int dense_ = 0;    // single systems whose Krylov products read A or its fp16 copy

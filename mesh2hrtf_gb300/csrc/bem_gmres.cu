@@ -9,12 +9,12 @@
 // default) are NumCalc's.
 //
 // Every system of the batch carries a small state machine (KState) in device
-// memory.  An iteration body runs kSteps Arnoldi steps for each system in
+// memory.  An iteration body runs up to kSteps Arnoldi steps for each system in
 // phase ARNOLDI and then the end of cycle for each system in phase UPDATE;
 // kernels skip the systems that are in another phase.  The body never needs
-// the host, so it is captured once as a CUDA graph and replayed; the host
-// reads the states after each replay and admits or retires systems between
-// replays.  The per-system arithmetic does not depend on the other systems of
+// the host, so the step and the end of cycle are each captured once as a CUDA
+// graph; the host replays the first as often as the body has steps and then the
+// second, reads the states and admits or retires systems between bodies.  The per-system arithmetic does not depend on the other systems of
 // the batch, so a system's result is the same alone and in any mix.
 //
 // Arnoldi step k (8 launches):
@@ -2962,54 +2962,63 @@ static int pc_window(bool c128, const KTable *d_tab, int mode, int gv, cudaStrea
     return !c128 && groups && single ? 1 : 0;
 }
 
-cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaStream_t st,
-                               int *launches_out, bool groups, bool blr, bool dense, const SideStream &side) {
+cudaError_t launch_krylov_step(int prec, const KTable *d_tab, cudaStream_t st, int *launches_out, bool groups, bool blr,
+                               bool dense, const SideStream &side) {
     KTable *tb = const_cast<KTable *>(d_tab);
     const bool c128 = prec == 0;
     if (!g_vec_grid) return cudaErrorNotReady;   // krylov_prepare() first
     const int gmv = g_mv_grid[c128 ? 0 : 1], gv = g_vec_grid;
     int nl = 0;
-    cudaError_t e = cudaSuccess;
     constexpr int kTmaThreads = 32 * (kTmaConsumers + 1);
-    for (int q = 0; q < kSteps; ++q) {
-        if (c128) body_launch(false, k_mv64<false>, gmv, 256, 0, st, tb, 0);
-        else {
-            if (dense) body_launch(false, k_mv_tma<false>, gmv, kTmaThreads, kTmaSmem, st, tb, 0);
-            else --nl;   // counted with the step's 8 below
-            if (groups) {
-                body_launch(dense, k_mv_grp_tc, gmv, 32 * (kTcWarps + 1), kTcSmem, st, tb, 0);
-                body_launch(true, k_mv_grp_umma, gmv, 32 * kUmWarps, kUmSmem, st, tb);
-                nl += 2;
-            }
-            if (blr) {
-                body_launch(dense || groups, k_mv_blr, g_blr_grid, kBlrThreads, 0, st, tb);
-                ++nl;
-            }
+    if (c128) body_launch(false, k_mv64<false>, gmv, 256, 0, st, tb, 0);
+    else {
+        if (dense) body_launch(false, k_mv_tma<false>, gmv, kTmaThreads, kTmaSmem, st, tb, 0);
+        else --nl;   // counted with the step's 8 below
+        if (groups) {
+            body_launch(dense, k_mv_grp_tc, gmv, 32 * (kTcWarps + 1), kTcSmem, st, tb, 0);
+            body_launch(true, k_mv_grp_umma, gmv, 32 * kUmWarps, kUmSmem, st, tb);
+            nl += 2;
         }
-        if (c128) {
-            body_launch(true, k_dot1<true>, gv, kThreads, 0, st, tb);
-            body_launch(true, k_axpy<1, true>, gv, kThreads, 0, st, d_tab);
-            body_launch(true, k_axpy<2, true>, gv, kThreads, 0, st, d_tab);
-        } else {
-            body_launch(true, k_dot1<false>, gv, kThreads, 0, st, tb);
-            body_launch(true, k_axpy<1, false>, gv, kThreads, 0, st, d_tab);
-            body_launch(true, k_axpy<2, false>, gv, kThreads, 0, st, d_tab);
+        if (blr) {
+            body_launch(dense || groups, k_mv_blr, g_blr_grid, kBlrThreads, 0, st, tb);
+            ++nl;
         }
-        if (c128) body_launch(true, k_scale<true, false>, gv, kThreads, 0, st, d_tab);
-        else body_launch(true, k_scale<false, false>, gv, kThreads, 0, st, d_tab);
-        // the rotations beside the window correction: both follow k_scale and
-        // precede the next product.  A system whose cycle ends here may see
-        // its phase change under the correction, whose result it then does
-        // not read (the cycle's update forms pcy, pcz and xh anew); a block of
-        // the correction decides as a whole whether it takes part.
-        cudaEventRecord(side.fork, st);
-        cudaStreamWaitEvent(side.st, side.fork, 0);
-        k_givens<<<1, kMaxSys, 0, side.st>>>(tb);
-        cudaEventRecord(side.join, side.st);
-        nl += pc_window(c128, d_tab, 0, gv, st, groups, dense || blr);
-        cudaStreamWaitEvent(st, side.join, 0);
-        nl += 8;
     }
+    if (c128) {
+        body_launch(true, k_dot1<true>, gv, kThreads, 0, st, tb);
+        body_launch(true, k_axpy<1, true>, gv, kThreads, 0, st, d_tab);
+        body_launch(true, k_axpy<2, true>, gv, kThreads, 0, st, d_tab);
+    } else {
+        body_launch(true, k_dot1<false>, gv, kThreads, 0, st, tb);
+        body_launch(true, k_axpy<1, false>, gv, kThreads, 0, st, d_tab);
+        body_launch(true, k_axpy<2, false>, gv, kThreads, 0, st, d_tab);
+    }
+    if (c128) body_launch(true, k_scale<true, false>, gv, kThreads, 0, st, d_tab);
+    else body_launch(true, k_scale<false, false>, gv, kThreads, 0, st, d_tab);
+    // the rotations beside the window correction: both follow k_scale and
+    // precede the next product.  A system whose cycle ends here may see
+    // its phase change under the correction, whose result it then does
+    // not read (the cycle's update forms pcy, pcz and xh anew); a block of
+    // the correction decides as a whole whether it takes part.
+    cudaEventRecord(side.fork, st);
+    cudaStreamWaitEvent(side.st, side.fork, 0);
+    k_givens<<<1, kMaxSys, 0, side.st>>>(tb);
+    cudaEventRecord(side.join, side.st);
+    nl += pc_window(c128, d_tab, 0, gv, st, groups, dense || blr);
+    cudaStreamWaitEvent(st, side.join, 0);
+    nl += 8;
+    if (launches_out) *launches_out = nl;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_krylov_cycle_end(int prec, const KTable *d_tab, cudaStream_t st, int *launches_out, bool groups,
+                                    bool blr, bool dense) {
+    KTable *tb = const_cast<KTable *>(d_tab);
+    const bool c128 = prec == 0;
+    if (!g_vec_grid) return cudaErrorNotReady;   // krylov_prepare() first
+    const int gmv = g_mv_grid[c128 ? 0 : 1], gv = g_vec_grid;
+    int nl = 0;
+    constexpr int kTmaThreads = 32 * (kTmaConsumers + 1);
     body_launch(false, k_trisolve, (kMaxSys + 3) / 4, 128, 0, st, d_tab);
     if (c128) body_launch(true, k_xupdate<true>, gv, kThreads, 0, st, d_tab);
     else body_launch(true, k_xupdate<false>, gv, kThreads, 0, st, d_tab);
@@ -3029,9 +3038,8 @@ cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaStream_t st,
     else body_launch(true, k_scale<false, true>, gv, kThreads, 0, st, d_tab);
     nl += pc_window(c128, d_tab, 1, gv, st, groups, dense || blr);
     nl += 10;
-    e = cudaGetLastError();
     if (launches_out) *launches_out = nl;
-    return e;
+    return cudaGetLastError();
 }
 
 }  // namespace bem

@@ -403,22 +403,23 @@ constexpr int kGrpCols = 256;
 
 // Arnoldi steps per iteration body.
 constexpr int kSteps = 8;
-// Enqueues one iteration body for the systems of *d_tab (device memory) on
-// st.  prec: 0 complex128, 1 complex64 matrices.
-// groups: include the shared-matrix (group) products, for batches that have
-// groups; blr: include the block low-rank product (k_mv_blr), for batches
-// with systems that have a block low-rank copy; dense: include the Krylov
-// product from A or its fp16 copy (k_mv_tma / k_mv64), for batches with
-// single systems without one (always for complex128).  Returns the number of
-// kernel launches enqueued through *launches_out.
+// Enqueue, for the systems of *d_tab (device memory), one Arnoldi step or the
+// end of cycle on st.  prec: 0 complex128, 1 complex64 matrices.  groups:
+// include the shared-matrix (group) products, for batches that have groups;
+// blr: include the block low-rank product (k_mv_blr), for batches with systems
+// that have a block low-rank copy; dense: include the Krylov product from A or
+// its fp16 copy (k_mv_tma / k_mv64), for batches with single systems without
+// one (always for complex128).  *launches_out: the kernel launches enqueued.
 // side: a second stream for the branch that runs beside the main one (joined
 // again before the next product), and the events that fork and join it.
 struct SideStream {
     cudaStream_t st;
     cudaEvent_t fork, join;
 };
-cudaError_t launch_krylov_body(int prec, const KTable *d_tab, cudaStream_t st,
-                               int *launches_out, bool groups, bool blr, bool dense, const SideStream &side);
+cudaError_t launch_krylov_step(int prec, const KTable *d_tab, cudaStream_t st, int *launches_out, bool groups, bool blr,
+                               bool dense, const SideStream &side);
+cudaError_t launch_krylov_cycle_end(int prec, const KTable *d_tab, cudaStream_t st, int *launches_out, bool groups,
+                                    bool blr, bool dense);
 // complex64 matrices: the product streams row segments with bulk copies
 // (TMA) in strips of `strip` rows (a multiple of kTmaRows, chosen per system
 // by the tuner; kTmaStrip by default); complex128: tiles of kMvRows rows.
