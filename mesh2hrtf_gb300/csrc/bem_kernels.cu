@@ -204,7 +204,7 @@ __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3]
 // 2 scalar FP32 operations and 6 special functions per two evaluations, and
 // about 45 per pair of entries); one entry at a time it was bound by
 // instruction issue at 79 per evaluation.  20480-triangle head, 10 kHz: k_far
-// 4.07 -> 3.33 ms (1280 triangles 50 us as before, 1536 quadrilaterals and their
+// 4.07 -> 3.33 ms (1280 triangles 50 us as before, 3072 quadrilaterals and their
 // images 690 -> 673).  Three blocks per SM with the column's data in shared
 // memory instead of two with it in registers: 3.77 ms.
 struct FarCol2 {
@@ -1039,7 +1039,11 @@ __device__ cplx<double> rhs_row(const DevMesh &m, const DevFreq &f, int i, const
 // the columns: far columns are integrated whole in their lane, subdivided ones
 // and the self pair by the warp, one at a time.  Integrating every column with
 // the warp left 28 of 32 lanes idle on the 4-point rule: 3072 quadrilaterals with
-// one image and 48 such columns 8.2 -> 1.5 ms.
+// one image and 48 such columns 8.2 -> 1.5 ms.  The rows beside those columns
+// subdivide many of them and are neighbours in the element order, so a block
+// takes rows that lie far apart: 1.49 -> 1.39 ms.  Sharing a block's subdivided
+// columns among its warps gave 1.28 but no shorter assembly; staging the
+// columns' points in shared memory 1.57, dealing them to a cluster 1.83.
 __global__ void __launch_bounds__(256) k_rhs(const __grid_constant__ AsmBatch tb) {
     __shared__ WarpScratch ws_all[8];
     const int sb = find_sys(tb.rhs_off, tb.B, blockIdx.x);
@@ -1058,7 +1062,7 @@ __global__ void __launch_bounds__(256) k_rhs(const __grid_constant__ AsmBatch tb
         b[i] = make_double2(z.re, z.im);
         return;
     }
-    const int i = blk * 8 + w;
+    const int i = w * (tb.rhs_off[sb + 1] - tb.rhs_off[sb]) + blk;   // neighbours in different blocks
     if (i >= n) return;
     WarpScratch &ws = ws_all[w];
     const double x[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
