@@ -11,8 +11,8 @@
 // needs no further set-up.
 //
 // Inversion: in-place Gauss-Jordan with partial pivoting, one block of kBlock
-// rows per cluster of CTAs that share its columns, entries in registers
-// (gauss_jordan_reg); the last, partial block of a system goes through shared
+// rows per CTA or per cluster of CTAs that share its columns, entries in
+// registers (gauss_jordan_one, gauss_jordan_cluster); the last, partial block of a system goes through shared
 // memory or a global workspace (gauss_jordan).  Inverses are stored transposed
 // so that the application (inside the Krylov kernels, bem_gmres.cu) reads them
 // coalesced.
@@ -131,34 +131,211 @@ __device__ void gauss_jordan(typename C2<T>::t *W, int ld, int nb, typename C2<T
     }
 }
 
-// The same on a full kBlock x kBlock block held in registers by CL CTAs of a
-// cluster: CTA r has the columns r kBlock / CL .. , thread t of NT its column
-// t % C (C = kBlock / CL) at rows kR (t / C) .. + kR - 1.  A step needs the
-// pivot column (published by the threads that hold it as soon as the step
-// before has updated it, in one of two buffers; the other CTAs fetch it through
-// distributed shared memory), the pivot with its inverse (one warp: square and
-// divisions on every warp took longer than the update) and the pivot row
-// (published by the threads that hold it).  Rows are not interchanged:
-// step k's pivot is the largest |a|^2 among the rows not used yet, lowest row
-// on ties, and with p_k its row the inverse is Ainv[k][p_c] = W[p_k][c].
+// The pivot of a column (v[q]: row lane + 32 q) by one warp: the largest |a|^2
+// among the rows not in used, lowest row on ties; nothing comparable (zero or
+// NaN) sets singular, and the lowest unused row serves.  Marks the row used.
+template <typename V>
+__device__ __forceinline__ int warp_pivot(const V (&v)[kBlock / 32], int lane, unsigned &used, int &singular) {
+    decltype(v[0].x + v[0].x) best = -1;
+    int p = kBlock;
+#pragma unroll
+    for (int q = 0; q < kBlock / 32; ++q) {
+        const auto m = v[q].x * v[q].x + v[q].y * v[q].y;
+        if (!((used >> q) & 1u) && m > best) {
+            best = m;
+            p = lane + 32 * q;
+        }
+    }
+    if constexpr (sizeof(best) == 4) {
+        // as whole numbers, in the same order: 0 for no candidate, else |a|^2's bits + 1
+        const unsigned key = p < kBlock ? __float_as_uint(best) + 1u : 0u, top = __reduce_max_sync(0xffffffffu, key);
+        p = (int)__reduce_min_sync(0xffffffffu, key == top ? (unsigned)p : (unsigned)kBlock);
+        best = top > 0u ? __uint_as_float(top - 1u) : -1.f;
+    } else {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const auto ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, p, o);
+            if (ob > best || (ob == best && oi < p)) { best = ob; p = oi; }
+        }
+    }
+    if (!(best > 0)) {
+        if (lane == 0) singular = 1;
+        if (p >= kBlock) {
+            int cand = kBlock;
+#pragma unroll
+            for (int q = kBlock / 32 - 1; q >= 0; --q)
+                if (!((used >> q) & 1u)) cand = lane + 32 * q;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
+            p = cand;
+        }
+    }
+    if (lane == (p & 31)) used |= 1u << (p >> 5);
+    return p;
+}
+
+// a - f r, in the order of operations of every step
+template <typename V> __device__ __forceinline__ V gj_update(V a, V f, V r) {
+    a.x = fma(-f.x, r.x, a.x);
+    a.x = fma(f.y, r.y, a.x);
+    a.y = fma(-f.x, r.y, a.y);
+    a.y = fma(-f.y, r.x, a.y);
+    return a;
+}
+
+// The same on a full kBlock x kBlock block held in registers by one CTA: thread
+// t of NT has columns t % C + c C (C = kBlock / NC) at rows kR (t / C) .. +
+// kR - 1.  A step
+// needs the pivot column, the pivot with its inverse, and the pivot row
+// (published by the threads that hold it).  Rows are not interchanged: step k's
+// pivot is the largest |a|^2 among the rows not used yet, lowest row on ties,
+// and with p_k its row the inverse is Ainv[k][p_c] = W[p_k][c].
 //
-// A full block in shared memory (three barriers a step, every entry loaded and
-// stored each step) was bound by shared-memory traffic: 306 us in complex64,
-// whatever the system's size; in registers 205 us.  complex128 is bound by
-// an SM's narrow FP64 pipe (4 FMA per entry and step), so its blocks spread
-// over four SMs: 40 blocks 3.9 ms in an L2 workspace, 1.24 ms now.
+// Warp 0 looks a step ahead: while the others update, it forms the next column
+// from its entries of the step before (published by their threads), finds its
+// pivot and inverts it, which needed a barrier of its own.  The column's factors
+// are loaded two rows at a time and serve NC columns: one column to a thread was
+// bound by those loads.  complex64, up to 152 blocks: 204 us as below on one
+// CTA, 199 with the look-ahead, 162 with two columns to a thread, 146 with the
+// pivot found by whole-number reductions; 1280 blocks 1.83 -> 1.34 ms.  What is
+// left is warp 0's chain.
+template <typename T, int NT, int NC>
+__device__ void gauss_jordan_one(const typename C2<T>::t *A, size_t lda, typename C2<T>::t *out, int *status) {
+    using V = typename C2<T>::t;
+    constexpr int C = kBlock / NC, G = NT / C, kR = kBlock / G;
+    static_assert(G * kR == kBlock && C % 32 == 0 && kR % 2 == 0, "threads cover the block, a warp one row group");
+    __shared__ __align__(16) V fcol[2][kBlock];   // the step's pivot column, by step parity
+    __shared__ __align__(16) V prev[2][kBlock];   // the next column before the step
+    __shared__ V rowb[kBlock], inv_s;
+    __shared__ int piv[kBlock], singular_s;
+    const int tid = threadIdx.x, lane = tid & 31, j = tid % C, i0 = tid / C * kR;
+    V a[NC][kR];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int q = 0; q < kR; ++q) a[c][q] = A[(size_t)(i0 + q) * lda + j + c * C];
+    if (j < 2) {
+#pragma unroll
+        for (int q = 0; q < kR; ++q) (j == 0 ? fcol[0] : prev[1])[i0 + q] = a[0][q];
+    }
+    if (tid == 0) singular_s = 0;
+    __syncthreads();
+    unsigned used = 0;   // warp 0, bit q: row lane + 32 q has been a pivot row
+    auto pivot = [&](int k, const V (&v)[kBlock / 32]) {
+        const int p = warp_pivot(v, lane, used, singular_s);
+        V b = v[0];
+#pragma unroll
+        for (int q = 1; q < kBlock / 32; ++q)
+            if ((p >> 5) == q) b = v[q];
+        if (lane == (p & 31)) {
+            piv[k] = p;
+            inv_s = cinv_pow2(b);
+        }
+    };
+    if (tid < 32) {
+        V v[kBlock / 32];
+#pragma unroll
+        for (int q = 0; q < kBlock / 32; ++q) v[q] = fcol[0][lane + 32 * q];
+        pivot(0, v);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < kBlock; ++k) {
+        const V *f = fcol[k & 1];
+        const int p = piv[k] - i0;   // the pivot row among this warp's rows
+        // the pivot row, scaled (its own column: 1 / pivot)
+        if (p >= 0 && p < kR) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                V r = a[c][0];
+#pragma unroll
+                for (int q = 1; q < kR; ++q)
+                    if (p == q) r = a[c][q];
+                if (j + c * C == k) { r.x = 1; r.y = 0; }
+                rowb[j + c * C] = cmul2(r, inv_s);
+            }
+        }
+        __syncthreads();
+        if (tid < 32 && k + 1 < kBlock) {
+            const V r = rowb[k + 1];
+            V v[kBlock / 32];
+#pragma unroll
+            for (int q = 0; q < kBlock / 32; ++q) {
+                const int i = lane + 32 * q;
+                v[q] = gj_update(prev[(k + 1) & 1][i], f[i], r);
+                if (i == piv[k]) v[q] = r;
+                fcol[(k + 1) & 1][i] = v[q];
+            }
+            pivot(k + 1, v);
+        }
+        V r[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            r[c] = rowb[j + c * C];
+            if (((j + c * C) >> 5) == (k >> 5)) {   // the warps with column k
+                if (j + c * C == k) {
+#pragma unroll
+                    for (int q = 0; q < kR; ++q) a[c][q].x = a[c][q].y = 0;
+                }
+            }
+        }
+        const float4 *f2 = reinterpret_cast<const float4 *>(f + i0);   // two rows to a load
+        static_assert(sizeof(V) == 8, "complex64");
+#pragma unroll
+        for (int q = 0; q < kR; q += 2) {
+            const float4 ff = f2[q / 2];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                a[c][q] = gj_update(a[c][q], make_float2(ff.x, ff.y), r[c]);
+                a[c][q + 1] = gj_update(a[c][q + 1], make_float2(ff.z, ff.w), r[c]);
+            }
+        }
+        if (p >= 0 && p < kR) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int q = 0; q < kR; ++q)
+                    if (p == q) a[c][q] = r[c];
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            if (j + c * C == k + 2) {
+#pragma unroll
+                for (int q = 0; q < kR; ++q) prev[k & 1][i0 + q] = a[c][q];
+            }
+        __syncthreads();
+    }
+    // row i was the pivot of step inv_p(i), column j holds the inverse's column
+    // p_j: Minv[c][r] (transposed) with r the step, c = piv[j]
+    int *step = reinterpret_cast<int *>(rowb);
+    if (tid < kBlock) step[piv[tid]] = tid;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int q = 0; q < kR; ++q) out[(size_t)piv[j + c * C] * kBlock + step[i0 + q]] = a[c][q];
+    if (tid == 0 && singular_s) atomicMax(status, 1);
+}
+
+// The same by CL CTAs of a cluster: CTA r has the columns r kBlock / CL .. .
+// The pivot column is published by the threads that hold it as soon as the step
+// before has updated it, in one of two buffers, and the other CTAs fetch it
+// through distributed shared memory; every CTA finds the pivot for itself.
+// For complex128, which an SM's narrow FP64 pipe bounds (4 FMA per entry and
+// step): 40 blocks 3.9 ms in an L2 workspace, 1.24 ms over four SMs each.
 template <typename T, int CL, int NT>
-__device__ void gauss_jordan_reg(const typename C2<T>::t *A, size_t lda, typename C2<T>::t *out, int *status) {
+__device__ void gauss_jordan_cluster(const typename C2<T>::t *A, size_t lda, typename C2<T>::t *out, int *status) {
     using V = typename C2<T>::t;
     constexpr int C = kBlock / CL, G = NT / C, kR = kBlock / G;
     static_assert(G * kR == kBlock && C % 32 == 0, "threads cover the block, a warp one row group");
     __shared__ __align__(16) V colb[2][kBlock];       // pivot column, by step parity (own CTA's threads)
-    __shared__ V col[CL > 1 ? kBlock : 1];   // the pivot column fetched from its CTA
+    __shared__ V col[kBlock];   // the pivot column fetched from its CTA
     __shared__ V rowb[C], inv_s;
     __shared__ int piv[kBlock], singular_s;
     const int tid = threadIdx.x, lane = tid & 31;
-    unsigned rank = 0;
-    if (CL > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    unsigned rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int j = tid % C, i0 = tid / C * kR, jg = (int)rank * C + j;   // own column (in the CTA, in the block)
     V a[kR];
 #pragma unroll
@@ -171,60 +348,29 @@ __device__ void gauss_jordan_reg(const typename C2<T>::t *A, size_t lda, typenam
     if (tid == 0) singular_s = 0;
 #pragma unroll 1
     for (int k = 0; k < kBlock; ++k) {
-        const V *pc = colb[k & 1];
-        if (CL > 1) {
-            // the column is complete in its CTA, and the others are done with
-            // the buffer of two steps ago
-            asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-            if (tid < kBlock) {
-                const unsigned src = (unsigned)__cvta_generic_to_shared(&colb[k & 1][tid]);
-                unsigned rem;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rem) : "r"(src), "r"(k / C));
-                V v;
-                if constexpr (sizeof(V) == 16)
-                    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(rem) : "memory");
-                else
-                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(rem) : "memory");
-                col[tid] = v;
-            }
-            pc = col;
+        // the column is complete in its CTA, and the others are done with
+        // the buffer of two steps ago
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+        if (tid < kBlock) {
+            const unsigned src = (unsigned)__cvta_generic_to_shared(&colb[k & 1][tid]);
+            unsigned rem;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rem) : "r"(src), "r"(k / C));
+            V v;
+            if constexpr (sizeof(V) == 16)
+                asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(rem) : "memory");
+            else
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(rem) : "memory");
+            col[tid] = v;
         }
         __syncthreads();
         if (tid < 32) {
-            T best = -1;
-            int p = kBlock;
+            V v[kBlock / 32];
 #pragma unroll
-            for (int q = 0; q < kBlock / 32; ++q) {
-                const V v = pc[lane + 32 * q];
-                const T m = v.x * v.x + v.y * v.y;
-                if (!((used >> q) & 1u) && m > best) {
-                    best = m;
-                    p = lane + 32 * q;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const T ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, p, o);
-                if (ob > best || (ob == best && oi < p)) { best = ob; p = oi; }
-            }
-            if (!(best > 0)) {
-                if (lane == 0) singular_s = 1;
-                // nothing comparable (NaN): the lowest unused row
-                if (p >= kBlock) {
-                    int cand = kBlock;
-#pragma unroll
-                    for (int q = kBlock / 32 - 1; q >= 0; --q)
-                        if (!((used >> q) & 1u)) cand = lane + 32 * q;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
-                    p = cand;
-                }
-            }
-            if (lane == (p & 31)) used |= 1u << (p >> 5);
+            for (int q = 0; q < kBlock / 32; ++q) v[q] = col[lane + 32 * q];
+            const int p = warp_pivot(v, lane, used, singular_s);
             if (lane == 0) {
                 piv[k] = p;
-                inv_s = cinv_pow2(pc[p]);
+                inv_s = cinv_pow2(col[p]);
             }
         }
         __syncthreads();
@@ -248,11 +394,7 @@ __device__ void gauss_jordan_reg(const typename C2<T>::t *A, size_t lda, typenam
         }
 #pragma unroll
         for (int q = 0; q < kR; ++q) {
-            const V f = pc[i0 + q];
-            a[q].x = fma(-f.x, r.x, a[q].x);
-            a[q].x = fma(f.y, r.y, a[q].x);
-            a[q].y = fma(-f.x, r.y, a[q].y);
-            a[q].y = fma(-f.y, r.x, a[q].y);
+            a[q] = gj_update(a[q], col[i0 + q], r);
         }
         if (p >= 0 && p < kR) {
 #pragma unroll
@@ -276,7 +418,7 @@ __device__ void gauss_jordan_reg(const typename C2<T>::t *A, size_t lda, typenam
     for (int q = 0; q < kR; ++q) out[(size_t)c * kBlock + step[i0 + q]] = a[q];
     if (tid == 0 && rank == 0 && singular_s) atomicMax(status, 1);
     // no CTA leaves while another may still read its column buffer
-    if (CL > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ int find_blk(const int *off, int B, int item) {
@@ -288,7 +430,7 @@ __device__ __forceinline__ int find_blk(const int *off, int B, int item) {
     return lo;
 }
 
-constexpr int kBinv32Threads = 1024;
+constexpr int kBinv32Threads = 512, kBinv32Cols = 2;
 constexpr int kBinv64Threads = 256, kBinv64Cluster = 4;
 
 // The system's last, partial block by one CTA on the nb x nb work array w
@@ -326,7 +468,7 @@ __global__ void __launch_bounds__(kBinv32Threads) k_binv32(const __grid_constant
     const int nb = min(kBlock, S.n - r0);
     float2 *out = (float2 *)S.Minv + (size_t)b * kBlock * kBlock;
     if (nb == kBlock)
-        gauss_jordan_reg<float, 1, kBinv32Threads>((const float2 *)S.A + (size_t)r0 * S.lda + r0, S.lda, out, S.status);
+        gauss_jordan_one<float, kBinv32Threads, kBinv32Cols>((const float2 *)S.A + (size_t)r0 * S.lda + r0, S.lda, out, S.status);
     else
         invert_partial<float>(S, r0, nb, smem, out);
 }
@@ -342,7 +484,7 @@ __global__ void __cluster_dims__(kBinv64Cluster, 1, 1) __launch_bounds__(kBinv64
     const int nb = min(kBlock, S.n - r0);
     double2 *out = (double2 *)S.Minv + (size_t)b * kBlock * kBlock;
     if (nb == kBlock)
-        gauss_jordan_reg<double, kBinv64Cluster, kBinv64Threads>((const double2 *)S.A + (size_t)r0 * S.lda + r0, S.lda,
+        gauss_jordan_cluster<double, kBinv64Cluster, kBinv64Threads>((const double2 *)S.A + (size_t)r0 * S.lda + r0, S.lda,
                                                                  out, S.status);
     else if (blockIdx.x % kBinv64Cluster == 0)
         invert_partial<double>(S, r0, nb, (double2 *)S.work + (size_t)b * kBlock * kBlock, out);
