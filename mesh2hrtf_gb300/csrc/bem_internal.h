@@ -156,7 +156,8 @@ inline size_t image_table_bytes(int n, int nref) {
 // k_near).  ctr: 4 device words, zero before the first use; the kernels leave
 // them zero.
 // Launch shapes of the assembly (persistent grids: resident blocks per SM of
-// k_far, at most kFarPerSmMax, and of k_near, at most 2); the results do not
+// k_far, at most kFarPerSmMax, and of k_near, at most 2, with twice as many of
+// its complex64 form, which keeps fewer registers); the results do not
 // depend on them.
 struct AsmShape {
     int far_per_sm = 2;

@@ -932,8 +932,12 @@ __device__ __forceinline__ void near_pair(const DevMeshView &mv, const DevFreq &
     }
 }
 
+// Bound by latency (each pair is a chain of subdivision levels, and the code is
+// long), so the float form takes four blocks per SM at 64 registers: 61440 pairs
+// 400 -> 280 us, 3840 pairs 30 -> 27 (three blocks 313, five 291).  The FP64 form
+// keeps two: its pipe is the limit.
 template <typename T>
-__global__ void __launch_bounds__(256, 2) k_near(const __grid_constant__ AsmBatch tb, unsigned *ctr) {
+__global__ void __launch_bounds__(256, std::is_same<T, float>::value ? 4 : 2) k_near(const __grid_constant__ AsmBatch tb, unsigned *ctr) {
     __shared__ WarpScratch ws_all[8];
     WarpScratch &ws = ws_all[threadIdx.y];
     const int total = tb.near_off[tb.B];
@@ -1041,10 +1045,11 @@ __device__ cplx<double> rhs_row(const DevMesh &m, const DevFreq &f, int i, const
 // the warp left 28 of 32 lanes idle on the 4-point rule: 3072 quadrilaterals with
 // one image and 48 such columns 8.2 -> 1.5 ms.  The rows beside those columns
 // subdivide many of them and are neighbours in the element order, so a block
-// takes rows that lie far apart: 1.49 -> 1.39 ms.  Sharing a block's subdivided
-// columns among its warps gave 1.28 but no shorter assembly; staging the
-// columns' points in shared memory 1.57, dealing them to a cluster 1.83.
-__global__ void __launch_bounds__(256) k_rhs(const __grid_constant__ AsmBatch tb) {
+// takes rows that lie far apart: 1.49 -> 1.39 ms; two blocks per SM at 128
+// registers instead of one at 255: 1.23.  Staging the columns' points in shared
+// memory (1.57 from 1.39) or dealing them to a cluster (1.83) cost more in
+// waits than they saved.
+__global__ void __launch_bounds__(256, 2) k_rhs(const __grid_constant__ AsmBatch tb) {
     __shared__ WarpScratch ws_all[8];
     const int sb = find_sys(tb.rhs_off, tb.B, blockIdx.x);
     const AsmSys &S = tb.sys[sb];
@@ -2301,9 +2306,10 @@ cudaError_t launch_assemble(const AsmBatch &t, int prec, unsigned *ctr, cudaStre
     dim3 block(32, 8);
     const int far_items = t.far_off[t.B], near_items = t.near_off[t.B];
     // persistent grids: far_per_sm resident blocks of k_far per SM (launch
-    // bounds allow kFarPerSm), near_per_sm of k_near (launch bounds allow 2)
+    // bounds allow kFarPerSm), near_per_sm of k_near, twice that for complex64 (its
+    // launch bounds allow 2 and 4)
     const int fps = std::max(1, std::min(shape.far_per_sm, kFarPerSm));
-    const int nps = std::max(1, std::min(shape.near_per_sm, 2));
+    const int nps = std::max(1, std::min(shape.near_per_sm, 2)) * (prec == 0 ? 1 : 2);
     const int gfar = std::max(1, std::min((far_items + 7) / 8, fps * sm_count()));
     const int gnear = std::max(1, std::min((near_items + 7) / 8, nps * sm_count()));
     // Systems that fill the GPU on their own take one single-system launch
