@@ -23,7 +23,7 @@ fp64_gpu  the plain FP64 GPU path on the first timed batch (the same 16
           frequencies, also one bem_solve_batch), against the mixed time of
           that batch, and the mixed path's relative L2 error against it.
 roofline  the dominant kernel (the matrix-vector products of the solve) over
-          the CUDA-event time of the product launches, against the measured
+          the device time of the product launches, against the measured
           HBM copy bandwidth; roofline.stages gives every stage of a solve a
           roofline time from its algorithmic work and the measured peaks
           (HBM copy, and the FP32 FMA / special-function / FP64 FMA issue
@@ -445,8 +445,8 @@ def main():
     # launch of the batched product covers every system still iterating; its
     # bytes are counted per system and product (Krylov products read the fp16
     # copy, N^2*4 + 2*N*16; refinement residuals the complex64 matrix,
-    # N^2*8 + 2*N*16), its time is the CUDA-event time of the launches inside
-    # the iteration bodies (events on the engine's stream).
+    # N^2*8 + 2*N*16), its time is the device time of the launches inside the
+    # iteration bodies (the global timer, read by the kernels).
     bytes_resid = by_c64
     mv_ms = sum(step[0]["matvec_ms"] for step in infos)
     n_mv = sum(i["n_matvec"] for step in infos for i in step)

@@ -1,9 +1,10 @@
 // bem_engine.h - host side of the batched Krylov engine (bem_gmres.cu).
 //
 // An Engine owns a device launch table (KTable), the systems' GMRES states,
-// the work-item lists of the kernels, and one CUDA graph of the iteration
-// body, captured at the first replay.  The table and states live in device
-// memory, so the graph stays valid while systems come and go: set_batch()
+// the work-item lists of the kernels, and the CUDA graphs of the Arnoldi step
+// and the end of cycle, captured at their first replay.  The table and states
+// live in device memory, so the graphs stay valid while systems come and go:
+// set_batch()
 // rewrites them between replays.
 #pragma once
 

@@ -290,8 +290,8 @@ cudaError_t launch_blr_compress(const BlrBatch &t, cudaStream_t st);
 
 // ---------------------------------------------------------------- Krylov engine
 // Restarted GMRES of one system as a state machine on the device.  An
-// iteration body (one captured graph) runs kSteps Arnoldi steps for every
-// system in phase ARNOLDI, then the cycle end for every system in phase
+// iteration body (replays of two captured graphs) runs up to kSteps Arnoldi
+// steps for every system in phase ARNOLDI, then the cycle end for every system in phase
 // UPDATE: y = H^{-1} g, x += d = M^{-1} V y, the refinement residual, the
 // convergence decision and the restart.  The residual is r = b - A x with
 // error-free products after the first cycle (and always for complex128);

@@ -9,7 +9,7 @@ graded) with 20 n^2 triangles (n = 59: 69620).  Sources: --rhs point
 sources 1 mm off seeded surface points, one right-hand side each.  Grid:
 --points quasi-uniform points (golden-angle spiral) on a 1.2 m sphere.
 The product's roofline: each shared-matrix product reads A once
-(N^2 * 8 bytes) for all right-hand sides; the engine's CUDA-event time of
+(N^2 * 8 bytes) for all right-hand sides; the engine's device time of
 the product launches over that.  --fp64-check also solves right-hand
 side 0 in FP64 and reports the mixed solution's relative L2 difference.
 """
