@@ -948,7 +948,8 @@ double bem_footprint_multi(int32_t n_elem, int32_t precision, int32_t restart, i
 double bem_mesh_footprint_bytes(int32_t n_elem, int32_t n_sym_planes) {
     const int n = std::max(n_elem, 1);
     const int nref = 1 << std::min(std::max(n_sym_planes, 0), 3);
-    // element tables: 1 + 12 + 3 + 3 + 1 + 1 words of 8 B, 3 + 3 + 10 + 12 + 1 + 3 + 12 of 4 B
+    // element tables: 1 + 12 + 3 + 3 + 1 + 1 words of 8 B, 3 + 3 + 10 + 12 + 1 + 3 + 10 of 4 B
+    // (44 counted: the estimate keeps room for allocation granularity)
     const double tables = (double)n * (4.0 + 20.0 * 8.0 + 44.0 * 4.0);
     const double near = (double)n * nref * 48.0 * sizeof(int2);   // the list's first allocation
     return tables + (double)bem::image_table_bytes(n, nref) + near;
@@ -1147,11 +1148,18 @@ bem_status bem_mesh_create(const bem_mesh_desc *d, bem_mesh_t *out) {
     if (e == cudaSuccess) e = up(&m->d_isqa, isqa);
     if (e == cudaSuccess) e = up(&m->d_n32, n32);
     if (e == cudaSuccess) {
-        std::vector<float4> row4(3 * (size_t)n);
-        for (int i = 0; i < n; ++i) {
-            row4[3 * (size_t)i] = make_float4(chi[i], chi[(size_t)n + i], chi[2 * (size_t)n + i], 0.f);
-            row4[3 * (size_t)i + 1] = make_float4(clo[i], clo[(size_t)n + i], clo[2 * (size_t)n + i], 0.f);
-            row4[3 * (size_t)i + 2] = make_float4(n32[i], n32[(size_t)n + i], n32[2 * (size_t)n + i], 0.f);
+        // two rows to a record, ready for packed arithmetic: each value beside
+        // its neighbour's, the centres negated (the last row stands in for a
+        // missing one)
+        std::vector<float4> row4(5 * (((size_t)n + 1) / 2));
+        for (size_t p = 0; p < ((size_t)n + 1) / 2; ++p) {
+            const size_t i = 2 * p, j = std::min(i + 1, (size_t)n - 1), N = (size_t)n;
+            float4 *r = &row4[5 * p];
+            r[0] = make_float4(-chi[i], -chi[j], -chi[N + i], -chi[N + j]);
+            r[1] = make_float4(-chi[2 * N + i], -chi[2 * N + j], -clo[i], -clo[j]);
+            r[2] = make_float4(-clo[N + i], -clo[N + j], -clo[2 * N + i], -clo[2 * N + j]);
+            r[3] = make_float4(n32[i], n32[j], n32[N + i], n32[N + j]);
+            r[4] = make_float4(n32[2 * N + i], n32[2 * N + j], 0.f, 0.f);
         }
         e = up(&m->d_row4, row4);
     }

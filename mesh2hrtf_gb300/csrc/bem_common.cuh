@@ -282,8 +282,8 @@ struct DevMesh {
     const float *q32;       // 12 rows (quads): vertex offsets from the centre
     const float *isqa32;    // 1 / sqrt(areael) in float (approximate ratios)
     const float *n32;       // 3 rows: centre normal in float
-    const float4 *row4;     // [n][3]: (chi, 0), (clo, 0), (n32, 0): a collocation
-                            // row's data in three 16-byte loads
+    const float4 *row4;     // two collocation rows' -chi, -clo and n32 in five
+                            // 16-byte loads, each value beside the other row's
     DevSym sym;             // symmetry-plane images (sym.nref = 1: none)
 };
 

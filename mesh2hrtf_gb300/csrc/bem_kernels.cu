@@ -204,9 +204,10 @@ __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3]
 // 2 scalar FP32 operations and 6 special functions per two evaluations, and
 // about 45 per pair of entries); one entry at a time it was bound by
 // instruction issue at 79 per evaluation.  20480-triangle head, 10 kHz: k_far
-// 4.07 -> 3.33 ms (1280 triangles 50 us as before, 3072 quadrilaterals and their
-// images 690 -> 673).  Three blocks per SM with the column's data in shared
-// memory instead of two with it in registers: 3.77 ms.
+// 4.07 -> 3.33 ms, and 3.17 with the rows' data stored as pairs (18 moves a pair
+// less); 1280 triangles 50 us as before, 3072 quadrilaterals and their images
+// 690 -> 665.  Three blocks per SM with the column's data in shared memory
+// instead of two with it in registers: 3.77 ms.
 struct FarCol2 {
     F2 a[3], b[3], n[3];
     F2 C[3];       // |s_g a + t_g b|^2 of points 1 .. 3 (point 0 is the centroid)
@@ -714,9 +715,9 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
             if (i != j || kref > 0) {
                 // the quadrature decision from the float distance, the exact
                 // FP64 one (a square root and a division) only near a threshold
-                const float4 rh = m.row4[3 * (size_t)i], rl = m.row4[3 * (size_t)i + 1];
-                const float d0 = (cjh[0] - rh.x) + (cjl[0] - rl.x), d1 = (cjh[1] - rh.y) + (cjl[1] - rl.y),
-                            d2 = (cjh[2] - rh.z) + (cjl[2] - rl.z);
+                const float *nr = reinterpret_cast<const float *>(m.row4 + 5 * (size_t)(i >> 1)) + (i & 1);   // -centre
+                const float d0 = (cjh[0] + nr[0]) + (cjl[0] + nr[6]), d1 = (cjh[1] + nr[2]) + (cjl[1] + nr[8]),
+                            d2 = (cjh[2] + nr[4]) + (cjl[2] + nr[10]);
                 const float q2 = (d0 * d0 + d1 * d1 + d2 * d2) * isq2;
                 bool near = false;
                 int order = 2;
@@ -758,13 +759,14 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
             const int i = i0 + r;
             if (i >= n) break;
             // the two rows' data (the same for the warp's 32 columns)
-            const float4 *row = m.row4 + 3 * (size_t)i, *row1 = i + 1 < n ? row + 3 : row;
-            const float4 h0 = row[0], l0 = row[1], n0 = row[2], h1 = row1[0], l1 = row1[1], n1 = row1[2];
-            const F2 D[3] = {vadd(vfma(pk2(h0.x, h1.x), fk.m1, dup2(cjh[0])), vfma(pk2(l0.x, l1.x), fk.m1, dup2(cjl[0]))),
-                             vadd(vfma(pk2(h0.y, h1.y), fk.m1, dup2(cjh[1])), vfma(pk2(l0.y, l1.y), fk.m1, dup2(cjl[1]))),
-                             vadd(vfma(pk2(h0.z, h1.z), fk.m1, dup2(cjh[2])), vfma(pk2(l0.z, l1.z), fk.m1, dup2(cjl[2])))};
+            const float4 *row = m.row4 + 5 * (size_t)(i >> 1);   // items start at even rows
+            const float4 v0 = row[0], v1 = row[1], v2 = row[2], v3 = row[3];
+            const float2 v4 = *reinterpret_cast<const float2 *>(row + 4);
+            const F2 D[3] = {vadd(vadd(dup2(cjh[0]), pk2(v0.x, v0.y)), vadd(dup2(cjl[0]), pk2(v1.z, v1.w))),
+                             vadd(vadd(dup2(cjh[1]), pk2(v0.z, v0.w)), vadd(dup2(cjl[1]), pk2(v2.x, v2.y))),
+                             vadd(vadd(dup2(cjh[2]), pk2(v1.x, v1.y)), vadd(dup2(cjl[2]), pk2(v2.z, v2.w)))};
             const F2 D2 = vfma(D[2], D[2], vfma(D[0], D[0], vmul(D[1], D[1])));
-            const F2 nx[3] = {pk2(n0.x, n1.x), pk2(n0.y, n1.y), pk2(n0.z, n1.z)};
+            const F2 nx[3] = {pk2(v3.x, v3.y), pk2(v3.z, v3.w), pk2(v4.x, v4.y)};
             float q2[2];
             unpk2(vmul(D2, dup2(isq2)), q2[0], q2[1]);
             // quadrature orders; 0: near or self
@@ -802,8 +804,8 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
                 else if (ord[h] > 2) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) unpk2(D[c], d[c][0], d[c][1]);
-                    const float2 v = far_entry_general(&mv, kref, j, d[0][h], d[1][h], d[2][h], h ? n1.x : n0.x,
-                                                       h ? n1.y : n0.y, h ? n1.z : n0.z, ord[h], fc);
+                    const float2 v = far_entry_general(&mv, kref, j, d[0][h], d[1][h], d[2][h], h ? v3.y : v3.x,
+                                                       h ? v3.w : v3.z, h ? v4.y : v4.x, ord[h], fc);
                     er[h] = v.x;
                     ei[h] = v.y;
                 }
