@@ -2615,7 +2615,13 @@ __global__ void __launch_bounds__(kPcgThreads, 3) k_pcwin_grp(const KTable *tb, 
         const KGroup g = tb->grp[q];
         const KSys &S = tb->sys[g.first];
         const int n = S.n, items = ceil_div(n, kItemRows);
-        // one answer per group and block: k_givens may run beside this
+        // items go round the blocks across the groups; the deal comes from the
+        // table alone, so that every block makes the same one
+        const unsigned shift = (unsigned)first_item % gridDim.x;
+        first_item += items;
+        // the phases, read once per group and block: k_givens may run beside
+        // this, and a block that sees a member's cycle ended leaves out rows
+        // that nobody reads
         __syncthreads();
         if (warp == 0) {
             const unsigned b = __ballot_sync(0xffffffffu, lane < g.count && pcw_active(tb->sys[g.first + min(lane, g.count - 1)], mode));
@@ -2624,10 +2630,7 @@ __global__ void __launch_bounds__(kPcgThreads, 3) k_pcwin_grp(const KTable *tb, 
         __syncthreads();
         const unsigned mask = active;
         if (!mask) continue;
-        // items go round the blocks across the groups
-        int it = (int)((blockIdx.x + gridDim.x - (unsigned)first_item % gridDim.x) % gridDim.x);
-        first_item += items;
-        for (; it < items; it += gridDim.x) {
+        for (int it = (int)((blockIdx.x + gridDim.x - shift) % gridDim.x); it < items; it += gridDim.x) {
             const int r0 = it * kItemRows + warp * kPcgRows, c0 = it * kItemRows / kPcWin * kPcWin;
             float sr[kPcgRows][kMaxGroup], si[kPcgRows][kMaxGroup];
 #pragma unroll
