@@ -106,8 +106,12 @@ __device__ void factor_diag(V (*D)[kPanel + 1], int kb, int *status) {
 #pragma unroll
                 for (int q = p; q < kPanel / 8; ++q) {
                     const int c = c0 + 8 * q;
-                    if (c > i) a[q] = cfnma(a[q], l, D[i][c]);
-                    if (c == i + 1 || r == i + 1) D[r][c] = a[q];
+                    if (c > i) {
+                        a[q] = cfnma(a[q], l, D[i][c]);
+                        // only what step i + 1 reads: column i of row i + 1 is
+                        // still being read by the row's other lanes
+                        if (c == i + 1 || r == i + 1) D[r][c] = a[q];
+                    }
                 }
             }
             __syncthreads();
