@@ -86,7 +86,7 @@ def _function(text, name):
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     text = SRC.read_text()
-    code = "\n".join(_function(text, f) for f in ("cdiv", "cfnma", "factor_diag"))
+    code = "\n".join(_function(text, f) for f in ("cdiv", "cnma", "factor_diag"))
     code = re.sub(r"#pragma unroll.*", "", code)
     d = tmp_path_factory.mktemp("lanes")
     (d / "lanes.cpp").write_text(HOST.replace("@@CODE@@", code))
@@ -110,3 +110,23 @@ def test_order_of_threads(lib, dt, kb, order):
     L, U = np.tril(lu, -1) + np.eye(kb), np.triu(lu)
     u = 2.0 ** -24 if dt == np.complex64 else 2.0 ** -53
     assert np.linalg.norm(L @ U - a) <= 8 * kb * u * np.linalg.norm(a, 2)
+
+
+@pytest.mark.parametrize("dt", [np.complex64, np.complex128])
+def test_an_update_rounds_once_at_the_entry(lib, dt):
+    """a - l u with |l u| far below |a| is within half a unit of a, and three
+    roundings of the product (two in it, one for a unit that the difference
+    may drop to), of its value."""
+    f = lib.factor_f if dt == np.complex64 else lib.factor_d
+    u = 2.0 ** -24 if dt == np.complex64 else 2.0 ** -53
+    rng = np.random.default_rng(8)
+    for _ in range(300):
+        D = np.zeros((32, 33), dt)
+        off = 0.03 * (rng.normal(size=2) + 1j * rng.normal(size=2))
+        a = np.array([[1 + 1j, off[0]], [off[1], 1.5 + 1.5j]]).astype(dt)
+        D[:2, :2] = a
+        assert f(D.ctypes.data_as(ctypes.c_void_p), 2, 0) == 0
+        l, d = D[1, 0].astype(np.clongdouble), D[1, 1].astype(np.clongdouble)
+        p = l * a[0, 1].astype(np.clongdouble)
+        e = d - (a[1, 1].astype(np.clongdouble) - p)
+        assert max(abs(e.real), abs(e.imag)) <= u + 3 * u * abs(p)   # half a unit in [1, 2)
