@@ -89,14 +89,23 @@ __device__ __forceinline__ void phase_sincos(float x, float *s, float *c) {
 // FP64 counterparts for the plain path, whose kernels are bound by GB300's
 // narrow FP64 pipe: what counts is the number of FP64 instructions.
 //
-// 1 / sqrt(x): the hardware's FP64 seed (about 2^-20 relative) and one
-// third-order step, y + y e (1/2 + 3/8 e) with e = 1 - x y^2: 5 instructions,
-// within 1.5 ulp.
-__device__ __forceinline__ double rsqrt_nr(double x) {
+// sqrt(x) and 1 / sqrt(x): the hardware's FP64 seed (about 2^-20 relative),
+// the third-order step of the binomial series of (1 - e)^(-1/2), e = 1 - x y^2
+// (Householder's iteration), and for the root one Heron step with its residual
+// fused, so that it is the correctly rounded one but for rare ties: 8
+// instructions.  Without the last step phases of k r = 58 carried 12 % more
+// error than with the library's root.  1 / sqrt(x) is within 1.5 ulp, as the
+// quotient of one by the rounded root.
+__device__ __forceinline__ double rsqrt_nr(double x, double *root) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    const double g = x * y, e = fma(-g, y, 1.0);
+    const double h = e * fma(0.375, e, 0.5);
+    const double u = fma(y, h, y), r = fma(g, h, g);
+    // u / 2 by its exponent
+    const double hu = __hiloint2double(__double2hiint(u) - (1 << 20), __double2loint(u));
+    *root = fma(hu, fma(-r, r, x), r);
+    return u;
 }
 
 // sin and cos of a phase (|x| below 10^9) by table look-up and a short
@@ -134,12 +143,14 @@ __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { phase_si
 __device__ __forceinline__ void vdup(F2 &r, float x) { r = pk2(x, x); }
 __device__ __forceinline__ void vdup(double &r, double x) { r = x; }
 // 1 / sqrt, and sin and cos of a phase, half by half (phase_sincos's steps)
-__device__ __forceinline__ F2 vrsqrt(F2 a) {
+__device__ __forceinline__ F2 vrsqrt(F2 a, F2 *root) {
     float lo, hi;
     unpk2(a, lo, hi);
-    return pk2(rsqrt_approx(lo), rsqrt_approx(hi));
+    const F2 u = pk2(rsqrt_approx(lo), rsqrt_approx(hi));
+    *root = vmul(a, u);
+    return u;
 }
-__device__ __forceinline__ double vrsqrt(double a) { return rsqrt_nr(a); }
+__device__ __forceinline__ double vrsqrt(double a, double *root) { return rsqrt_nr(a, root); }
 // Constants of phase_sincos in packed form.
 template <typename R> struct ScConst {};
 template <> struct ScConst<F2> {
@@ -405,14 +416,13 @@ __device__ __forceinline__ void map_point(const Elem64 &e, double s, double t, c
     double nx = dxs[1] * dxt[2] - dxt[1] * dxs[2];
     double ny = dxs[2] * dxt[0] - dxt[2] * dxs[0];
     double nz = dxs[0] * dxt[1] - dxt[0] * dxs[1];
-    const double n2 = nx * nx + ny * ny + nz * nz, il = rsqrt_nr(n2);
+    double len;
+    const double il = rsqrt_nr(nx * nx + ny * ny + nz * nz, &len);
     q.ny[0] = nx * il; q.ny[1] = ny * il; q.ny[2] = nz * il;
-    q.wj = w * (n2 * il);
+    q.wj = w * len;
 #pragma unroll
     for (int k = 0; k < 3; ++k) q.d[k] = y[k] - x[k];
-    const double r2 = q.d[0] * q.d[0] + q.d[1] * q.d[1] + q.d[2] * q.d[2];
-    q.ir = rsqrt_nr(r2);
-    q.r = r2 * q.ir;
+    q.ir = rsqrt_nr(q.d[0] * q.d[0] + q.d[1] * q.d[1] + q.d[2] * q.d[2], &q.r);
 #pragma unroll
     for (int a = 0; a < 4; ++a) q.sh[a] = sh[a];
 }

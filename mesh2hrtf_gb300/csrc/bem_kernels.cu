@@ -276,8 +276,8 @@ __device__ __forceinline__ F2 dot2(const F2 x[3], const F2 y[3]) {
 template <int BC>
 __device__ __forceinline__ void far_point2(const FarConst &k, const FusedCol2 &c, F2 r2, F2 dny, F2 dnx, F2 nn, F2 wj,
                                            FarSum2 &o) {
-    const F2 u = vrsqrt(r2), r = vmul(r2, u);
-    F2 sn, cs, fr, fi, amp;
+    F2 r, sn, cs, fr, fi, amp;
+    const F2 u = vrsqrt(r2, &r);
     vsincos(k.sc, vmul(c.wr, r), sn, cs);
     if (BC == 1) {
         // -tau - i b z1 re2, z1 = -1/r + i wr, re2 = -d.n_x / r
@@ -396,10 +396,11 @@ __device__ __forceinline__ void far_col64(const DevMesh &m, int j, FarCol64 &e) 
         e.n[k] = e.a[p] * e.b[q] - e.b[p] * e.a[q];
         n2 = fma(e.n[k], e.n[k], n2);
     }
-    const double il = rsqrt_nr(n2);
+    double len;
+    const double il = rsqrt_nr(n2, &len);
 #pragma unroll
     for (int k = 0; k < 3; ++k) e.n[k] *= il;
-    e.J4 = n2 * il * (1.0 / kPI4);
+    e.J4 = len * (1.0 / kPI4);
 }
 
 // Points o0 .. o0 + np - 1 of the triangle rules; D = centroid - x.
@@ -422,9 +423,9 @@ __device__ __forceinline__ cplx<double> far_tri64(const FarCol64 &e, const doubl
         // D2 + s (2 D.a + s a.a + 2 t a.b) + t (2 D.b + t b.b)
         const double r2 = fma(s, fma(s, e.aa, fma(2.0 * t, e.ab, Da2)), fma(t, fma(t, e.bb, Db2), D2));
         const double dnx = fma(t, bnx, fma(s, anx, dnx0));
-        const double u = rsqrt_nr(r2), u2 = u * u;
-        double sn, cs;
-        phase_sincos(c.wr * (r2 * u), &sn, &cs);
+        double r, sn, cs;
+        const double u = rsqrt_nr(r2, &r), u2 = u * u;
+        phase_sincos(c.wr * r, &sn, &cs);
         double fr, fi, amp;
         if (BC == 1) {
             const double du = dnx * u;
@@ -438,7 +439,7 @@ __device__ __forceinline__ cplx<double> far_tri64(const FarCol64 &e, const doubl
             amp = w * e.J4 * u2;
             if (BC == 2) {
                 // + Y (1 + i b tau z1 re2) / u
-                const double bt = c.b * c.tau, r = r2 * u;
+                const double bt = c.b * c.tau;
                 const double pr = fma(bt * c.wr, dnx, r), pi = bt * u * dnx;
                 fr += c.yr * pr - c.yi * pi;
                 fi += c.yr * pi + c.yi * pr;
@@ -1648,8 +1649,8 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
             w = e.v[30 + g];
         }
         const R r2 = vfma(d[2], d[2], vfma(d[0], d[0], vmul(d[1], d[1])));
-        R u = vrsqrt(r2), sn, cs;
-        vsincos(sc, vmul(wr, vmul(r2, u)), sn, cs);
+        R r, sn, cs, u = vrsqrt(r2, &r);
+        vsincos(sc, vmul(wr, r), sn, cs);
         if constexpr (std::is_same<T, float>::value) {
             float lo, hi;
             unpk2(u, lo, hi);

@@ -1,0 +1,65 @@
+"""The FP64 path's own square root, as the kernels compile it: over exponents of
+-300 .. 300 the root is the correctly rounded one (its last step adds a fused
+residual good to 2^-51 of the correction, so a wrong rounding needs a value
+that close to a tie), and the inverse is within 1.5 units in the last place."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from mesh2hrtf_gb300 import build
+
+pytestmark = pytest.mark.gpu
+
+CODE = r"""
+#include "bem_common.cuh"
+__global__ void k_root(int n, const double *x, double *root, double *inv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) inv[i] = bem::rsqrt_nr(x[i], root + i);
+}
+static double *up(int n, const double *h) {
+    double *d = nullptr;
+    cudaMalloc(&d, sizeof(double) * n);
+    if (h) cudaMemcpy(d, h, sizeof(double) * n, cudaMemcpyHostToDevice);
+    return d;
+}
+static void down(int n, double *d, double *h) {
+    if (h) cudaMemcpy(h, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+}
+extern "C" int run_root(int n, const double *x, double *root, double *inv) {
+    double *a = up(n, x), *b = up(n, nullptr), *c = up(n, nullptr);
+    k_root<<<(n + 255) / 256, 256>>>(n, a, b, c);
+    down(n, a, nullptr); down(n, b, root); down(n, c, inv);
+    return (int)cudaGetLastError();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("functions")
+    src, so = str(d / "functions.cu"), str(d / "functions.so")
+    with open(src, "w") as f:
+        f.write(CODE)
+    subprocess.run([build.nvcc(), "-shared", "-o", so, src, "-O3", "-std=c++17", *build.ARCH, "-Xcompiler", "-fPIC",
+                    "-I", build.CSRC, "-I", os.path.join(build.ROOT, "include")], check=True)
+    return ctypes.CDLL(so)
+
+
+def _p(a):
+    return a.ctypes.data_as(ctypes.c_void_p)
+
+
+def test_square_root(lib):
+    rng = np.random.default_rng(1)
+    x = np.ldexp(rng.uniform(1.0, 2.0, 1 << 20), rng.integers(-300, 301, 1 << 20))
+    x[:64] = np.ldexp(1.0, np.arange(64) - 32)
+    root, inv = np.zeros_like(x), np.zeros_like(x)
+    assert lib.run_root(len(x), _p(x), _p(root), _p(inv)) == 0
+    assert np.array_equal(root, np.sqrt(x))
+    e = inv.astype(np.longdouble) * np.sqrt(x.astype(np.longdouble)) - 1
+    unit = np.ldexp(1.0, np.frexp(inv)[1] - 53).astype(np.longdouble) / inv
+    assert (np.abs(e) <= 1.5 * unit).all()
