@@ -355,22 +355,25 @@ __device__ __forceinline__ void far_quad2(const FarConst &k, float (*st)[32], in
     }
 }
 
-// FP64 regular pair on a flat triangle, arranged for the fewest FP64
-// instructions (the plain path is bound by GB300's narrow FP64 pipe): the
-// column's edge vectors, normal, Jacobian and, for the 4-point rule,
-// |s_g a + t_g b|^2 are formed once per thread; a point's squared distance is
-// |D|^2 + 2 s D.a + 2 t D.b + |s a + t b|^2 (the terms' cancellation costs at
-// most a factor of ten of the rounding at the smallest ratio, 1.3), and with
+// FP64 regular pair on a flat triangle, arranged for few FP64 instructions
+// (the plain path is bound by GB300's narrow FP64 pipe): the column's edge
+// vectors, normal, Jacobian and centroid, in two parts, are formed once per
+// thread; a point's vector d is the difference D of the centroid's high part
+// and x plus the point's offset, two roundings, D's exact for near pairs.  With
 // P = (D.n_y)(d.n_x), u = 1/r, E = n_x.n_y - 3 P u^2 the velocity entry's factor is
 //   u (b wr E - tau D.n_y u) + i u (b u (E + k^2 P) + tau wr D.n_y).
-// 44 FP64 instructions per point (the general form through map_point and the
+// 53 FP64 instructions per point (the general form through map_point and the
 // library's square roots, divisions and sincos took about 250).  5120-triangle
-// head, 5 kHz: k_far 33.0 -> 11.9 ms; entries as close to 80-bit ones as
-// before (5.1e-15 against 5.0e-15 at 16 kHz, 1.00e-15 against 1.04e-15 at 4 kHz).
+// head, 5 kHz: k_far 33.0 -> 12.8 ms.  Mean errors against 80-bit entries, this
+// and the general form, beyond a ratio of 4.5 and below 4, k = 73: head 1.35e-15
+// and 1.50e-15, 8.6e-16 and 9.1e-16; sphere flattened to a tenth 8.4e-16 and
+// 9.0e-16, 2.4e-16 and 3.0e-16.  |D|^2 + 2 s D.a + ... for the squared distance
+// (7 instructions less) loses (|D| / r)^2 units where a long thin
+// triangle's point comes close to x.
 struct FarCol64 {
-    double c[3];         // centroid
+    double c[3], cl[3];  // centroid, high and low part
     double a[3], b[3], n[3];
-    double aa, ab, bb;   // a.a, a.b, b.b
+    double cln;          // cl . n
     double J4;           // J / (4 pi)
 };
 struct FusedCol64 {
@@ -379,16 +382,15 @@ struct FusedCol64 {
 
 __device__ __forceinline__ void far_col64(const DevMesh &m, int j, FarCol64 &e) {
     double n2 = 0.0;
-    e.aa = e.ab = e.bb = 0.0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const double p2 = m.v64[(6 + k) * m.n + j];
         e.a[k] = m.v64[k * m.n + j] - p2;
         e.b[k] = m.v64[(3 + k) * m.n + j] - p2;
-        e.c[k] = p2 + (e.a[k] + e.b[k]) * (1.0 / 3.0);
-        e.aa = fma(e.a[k], e.a[k], e.aa);
-        e.ab = fma(e.a[k], e.b[k], e.ab);
-        e.bb = fma(e.b[k], e.b[k], e.bb);
+        const double o = (e.a[k] + e.b[k]) * (1.0 / 3.0);
+        e.c[k] = p2 + o;
+        const double p = e.c[k] - o;   // the sum's error (Knuth)
+        e.cl[k] = (p2 - p) + (o - (e.c[k] - p));
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -400,29 +402,26 @@ __device__ __forceinline__ void far_col64(const DevMesh &m, int j, FarCol64 &e) 
     const double il = rsqrt_nr(n2, &len);
 #pragma unroll
     for (int k = 0; k < 3; ++k) e.n[k] *= il;
+    e.cln = e.cl[0] * e.n[0] + e.cl[1] * e.n[1] + e.cl[2] * e.n[2];
     e.J4 = len * (1.0 / kPI4);
 }
 
-// Points o0 .. o0 + np - 1 of the triangle rules; D = centroid - x.
+// Points o0 .. o0 + np - 1 of the triangle rules; D = centroid's high part - x.
 template <int BC>
 __device__ __forceinline__ cplx<double> far_tri64(const FarCol64 &e, const double D[3], const double nx[3], int o0,
                                                   int np, const FusedCol64 &c) {
-    const double D2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2];
-    const double dny = D[0] * e.n[0] + D[1] * e.n[1] + D[2] * e.n[2];
-    const double dnx0 = D[0] * nx[0] + D[1] * nx[1] + D[2] * nx[2];
-    const double anx = e.a[0] * nx[0] + e.a[1] * nx[1] + e.a[2] * nx[2];
-    const double bnx = e.b[0] * nx[0] + e.b[1] * nx[1] + e.b[2] * nx[2];
+    const double dny = fma(D[2], e.n[2], fma(D[1], e.n[1], fma(D[0], e.n[0], e.cln)));
     const double nn = e.n[0] * nx[0] + e.n[1] * nx[1] + e.n[2] * nx[2];
-    const double Da2 = 2.0 * (D[0] * e.a[0] + D[1] * e.a[1] + D[2] * e.a[2]);
-    const double Db2 = 2.0 * (D[0] * e.b[0] + D[1] * e.b[1] + D[2] * e.b[2]);
     const double ct = -c.tau * dny, cw = c.tau * c.wr * dny, bwr = c.b * c.wr;
     double ar = 0.0, ai = 0.0;
 #pragma unroll 2
     for (int g = 0; g < np; ++g) {
         const double s = c_far64[o0 + g][0], t = c_far64[o0 + g][1], w = c_far64[o0 + g][2];
-        // D2 + s (2 D.a + s a.a + 2 t a.b) + t (2 D.b + t b.b)
-        const double r2 = fma(s, fma(s, e.aa, fma(2.0 * t, e.ab, Da2)), fma(t, fma(t, e.bb, Db2), D2));
-        const double dnx = fma(t, bnx, fma(s, anx, dnx0));
+        double d[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d[k] = D[k] + fma(t, e.b[k], fma(s, e.a[k], e.cl[k]));
+        const double r2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+        const double dnx = fma(d[2], nx[2], fma(d[1], nx[1], d[0] * nx[0]));
         double r, sn, cs;
         const double u = rsqrt_nr(r2, &r), u2 = u * u;
         phase_sincos(c.wr * r, &sn, &cs);
