@@ -1500,10 +1500,14 @@ template <typename T> struct ProjLane;
 template <> struct ProjLane<float> { using R = F2; static constexpr int kP = 2, kPart = 2; };
 template <> struct ProjLane<double> { using R = double; static constexpr int kP = 1, kPart = 4; };
 
-// A staged element.  v[0..2] centre (float: high parts, v[3..5] low parts);
-// triangles: 6 a, 9 b, 12 n; quadrilaterals, per point g: 6 + 3 g offset (FP64:
-// position), 18 + 3 g normal, 30 + g weight.  Per right-hand side W (re, im,
-// -im, -re) and, where some right-hand side has nodal velocities, V of the points.
+// A staged element.  Float triangles: v[0..2] centre, high parts, v[3..5] low
+// parts, 6 a, 9 b, 12 n.  Else, per point g: 6 + 3 g position (float: offset
+// from the centre, staged as above), 18 + 3 g normal (FP64 triangles: 18 n),
+// 30 + g weight (quadrilaterals).  FP64 subtracts positions, as map_point does:
+// an offset from the centroid leaves the rounding of the centroid and of the
+// difference in all points of the element (scattered fields 1 m away at k = 73
+// up to 1.4 times as far from 80-bit ones).  Per right-hand side W (re, im, -im,
+// -re) and, where some right-hand side has nodal velocities, V of the points.
 template <typename T, int NR> struct ProjElem {
     typename ProjLane<T>::R v[34], W[NR][4], V[NR][4][3];
     float hi[3], lo[3], isq2;
@@ -1541,10 +1545,8 @@ __device__ void proj_stage(const ProjSys *sys, int nr, const DevMesh &m, const D
             far_col64(mk, j, f);
             J = f.J4 * kPI4;
             for (int k = 0; k < 3; ++k) {
-                if (g == 0) o.v[6 + k] = f.a[k];
-                if (g == 1) o.v[9 + k] = f.b[k];
-                if (g == 2) o.v[12 + k] = f.n[k];
-                if (g == 3) o.v[k] = f.c[k];
+                o.v[6 + 3 * g + k] = f.c[k] + fma(c_far64[g][1], f.b[k], fma(c_far64[g][0], f.a[k], f.cl[k]));
+                if (g == 0) o.v[18 + k] = f.n[k];
             }
         }
         fac = J * i4pi;
@@ -1622,30 +1624,36 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
     Ti = P0r = P0i = Tr;
 #pragma unroll
     for (int k = 0; k < 3; ++k) G0r[k] = G0i[k] = Tr;
-    if (TRI) dny = vfma(D[2], e.v[14], vfma(D[0], e.v[12], vmul(D[1], e.v[13])));
+    constexpr bool kFlat = TRI && std::is_same<T, float>::value;   // offsets from the centroid
+    constexpr int kN = kFlat ? 12 : 18;
+    if (TRI) {
+        R c[3];   // the centroid (FP64: the rule's first point) - x
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if constexpr (kFlat) c[k] = D[k];
+            else c[k] = vadd(D[k], e.v[6 + k]);
+        }
+        dny = vfma(c[2], e.v[kN + 2], vfma(c[0], e.v[kN], vmul(c[1], e.v[kN + 1])));
+    }
     constexpr int kUnroll = std::is_same<T, float>::value ? 4 : 1;   // FP64: pipe bound, registers short
 #pragma unroll kUnroll
     for (int g = 0; g < 4; ++g) {
         R d[3], w;
-        if constexpr (TRI) {
-            R ss, tt;
-            if constexpr (std::is_same<T, float>::value) {
-                const float2 s2 = c_far4d[g][0], t2 = c_far4d[g][1], w2 = c_far4d[g][2];
-                ss = pk2(s2.x, s2.y);
-                tt = pk2(t2.x, t2.y);
-                w = pk2(w2.x, w2.y);
-            } else {
-                ss = c_far64[g][0];
-                tt = c_far64[g][1];
-                w = c_far64[g][2];
-            }
+        if constexpr (kFlat) {
+            const float2 s2 = c_far4d[g][0], t2 = c_far4d[g][1], w2 = c_far4d[g][2];
+            const R ss = pk2(s2.x, s2.y), tt = pk2(t2.x, t2.y);
+            w = pk2(w2.x, w2.y);
 #pragma unroll
             for (int k = 0; k < 3; ++k) d[k] = vfma(tt, e.v[9 + k], vfma(ss, e.v[6 + k], D[k]));
         } else {
 #pragma unroll
             for (int k = 0; k < 3; ++k) d[k] = vadd(D[k], e.v[6 + 3 * g + k]);
-            dny = vfma(d[2], e.v[18 + 3 * g + 2], vfma(d[0], e.v[18 + 3 * g], vmul(d[1], e.v[18 + 3 * g + 1])));
-            w = e.v[30 + g];
+            if constexpr (TRI) {
+                w = c_far64[g][2];
+            } else {
+                dny = vfma(d[2], e.v[18 + 3 * g + 2], vfma(d[0], e.v[18 + 3 * g], vmul(d[1], e.v[18 + 3 * g + 1])));
+                w = e.v[30 + g];
+            }
         }
         const R r2 = vfma(d[2], d[2], vfma(d[0], d[0], vmul(d[1], d[1])));
         R r, sn, cs, u = vrsqrt(r2, &r);
@@ -1700,8 +1708,8 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
         P0i = vmul(dny, Ti);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            G0r[k] = vfma(Tr, e.v[12 + k], G0r[k]);
-            G0i[k] = vfma(Ti, e.v[12 + k], G0i[k]);
+            G0r[k] = vfma(Tr, e.v[kN + k], G0r[k]);
+            G0i[k] = vfma(Ti, e.v[kN + k], G0i[k]);
         }
     }
 #pragma unroll
@@ -1909,7 +1917,7 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
                     float d[3];
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        D[c] = tri ? e.v[c] - X[c] : -X[c];
+                        D[c] = -X[c];
                         d[c] = (e.hi[c] - xh[0][c]) + (e.lo[c] - xl[0][c]);
                     }
                     q2[0] = (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]) * e.isq2;
