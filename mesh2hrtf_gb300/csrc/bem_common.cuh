@@ -14,6 +14,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+#include <vector>
+
 #include "bem_f32x2.cuh"
 #include "bem_internal.h"
 
@@ -108,18 +111,33 @@ __device__ __forceinline__ double rsqrt_nr(double x, double *root) {
     return u;
 }
 
-// sin and cos of a phase (|x| below 10^9) by table look-up and a short
-// Taylor polynomial (P. T. P. Tang, "Table-driven implementation of the
-// exponential function", ACM TOMS 15, 1989, applied to the circle):
-// x = (q + f) 2 pi / 1024, q an integer, |f| <= 1/2; with the table's
-// (sin, cos) of q 2 pi / 1024 and the polynomials of f 2 pi / 1024
-// (|angle| <= 0.0031: the first terms left out are below 1e-17) the angle sum
-// takes 16 FP64 instructions, against about 35 of the general library
-// routine, whose large-argument branch is never needed here.  The
-// fraction keeps the product's low part (1024 / 2 pi in two doubles), so the
-// result is within about 2 ulp of 1.
+// sin and cos of a phase by table look-up and a short Taylor polynomial
+// (P. T. P. Tang, "Table-driven implementation of the exponential function",
+// ACM TOMS 15, 1989, applied to the circle): x = (q + f) 2 pi / 1024, q an
+// integer, |f| <= 1/2; with the table's (sin, cos) of q 2 pi / 1024, in two parts
+// each, and the polynomials of f 2 pi / 1024 (|angle| <= 0.0031: the first terms
+// left out are below 1e-17) the angle sum takes 16 FP64 instructions, against
+// about 35 of the general library routine.  The fraction keeps the product's low
+// part (1024 / 2 pi in two doubles) up to |x| = 2^43, so the result is the rounded
+// one plus at most 2^-58.
 constexpr int kScTab = 1024;
-__device__ double2 g_sctab[kScTab];   // (sin, cos)(2 pi q / kScTab), init_device_tables
+__device__ double2 g_sctab[kScTab][2];   // (sin, cos)(2 pi q / kScTab), high and low part
+
+inline cudaError_t init_sincos_table() {
+    std::vector<double2> tab(2 * kScTab);
+    for (int q = 0; q < kScTab; ++q) {
+        const long double ang = (long double)q * 6.283185307179586476925286766559005768L / kScTab;
+        const long double s = sinl(ang), c = cosl(ang);
+        tab[2 * q] = make_double2((double)s, (double)c);
+        tab[2 * q + 1] = make_double2((double)(s - (double)s), (double)(c - (double)c));
+    }
+    // exact on the axes, where the long double angle is not
+    for (int q = 0; q < 4; ++q) {
+        tab[q * (kScTab / 2)] = make_double2(q == 1 ? 1.0 : q == 3 ? -1.0 : 0.0, q == 0 ? 1.0 : q == 2 ? -1.0 : 0.0);
+        tab[q * (kScTab / 2) + 1] = make_double2(0.0, 0.0);
+    }
+    return cudaMemcpyToSymbol(g_sctab, tab.data(), tab.size() * sizeof(double2));
+}
 
 __device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
     constexpr double kShift = 6755399441055744.0;            // 1.5 * 2^52
@@ -129,12 +147,13 @@ __device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
     const double t = fma(x, kHi, kShift);
     const double q = t - kShift;
     const double f = fma(x, kLo, fma(x, kHi, -q));
-    const double2 sc = g_sctab[__double2loint(t) & (kScTab - 1)];
+    const double2 *tab = g_sctab[__double2loint(t) & (kScTab - 1)];
+    const double2 sc = tab[0], lo = tab[1];
     const double f2 = f * f;
     const double sr = f * fma(f2, fma(f2, a * a * a * a * a / 120.0, -a * a * a / 6.0), a);
     const double cm = f2 * fma(f2, a * a * a * a / 24.0, -a * a / 2.0);   // cos - 1
-    *s = sc.x + fma(sc.y, sr, sc.x * cm);
-    *c = sc.y + fma(-sc.x, sr, sc.y * cm);
+    *s = sc.x + fma(sc.y, sr, fma(sc.x, cm, lo.x));
+    *c = sc.y + fma(-sc.x, sr, fma(sc.y, cm, lo.y));
 }
 
 __device__ __forceinline__ void sincos_t(double x, double *s, double *c) { phase_sincos(x, s, c); }

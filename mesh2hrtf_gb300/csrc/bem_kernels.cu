@@ -2210,15 +2210,7 @@ cudaError_t init_device_tables() {
         far64[g][3] = 0.0;
     }
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far64, far64, sizeof(far64));
-    std::vector<double2> sctab(kScTab);
-    for (int q = 0; q < kScTab; ++q) {
-        const long double ang = (long double)q * 6.283185307179586476925286766559005768L / kScTab;
-        sctab[q] = make_double2((double)sinl(ang), (double)cosl(ang));
-    }
-    // exact on the axes, where the long double angle is not
-    for (int q = 0; q < 4; ++q)
-        sctab[q * (kScTab / 4)] = make_double2(q == 1 ? 1.0 : q == 3 ? -1.0 : 0.0, q == 0 ? 1.0 : q == 2 ? -1.0 : 0.0);
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_sctab, sctab.data(), sctab.size() * sizeof(double2));
+    if (e == cudaSuccess) e = init_sincos_table();
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_glxf, glxf, sizeof(glxf));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_glwf, glwf, sizeof(glwf));
     return e;
