@@ -119,7 +119,9 @@ __device__ __forceinline__ double rsqrt_nr(double x, double *root) {
 // left out are below 1e-17) the angle sum takes 16 FP64 instructions, against
 // about 35 of the general library routine.  The fraction keeps the product's low
 // part (1024 / 2 pi in two doubles) up to |x| = 2^43, so the result is the rounded
-// one plus at most 2^-58.
+// one plus at most 2^-58.  Larger phases, whose q would leave the shift's range,
+// go to the library: a test and a call in the loop over a far pair's points
+// (53 FP64 instructions each) cost it 4 %, so there the pair is tested.
 constexpr int kScTab = 1024;
 __device__ double2 g_sctab[kScTab][2];   // (sin, cos)(2 pi q / kScTab), high and low part
 
@@ -139,6 +141,7 @@ inline cudaError_t init_sincos_table() {
     return cudaMemcpyToSymbol(g_sctab, tab.data(), tab.size() * sizeof(double2));
 }
 
+// |x| below 2^43 (phase_reach, or sincos_t, which looks for itself)
 __device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
     constexpr double kShift = 6755399441055744.0;            // 1.5 * 2^52
     constexpr double kHi = 162.97466172610083;               // 1024 / (2 pi), high and low part
@@ -156,7 +159,27 @@ __device__ __forceinline__ void phase_sincos(double x, double *s, double *c) {
     *c = sc.y + fma(-sc.x, sr, fma(sc.y, cm, lo.y));
 }
 
-__device__ __forceinline__ void sincos_t(double x, double *s, double *c) { phase_sincos(x, s, c); }
+__device__ __noinline__ double2 sincos_large(double x) {
+    double2 r;
+    sincos(x, &r.x, &r.y);
+    return r;
+}
+__device__ __forceinline__ void sincos_t(double x, double *s, double *c) {
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x42A00000) {   // 2^43 or more, or not finite
+        const double2 r = sincos_large(x);
+        *s = r.x;
+        *c = r.y;
+    } else {
+        phase_sincos(x, s, c);
+    }
+}
+// Coordinates (the larger components of points x and y, as high words without
+// the sign) whose phase k |x - y| phase_sincos can take: both below
+// phase_reach(k) = 2^41 / |k|, so that k |x - y| < 2 sqrt(3) 2^41.
+__device__ __forceinline__ int phase_reach(double k) { return __double2hiint(2199023255552.0 / fabs(k)); }
+__device__ __forceinline__ int max_hi(double x, double y, double z) {
+    return max(__double2hiint(x) & 0x7fffffff, max(__double2hiint(y) & 0x7fffffff, __double2hiint(z) & 0x7fffffff));
+}
 __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { phase_sincos(x, s, c); }
 // ------------------------------------------------------------ packed or FP64 operands
 __device__ __forceinline__ void vdup(F2 &r, float x) { r = pk2(x, x); }

@@ -364,7 +364,7 @@ __device__ __forceinline__ void far_quad2(const FarConst &k, float (*st)[32], in
 //   u (b wr E - tau D.n_y u) + i u (b u (E + k^2 P) + tau wr D.n_y).
 // 53 FP64 instructions per point (the general form through map_point and the
 // library's square roots, divisions and sincos took about 250).  5120-triangle
-// head, 5 kHz: k_far 33.0 -> 12.8 ms.  Mean errors against 80-bit entries, this
+// head, 5 kHz: k_far 33.0 -> 12.9 ms.  Mean errors against 80-bit entries, this
 // and the general form, beyond a ratio of 4.5 and below 4, k = 73: head 1.35e-15
 // and 1.50e-15, 8.6e-16 and 9.1e-16; sphere flattened to a tenth 8.4e-16 and
 // 9.0e-16, 2.4e-16 and 3.0e-16.  |D|^2 + 2 s D.a + ... for the squared distance
@@ -375,6 +375,7 @@ struct FarCol64 {
     double a[3], b[3], n[3];
     double cln;          // cl . n
     double J4;           // J / (4 pi)
+    int far;             // the vertices' largest component (max_hi)
 };
 struct FusedCol64 {
     double yr, yi, tau, b, k2, wr;
@@ -382,9 +383,11 @@ struct FusedCol64 {
 
 __device__ __forceinline__ void far_col64(const DevMesh &m, int j, FarCol64 &e) {
     double n2 = 0.0;
+    e.far = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const double p2 = m.v64[(6 + k) * m.n + j];
+        e.far = max(e.far, max_hi(m.v64[k * m.n + j], m.v64[(3 + k) * m.n + j], p2));
         e.a[k] = m.v64[k * m.n + j] - p2;
         e.b[k] = m.v64[(3 + k) * m.n + j] - p2;
         const double o = (e.a[k] + e.b[k]) * (1.0 / 3.0);
@@ -707,6 +710,8 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
         FarCol64 e4;
         if (tri) far_col64(mk, j, e4);
         const FusedCol64 fc = {admj.re, admj.im, f.tao, f.beta_im, f.k * f.k, f.wr};
+        const int reach = phase_reach(f.wr);
+        const bool fits = tri && e4.far < reach;
 #pragma unroll 1
         for (int r = 0; r < rpt; ++r) {
             const int i = i0 + r;
@@ -728,7 +733,7 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
                 if (!near) {
                     const double x64[3] = {m.c64[i], m.c64[n + i], m.c64[2 * n + i]};
                     const double nx64[3] = {m.n64[i], m.n64[n + i], m.n64[2 * n + i]};
-                    if (tri) {
+                    if (fits && max_hi(x64[0], x64[1], x64[2]) < reach) {
                         val = far_entry_tri64(e4, x64, nx64, order, bcj, fc);
                     } else {
                         Elem64 e;
@@ -1511,7 +1516,7 @@ template <> struct ProjLane<double> { using R = double; static constexpr int kP 
 template <typename T, int NR> struct ProjElem {
     typename ProjLane<T>::R v[34], W[NR][4], V[NR][4][3];
     float hi[3], lo[3], isq2;
-    int nv, iv;
+    int nv, iv, far;   // far: the vertices' largest component (FP64; max_hi)
 };
 
 template <typename T>
@@ -1583,6 +1588,11 @@ __device__ void proj_stage(const ProjSys *sys, int nr, const DevMesh &m, const D
                 vdup(o.v[k], o.hi[k]);
                 vdup(o.v[3 + k], o.lo[k]);
             }
+        }
+        o.far = 0;
+        if constexpr (std::is_same<T, double>::value) {
+            for (int a = 0; a < nv; ++a)
+                o.far = max(o.far, max_hi(mk.v64[3 * a * n + j], mk.v64[(3 * a + 1) * n + j], mk.v64[(3 * a + 2) * n + j]));
         }
     }
     bool any = false;
@@ -1726,7 +1736,8 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
     }
 }
 
-// A not subdivided pair of a higher Gauss order, by one lane.
+// A not subdivided pair of a higher Gauss order, or of a phase beyond
+// phase_sincos's range, by one lane.
 template <typename T>
 __device__ __noinline__ ProjAcc<T> proj_whole(const ProjSys *Sp, int kref, int j, int order, int p) {
     const ProjSys &S = *Sp;
@@ -1891,6 +1902,11 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
         for (int c = 0; c < 3; ++c) acc[r].gr[c] = acc[r].gi[c] = acc[r].pr;
     }
     if (NR == 1) nr = 1;
+    int reach = 0;   // FP64: phases of elements within it fit phase_sincos
+    if constexpr (P == 1) {
+        reach = phase_reach(wrs);
+        if (max_hi(X[0], X[1], X[2]) >= reach) reach = 0;
+    }
     int err = kDevOk;
     for (int kref = 0; kref < m.sym.nref; ++kref) {
         const DevMesh mk = image_mesh(m, kref);
@@ -1938,7 +1954,7 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
                         }
                         if (near) ord[h] = 0;
                     }
-                    if (ord[h] == 2) far |= 1u << h;
+                    if (ord[h] == 2 && (P == 2 || e.far < reach)) far |= 1u << h;
                 }
                 if (__any_sync(0xffffffffu, far != 0)) {
                     if (tri) {
@@ -1953,7 +1969,7 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
 #pragma unroll
                 for (int h = 0; h < P; ++h) {
                     const bool pv = p0 + 32 * h < npts;
-                    if (pv && ord[h] > 2)
+                    if (pv && ord[h] != 0 && !((far >> h) & 1u))
 #pragma unroll 1
                         for (int r = 0; r < nr; ++r)
                             racc_at<T, NR>(acc, r, h, proj_whole<T>(&tb.sys[sb + r], kref, base + q, ord[h], p0 + 32 * h));

@@ -7,7 +7,7 @@ in the last place.
 
 Sine and cosine: the table's two parts are good to 2^-64 or more, the angle sum's
 corrections (below 2^-8) carry three roundings and the result one: half a unit in
-the last place plus 2^-58, up to phases of 2^43."""
+the last place plus 2^-58, up to phases of 2^43; the library's two units beyond."""
 import ctypes
 import os
 import subprocess
@@ -15,7 +15,8 @@ import subprocess
 import numpy as np
 import pytest
 
-from mesh2hrtf_gb300 import build
+from mesh2hrtf_gb300 import build, capi
+from oracle import oracle_py as oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -82,15 +83,51 @@ def test_square_root(lib):
     assert (np.abs(e) <= 1.5 * unit).all()
 
 
-def test_sine_and_cosine(lib):
+@pytest.mark.parametrize("large", [False, True])
+def test_sine_and_cosine(lib, large):
     rng = np.random.default_rng(2)
     n = 1 << 16
-    x = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-20, 43, n)) * rng.choice([-1.0, 1.0], n)
-    q = rng.integers(-4000, 4000, n // 2)
-    x[: n // 2] = (q + 0.5 * (q & 1)) * (2 * np.pi / 1024)   # cells' centres and borders
-    x[0] = 0.0
+    lo, hi = (43, 200) if large else (-20, 43)
+    x = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(lo, hi, n)) * rng.choice([-1.0, 1.0], n)
+    if not large:
+        q = rng.integers(-4000, 4000, n // 2)
+        x[: n // 2] = (q + 0.5 * (q & 1)) * (2 * np.pi / 1024)   # cells' centres and borders
+        x[0] = 0.0
     s, c = np.zeros(n), np.zeros(n)
     assert lib.run_sincos(n, _p(x), _p(s), _p(c)) == 0
     for got, f in ((s, np.sin), (c, np.cos)):
         e = np.abs(got - f(x.astype(np.longdouble)))
-        assert (e <= 0.5 * np.ldexp(1.0, np.frexp(got)[1] - 53) + 2.0**-58).all()
+        unit = np.ldexp(1.0, np.frexp(got)[1] - 53)
+        assert (e <= (2 * unit if large else 0.5 * unit + 2.0**-58)).all()
+
+
+@pytest.mark.parametrize("quad", [False, True])
+def test_distances_beyond_the_table(quad):
+    """Phases of 1e18: in double precision all points of a small element are at
+    the same distance of a point 5e14 away, so its entries and fields there have
+    the oracle's sizes, whatever the phase."""
+    shape = np.array([[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]] if quad else [[0, 0, 0], [1, 0, 0], [0, 1, 0]], float)
+    c = len(shape)
+    row = np.array([3e14, 0, 4e14]) + 1e3 * (shape + shape[:, [1, 2, 0]])
+    v, k = np.concatenate([1e-4 * shape, row]), 2000.0
+    pts = np.array([[-3e14, 0, 4e14], [1e14, 2e14, -5e14]])
+    weak = dict(point_sources=[[5.0, 0, 0]], point_amps=[1e-60])
+    for n in (2, 1):
+        f = np.arange(n * c, dtype=np.int32).reshape(n, c)
+        bcv = np.zeros((n, 4), complex)
+        bcv[0, :c] = 1.0
+        om, of = oracle.OracleMesh(v[: n * c], f, None, bcv), oracle.OracleFreq(k, *weak.values())
+        m = capi.Mesh(v[: n * c], f)
+        s = capi.Solver(m, precision=capi.PREC_FP64)
+        s.assemble(capi.Frequency(k, n, bc_value=bcv, **weak))
+        if n == 2:
+            A, want = s.system()[0], oracle.assemble(om, of)[0]
+            assert abs(abs(A[1, 0]) - abs(want[1, 0])) <= 1e-9 * abs(want[1, 0])
+        else:
+            s.solve()
+            pot, grad = s.project(pts)
+            q, g = oracle.project(om, of, *oracle.boundary_fields(om, s.solution()), pts)
+            assert (abs(abs(pot) - abs(q)) <= 1e-9 * abs(q)).all()
+            assert (abs(abs(grad) - abs(g)) <= 1e-9 * abs(g).max(axis=1)[:, None]).all()
+        s.close()
+        m.close()
