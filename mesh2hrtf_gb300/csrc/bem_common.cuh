@@ -192,7 +192,6 @@ __device__ __forceinline__ F2 vrsqrt(F2 a, F2 *root) {
     *root = vmul(a, u);
     return u;
 }
-__device__ __forceinline__ double vrsqrt(double a, double *root) { return rsqrt_nr(a, root); }
 // Constants of phase_sincos in packed form.
 template <typename R> struct ScConst {};
 template <> struct ScConst<F2> {

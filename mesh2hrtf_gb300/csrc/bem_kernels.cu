@@ -1666,15 +1666,19 @@ __device__ __forceinline__ void proj_far(const ProjElem<T, NR> &e, int nr, const
             }
         }
         const R r2 = vfma(d[2], d[2], vfma(d[0], d[0], vmul(d[1], d[1])));
-        R r, sn, cs, u = vrsqrt(r2, &r);
-        vsincos(sc, vmul(wr, r), sn, cs);
+        // points out of the mask: zero distance, before anything is formed from
+        // it (such a point may lie on this rule's, or beyond phase_sincos)
+        R r, sn, cs, u;
         if constexpr (std::is_same<T, float>::value) {
             float lo, hi;
-            unpk2(u, lo, hi);
-            u = pk2((mask & 1u) ? lo : 0.f, (mask & 2u) ? hi : 0.f);
+            unpk2(r2, lo, hi);
+            u = pk2((mask & 1u) ? rsqrt_approx(lo) : 0.f, (mask & 2u) ? rsqrt_approx(hi) : 0.f);
+            r = vmul(r2, u);
         } else {
-            u = mask ? u : 0.0;
+            u = rsqrt_nr(r2, &r);
+            if (!mask) u = r = 0.0;
         }
+        vsincos(sc, vmul(wr, r), sn, cs);
         const R A = vmul(u, u), B = vmul(wr, u), nB = vmul(nwr, u), p = vmul(w, u);
         const R Gr = vmul(p, cs), Gi = vmul(p, sn);
         const R hr = vfma(Gi, B, vmul(Gr, A)), hi = vfma(Gr, nB, vmul(Gi, A));   // G alpha
