@@ -305,18 +305,33 @@ __device__ __forceinline__ void far_point2(const FarConst &k, const FusedCol2 &c
     o.ai = vfma(cs, qi, vfma(sn, qr, o.ai));
 }
 
-template <int BC>
+// DIFF: the squared distance from the difference of the points, as every other
+// pair's, for meshes with symmetry images.  Where a long thin triangle's point is
+// closer than its centroid, the expanded sum loses (|D| / r)^2 units, and
+// images come close at their plane.
+template <int BC, bool DIFF>
 __device__ __forceinline__ void far_tri2(const FarConst &k, const FarCol2 &e, const F2 D[3], F2 D2, const F2 nx[3],
                                          const FusedCol2 &c, FarSum2 &o) {
     const F2 dny = dot2(D, e.n), dnx = dot2(D, nx), nn = dot2(e.n, nx);
     const F2 anx = dot2(e.a, nx), bnx = dot2(e.b, nx);
-    F2 Da = dot2(D, e.a), Db = dot2(D, e.b);
-    Da = vadd(Da, Da);   // exact: 2 s D.a = s (2 D.a)
-    Db = vadd(Db, Db);
+    F2 Da, Db;
+    if (!DIFF) {
+        Da = dot2(D, e.a);
+        Db = dot2(D, e.b);
+        Da = vadd(Da, Da);   // exact: 2 s D.a = s (2 D.a)
+        Db = vadd(Db, Db);
+    }
+    auto r2 = [&](F2 s, F2 t, F2 C) {
+        if (!DIFF) return vfma(s, Da, vfma(t, Db, vadd(D2, C)));
+        F2 d[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) d[q] = vfma(t, e.b[q], vfma(s, e.a[q], D[q]));
+        return dot2(d, d);
+    };
     far_point2<BC>(k, c, D2, dny, dnx, nn, e.wJ0, o);
-    far_point2<BC>(k, c, vfma(k.p, Da, vfma(k.p, Db, vadd(D2, e.C[0]))), dny, vfma(k.p, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
-    far_point2<BC>(k, c, vfma(k.q, Da, vfma(k.p, Db, vadd(D2, e.C[1]))), dny, vfma(k.p, bnx, vfma(k.q, anx, dnx)), nn, e.wJ1, o);
-    far_point2<BC>(k, c, vfma(k.p, Da, vfma(k.q, Db, vadd(D2, e.C[2]))), dny, vfma(k.q, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
+    far_point2<BC>(k, c, r2(k.p, k.p, e.C[0]), dny, vfma(k.p, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
+    far_point2<BC>(k, c, r2(k.q, k.p, e.C[1]), dny, vfma(k.p, bnx, vfma(k.q, anx, dnx)), nn, e.wJ1, o);
+    far_point2<BC>(k, c, r2(k.p, k.q, e.C[2]), dny, vfma(k.q, bnx, vfma(k.p, anx, dnx)), nn, e.wJ1, o);
 }
 
 // The same for a quadrilateral column, whose four points (offset from the
@@ -675,7 +690,7 @@ __device__ __noinline__ float2 far_entry_general(const DevMeshView *mv, int kref
 // kref = 0 writes the entries; the images add theirs (reflection factor
 // applied, NC_AssembleTBEM, NC_EquationSystem.cpp:181-206) in image order.
 // Near images and the self pair contribute zero here; k_near adds them.
-template <typename T>
+template <typename T, bool IMG>
 __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f,
                                          typename Vec2<T>::type *__restrict__ A, size_t lda, int tx, int i0, int kref,
                                          const FarConst &fk, float (*st)[32]) {
@@ -791,9 +806,14 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
             FarSum2 o = {dup2(0.f), dup2(0.f), dup2(0.f)};
             if (ord[0] == 2 || ord[1] == 2) {
                 if (tri) {
-                    if (bcj == 0) far_tri2<0>(fk, e2, D, D2, nx, f2, o);
-                    else if (bcj == 1) far_tri2<1>(fk, e2, D, D2, nx, f2, o);
-                    else far_tri2<2>(fk, e2, D, D2, nx, f2, o);
+                    auto points = [&](auto diff) {
+                        constexpr bool kDiff = decltype(diff)::value;
+                        if (bcj == 0) far_tri2<0, kDiff>(fk, e2, D, D2, nx, f2, o);
+                        else if (bcj == 1) far_tri2<1, kDiff>(fk, e2, D, D2, nx, f2, o);
+                        else far_tri2<2, kDiff>(fk, e2, D, D2, nx, f2, o);
+                    };
+                    if (IMG && m.sym.nref > 1) points(std::true_type());
+                    else points(std::false_type());
                 } else {
                     if (bcj == 0) far_quad2<0>(fk, st, lane, D, nx, f2, o);
                     else if (bcj == 1) far_quad2<1>(fk, st, lane, D, nx, f2, o);
@@ -843,7 +863,7 @@ __global__ void __launch_bounds__(256, kFarPerSm) k_far(const __grid_constant__ 
         const int ntx = (S.m.n + 31) / 32;
         const int nref = IMG ? S.m.sym.nref : 1;
         for (int kref = 0; kref < nref; ++kref)
-            far_tile<T>(S.m, S.f, (typename Vec2<T>::type *)S.A, S.lda, local % ntx, local / ntx * far_rows(S.m.n), kref,
+            far_tile<T, IMG>(S.m, S.f, (typename Vec2<T>::type *)S.A, S.lda, local % ntx, local / ntx * far_rows(S.m.n), kref,
                         fk, st[std::is_same<T, float>::value ? threadIdx.y : 0]);
     }
 }

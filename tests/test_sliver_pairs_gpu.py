@@ -1,10 +1,12 @@
-"""FP64 matrix entries where a far pair's quadrature point is much closer than
+"""Matrix entries where a far pair's quadrature point is much closer than
 its centroid: a long thin triangle (1 : 500) whose distance ratio asks for the
 4-point rule, collocation points 3e-4 and 3e-3 of its length beside two of the
 rule's points, against the same rule in extended precision.
 
-Bar: a point's vector d = y - x has an error of 3 u (|y| + |x|), u = 2^-53, with
-both within the length of 1, so r and the products with the normals are good to
+FP64, and mixed precision with a symmetry plane (far enough for the images to
+be below the bar).  Bar: a point's vector d = y - x has an error of
+3 u (|y| + |x|), u the unit roundoff, with both within the length of 1 (float
+works with vectors from the centroid), so r and the products with the normals are good to
 6 u / r of themselves; an entry's terms go with up to 1 / r^3, with a distance
 and two products in them, and some forty operations more:
 (8 * 6 u / r + 64 u) of the sum of the terms' sizes."""
@@ -54,15 +56,18 @@ def _entry(p, x, nx, k, tau=1):
 
 @pytest.mark.parametrize("seed", [4, 5, 6])
 @pytest.mark.parametrize("k", [2.0, 60.0])
-def test_entries(k, seed):
+@pytest.mark.parametrize("prec,sym,u", [(capi.PREC_FP64, (0, 0, 0), 2.0**-53), (capi.PREC_MIXED, (0, 1, 0), 2.0**-24)])
+def test_entries(prec, sym, u, k, seed):
     v, f = _mesh(np.random.default_rng(seed))
-    m = capi.Mesh(v, f)
-    s = capi.Solver(m, precision=capi.PREC_FP64)
+    if any(sym):
+        v = v + [0, 40.0, 0]
+    m = capi.Mesh(v, f, sym_planes=sym)
+    s = capi.Solver(m, precision=prec)
     s.assemble(capi.Frequency(k, len(f), point_sources=[[9.0, 9.0, 9.0]], point_amps=[1.0]))
     A, _ = s.system()
     s.close()
     m.close()
-    u, p = 2.0**-53, v[f[0]].astype(L)
+    p = v[f[0]].astype(L)
     a, b = p[0] - p[2], p[1] - p[2]
     for i in range(1, len(f)):
         q = v[f[i]]
