@@ -942,8 +942,11 @@ __global__ void __launch_bounds__(32 * (kGrpWarps + 1), 1) k_mv_grp(KTable *tb, 
             return v;
         };
         const int c1 = (len & 1) && lane == (len2 & 31) ? len2 + 1 : len2;
-        if (mymask && tb->sys[mt.first].n >= kGrpBiasedMin) {
-            float asum[RW], xmax[MW];
+        bool biased = mymask && tb->sys[mt.first].n >= kGrpBiasedMin;
+        float asum[RW], xmax[MW];
+        // twice the bound, with room for its rounding
+        auto bound = [&](int r, int q) { return 2.001f * asum[r] * xmax[q]; };
+        if (biased) {
 #pragma unroll
             for (int r = 0; r < RW; ++r) {
                 asum[r] = 0.f;
@@ -952,6 +955,7 @@ __global__ void __launch_bounds__(32 * (kGrpWarps + 1), 1) k_mv_grp(KTable *tb, 
                     asum[r] += (fabsf(a.x) + fabsf(a.y)) + (fabsf(a.z) + fabsf(a.w));
                 }
             }
+            float most = 0.f;
 #pragma unroll
             for (int q = 0; q < MW; ++q) {
                 xmax[q] = 0.f;
@@ -960,11 +964,15 @@ __global__ void __launch_bounds__(32 * (kGrpWarps + 1), 1) k_mv_grp(KTable *tb, 
                     const float4 x = load(xrow(q), c);
                     xmax[q] = fmaxf(xmax[q], fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
                 }
+#pragma unroll
+                for (int r = 0; r < RW; ++r) most = fmaxf(most, bound(r, q));
             }
-            // twice the bound, with room for its rounding; the cap keeps the bias
-            // finite (sums near the type's end lose the error term there)
+            // near the type's end the bias would not be finite: two-sums there
+            biased = !__any_sync(0xffffffffu, !(most < 4e37f));
+        }
+        if (biased) {
             auto bias = [&](int r, int q) {
-                const float b = fminf(2.001f * asum[r] * xmax[q], 4e37f);
+                const float b = bound(r, q);
                 return pk2(b, b);
             };
             F2 s[RW][MW], e[RW][MW];
