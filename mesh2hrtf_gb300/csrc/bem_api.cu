@@ -481,8 +481,8 @@ bem_status batch_ctx(BatchCtx **out) {
         auto c = std::make_unique<BatchCtx>();
         CU(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
         for (auto &e : c->ev) CU(cudaEventCreate(&e));
-        CU(cudaMalloc(&c->ctr, 4 * sizeof(unsigned)));
-        CU(cudaMemset(c->ctr, 0, 4 * sizeof(unsigned)));
+        CU(cudaMalloc(&c->ctr, 2 * sizeof(unsigned)));
+        CU(cudaMemset(c->ctr, 0, 2 * sizeof(unsigned)));
         t_batch = std::move(c);
     }
     *out = t_batch.get();
@@ -1272,7 +1272,7 @@ bem_status bem_solver_create(bem_mesh_t mesh, const bem_solver_params *p, bem_so
         s->xr.resize(n_rhs - 1);
         s->xfreq.resize(n_rhs - 1);
         bem::solver_layout(n, prec, m, pc, s->block, &s->d, n_rhs, s->xr.data(), kcopy);
-        e = cudaMemset(s->d.ctr, 0, 4 * sizeof(unsigned));
+        e = cudaMemset(s->d.ctr, 0, 2 * sizeof(unsigned));
     }
     if (e != cudaSuccess)
         return fail(e == cudaErrorMemoryAllocation ? BEM_ERR_OUT_OF_HBM : BEM_ERR_CUDA, "solver allocation: %s",

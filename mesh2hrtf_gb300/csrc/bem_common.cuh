@@ -219,9 +219,6 @@ __device__ __forceinline__ void vsincos(const ScConst<double> &, double x, doubl
     phase_sincos(x, &s, &c);
 }
 
-__device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
-__device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
-
 // ------------------------------------------------------------ quadrature
 // Triangle rules on the (1,0),(0,1),(0,0) reference triangle (weights sum to
 // 0.5): Strang-Fix 4-point (order 2), Radon 7-point (order 3), 13-point
@@ -247,9 +244,8 @@ struct QuadTables {
 // header.
 __constant__ QuadTables c_quad;
 __constant__ float c_trif[24][3];
-// The 4-point rule's (s - 1/3, t - 1/3, 2 (s - 1/3), 2 (t - 1/3)): operands of
-// the expanded squared distance of the order-2 far pairs.
-__constant__ float c_far4[4][4];
+// The 4-point rule's (s - 1/3, t - 1/3), operands of the order-2 far pairs.
+__constant__ float c_far4[4][2];
 // (s - 1/3, t - 1/3, weight) in double for the FP64 pairs on flat triangles:
 // every triangle rule's points, in the order of QuadTables::tri
 __constant__ double c_far64[24][4];

@@ -153,8 +153,8 @@ inline size_t image_table_bytes(int n, int nref) {
 }
 // A = assembled TBEM matrices of the batch, complex128 (prec 0) or complex64
 // (prec 1): regular pairs (persistent k_far), then the near lists (persistent
-// k_near).  ctr: 4 device words, zero before the first use; the kernels leave
-// them zero.
+// k_near).  ctr: 2 device words, the queue of k_near, zero before the first
+// use; the kernel leaves them zero.
 // Launch shapes of the assembly (persistent grids: resident blocks per SM of
 // k_far, at most kFarPerSmMax, and of k_near, at most 2, with twice as many of
 // its complex64 form, which keeps fewer registers); the results do not

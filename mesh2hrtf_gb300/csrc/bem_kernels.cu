@@ -162,7 +162,7 @@ __device__ __forceinline__ void tri_points(const Elem32 &e, float dny, float dnx
     }
 }
 
-// Matrix entry of a regular pair in float with a fixed Gauss order.  Flat
+// Matrix entry of a regular pair in float with a Gauss order above 2.  Flat
 // triangles: n_y is constant and d.n_y = D.n_y at every point; d.n_x is
 // affine in (s, t).
 __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3], int order, const FusedCol &c) {
@@ -173,8 +173,7 @@ __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3]
         const float anx = e.a[0] * nx[0] + e.a[1] * nx[1] + e.a[2] * nx[2];
         const float bnx = e.b[0] * nx[0] + e.b[1] * nx[1] + e.b[2] * nx[2];
         const float nn = e.n[0] * nx[0] + e.n[1] * nx[1] + e.n[2] * nx[2];
-        if (order <= 2) tri_points<4, 0>(e, dny, dnx0, anx, bnx, nn, c, ar, ai);
-        else if (order == 3) tri_points<7, 4>(e, dny, dnx0, anx, bnx, nn, c, ar, ai);
+        if (order == 3) tri_points<7, 4>(e, dny, dnx0, anx, bnx, nn, c, ar, ai);
         else tri_points<13, 11>(e, dny, dnx0, anx, bnx, nn, c, ar, ai);
     } else {
         const int np = quad_count(order);
@@ -655,8 +654,10 @@ __global__ void __launch_bounds__(256) k_near_list(DevMeshView mv, const float4 
 //
 // Rows per item (an item is one warp's 32 columns x far_rows rows): the more,
 // the further the column's preparation is spread; small systems take fewer so
-// that the 2432 warps of the grid get about six items or more each (with one
-// or two the last round would leave most of them idle).
+// that the 2432 warps of the grid (two blocks of eight on each of 152 SMs) get
+// about six items or more each (with one or two the last round would leave most
+// of them idle).  The host and the kernel both form it, so it goes by the
+// number and not by the device; entries do not depend on it.
 __host__ __device__ inline int far_rows(int n) {
     const long long e = (long long)n * n / (32 * 6 * 2432);   // rows for six items per warp
     return e >= 16 ? 16 : e >= 8 ? 8 : e >= 4 ? 4 : 2;
@@ -673,7 +674,7 @@ __device__ __noinline__ int far_order_exact(const DevMeshView *mv, int kref, int
     const double rd = ratio0_exact(image_mesh(m, kref), j, x64);
     return rd < kTolf ? 0 : gauss_order(rd);
 }
-// Entry of a quadrilateral column or of a Gauss order above 2.
+// Entry of a Gauss order above 2.
 __device__ __noinline__ float2 far_entry_general(const DevMeshView *mv, int kref, int j, float D0, float D1, float D2,
                                                  float nx0, float nx1, float nx2, int order, FusedCol fc) {
     const DevMesh m = image_mesh(to_dev(*mv), kref);
@@ -1519,7 +1520,10 @@ constexpr int kProjSlice = 256;   // most elements per slice
 constexpr int kProjStep = 16;     // fewest elements per slice
 // elements staged at a time (the stage and the subdivision scratch share 48 KB)
 __host__ __device__ constexpr int proj_chunk(int nr) { return nr <= 2 ? 16 : 8; }
-constexpr int kProjSlots = 304;   // resident blocks: 2 on each of 152 SMs
+// Resident blocks, 2 on each of 152 SMs: a number and not the device's own, since
+// the split decides the order of a field's sums and a result should not depend
+// on the device.
+constexpr int kProjSlots = 304;
 
 template <typename T> struct ProjLane;
 template <> struct ProjLane<float> { using R = F2; static constexpr int kP = 2, kPart = 2; };
@@ -2072,7 +2076,8 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
 // that finishes the point.  The additions and conversions run on an SM's
 // narrow FP64 pipe, so few points (up to kSumSpread) go 4 to a block to reach
 // more SMs: 64 points x 320 slices on 2 SMs took 56 us, on 16 they take 15.
-constexpr int kSumSpread = 2432;   // 4 points per block: up to 4 blocks per SM
+// (4 blocks on each of 152 SMs, as a number for the reason given at kProjSlots)
+constexpr int kSumSpread = 2432;
 __host__ __device__ inline int sum_points(int npts) { return npts <= kSumSpread ? 4 : 32; }
 
 template <typename T>
@@ -2227,12 +2232,10 @@ cudaError_t init_device_tables() {
     q.far2_sq = (float)((q.order_thr[2] * (1.0 + 3e-5)) * (q.order_thr[2] * (1.0 + 3e-5)));
     cudaError_t e = cudaMemcpyToSymbol(c_quad, &q, sizeof(q));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_trif, trif, sizeof(trif));
-    float far4[4][4];
+    float far4[4][2];
     for (int g = 0; g < 4; ++g) {
         far4[g][0] = trif[g][0] - (1.0f / 3.0f);
         far4[g][1] = trif[g][1] - (1.0f / 3.0f);
-        far4[g][2] = 2.0f * far4[g][0];
-        far4[g][3] = 2.0f * far4[g][1];
     }
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_far4, far4, sizeof(far4));
     float2 far4d[4][3];
@@ -2394,8 +2397,8 @@ cudaError_t launch_assemble(const AsmBatch &t, int prec, unsigned *ctr, cudaStre
         far(t, gfar);
     }
     if (near_items) {
-        if (prec == 0) k_near<double><<<gnear, block, 0, st>>>(t, ctr + 2);
-        else k_near<float><<<gnear, block, 0, st>>>(t, ctr + 2);
+        if (prec == 0) k_near<double><<<gnear, block, 0, st>>>(t, ctr);
+        else k_near<float><<<gnear, block, 0, st>>>(t, ctr);
     }
     return cudaGetLastError();
 }

@@ -170,14 +170,14 @@ void bem_server_s::run() {
     cudaStreamCreateWithFlags(&st_k, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&st_a, cudaStreamNonBlocking);
     unsigned *ctr = nullptr;
-    cudaMalloc(&ctr, 4 * sizeof(unsigned));
+    cudaMalloc(&ctr, 2 * sizeof(unsigned));
     // pinned status words of the requests in preparation (assembly, block
     // inverse): at most max_active requests are in preparation at once
     int *h_pool = nullptr;
     cudaMallocHost(&h_pool, 2 * sizeof(int) * bem::kMaxSys);
     std::vector<int> free_slots;
     for (int i = bem::kMaxSys - 1; i >= 0; --i) free_slots.push_back(i);
-    cudaMemset(ctr, 0, 4 * sizeof(unsigned));
+    cudaMemset(ctr, 0, 2 * sizeof(unsigned));
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     cudaEventCreate(&pe0);
     cudaEventCreate(&pe1);

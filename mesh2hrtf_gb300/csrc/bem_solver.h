@@ -82,7 +82,7 @@ struct SolverBufs {
     void *Minv = nullptr, *Mwork = nullptr;
     void *pcy = nullptr, *pcz = nullptr;   // window correction vectors
     int *status = nullptr;
-    unsigned *ctr = nullptr;   // 4 words: work queues of the persistent assembly kernels
+    unsigned *ctr = nullptr;   // 2 words: the work queue of k_near
     double *phi = nullptr, *vel = nullptr;
     float *phi32 = nullptr, *vel32 = nullptr;
     int *ivi = nullptr;
