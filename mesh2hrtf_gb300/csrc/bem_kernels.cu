@@ -772,9 +772,11 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
         fc.b = PT.beta_im;
         fc.k2 = PT.k * PT.k;
         fc.wr = PT.wr;
-        const FusedCol2 f2 = {dup2(fc.wr), dup2(fc.b), dup2(fc.b * fc.wr), dup2(fc.k2), dup2(-fc.tau),
-                              dup2(fc.tau * fc.wr), dup2(fc.yr), dup2(fc.yi), dup2(-fc.yi), dup2(fc.b * fc.tau),
-                              dup2(fc.b * fc.tau * fc.wr)};
+        // products of the constants rounded once: b wr is +-1 up to FP64's rounding
+        const double b = f.beta_im, wr = f.wr, tau = f.tao;
+        const FusedCol2 f2 = {dup2(fc.wr), dup2(fc.b), dup2((float)(b * wr)), dup2((float)(f.k * f.k)), dup2(-fc.tau),
+                              dup2((float)(tau * wr)), dup2(fc.yr), dup2(fc.yi), dup2(-fc.yi), dup2((float)(b * tau)),
+                              dup2((float)(b * tau * wr))};
 #pragma unroll 1
         for (int r = 0; r < rpt; r += 2) {
             const int i = i0 + r;
