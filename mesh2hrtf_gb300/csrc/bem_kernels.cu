@@ -1520,6 +1520,12 @@ __global__ void __launch_bounds__(256, 2) k_project(const __grid_constant__ Proj
 // elements 17.1 -> 5.8 ms.
 constexpr int kProjSlice = 256;   // most elements per slice
 constexpr int kProjStep = 16;     // fewest elements per slice
+// Elements of a slice whose terms are added one by one, each with two roundings at
+// the sum's size; the runs are then added up.  One sum over a slice (476 elements
+// where the scratch holds 43 slices) left gradients near the surface up to a fifth
+// further from 64-bit ones than single roundings had; runs of 64 leave them 0.6 ..
+// 0.9 of that, in the same time.
+constexpr int kProjRun = 64;
 // elements staged at a time (the stage and the subdivision scratch share 48 KB)
 __host__ __device__ constexpr int proj_chunk(int nr) { return nr <= 2 ? 16 : 8; }
 // Resident blocks, 2 on each of 152 SMs: a number and not the device's own, since
@@ -1645,6 +1651,21 @@ __device__ void proj_stage(const ProjSys *sys, int nr, const DevMesh &m, const D
 }
 
 template <typename R> struct RAcc { R pr, pi, gr[3], gi[3]; };
+template <typename R> __device__ __forceinline__ void racc_zero(RAcc<R> &a) {
+    vdup(a.pr, 0);
+    a.pi = a.pr;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a.gr[k] = a.gi[k] = a.pr;
+}
+template <typename R> __device__ __forceinline__ void racc_sum(RAcc<R> &a, const RAcc<R> &b) {
+    a.pr = vadd(a.pr, b.pr);
+    a.pi = vadd(a.pi, b.pi);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a.gr[k] = vadd(a.gr[k], b.gr[k]);
+        a.gi[k] = vadd(a.gi[k], b.gi[k]);
+    }
+}
 
 // The 4-point rule of a staged element at the lane's points, for the points
 // with their bit in mask, added to the right-hand sides' sums.
@@ -1923,14 +1944,23 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
     m3 = opaque2(T(-3));
     ScConst<R> sc;
     sc.init();
-    RAcc<R> acc[NR];
+    // sums of up to kProjRun elements; of those before them, in local memory,
+    // which the compiler is to leave there (in registers they push the loop's
+    // own values out)
+    RAcc<R> acc[NR], sum_s[NR], *sum = sum_s;
+    asm volatile("" : "+l"(sum)::"memory");
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        vdup(acc[r].pr, 0);
-        acc[r].pi = acc[r].pr;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc[r].gr[c] = acc[r].gi[c] = acc[r].pr;
+        racc_zero(acc[r]);
+        racc_zero(sum[r]);
     }
+    auto flush = [&]() {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            racc_sum(sum[r], acc[r]);
+            racc_zero(acc[r]);
+        }
+    };
     if (NR == 1) nr = 1;
     int reach = 0;   // FP64: phases of elements within it fit phase_sincos
     if constexpr (P == 1) {
@@ -2016,15 +2046,17 @@ __global__ void __launch_bounds__(256, NR <= 2 ? 2 : 1) k_project_pts(const __gr
                     }
                 }
             }
+            if ((base + kChunk - j0) % kProjRun == 0) flush();
         }
     }
+    flush();
     if (err != kDevOk && lane == 0) atomicMax(S.status, err);
     // the element parts of a point group meet in shared memory, in order
     R *red = reinterpret_cast<R *>(ws_all);   // [warp][8][lane]
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
         if (r >= nr) break;
-        RAcc<R> &a = acc[r];
+        RAcc<R> a = sum[r];
         if (ewb > 1) {
             __syncthreads();
             if (ew > 0) {
