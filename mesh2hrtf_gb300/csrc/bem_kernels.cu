@@ -1822,6 +1822,15 @@ __device__ __noinline__ ProjAcc<T> proj_whole(const ProjSys *Sp, int kref, int j
         }
         Elem32 e;
         load_elem32(mk, j, xhi, xlo, e);
+        if (nv == 3 && !iv) {   // the unknown once per pair, the points' constants in the code
+            float2 P = make_float2(0.f, 0.f), U[3] = {P, P, P}, Tn = P;
+            const float dny = e.D[0] * e.n[0] + e.D[1] * e.n[1] + e.D[2] * e.n[2];
+            if (order == 3) proj_tri_points<7, 4>(e, dny, k * k, wr, P, U, Tn);
+            else proj_tri_points<13, 11>(e, dny, k * k, wr, P, U, Tn);
+            acc.p = ph * cplx<float>{P.x, P.y};
+            for (int q = 0; q < 3; ++q) acc.g[q] = ph * cplx<float>{fmaf(Tn.x, e.n[q], U[q].x), fmaf(Tn.y, e.n[q], U[q].y)};
+            return acc;
+        }
         for (int g = 0; g < np; ++g) {
             float s, t, w;
             sub_point_f(nv, order, g, 0.f, 0.f, 1.f, s, t, w);
@@ -2340,7 +2349,12 @@ void asm_batch_finish(AsmBatch &t) {
 // more where that leaves SMs idle, down to kProjStep elements; the number of
 // blocks is then rounded down to whole rounds of the resident ones (2 per SM
 // of 152; 26 slices of 24 blocks ran a third round for 16 of them: 11950 points
-// on 20480 elements 2.43 ms, with whole rounds 2.15), and the scratch may hold fewer.
+// on 20480 elements 2.43 ms, with whole rounds 2.15), and the scratch may hold
+// fewer.  Where it leaves less than a round of blocks, as for many points on a
+// small mesh, blocks take fewer groups, whose elements their warps then share:
+// points near the surface, with their subdivided pairs and higher orders, often
+// follow one another and would hold up a few blocks (2000 triangles, 10550
+// points of which 500 are near: 4.8 -> 0.73 ms).
 void proj_batch_finish(ProjBatch &t, int prec) {
     t.fld_off[0] = t.pt_off[0] = t.lp_off[0] = t.ps_off[0] = 0;
     const int gpts = 32 * (prec == 0 ? ProjLane<double>::kP : ProjLane<float>::kP);
@@ -2352,12 +2366,20 @@ void proj_batch_finish(ProjBatch &t, int prec) {
         const int G = ceil_div(S.npts, gpts);
         S.pgb = 8;
         while (S.pgb > 1 && 14 * (ceil_div(G, S.pgb) * S.pgb - G) >= G) S.pgb /= 2;
-        const int GB = G > 0 ? ceil_div(G, S.pgb) : 1;
+        int GB = G > 0 ? ceil_div(G, S.pgb) : 1;
         S.pstride = G * gpts;
         const long long fit = G > 0 && S.part ? S.part_cap / ((long long)part * S.pstride) : 0;
         const long long least = ceil_div(S.m.n, kProjSlice), most = ceil_div(S.m.n, kProjStep);
-        long long nsl = std::max(least, std::min<long long>(most, ceil_div(4 * kProjSlots, GB)));
-        nsl = std::min(nsl, fit);
+        auto slices = [&]() {
+            const long long nsl = std::max(least, std::min<long long>(most, ceil_div(4 * kProjSlots, GB)));
+            return std::min(nsl, fit);
+        };
+        long long nsl = slices();
+        while (S.pgb > 1 && nsl * GB < kProjSlots) {
+            S.pgb /= 2;
+            GB = ceil_div(G, S.pgb);
+            nsl = slices();
+        }
         const long long rounds = nsl * GB / kProjSlots;
         if (rounds > 0 && rounds <= 4) nsl = std::max(std::min(least, fit), rounds * kProjSlots / GB);
         S.per = nsl > 0 ? ceil_div(S.m.n, nsl) : 0;
