@@ -2350,11 +2350,13 @@ void asm_batch_finish(AsmBatch &t) {
 // blocks is then rounded down to whole rounds of the resident ones (2 per SM
 // of 152; 26 slices of 24 blocks ran a third round for 16 of them: 11950 points
 // on 20480 elements 2.43 ms, with whole rounds 2.15), and the scratch may hold
-// fewer.  Where it leaves less than a round of blocks, as for many points on a
+// fewer.  Where it leaves less than two rounds of blocks, as for many points on a
 // small mesh, blocks take fewer groups, whose elements their warps then share:
 // points near the surface, with their subdivided pairs and higher orders, often
 // follow one another and would hold up a few blocks (2000 triangles, 10550
-// points of which 500 are near: 4.8 -> 0.73 ms).
+// points of which 500 are near: 4.8 -> 0.73 ms; 4000 points along the surface
+// of 5120 triangles 1.6 -> 0.63 ms, with one round 0.84).  It costs up to 8 % where all
+// points are far (1730 points on 5120 triangles 166 -> 180 us).
 void proj_batch_finish(ProjBatch &t, int prec) {
     t.fld_off[0] = t.pt_off[0] = t.lp_off[0] = t.ps_off[0] = 0;
     const int gpts = 32 * (prec == 0 ? ProjLane<double>::kP : ProjLane<float>::kP);
@@ -2375,7 +2377,7 @@ void proj_batch_finish(ProjBatch &t, int prec) {
             return std::min(nsl, fit);
         };
         long long nsl = slices();
-        while (S.pgb > 1 && nsl * GB < kProjSlots) {
+        while (S.pgb > 1 && nsl * GB < 2 * kProjSlots) {
             S.pgb /= 2;
             GB = ceil_div(G, S.pgb);
             nsl = slices();
