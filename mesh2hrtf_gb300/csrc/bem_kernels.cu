@@ -378,7 +378,7 @@ __device__ __forceinline__ void far_quad2(const FarConst &k, float (*st)[32], in
 //   u (b wr E - tau D.n_y u) + i u (b u (E + k^2 P) + tau wr D.n_y).
 // 53 FP64 instructions per point (the general form through map_point and the
 // library's square roots, divisions and sincos took about 250).  5120-triangle
-// head, 5 kHz: k_far 33.0 -> 12.9 ms.  Mean errors against 80-bit entries, this
+// head, 5 kHz: k_far 33.0 -> 13.1 ms.  Mean errors against 80-bit entries, this
 // and the general form, beyond a ratio of 4.5 and below 4, k = 73: head 1.35e-15
 // and 1.50e-15, 8.6e-16 and 9.1e-16; sphere flattened to a tenth 8.4e-16 and
 // 9.0e-16, 2.4e-16 and 3.0e-16.  |D|^2 + 2 s D.a + ... for the squared distance
@@ -1487,9 +1487,8 @@ __global__ void __launch_bounds__(256, 2) k_project(const __grid_constant__ Proj
 
 // Projection with lanes = evaluation points.  A block takes some groups of
 // points (32 lanes x kP points per lane) and a slice of the elements, which it
-// stages kProjChunk at a time in shared memory; its 8 warps are pgb point
-// groups x 8 / pgb element parts (pgb < 8 when there are few groups, so that
-// a call for a few points still spreads over the SMs).  An element's data is
+// stages proj_chunk at a time in shared memory; its 8 warps are pgb point
+// groups x 8 / pgb element parts (proj_batch_finish).  An element's data is
 // the same for all lanes: one broadcast read serves 32 kP points.
 //
 // In float a lane holds two points and the 4-point rule runs in packed
@@ -1513,11 +1512,11 @@ __global__ void __launch_bounds__(256, 2) k_project(const __grid_constant__ Proj
 // Points of higher order and subdivided pairs take proj_whole and
 // warp_subdivide.  Partial sums go to ProjSys::part per (slice, point);
 // k_project_sum adds the slices (FP64) and finishes the point.  In float, 11950
-// points on 20480 elements 3.87 -> 2.15 ms (41 instructions per evaluation,
+// points on 20480 elements 3.87 -> 2.14 ms (41 instructions per evaluation,
 // FMA pipe 64 % active on a smaller case), 64 points on 5120 elements 225 ->
 // 17 us (40 warps swept the elements before), 3072 quadrilaterals with an
-// image and velocities, 1730 points 1.63 -> 0.18 ms; FP64, 1730 points on 5120
-// elements 17.1 -> 5.8 ms.
+// image and velocities, 1730 points 1.63 -> 0.19 ms; FP64, 1730 points on 5120
+// elements 17.1 -> 4.3 ms.
 constexpr int kProjSlice = 256;   // most elements per slice
 constexpr int kProjStep = 16;     // fewest elements per slice
 // Elements of a slice whose terms are added one by one, each with two roundings at
