@@ -363,6 +363,11 @@ bem_status upload_freq(bem_solver_t s, const bem_frequency_desc *f, cudaStream_t
     F.wrf = (float)F.wr;
     F.taof = (float)F.tao;
     F.beta_imf = (float)F.beta_im;
+    F.k2f = (float)(F.k * F.k);
+    F.bwrf = (float)(F.beta_im * F.wr);
+    F.twrf = (float)(F.tao * F.wr);
+    F.btf = (float)(F.beta_im * F.tao);
+    F.btwf = (float)(F.beta_im * F.tao * F.wr);
     const std::vector<int> &ext = s->mesh->ext_of_int;
     std::vector<int> cols, bct;
     std::vector<double> bcv, adm, src;

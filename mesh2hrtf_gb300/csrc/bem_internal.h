@@ -54,6 +54,9 @@ constexpr int kMaxElements = (1 << kNearColBits) - 1;
 struct DevFreq {
     double k, wr, tao, beta_im;
     float kf, wrf, taof, beta_imf;   // the same in float
+    // products, rounded once: k^2, beta wr (+-1 up to FP64's rounding), tao wr,
+    // beta tao, beta tao wr
+    float k2f, bwrf, twrf, btf, btwf;
     const int *bc_type;        // [n] or nullptr (all velocity)
     const double *bc_val;      // [4][n] complex (row a = node a), or nullptr
     const double *adm;         // [n] complex, or nullptr

@@ -772,11 +772,8 @@ __device__ __forceinline__ void far_tile(const DevMeshView &mv, const DevFreq &f
         fc.b = PT.beta_im;
         fc.k2 = PT.k * PT.k;
         fc.wr = PT.wr;
-        // products of the constants rounded once: b wr is +-1 up to FP64's rounding
-        const double b = f.beta_im, wr = f.wr, tau = f.tao;
-        const FusedCol2 f2 = {dup2(fc.wr), dup2(fc.b), dup2((float)(b * wr)), dup2((float)(f.k * f.k)), dup2(-fc.tau),
-                              dup2((float)(tau * wr)), dup2(fc.yr), dup2(fc.yi), dup2(-fc.yi), dup2((float)(b * tau)),
-                              dup2((float)(b * tau * wr))};
+        const FusedCol2 f2 = {dup2(fc.wr), dup2(fc.b), dup2(f.bwrf), dup2(f.k2f), dup2(-fc.tau),
+                              dup2(f.twrf), dup2(fc.yr), dup2(fc.yi), dup2(-fc.yi), dup2(f.btf), dup2(f.btwf)};
 #pragma unroll 1
         for (int r = 0; r < rpt; r += 2) {
             const int i = i0 + r;
