@@ -195,7 +195,7 @@ __device__ __forceinline__ float2 far_entry_f(const Elem32 &e, const float nx[3]
 // in packed FP32, with the column element's data hoisted out of the row loop:
 // point g's squared distance is |D|^2 + 2 s_g D.a + 2 t_g D.b + C_g with
 // C_g = |s_g a + t_g b|^2 (at the order-2 ratio, |D| > 4 sqrt(area), the terms
-// do not cancel).  The distance, the phase and its reduction are rounded
+// do not cancel on elements that are not long and thin; see far_tri2).  The distance, the phase and its reduction are rounded
 // operation by operation (the phase's rounding is the entry's error); the
 // kernel terms of fused_point are regrouped around u = 1/r as in far_tri64.
 //
